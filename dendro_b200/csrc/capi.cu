@@ -98,6 +98,12 @@ using namespace dg;
 namespace {
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// The objects made so far on s are complete and may be used on any stream.
+dg_status finish_stream(cudaStream_t s) {
+  DG_CUDA(cudaStreamSynchronize(s));
+  return DG_OK;
+}
+
 template <class T>
 dg_status upload(DBuf<T>& buf, const T* host, int64_t n) {
   DG_TRY(buf.alloc(n));
@@ -140,6 +146,7 @@ dg_status dg_points2octree(const double* pts, int64_t n, int pts_on_device, uint
                            dg_octree** out) {
   DG_CHECK(out && (pts || n == 0) && n >= 0, DG_EINVAL, "points2octree: bad arguments");
   DG_CHECK(max_depth <= kMaxDepth, DG_EDEPTH, "points2octree: maxDepth must be <= 19");
+  PoolScope scope(nullptr);
   auto* t = new dg_octree();
   DBuf<double> dp;
   const double* src = pts;
@@ -149,6 +156,7 @@ dg_status dg_points2octree(const double* pts, int64_t n, int pts_on_device, uint
     src = dp.p;
   }
   dg_status st = points_to_octree(src, n, max_depth, max_num_pts, t, nullptr);
+  if (!st) st = finish_stream(nullptr);
   if (st) { delete t; return st; }
   *out = t;
   return DG_OK;
@@ -157,6 +165,7 @@ dg_status dg_points2octree(const double* pts, int64_t n, int pts_on_device, uint
 dg_status dg_octree_from_octants(const dg_octant* octs, int64_t n, int on_device, uint32_t max_depth, dg_octree** out) {
   DG_CHECK(out && octs && n > 0, DG_EINVAL, "octree_from_octants: bad arguments");
   DG_CHECK(max_depth <= kMaxDepth, DG_EDEPTH, "octree_from_octants: maxDepth must be <= 19");
+  PoolScope scope(nullptr);
   DBuf<dg_octant> d;
   const dg_octant* src = octs;
   if (!on_device) {
@@ -185,8 +194,10 @@ dg_status dg_octree_from_octants(const dg_octant* octs, int64_t n, int on_device
 
 dg_status dg_balance_octree(const dg_octree* in, dg_octree** out) {
   DG_CHECK(in && out, DG_EINVAL, "balance: bad arguments");
+  PoolScope scope(nullptr);
   auto* t = new dg_octree();
   dg_status st = balance_octree(in, t, nullptr);
+  if (!st) st = finish_stream(nullptr);
   if (st) { delete t; return st; }
   *out = t;
   return DG_OK;
@@ -194,8 +205,10 @@ dg_status dg_balance_octree(const dg_octree* in, dg_octree** out) {
 
 dg_status dg_coarsen_octree(const dg_octree* in, dg_octree** out) {
   DG_CHECK(in && out, DG_EINVAL, "coarsen: bad arguments");
+  PoolScope scope(nullptr);
   auto* t = new dg_octree();
   dg_status st = coarsen_octree(in, t, nullptr);
+  if (!st) st = finish_stream(nullptr);
   if (st) { delete t; return st; }
   *out = t;
   return DG_OK;
@@ -206,6 +219,7 @@ uint32_t dg_octree_max_depth(const dg_octree* t) { return t ? t->max_depth : 0; 
 
 dg_status dg_octree_export(const dg_octree* t, dg_octant* host_out) {
   DG_CHECK(t && host_out, DG_EINVAL, "octree_export: bad arguments");
+  PoolScope scope(nullptr);
   DBuf<dg_octant> d;
   DG_TRY(d.alloc(t->n));
   keys_to_octants<<<grid_for(t->n, 256), 256>>>(t->keys.p, t->n, d.p, 0u);
@@ -214,13 +228,15 @@ dg_status dg_octree_export(const dg_octree* t, dg_octant* host_out) {
   return DG_OK;
 }
 
-void dg_octree_destroy(dg_octree* t) { delete t; }
+void dg_octree_destroy(dg_octree* t) { delete_drained(t); }
 
 // -------------------------------------------------------------------- mesh
 dg_status dg_da_create(const dg_octree* balanced, dg_da** out) {
   DG_CHECK(balanced && out, DG_EINVAL, "da_create: bad arguments");
+  PoolScope scope(nullptr);
   auto* da = new dg_da();
   dg_status st = build_mesh(balanced, da, nullptr);
+  if (!st) st = finish_stream(nullptr);
   if (st) { delete da; return st; }
   *out = da;
   return DG_OK;
@@ -232,6 +248,7 @@ dg_status dg_da_create_from_maps(int64_t E, int64_t N, uint32_t max_depth, const
   DG_CHECK(out && nlist && level && cnum && hmask && node_xyz && elem_xyz && E > 0 && N > 0, DG_EINVAL,
            "da_create_from_maps: bad arguments");
   DG_CHECK(max_depth + 1 <= kMaxEmbeddedDepth, DG_EDEPTH, "da_create_from_maps: maxDepth must be <= 18");
+  PoolScope scope(nullptr);
   auto* da = new dg_da();
   da->D = max_depth + 1;
   da->E = E;
@@ -255,10 +272,10 @@ dg_status dg_da_create_from_maps(int64_t E, int64_t N, uint32_t max_depth, const
   if (!st) st = upload(da->meta, meta.data(), E);
   if (!st) st = upload(da->ekey, ek.data(), E);
   if (!st) st = upload(da->nkey, nk.data(), N);
-  if (!st) st = build_tiles(da, nullptr);
   // octets: the corners a hanging vertex needs are nodes its own element
   // lists, so a mesh of any subset of elements has them
   if (!st) st = build_octets(da, nullptr);
+  if (!st) st = finish_stream(nullptr);
   if (st) { delete da; return st; }
   *out = da;
   return DG_OK;
@@ -274,7 +291,7 @@ dg_status dg_da_sizes(const dg_da* da, int64_t* elements, int64_t* nodes, int64_
 
 uint32_t dg_da_max_depth(const dg_da* da) { return da ? da->D : 0; }
 
-int64_t dg_da_octets(const dg_da* da) { return da ? da->octs.n : 0; }
+int64_t dg_da_octets(const dg_da* da) { return da && da->meshes == 1 ? da->octs.n : 0; }
 
 dg_status dg_da_load_vector(const dg_da* da, const double* force, double* b, int on_device) {
   DG_CHECK(da && force && b, DG_EINVAL, "da_load_vector: bad arguments");
@@ -369,7 +386,7 @@ dg_status dg_da_element_centers(const dg_da* da, double* host_out) {
   return DG_OK;
 }
 
-void dg_da_destroy(dg_da* da) { delete da; }
+void dg_da_destroy(dg_da* da) { delete_drained(da); }
 
 // --------------------------------------------------------------- operators
 dg_status dg_mat_create_lapmass(dg_da* da, const double* coef, dg_mat** out) {
@@ -414,6 +431,7 @@ dg_status dg_mat_create_elasticity(dg_da* da, double mu, double lambda, const ui
       st = node_boundary_flags(da, A->dirichlet.p, nullptr);
     }
   }
+  if (!st) st = ensure_octet_chunks(da, nullptr);
   if (st) { delete A; return st; }
   *out = A;
   return DG_OK;
@@ -512,6 +530,7 @@ dg_status dg_mat_set_kernel(dg_mat* A, int prec, int variant) {
   DG_CHECK(A && A->kind == 0, DG_EINVAL, "set_kernel: scalar operator expected");
   DG_CHECK(variant >= 0 && variant < matvec_variant_count(), DG_EINVAL, "set_kernel: variant out of range");
   DG_CHECK(prec == DG_PREC_F64 || prec == DG_PREC_F32, DG_EINVAL, "set_kernel: precision");
+  DG_TRY(matvec_variant_tables(A->da, variant, nullptr));
   (prec == DG_PREC_F64 ? A->da->tuned_f64 : A->da->tuned_f32) = variant;
   return DG_OK;
 }

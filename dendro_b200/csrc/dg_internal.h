@@ -44,6 +44,7 @@ struct OctetSet {
   // touch (bit 31: another chunk touches the node too) and the range of
   // element ids of its children; per octet the chunk-local index of each
   // lattice node (0xffff: none) and of each present child's element.
+  bool chunks_tried = false;  // chunks built, or found not to fit
   int64_t nchunk = 0;
   uint32_t max_nodes = 0, max_erange = 0;
   DBuf<uint32_t> cptr;    // [nchunk + 1]
@@ -83,13 +84,14 @@ struct dg_octree {
 struct dg_da {
   uint32_t D = 0;        // embedded depth = maxDepth + 1
   int64_t E = 0, N = 0, P = 0;
+  int meshes = 1;            // independent meshes concatenated into this one
   dg::DBuf<uint32_t> nl;     // [8][E] node ids, vertex-major
   dg::DBuf<uint32_t> meta;   // [E] packed level / child number / hanging mask / type
   dg::DBuf<uint64_t> ekey;   // [E] element octant keys (embedded space)
   dg::DBuf<uint64_t> nkey;   // [N] node anchor Morton keys (embedded space), sorted
   // element tiles of the shared-memory operator kernels: the scalar warp-tile
-  // operator's (kWarpTile elements per tile, built with the mesh) and the
-  // multi-right-hand-side one's (kMultiTile elements per tile, built on first use)
+  // operator's (kWarpTile elements per tile) and the multi-right-hand-side
+  // one's (kMultiTile elements per tile), both built on first use
   dg::TileSet tiles_w, tiles_mr;
   dg::OctetSet octs;  // elements grouped by parent (octet operator kernel)
   dg::CompressedMap cmap;  // compressed element map (on request)
@@ -155,11 +157,12 @@ dg_status mlp_adam(float* p, const float* g, float* m1, float* m2, int step, flo
 // returns the total through *total (host) when not null.
 dg_status scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* total, cudaStream_t s);
 // Keys-only stable LSD radix sort of n uint64 keys on bits
-// [start_bit, start_bit + bits).  Sorted keys end in `keys`; tmp holds n keys.
-dg_status radix_sort_u64(uint64_t* keys, uint64_t* tmp, int64_t n, int bits, cudaStream_t s,
+// [start_bit, start_bit + bits).  Sorted keys end in `keys` (the two buffers,
+// of n keys each, may be swapped).
+dg_status radix_sort_u64(DBuf<uint64_t>& keys, DBuf<uint64_t>& tmp, int64_t n, int bits, cudaStream_t s,
                          int start_bit = 0);
-// Remove adjacent duplicates in place; returns the new length.
-dg_status unique_u64(uint64_t* keys, int64_t n, int64_t* n_out, cudaStream_t s);
+// Remove adjacent duplicates (through tmp, swapped with keys); returns the new length.
+dg_status unique_u64(DBuf<uint64_t>& keys, DBuf<uint64_t>& tmp, int64_t n, int64_t* n_out, cudaStream_t s);
 
 // ---- octree (octree.cu) ----
 dg_status points_to_octree(const double* d_pts, int64_t n, uint32_t D, uint32_t m, dg_octree* out,
@@ -175,8 +178,14 @@ dg_status build_mesh(const dg_octree* tree, dg_da* da, cudaStream_t s);
 void set_wait_limit(long long cycles);
 long long wait_limit();  // clock cycles a bounded device wait may take
 dg_status device_wait_status(cudaStream_t s);
-dg_status build_tiles(dg_da* da, cudaStream_t s);  // da->tiles_w (kWarpTile)
-dg_status build_octets(dg_da* da, cudaStream_t s);  // da->octs (octet.cu)
+dg_status build_octets(dg_da* da, cudaStream_t s);  // da->octs from nl and meta (octet.cu)
+// Tables that only some launch shapes read, built when one of those is chosen
+// (not inside a stream capture: they allocate and synchronise s): the warp
+// tiles (da->tiles_w), the octets' records, the octet chunks (none when a
+// chunk's elements are too far apart).
+dg_status ensure_tiles(dg_da* da, cudaStream_t s);
+dg_status ensure_octet_records(dg_da* da, cudaStream_t s);
+dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s);
 // da->cmap with narrow quotients of qbits (1..16) bits (cmap.cu); nl_out
 // [8][E] receives the map decoded from it
 dg_status build_cmap(dg_da* da, int qbits, cudaStream_t s);
@@ -229,6 +238,7 @@ dg_status lapmass_residual_f32(const dg_mat* A, const float* x, const float* b, 
                                const Type1Set* t1 = nullptr);
 const char* matvec_variant_name(int v);
 int matvec_variant_count();
+dg_status matvec_variant_tables(dg_da* da, int v, cudaStream_t s);
 // Y = A X for nrhs vectors (node-major [N][nrhs], FP32) on the tensor cores;
 // split 1: TF32 products, 3: high/low TF32 split (FP32-level accuracy).
 dg_status mrhs_apply(const dg_mat* A, const float* X, float* Y, int nrhs, int split, cudaStream_t s);

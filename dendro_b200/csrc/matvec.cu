@@ -2232,13 +2232,23 @@ static dg_status allow_dynamic_smem(const void* kern, size_t bytes) {
 constexpr int kNumVariants = int(sizeof(kVariants) / sizeof(kVariants[0]));
 
 // Whether the mesh has the structure a launch shape of this kind reads:
-// octets, octet chunks, warp tiles or the compressed map.
+// octets, octet records, octet chunks, warp tiles or the compressed map.
 static bool variant_runs(int k, const dg_da* da) {
   if (k == 16) return da->cmap.qbits != 0;
   if ((k == 6 || k >= 10) && da->octs.n == 0) return false;
+  if ((k == 10 || k == 11) && da->octs.rec.n == 0) return false;
   if (k >= 7 && k <= 9 && da->octs.nchunk == 0) return false;
   if (k >= 2 && k <= 5 && da->tiles_w.ntiles == 0) return false;
   return true;
+}
+
+// The tables that launch shape v reads and a new mesh does not have.
+dg_status matvec_variant_tables(dg_da* da, int v, cudaStream_t s) {
+  const int k = kVariants[v].kind;
+  if (k == 10 || k == 11) return ensure_octet_records(da, s);
+  if (k >= 7 && k <= 9) return ensure_octet_chunks(da, s);
+  if (k >= 2 && k <= 5) return ensure_tiles(da, s);
+  return DG_OK;
 }
 
 template <class T, class CT>
@@ -2425,17 +2435,27 @@ static int forced_variant() {
 // then per variant the best of two timed launches, each after overwriting a
 // buffer larger than L2 so that the mesh streams from HBM as it does for
 // meshes larger than L2.  y is used as scratch and left zero.  Inside a
-// capture an untuned mesh gets the default warp-tile shape.
-constexpr int kDefaultVariant = 5;  // "warp-tile 32 elems, 5 CTAs/SM"
+// capture an untuned mesh gets the default octet shape.  Timed are the shapes
+// that are fastest on some mesh: the element kernel (small meshes), the octet
+// kernels with the next ids in flight (the others), and the compressed-map
+// kernel where its map has been built; the tile, chunk, lane and quad shapes
+// need tables of their own and were 1.2 to 2 times slower on the benchmark
+// mesh, so they run only when fixed by the caller.
+constexpr int kDefaultVariant = 28;  // "octet b128, next ids in flight, 4 CTAs/SM"
+static bool variant_timed(int v) {
+  const int k = kVariants[v].kind;
+  return k == 0 || k == 6 || k == 12 || k == 13 || k >= 15;
+}
 template <class T, class CT>
-static dg_status pick_variant(const dg_da* da, int& choice, const CT* ca, const CT* cb, const T* x, T* y,
+static dg_status pick_variant(dg_da* da, int& choice, const CT* ca, const CT* cb, const T* x, T* y,
                               cudaStream_t s, int* v_out) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (choice < 0 || forced_variant() >= 0) DG_CUDA(cudaStreamIsCapturing(s, &cap));
   if (forced_variant() >= 0) {
     *v_out = forced_variant();
+    if (cap == cudaStreamCaptureStatusNone) DG_TRY(matvec_variant_tables(da, *v_out, s));
     return DG_OK;
   }
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  DG_CUDA(cudaStreamIsCapturing(s, &cap));
   if (choice < 0 && cap != cudaStreamCaptureStatusNone) {  // no timing inside a graph capture
     *v_out = kDefaultVariant;
     return DG_OK;
@@ -2452,7 +2472,7 @@ static dg_status pick_variant(const dg_da* da, int& choice, const CT* ca, const 
     DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
     DG_TRY((launch_variant<T, CT>(0, da, ca, cb, x, y, s)));
     for (int v = 0; v < kNumVariants; ++v) {
-      if (!variant_runs(kVariants[v].kind, da)) continue;
+      if (!variant_timed(v) || !variant_runs(kVariants[v].kind, da)) continue;
       for (int trial = 0; trial < 2; ++trial) {
         DG_CUDA(cudaMemsetAsync(flush.p, trial + 1, flush_bytes, s));
         DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
@@ -2571,6 +2591,7 @@ struct HostPipe {
 };
 
 constexpr int kPipeGroups = 16;
+constexpr int kPipeVariant = 5;  // "warp-tile 32 elems, 5 CTAs/SM"
 constexpr int64_t kPipeMinElements = int64_t(1) << 20;
 
 static dg_status build_host_pipe(const dg_da* da, HostPipe& P) {
@@ -2719,19 +2740,20 @@ static bool page_locked(const void* p) {
 
 dg_status lapmass_apply_host_pipelined_f64(dg_mat* A, const double* hx, double* hy) {
   dg_da* da = A->da;
-  if (A->kind != 0 || da->E < kPipeMinElements || da->tiles_w.ntiles == 0 || da->tuned_f64 < 0) return DG_ENOTIMPL;
+  if (A->kind != 0 || da->E < kPipeMinElements || da->tuned_f64 < 0) return DG_ENOTIMPL;
   // pageable buffers: each chunk copy would block the host until its group
   // has run, serialising the pipeline, so the caller copies, applies, copies
   if (!page_locked(hx) || !page_locked(hy)) return DG_ENOTIMPL;
   if (!A->pipe) {
     auto P = std::make_shared<HostPipe>();
+    DG_TRY(ensure_tiles(da, nullptr));
     DG_TRY(build_host_pipe(da, *P));
     A->pipe = P;
   }
   HostPipe& P = *A->pipe;
-  // the mesh's tuned shape when it is a plain warp-tile one, else the default
+  // the mesh's shape when it is a plain warp-tile one, else the widest of them
   const int kind = kVariants[da->tuned_f64].kind;
-  P.variant = (kind >= 2 && kind <= 4) ? da->tuned_f64 : kDefaultVariant;
+  P.variant = (kind >= 2 && kind <= 4) ? da->tuned_f64 : kPipeVariant;
   DG_TRY(enqueue_host_pipe(A, P, hx, hy));
   DG_CUDA(cudaStreamSynchronize(P.sk));
   return DG_OK;

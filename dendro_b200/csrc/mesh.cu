@@ -8,7 +8,10 @@
 //    hanging masks, child numbers and element types (DA::buildNodeList,
 //    src/oda/private/odaBuildNlist.C:47-856; GET_ETYPE_BLOCK,
 //    include/oda/odaUtils.h:334).
-#include "dg_internal.h"
+#include <utility>
+
+#include "octet.cuh"
+#include "prim.cuh"
 
 namespace dg {
 
@@ -41,111 +44,327 @@ __device__ __forceinline__ int64_t find_exact(const uint64_t* __restrict__ a, in
   return (lo < n && a[lo] == key) ? lo : -1;
 }
 
-// Embedded element keys (level + 1, same anchors) and pseudo-octant counts.
-__global__ void embed_and_count(const uint64_t* __restrict__ k, int64_t n, uint32_t D, uint64_t* __restrict__ ekey,
-                                uint32_t* __restrict__ cnt) {
-  const uint32_t top = 1u << D;
-  for (int64_t i = gtid(); i < n; i += gstride()) {
-    uint64_t m = okey_m(k[i]);
-    uint32_t l = okey_l(k[i]);
-    ekey[i] = okey(m, l + 1);
-    uint32_t x, y, z;
-    demorton(m, x, y, z);
-    uint32_t blen = top - (1u << (D - l));
-    uint32_t px = x == blen, py = y == blen, pz = z == blen;
-    cnt[i] = px + py + pz + (px & py) + (px & pz) + (py & pz) + (px & py & pz);
+// Hash map of 64-bit keys to 32-bit values: slots (key, value) of 16 bytes,
+// so that a look-up that hits on its first probe reads one 32-byte sector.
+// (Binary searches over the sorted node keys took 22 dependent loads each.)
+struct KeyMap {
+  ulonglong2* slot;  // key kNoKey: empty
+  uint64_t cap;
+};
+__device__ __forceinline__ void map_insert(const KeyMap& M, uint64_t key, uint32_t val) {
+  // keys are distinct and fill at most half the slots, so this ends
+  uint64_t h = hash_slot(key, M.cap);
+  while (atomicCAS(&M.slot[h].x, kNoKey, key) != kNoKey) h = h + 1 == M.cap ? 0 : h + 1;
+  M.slot[h].y = val;
+}
+// The value of `key`, kNoNode when it is not there; `cur` is the slot at
+// hash_slot(key), read by the caller (so that several reads overlap).
+__device__ __forceinline__ uint32_t map_resolve(const KeyMap& M, uint64_t key, uint64_t h, ulonglong2 cur) {
+  while (cur.x != key) {
+    if (cur.x == kNoKey) return kNoNode;
+    h = h + 1 == M.cap ? 0 : h + 1;
+    cur = M.slot[h];
   }
+  return uint32_t(cur.y);
+}
+__device__ __forceinline__ uint32_t map_find(const KeyMap& M, uint64_t key) {
+  const uint64_t h = hash_slot(key, M.cap);
+  return map_resolve(M, key, h, M.slot[h]);
 }
 
-__global__ void emit_pseudo(const uint64_t* __restrict__ k, int64_t n, uint32_t D, const uint32_t* __restrict__ pos,
-                            uint64_t* __restrict__ out) {
-  const uint32_t top = 1u << D;
-  for (int64_t i = gtid(); i < n; i += gstride()) {
-    uint64_t m = okey_m(k[i]);
-    uint32_t l = okey_l(k[i]);
-    uint32_t x, y, z;
-    demorton(m, x, y, z);
-    uint32_t blen = top - (1u << (D - l));
-    bool px = x == blen, py = y == blen, pz = z == blen;
-    uint64_t* o = out + pos[i];
-    int c = 0;
-    if (px) o[c++] = okey(morton(top, y, z), l + 1);
-    if (py) o[c++] = okey(morton(x, top, z), l + 1);
-    if (pz) o[c++] = okey(morton(x, y, top), l + 1);
-    if (px && py) o[c++] = okey(morton(top, top, z), l + 1);
-    if (px && pz) o[c++] = okey(morton(top, y, top), l + 1);
-    if (py && pz) o[c++] = okey(morton(x, top, top), l + 1);
-    if (px && py && pz) o[c++] = okey(morton(top, top, top), l + 1);
+// Per octant its positive-boundary pseudo-octants (embedded keys); the
+// octant's own embedded key (level + 1, same anchor) goes to ekey.
+struct PseudoOctants {
+  const uint64_t* __restrict__ k;
+  uint32_t D;
+  uint64_t* __restrict__ ekey;
+  uint64_t* __restrict__ out;
+  __device__ uint32_t touching(int64_t i, uint32_t& x, uint32_t& y, uint32_t& z) const {
+    demorton(okey_m(k[i]), x, y, z);
+    const uint32_t blen = (1u << D) - (1u << (D - okey_l(k[i])));
+    return (x == blen) | (y == blen) << 1 | (z == blen) << 2;
   }
+  __device__ uint32_t count(int64_t i) const {
+    uint32_t x, y, z;
+    return (1u << __popc(touching(i, x, y, z))) - 1u;  // the non-empty subsets of the touched faces
+  }
+  __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
+    ekey[i] = k[i] + 1;
+    if (!c) return;
+    uint32_t x, y, z;
+    const uint32_t f = touching(i, x, y, z), top = 1u << D;
+    uint64_t* o = out + off;
+    for (uint32_t s = 1; s < 8; ++s)
+      if ((s & f) == s)
+        *o++ = okey(morton((s & 1) ? top : x, (s & 2) ? top : y, (s & 4) ? top : z), okey_l(k[i]) + 1);
+  }
+};
+
+// Embedded key of the parent of an octant with (unembedded) key k.
+__device__ __forceinline__ uint64_t embedded_parent(uint64_t k, uint32_t D) {
+  const uint32_t l = okey_l(k);
+  return okey(okey_m(k) & ~((1ull << (3u * (D - l + 1))) - 1ull), l);
+}
+// The parents of the octants, once per run of siblings.
+struct ParentRuns {
+  const uint64_t* __restrict__ k;
+  uint32_t D;
+  uint64_t* __restrict__ out;
+  __device__ uint32_t count(int64_t i) const {
+    return i == 0 || embedded_parent(k[i], D) != embedded_parent(k[i - 1], D) ? 1u : 0u;
+  }
+  __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
+    if (c) out[off] = embedded_parent(k[i], D);
+  }
+};
+
+// Per octet (parent with leaf children): the element ids of its children, its
+// meta word, and its place in the map of octet keys; *covered counts the
+// children, all E elements when no octant lies inside another.
+__global__ void octet_children(const uint64_t* __restrict__ okeys, int64_t n, uint32_t Dp,
+                               const uint64_t* __restrict__ ekey, int64_t E, uint32_t* __restrict__ ometa,
+                               uint32_t* __restrict__ oelem, KeyMap M, uint32_t* __restrict__ covered) {
+  uint32_t mine = 0;
+  for (int64_t o = gtid(); o < n; o += gstride()) {
+    const uint64_t k = okeys[o], am = okey_m(k);
+    const uint32_t m = okey_l(k) + 1;
+    const uint32_t sh = 3u * (Dp - m);
+    int64_t lo = 0, hi = E;  // the first element at or after the parent's anchor
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (ekey[mid] < okey(am, 0)) lo = mid + 1;
+      else hi = mid;
+    }
+    uint32_t mask = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const uint64_t ck = okey(am + (uint64_t(c) << sh), m);
+      const bool leaf = lo < E && ekey[lo] == ck;
+      oelem[int64_t(c) * n + o] = leaf ? uint32_t(lo) : kNoNode;
+      if (leaf) {
+        mask |= 1u << c;
+        ++lo;
+      } else if (c < 7) {  // refined: past the child's own elements
+        lo = gallop(ekey, lo, E, okey(am + (uint64_t(c + 1) << sh), 0));
+      }
+    }
+    ometa[o] = m | (mask << 8);
+    map_insert(M, k, uint32_t(o));
+    mine += __popc(mask);
+  }
+  atomicAdd(covered, mine);
 }
 
-// NODE flag: the anchor is hanging when the parent of a same-level neighbour
-// across the parent's faces/edges holding the anchor is an octant.
-__global__ void flag_nodes(const uint64_t* __restrict__ all, int64_t n, uint32_t Dp, uint32_t* __restrict__ flag) {
-  for (int64_t i = gtid(); i < n; i += gstride()) {
-    uint64_t k = all[i];
-    uint32_t m = okey_l(k);
+// Whether the octant q (an embedded key inside the domain, level >= 1) is an
+// element: its parent is an octet with that child.
+__device__ __forceinline__ bool is_element(const KeyMap& M, const uint32_t* __restrict__ ometa, uint64_t q,
+                                           uint32_t Dp) {
+  const uint32_t l = okey_l(q);
+  const uint64_t m = okey_m(q);
+  const uint32_t o = map_find(M, okey(m & ~((1ull << (3u * (Dp - l + 1))) - 1ull), l - 1));
+  return o != kNoNode && ((ometa_cmask(ometa[o]) >> uint32_t((m >> (3u * (Dp - l))) & 7u)) & 1u);
+}
+
+// NODE flags of the elements (flagNodesType3): the anchor of child c is
+// hanging when one of the parent's same-size neighbours across the faces and
+// edges of the parent that hold the anchor is an element.  8 lanes per octet:
+// lane S looks up the neighbour towards the axes of S, lane c combines them.
+__global__ void flag_elements(const uint64_t* __restrict__ okeys, int64_t n, uint32_t Dp,
+                              const uint32_t* __restrict__ ometa, const uint32_t* __restrict__ oelem, KeyMap M,
+                              uint8_t* __restrict__ flag) {
+  const int64_t nr = (8 * n + 31) & ~int64_t(31);
+  for (int64_t t = gtid(); t < nr; t += gstride()) {
+    const int64_t o = t >> 3;
+    const uint32_t c = uint32_t(t & 7);
+    bool coarse = false;
+    uint32_t e = kNoNode;
+    if (o < n) {
+      e = oelem[int64_t(c) * n + o];
+      const uint64_t k = okeys[o];
+      const uint32_t pl = okey_l(k);
+      if (pl >= 1 && c != 0 && c != 7) {
+        uint32_t x, y, z;
+        demorton(okey_m(k), x, y, z);
+        const uint32_t S = 1u << (Dp - pl);
+        if (!(((c & 1) && !x) || ((c & 2) && !y) || ((c & 4) && !z)))
+          coarse = is_element(M, ometa, okey(morton(x - ((c & 1) ? S : 0), y - ((c & 2) ? S : 0), z - ((c & 4) ? S : 0)), pl), Dp);
+      }
+    }
+    const uint32_t L = __ballot_sync(0xffffffffu, coarse) >> (threadIdx.x & 24);
+    if (e == kNoNode) continue;
     bool hanging = false;
-    if (m != 1 && m != 0) {
+    if (c != 0 && c != 7)
+#pragma unroll
+      for (uint32_t S = 1; S < 7; ++S) hanging = hanging || (!(S & c) && ((L >> S) & 1u));
+    flag[e] = hanging ? 0 : 1;
+  }
+}
+
+// The same for the pseudo-octants (their neighbours may be pseudo-octants).
+__global__ void flag_pseudo(const uint64_t* __restrict__ ps, int64_t P, uint32_t Dp,
+                            const uint32_t* __restrict__ ometa, KeyMap M, uint8_t* __restrict__ flag) {
+  const uint64_t outside = okey(1ull << (3u * (Dp - 1)), 0);
+  for (int64_t i = gtid(); i < P; i += gstride()) {
+    const uint64_t k = ps[i];
+    const uint32_t m = okey_l(k);
+    bool hanging = false;
+    if (m > 1) {
       uint32_t x, y, z;
       demorton(okey_m(k), x, y, z);
-      uint32_t s = 1u << (Dp - m);
-      uint32_t c = ((x >> (Dp - m)) & 1u) | (((y >> (Dp - m)) & 1u) << 1) | (((z >> (Dp - m)) & 1u) << 2);
+      const uint32_t s = 1u << (Dp - m);
+      const uint32_t c = uint32_t((okey_m(k) >> (3u * (Dp - m))) & 7u);
       if (c != 0 && c != 7) {
-        uint32_t zero = (~c) & 7u;
-        uint32_t pmask = ~((2u * s) - 1u);
+        const uint32_t zero = (~c) & 7u, pmask = ~((2u * s) - 1u);
         for (uint32_t S = 1; S < 8 && !hanging; ++S) {
           if ((S & zero) != S) continue;
           if (((S & 1) && !x) || ((S & 2) && !y) || ((S & 4) && !z)) continue;
-          uint32_t nx = x - ((S & 1) ? s : 0), ny = y - ((S & 2) ? s : 0), nz = z - ((S & 4) ? s : 0);
-          uint64_t pk = okey(morton(nx & pmask, ny & pmask, nz & pmask), m - 1);
-          if (find_exact(all, n, pk) >= 0) hanging = true;
+          const uint32_t nx = x - ((S & 1) ? s : 0), ny = y - ((S & 2) ? s : 0), nz = z - ((S & 4) ? s : 0);
+          const uint64_t q = okey(morton(nx & pmask, ny & pmask, nz & pmask), m - 1);
+          hanging = q >= outside ? find_exact(ps, P, q) >= 0 : is_element(M, ometa, q, Dp);
         }
       }
     }
-    flag[i] = hanging ? 0u : 1u;
+    flag[i] = hanging ? 0 : 1;
   }
 }
 
-__global__ void emit_node_keys(const uint64_t* __restrict__ all, int64_t n, const uint32_t* __restrict__ flag,
-                               const uint32_t* __restrict__ pos, uint64_t* __restrict__ nkey) {
-  for (int64_t i = gtid(); i < n; i += gstride())
-    if (flag[i]) nkey[pos[i]] = okey_m(all[i]);
-}
+// The nodes: octants flagged NODE, elements then pseudo-octants, in key
+// order (pseudo-octants lie outside the domain child of the embedded root, so
+// they sort after every element); each node's key goes to the map too.
+struct NodeKeys {
+  const uint8_t* __restrict__ flag;
+  const uint64_t* __restrict__ ekey;
+  int64_t E;
+  const uint64_t* __restrict__ ps;
+  uint64_t* __restrict__ nkey;
+  KeyMap M;
+  __device__ uint32_t count(int64_t i) const { return flag[i]; }
+  __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
+    if (!c) return;
+    const uint64_t m = okey_m(i < E ? ekey[i] : ps[i - E]);
+    nkey[off] = m;
+    map_insert(M, m, off);
+  }
+};
 
-// Element -> node map, hanging mask, child number, element type.
-__global__ void build_nlist(const uint64_t* __restrict__ ekey, int64_t E, uint32_t Dp, const uint64_t* __restrict__ nkey,
-                            int64_t N, uint32_t* __restrict__ nl, uint32_t* __restrict__ meta, uint32_t* __restrict__ err) {
-  for (int64_t e = gtid(); e < E; e += gstride()) {
-    uint64_t k = ekey[e];
-    uint32_t m = okey_l(k);
-    uint32_t x, y, z;
-    demorton(okey_m(k), x, y, z);
-    uint32_t s = 1u << (Dp - m);
-    uint32_t pm = ~((2u * s) - 1u);
-    uint32_t px = x & pm, py = y & pm, pz = z & pm;
-    uint32_t mask = 0;
-    for (uint32_t v = 0; v < 8; ++v) {
-      uint32_t vx = x + ((v & 1) ? s : 0), vy = y + ((v & 2) ? s : 0), vz = z + ((v & 4) ? s : 0);
-      int64_t id = find_exact(nkey, N, morton(vx, vy, vz));
-      if (id < 0) {
-        mask |= 1u << v;
-        id = find_exact(nkey, N, morton(px + ((v & 1) ? 2 * s : 0), py + ((v & 2) ? 2 * s : 0),
-                                        pz + ((v & 4) ? 2 * s : 0)));
-        if (id < 0) {
-          atomicOr(err, 1u);
-          id = 0;
-        }
+// Children of an octet that have lattice point p as a vertex.
+__host__ __device__ constexpr uint32_t lat_children(int p) {
+  uint32_t t = 0;
+  for (int c = 0; c < 8; ++c) {
+    bool in = true;
+    for (int a = 0; a < 3; ++a) {
+      const int d = oct_coord(p, a) - ((c >> a) & 1);
+      in = in && (d == 0 || d == 1);
+    }
+    if (in) t |= 1u << c;
+  }
+  return t;
+}
+// Corners of the octet that a hanging point p interpolates from.
+__host__ __device__ constexpr uint32_t lat_corners(int p) {
+  uint32_t t = 0;
+  for (int v = 0; v < 8; ++v) {
+    bool in = true;
+    for (int a = 0; a < 3; ++a) in = in && (oct_coord(p, a) == 1 || oct_coord(p, a) == 2 * ((v >> a) & 1));
+    if (in) t |= 1u << (2 * (v & 1) + 6 * ((v >> 1) & 1) + 18 * ((v >> 2) & 1));
+  }
+  return t;
+}
+struct LatticeTables {
+  uint32_t children[32], corners[32];
+  constexpr LatticeTables() : children(), corners() {
+    for (int p = 0; p < 27; ++p) {
+      children[p] = lat_children(p);
+      corners[p] = lat_corners(p);
+    }
+  }
+};
+__constant__ LatticeTables c_lat = LatticeTables();
+
+// Element -> node map, hanging masks, element types and the octets' lattice
+// ids from one look-up per lattice point: a warp per octet, lane p looks up
+// point p (27 look-ups per octet instead of 64 and more per 8 elements); a
+// vertex without a node hangs and lists its parent's vertex, an octet corner
+// (DA::buildNodeList).  A CTA works 32 octets and writes their rows together.
+// One look-up is a random 32-byte sector, so each warp issues the first probe
+// of its 4 octets before it follows any of them.
+constexpr int kLatOctets = 32;
+__global__ void __launch_bounds__(256) octet_lattice(const uint64_t* __restrict__ okeys, int64_t n, uint32_t Dp,
+                                                     const uint32_t* __restrict__ ometa,
+                                                     const uint32_t* __restrict__ oelem, KeyMap M, int64_t E,
+                                                     uint32_t* __restrict__ oid, uint32_t* __restrict__ nl,
+                                                     uint32_t* __restrict__ meta, uint32_t* __restrict__ err) {
+  __shared__ uint32_t sid[27][kLatOctets + 1], shang[kLatOctets];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  constexpr int kPer = kLatOctets / 8;  // octets per warp
+  const uint32_t touch = lane < 27 ? c_lat.children[lane] : 0u, corner = lane < 27 ? c_lat.corners[lane] : 0u;
+  constexpr uint32_t kNever = (1u << 0) | (1u << 2) | (1u << 6) | (1u << 8) | (1u << 13) | (1u << 18) | (1u << 20) |
+                              (1u << 24) | (1u << 26);  // corners and the centre do not hang
+  for (int64_t o0 = int64_t(blockIdx.x) * kLatOctets; o0 < n; o0 += int64_t(gridDim.x) * kLatOctets) {
+    uint64_t key[kPer], h[kPer];
+    ulonglong2 cur[kPer];
+    uint32_t cm[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int64_t o = o0 + w * kPer + j;
+      cm[j] = 0;
+      key[j] = h[j] = 0;
+      cur[j] = make_ulonglong2(kNoKey, 0);
+      if (o < n && lane < 27) {
+        const uint64_t k = okeys[o];
+        cm[j] = ometa_cmask(ometa[o]);
+        uint32_t x, y, z;
+        demorton(okey_m(k), x, y, z);
+        const uint32_t s = 1u << (Dp - okey_l(k) - 1);
+        key[j] = morton(x + s * (lane % 3), y + s * ((lane / 3) % 3), z + s * (lane / 9));
+        h[j] = hash_slot(key[j], M.cap);
+        cur[j] = M.slot[h[j]];
       }
-      nl[int64_t(v) * E + e] = uint32_t(id);
     }
-    uint32_t c = ((x >> (Dp - m)) & 1u) | (((y >> (Dp - m)) & 1u) << 1) | (((z >> (Dp - m)) & 1u) << 2);
-    uint32_t t = mask ? c_etype_lut[c][mask] : 0u;
-    if (t == 255u) {
-      atomicOr(err, 2u);
-      t = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t id = map_resolve(M, key[j], h[j], cur[j]);
+      const bool present = (cm[j] & touch) != 0u, found = id != kNoNode;
+      const uint32_t hang = __ballot_sync(0xffffffffu, present && !found);
+      const uint32_t need = __reduce_or_sync(0xffffffffu, ((hang >> lane) & 1u) ? corner : 0u);
+      const bool use = (present && found) || ((need >> lane) & 1u);
+      if (((need >> lane) & 1u) && !found) atomicOr(err, 1u);
+      if (lane < 27) sid[lane][w * kPer + j] = use ? id : kNoNode;
+      if (lane == 0) {
+        shang[w * kPer + j] = hang;
+        if (hang & kNever) atomicOr(err, 2u);
+      }
     }
-    meta[e] = meta_pack(m, c, mask, t);
+    __syncthreads();
+    for (int i = tid; i < 27 * kLatOctets; i += 256) {
+      const int p = i / kLatOctets, j = i % kLatOctets;
+      if (o0 + j < n) oid[int64_t(p) * n + o0 + j] = sid[p][j];
+    }
+    {
+      const int j = tid >> 3, c = tid & 7;
+      const int64_t o = o0 + j;
+      const uint32_t e = o < n ? oelem[int64_t(c) * n + o] : kNoNode;
+      if (e != kNoNode) {
+        const uint32_t hang = shang[j];
+        uint32_t mask = 0;
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          int p = ((c & 1) + (v & 1)) + 3 * (((c >> 1) & 1) + ((v >> 1) & 1)) + 9 * ((c >> 2) + (v >> 2));
+          if ((hang >> p) & 1u) {
+            mask |= 1u << v;
+            p = 2 * (v & 1) + 6 * ((v >> 1) & 1) + 18 * (v >> 2);
+          }
+          nl[int64_t(v) * E + e] = sid[p][j];
+        }
+        uint32_t t = mask ? c_etype_lut[c][mask] : 0u;
+        if (t == 255u) {
+          atomicOr(err, 2u);
+          t = 0;
+        }
+        meta[e] = meta_pack(ometa_lev(ometa[o]), uint32_t(c), mask, t);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -407,52 +626,81 @@ dg_status build_mesh(const dg_octree* tree, dg_da* da, cudaStream_t s) {
            "mesh: maxDepth above 18 is not supported (the embedded depth's keys would exceed 64 bits)");
   DG_CHECK(E >= 1, DG_EINVAL, "empty octree");
   DG_TRY(upload_etype_lut());
+  DG_CHECK(E < (int64_t(1) << 31), DG_EINVAL, "mesh above 2^31 elements");
   const uint32_t Dp = D + 1;
+  const int bits = int(3 * Dp + 5);
+  OctetSet& O = da->octs;
   da->D = Dp;
   da->E = E;
-  DBuf<uint32_t> cnt;
-  DG_TRY(cnt.alloc(E));
-  DBuf<uint64_t> ekey;
-  DG_TRY(ekey.alloc(E));
-  unsigned g = grid_for(E, 256);
-  embed_and_count<<<g, 256, 0, s>>>(tree->keys.p, E, D, ekey.p, cnt.p);
-  uint32_t P = 0;
-  DG_TRY(scan_u32(cnt.p, cnt.p, E, &P, s));
+  DG_TRY(da->ekey.alloc(E));
+  const int64_t nb = tile_blocks(E);
+  DBuf<uint32_t> sums, cnt;  // cnt: [0] pseudo-octants, [1] sibling runs, [2] octets, [3] nodes, [4] children, [5] errors
+  DG_TRY(sums.alloc(2 * nb));
+  DG_TRY(cnt.alloc(6));
+  DG_CUDA(cudaMemsetAsync(cnt.p, 0, 24, s));
+  PseudoOctants pf{tree->keys.p, D, da->ekey.p, nullptr};
+  ParentRuns rf{tree->keys.p, D, nullptr};
+  DG_TRY(tile_scan(pf, ItemCount{E}, sums.p, cnt.p, s));
+  DG_TRY(tile_scan(rf, ItemCount{E}, sums.p + nb, cnt.p + 1, s));
+  uint32_t h[6];
+  DG_TRY(read_words(cnt.p, h, 2, s));
+  const int64_t P = h[0], runs = h[1];
   da->P = P;
-  const int64_t n = E + P;
-  DBuf<uint64_t> all, tmp;
-  DG_TRY(all.alloc(n));
-  DG_TRY(tmp.alloc(P > 0 ? P : 1));
-  DG_CUDA(cudaMemcpyAsync(all.p, ekey.p, 8 * E, cudaMemcpyDeviceToDevice, s));
-  emit_pseudo<<<g, 256, 0, s>>>(tree->keys.p, E, D, cnt.p, all.p + E);
+  DBuf<uint64_t> ps, pt, okeys, ot;
+  DG_TRY(ps.alloc(P));
+  DG_TRY(pt.alloc(P));
+  DG_TRY(okeys.alloc(runs));
+  DG_TRY(ot.alloc(runs));
+  pf.out = ps.p;
+  rf.out = okeys.p;
+  DG_TRY(tile_emit(pf, ItemCount{E}, sums.p, s));
+  DG_TRY(tile_emit(rf, ItemCount{E}, sums.p + nb, s));
+  DG_TRY(radix_sort_u64(ps, pt, P, bits, s));
+  DG_TRY(radix_sort_u64(okeys, ot, runs, bits, s));
+  const UniqueKeys uq{okeys.p, ot.p};
+  DG_TRY(tile_scan(uq, ItemCount{runs}, sums.p, cnt.p + 2, s));
+  DG_TRY(tile_emit(uq, ItemCount{runs}, sums.p, s));
+  std::swap(okeys, ot);
+  DG_TRY(read_words(cnt.p, h, 3, s));
+  const int64_t n = h[2];
+  O.n = n;
+  DG_TRY(O.meta.alloc(n));
+  DG_TRY(O.elem.alloc(8 * n));
+  DBuf<ulonglong2> oslots, nslots;
+  DG_TRY(oslots.alloc(2 * n));
+  DG_CUDA(cudaMemsetAsync(oslots.p, 0xff, sizeof(ulonglong2) * size_t(oslots.n), s));
+  const KeyMap om{oslots.p, uint64_t(oslots.n)};
+  octet_children<<<grid_for(n, 128), 128, 0, s>>>(okeys.p, n, Dp, da->ekey.p, E, O.meta.p, O.elem.p, om,
+                                                  cnt.p + 4);
+  DBuf<uint8_t> flag;
+  DG_TRY(flag.alloc(E + P));
+  flag_elements<<<grid_for(8 * n, 256), 256, 0, s>>>(okeys.p, n, Dp, O.meta.p, O.elem.p, om, flag.p);
+  if (P) flag_pseudo<<<grid_for(P, 128), 128, 0, s>>>(ps.p, P, Dp, O.meta.p, om, flag.p + E);
   DG_CUDA(cudaGetLastError());
-  // pseudo-octants lie outside the domain child of the embedded root, so they
-  // sort after every element; sorting them alone keeps `all` sorted
-  DG_TRY(radix_sort_u64(all.p + E, tmp.p, P, int(3 * Dp + 5), s));
-  DBuf<uint32_t> flag, pos;
-  DG_TRY(flag.alloc(n));
-  DG_TRY(pos.alloc(n));
-  flag_nodes<<<grid_for(n, 256), 256, 0, s>>>(all.p, n, Dp, flag.p);
-  uint32_t N = 0;
-  DG_TRY(scan_u32(flag.p, pos.p, n, &N, s));
+  NodeKeys nf{flag.p, da->ekey.p, E, ps.p, nullptr, {}};
+  DBuf<uint32_t> nsums;
+  DG_TRY(nsums.alloc(tile_blocks(E + P)));
+  DG_TRY(tile_scan(nf, ItemCount{E + P}, nsums.p, cnt.p + 3, s));
+  DG_TRY(read_words(cnt.p, h, 5, s));
+  DG_CHECK(h[4] == uint32_t(E), DG_EUNBALANCED, "octants inside one another: octree not linear");
+  const int64_t N = h[3];
   da->N = N;
   DG_TRY(da->nkey.alloc(N));
-  emit_node_keys<<<grid_for(n, 256), 256, 0, s>>>(all.p, n, flag.p, pos.p, da->nkey.p);
+  DG_TRY(nslots.alloc(2 * N));
+  DG_CUDA(cudaMemsetAsync(nslots.p, 0xff, sizeof(ulonglong2) * size_t(nslots.n), s));
+  nf.nkey = da->nkey.p;
+  nf.M = KeyMap{nslots.p, uint64_t(nslots.n)};
+  DG_TRY(tile_emit(nf, ItemCount{E + P}, nsums.p, s));
   DG_TRY(da->nl.alloc(8 * E));
   DG_TRY(da->meta.alloc(E));
-  DBuf<uint32_t> err;
-  DG_TRY(err.alloc(1));
-  DG_CUDA(cudaMemsetAsync(err.p, 0, 4, s));
-  build_nlist<<<g, 256, 0, s>>>(ekey.p, E, Dp, da->nkey.p, N, da->nl.p, da->meta.p, err.p);
+  DG_TRY(O.id.alloc(27 * n));
+  octet_lattice<<<grid_for(n, kLatOctets, 8), 256, 0, s>>>(okeys.p, n, Dp, O.meta.p, O.elem.p, nf.M, E, O.id.p,
+                                                           da->nl.p, da->meta.p, cnt.p + 5);
   DG_CUDA(cudaGetLastError());
-  uint32_t herr = 0;
-  DG_CUDA(cudaMemcpyAsync(&herr, err.p, 4, cudaMemcpyDeviceToHost, s));
-  DG_CUDA(cudaStreamSynchronize(s));
-  DG_CHECK(!(herr & 1u), DG_EUNBALANCED, "hanging vertex without a parent node: octree not 2:1 balanced");
-  DG_CHECK(!(herr & 2u), DG_EUNBALANCED, "hanging configuration outside the 18 element types");
-  da->ekey = std::move(ekey);
-  DG_TRY(build_tiles(da, s));
-  return build_octets(da, s);
+  DG_TRY(read_words(cnt.p, h, 6, s));
+  DG_CHECK(!(h[5] & 1u), DG_EUNBALANCED, "hanging vertex without a parent node: octree not 2:1 balanced");
+  DG_CHECK(!(h[5] & 2u), DG_EUNBALANCED, "hanging configuration outside the 18 element types");
+  return DG_OK;
 }
 
 template <int TE>
@@ -473,8 +721,6 @@ dg_status build_tile_set(const dg_da* da, int te, TileSet& ts, cudaStream_t s) {
   DG_CHECK(da->N < (int64_t(1) << 31), DG_EINVAL, "mesh above 2^31 nodes");
   DG_CHECK(te == kMultiTile || te == kWarpTile, DG_EINVAL, "unsupported tile size");
   const int64_t E = da->E, nt = (E + te - 1) / te, S = 8 * int64_t(te);
-  ts.te = te;
-  ts.ntiles = nt;
   DBuf<uint32_t> tmp, cnt, touch;
   DG_TRY(tmp.alloc(nt * S));
   DG_TRY(cnt.alloc(nt));
@@ -531,10 +777,18 @@ dg_status build_tile_set(const dg_da* da, int te, TileSet& ts, cudaStream_t s) {
     ts.inc.reset();
     ts.nend.reset();
   }
+  ts.te = te;
+  ts.ntiles = nt;
   return DG_OK;
 }
 
-dg_status build_tiles(dg_da* da, cudaStream_t s) { return build_tile_set(da, kWarpTile, da->tiles_w, s); }
+dg_status ensure_tiles(dg_da* da, cudaStream_t s) {
+  if (da->tiles_w.ntiles) return DG_OK;
+  PoolScope scope(s);
+  DG_TRY(build_tile_set(da, kWarpTile, da->tiles_w, s));
+  DG_CUDA(cudaStreamSynchronize(s));
+  return DG_OK;
+}
 
 uint32_t etype_mask(int c, int t) { return kEtypeMask[c & 7][t % 18]; }
 

@@ -868,9 +868,10 @@ dg_status mrhs_apply(const dg_mat* A, const float* X, float* Y, int R, int split
                                           : 3;
   }
   if (split == 0 || form == 5) {
-    DG_CHECK(R % 32 == 0 && da->octs.n > 0, DG_EINVAL, "mat_mult_multi: the octet form takes nrhs a multiple of 32");
+    DG_CHECK(R % 32 == 0 && da->octs.n > 0 && da->meshes == 1, DG_EINVAL, "mat_mult_multi: the octet form takes nrhs a multiple of 32");
     return mrhs_octet_apply<float>(A, A->has_coef ? A->coef32.p : nullptr, X, Y, R, s);
   }
+  if (form != 2) DG_TRY(ensure_tiles(da, s));
   if (form >= 3 && R % 32 == 0) {
     static float4* ftbls[64] = {};  // frame tables, one per device, kept for the process
     if (!ftbls[dev]) {

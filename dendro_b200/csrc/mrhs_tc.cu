@@ -517,12 +517,13 @@ dg_status mrhs_tc_apply(const dg_mat* A, const float* X, float* Y, int R, int pa
   dg_da* da = A->da;
   OctetSet& O = da->octs;
   DG_CHECK(A->kind == 0, DG_EINVAL, "mat_mult_multi: scalar operator expected");
-  DG_CHECK(R > 0 && R % kTcRhs == 0 && O.n > 0, DG_EINVAL,
+  DG_CHECK(R > 0 && R % kTcRhs == 0 && O.n > 0 && da->meshes == 1, DG_EINVAL,
            "mat_mult_multi: the tensor-memory form takes nrhs a multiple of 64 on a mesh with octets");
   DG_CHECK(passes == 1 || passes == 3, DG_EINVAL, "mat_mult_multi: passes must be 1 or 3");
   DG_CHECK((reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0, DG_EINVAL,
            "mat_mult_multi: X and Y must be 16-byte aligned");
   const unsigned pg = unsigned(std::min<int64_t>((O.n + 256) / 256, int64_t(sm_count()) * 8));
+  DG_TRY(ensure_octet_records(da, s));
   if (!A->tc_coef.p) DG_TRY(A->tc_coef.alloc((O.n + 1) * kTcCoef));
   const float* ca = A->has_coef ? A->coef32.p : nullptr;
   const float* cb = A->has_coef ? A->coef32.p + da->E : nullptr;

@@ -1,11 +1,14 @@
-// Builds the octet tables of a mesh (OctetSet, octet.cuh): elements grouped by
-// their parent octant, the node id of every lattice point of the parent, the
-// element id of every present child.  One-time set-up after the element ->
-// node map (build_nlist, mesh.cu) exists.
+// Octet tables of a mesh (OctetSet, octet.cuh): elements grouped by their
+// parent octant, the node id of every lattice point of the parent, the element
+// id of every present child.  A mesh built from an octree has them from the
+// octet look-ups that make its element -> node map (mesh.cu); here they are
+// made from a given map (meshes built from maps), and the tables on top of
+// them, chunks and records, for the kernels that read those.
 #include <algorithm>
 #include <vector>
 
 #include "octet.cuh"
+#include "prim.cuh"
 
 namespace dg {
 namespace {
@@ -389,10 +392,9 @@ dg_status build_octets(dg_da* da, cudaStream_t s) {
   DG_TRY(tmp.alloc(E));
   octet_parent_keys<<<grid_for(E, 256), 256, 0, s>>>(da->ekey.p, E, Dp, pk.p);
   DG_CUDA(cudaGetLastError());
-  DG_TRY(radix_sort_u64(pk.p, tmp.p, E, int(3 * Dp + 5), s));
+  DG_TRY(radix_sort_u64(pk, tmp, E, int(3 * Dp + 5), s));
   int64_t n = 0;
-  DG_TRY(unique_u64(pk.p, E, &n, s));
-  O.n = n;
+  DG_TRY(unique_u64(pk, tmp, E, &n, s));
   DG_TRY(O.meta.alloc(n));
   DG_TRY(O.id.alloc(27 * n));
   DG_TRY(O.elem.alloc(8 * n));
@@ -411,15 +413,32 @@ dg_status build_octets(dg_da* da, cudaStream_t s) {
   octet_corners<<<grid_for(n, 256), 256, 0, s>>>(pk.p, n, Dp, da->nkey.p, da->N, hang.p, node.p, O.id.p, err.p);
   DG_CUDA(cudaGetLastError());
   uint32_t herr = 0;
-  DG_CUDA(cudaMemcpyAsync(&herr, err.p, 4, cudaMemcpyDeviceToHost, s));
-  DG_CUDA(cudaStreamSynchronize(s));
+  DG_TRY(read_words(err.p, &herr, 1, s));
   DG_CHECK(!(herr & 1u), DG_EUNBALANCED, "octets: element without its parent entry");
   DG_CHECK(!(herr & 2u), DG_EUNBALANCED, "octets: a lattice point hangs for one child and is a node for another");
   DG_CHECK(!(herr & 4u), DG_EUNBALANCED, "octets: a parent corner needed by a hanging point is not a node");
-  DG_TRY(O.rec.alloc((n + 1) * kOctRec));
-  octet_records<<<grid_for(n + 1, 256), 256, 0, s>>>(n, O.meta.p, O.id.p, O.rec.p);
+  O.n = n;
+  return DG_OK;
+}
+
+dg_status ensure_octet_records(dg_da* da, cudaStream_t s) {
+  OctetSet& O = da->octs;
+  if (O.rec.n || !O.n) return DG_OK;
+  PoolScope scope(s);
+  DG_TRY(O.rec.alloc((O.n + 1) * kOctRec));
+  octet_records<<<grid_for(O.n + 1, 256), 256, 0, s>>>(O.n, O.meta.p, O.id.p, O.rec.p);
   DG_CUDA(cudaGetLastError());
-  return build_chunks(da, s);
+  DG_CUDA(cudaStreamSynchronize(s));
+  return DG_OK;
+}
+
+dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s) {
+  if (da->octs.chunks_tried || !da->octs.n) return DG_OK;
+  PoolScope scope(s);
+  DG_TRY(build_chunks(da, s));
+  da->octs.chunks_tried = true;
+  DG_CUDA(cudaStreamSynchronize(s));
+  return DG_OK;
 }
 
 }  // namespace dg

@@ -4,9 +4,12 @@
 // of coarsening (coarsenOctree, src/oct/Coarsen.C:53-104).
 //
 // All three are integer key manipulations on Morton keys: sort, adjacent
-// unique, per-key arithmetic and binary search.  Outputs are bit-exact with
-// the reference's octant lists (anchors and levels, Morton order).
-#include "dg_internal.h"
+// unique, a hash set and per-key arithmetic.  Outputs are bit-exact with the
+// reference's octant lists (anchors and levels, Morton order).  Counts stay on
+// the device; each operation reads one of them back, to size its output.
+#include <algorithm>
+
+#include "prim.cuh"
 
 namespace dg {
 
@@ -85,87 +88,155 @@ __device__ __forceinline__ void gap_bounds(const uint64_t* __restrict__ lk, int6
   hi = (k == u) ? (1ull << (3u * D)) : okey_m(lk[k]);
 }
 
-__global__ void count_gaps(const uint64_t* __restrict__ lk, int64_t u, uint32_t D, uint32_t* __restrict__ cnt) {
-  for (int64_t k = gtid(); k <= u; k += gstride()) {
+// Item k of u + 1: the octants of the gap before leaf k, then the leaf.
+struct Gaps {
+  const uint64_t* __restrict__ lk;
+  const uint32_t* __restrict__ nu;  // number of leaves u
+  uint32_t D;
+  uint64_t* __restrict__ out;
+  __device__ uint32_t count(int64_t k) const {
+    const int64_t u = *nu;
     uint64_t lo, hi;
     gap_bounds(lk, u, k, D, lo, hi);
-    cnt[k] = gap_blocks(lo, hi, D, nullptr) + (k < u ? 1u : 0u);
+    return gap_blocks(lo, hi, D, nullptr) + (k < u ? 1u : 0u);
   }
-}
-
-__global__ void emit_gaps(const uint64_t* __restrict__ lk, int64_t u, uint32_t D, const uint32_t* __restrict__ pos,
-                          uint64_t* __restrict__ out) {
-  for (int64_t k = gtid(); k <= u; k += gstride()) {
+  __device__ void emit(int64_t k, uint32_t off, uint32_t) const {
+    const int64_t u = *nu;
     uint64_t lo, hi;
     gap_bounds(lk, u, k, D, lo, hi);
-    uint32_t c = gap_blocks(lo, hi, D, out + pos[k]);
-    if (k < u) out[pos[k] + c] = lk[k];
+    const uint32_t c = gap_blocks(lo, hi, D, out + off);
+    if (k < u) out[off + c] = lk[k];
   }
-}
+};
 
 // -------------------------------------------------------------- balance --
-__global__ void level_composite(const uint64_t* __restrict__ ok, int64_t n, uint32_t D, uint64_t* __restrict__ out,
-                                uint32_t* __restrict__ hist) {
-  __shared__ uint32_t h[32];
-  if (threadIdx.x < 32) h[threadIdx.x] = 0;
-  __syncthreads();
-  for (int64_t i = gtid(); i < n; i += gstride()) {
-    uint32_t l = okey_l(ok[i]);
-    uint64_t lk = okey_m(ok[i]) >> (3u * (D - l));
-    out[i] = (uint64_t(l) << 59) | lk;
-    atomicAdd(&h[l], 1u);
+// The internal octants U of the balanced octree, as a set: the parents of the
+// input's leaves, and for every internal octant u at level l the parents of
+// its 26 neighbours of level l (an internal octant's neighbours must exist, so
+// their parents are internal).  Along an axis those are u's parent and the
+// parent's neighbour on u's side of it, so 8 cells at level l - 1 and not 27
+// octants at level l, which halves and more what is looked up; the set is a
+// hash table, because sorting each level's candidates (8 passes over 27 keys
+// per internal octant) was two thirds of the kernel time.  Levels are worked
+// from the finest up, one launch each, with all counts on the device.
+struct InternalSet {
+  uint64_t* table;     // [cap] okeys, kNoKey empty
+  uint64_t cap;
+  uint64_t* list;      // [lcap] the set's members in order of insertion
+  uint32_t lcap;
+  uint32_t* count;     // [0] members from leaves, [1] flag: table or list full, [2 + l] members of level l added
+                       // below leaves' parents
+};
+
+// Lanes whose key is new to the set; a full table raises the flag.
+__device__ __forceinline__ bool set_insert(const InternalSet& S, uint64_t key) {
+  uint64_t h = hash_slot(key, S.cap);
+  for (int probe = 0; probe < kMaxProbes; ++probe) {
+    uint64_t cur = *reinterpret_cast<volatile uint64_t*>(S.table + h);
+    if (cur == kNoKey)
+      cur = atomicCAS(reinterpret_cast<unsigned long long*>(S.table + h), kNoKey, key);
+    if (cur == kNoKey) return true;
+    if (cur == key) return false;
+    h = h + 1 == S.cap ? 0 : h + 1;
   }
-  __syncthreads();
-  if (threadIdx.x < 32 && h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], h[threadIdx.x]);
+  S.count[1] = 1u;
+  return false;
+}
+// Append `key` of the lanes with `is_new` behind the first `base` members,
+// counting them in *ctr: one atomic per warp.  All lanes of the warp call it.
+__device__ __forceinline__ void set_append(const InternalSet& S, bool is_new, uint64_t key, uint32_t base,
+                                           uint32_t* ctr) {
+  const uint32_t m = __ballot_sync(0xffffffffu, is_new);
+  if (!m) return;
+  const int lane = threadIdx.x & 31;
+  uint32_t at = 0;
+  if (lane == __ffs(m) - 1) at = atomicAdd(ctr, uint32_t(__popc(m)));
+  at = base + __shfl_sync(0xffffffffu, at, __ffs(m) - 1) + uint32_t(__popc(m & ((1u << lane) - 1u)));
+  if (!is_new) return;
+  if (at < S.lcap) S.list[at] = key;
+  else S.count[1] = 1u;
 }
 
-__global__ void strip_level(uint64_t* __restrict__ k, int64_t n) {
-  for (int64_t i = gtid(); i < n; i += gstride()) k[i] &= (1ull << 59) - 1ull;
+__device__ __forceinline__ uint64_t parent_key(uint64_t ok, uint32_t D) {
+  uint32_t l = okey_l(ok);
+  uint32_t pl = l ? l - 1 : 0;
+  uint64_t m = okey_m(ok) & ~((1ull << (3u * (D - pl))) - 1ull);
+  return okey(m, pl);
 }
 
-// Adjacent-unique parents of sorted level-l keys (parent key = key >> 3).
-__global__ void mark_parent_unique(const uint64_t* __restrict__ k, int64_t n, uint32_t* __restrict__ flag) {
-  for (int64_t i = gtid(); i < n; i += gstride()) flag[i] = (i == 0 || (k[i] >> 3) != (k[i - 1] >> 3)) ? 1u : 0u;
-}
-__global__ void scatter_parents(const uint64_t* __restrict__ k, int64_t n, const uint32_t* __restrict__ flag,
-                                const uint32_t* __restrict__ pos, uint64_t* __restrict__ out) {
-  for (int64_t i = gtid(); i < n; i += gstride())
-    if (flag[i]) out[pos[i]] = k[i] >> 3;
-}
-
-// The 3x3x3 block of level-l octants around each parent (the parent and its
-// 26 same-level neighbours), clipped to the domain; sentinel ~0 elsewhere.
-__global__ void block27(const uint64_t* __restrict__ u, int64_t nu, uint32_t l, uint64_t* __restrict__ out) {
-  const int64_t side = int64_t(1) << l;
-  for (int64_t t = gtid(); t < nu * 27; t += gstride()) {
-    int64_t i = t / 27;
-    int r = int(t - i * 27);
-    int dx = r % 3 - 1, dy = (r / 3) % 3 - 1, dz = r / 9 - 1;
-    uint32_t x, y, z;
-    demorton(u[i], x, y, z);
-    int64_t nx = int64_t(x) + dx, ny = int64_t(y) + dy, nz = int64_t(z) + dz;
-    bool ok = nx >= 0 && ny >= 0 && nz >= 0 && nx < side && ny < side && nz < side;
-    out[t] = ok ? morton(uint32_t(nx), uint32_t(ny), uint32_t(nz)) : ~0ull;
+__global__ void balance_leaf_parents(const uint64_t* __restrict__ leaf, int64_t n, uint32_t D, InternalSet S) {
+  const int64_t nr = (n + 31) & ~int64_t(31);  // whole warps
+  for (int64_t i = gtid(); i < nr; i += gstride()) {
+    bool fresh = false;
+    uint64_t pk = 0;
+    if (i < n && okey_l(leaf[i]) > 0) {
+      pk = parent_key(leaf[i], D);
+      // siblings are mostly adjacent: only the first of a run inserts
+      if (i == 0 || okey_l(leaf[i - 1]) == 0 || parent_key(leaf[i - 1], D) != pk) fresh = set_insert(S, pk);
+    }
+    set_append(S, fresh, pk, 0u, S.count);
   }
 }
 
-__device__ __forceinline__ bool contains_sorted(const uint64_t* __restrict__ a, int64_t n, uint64_t key) {
-  int64_t lo = 0, hi = n;
-  while (lo < hi) {
-    int64_t mid = (lo + hi) >> 1;
-    if (a[mid] < key) lo = mid + 1; else hi = mid;
+// The members of level l (those among the leaves' parents, and those that the
+// level below added) add theirs at level l - 1; 8 lanes per member.
+__global__ void balance_level(uint32_t l, uint32_t D, InternalSet S) {
+  const uint32_t n0 = min(S.count[0], S.lcap);
+  uint32_t base = n0;
+  for (uint32_t k = l + 1; k < D; ++k) base += S.count[2 + k];
+  const uint32_t nl = S.count[2 + l];
+  const uint32_t wbase = base + nl;
+  const int64_t items = (int64_t(n0) + nl) * 8, nr = (items + 31) & ~int64_t(31);
+  const int64_t side = int64_t(1) << (l - 1);
+  for (int64_t t = gtid(); t < nr; t += gstride()) {
+    bool fresh = false;
+    uint64_t key = 0;
+    if (t < items) {
+      const uint32_t j = uint32_t(t >> 3);
+      const uint64_t at = j < n0 ? j : uint64_t(base) + (j - n0);
+      const uint64_t u = at < S.lcap ? S.list[at] : 0ull;
+      if (at < S.lcap && okey_l(u) == l) {
+        uint32_t c[3];
+        demorton(okey_m(u) >> (3u * (D - l)), c[0], c[1], c[2]);
+        bool in = true;
+        uint32_t q[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          int64_t p = int64_t(c[a] >> 1);
+          if ((t >> a) & 1) p += (c[a] & 1u) ? 1 : -1;
+          in = in && p >= 0 && p < side;
+          q[a] = uint32_t(p);
+        }
+        if (in) {
+          key = okey(morton(q[0], q[1], q[2]) << (3u * (D - l + 1)), l - 1);
+          fresh = set_insert(S, key);
+        }
+      }
+    }
+    set_append(S, fresh, key, wbase, S.count + 2 + (l - 1));
   }
-  return lo < n && a[lo] == key;
 }
 
-// Leaves at level l: children of internal level-(l-1) octants that are not
-// internal themselves.  Writes octant keys at depth D, or ~0 for internal.
-__global__ void emit_children(const uint64_t* __restrict__ up, int64_t nup, const uint64_t* __restrict__ uc,
-                              int64_t nuc, uint32_t l, uint32_t D, uint64_t* __restrict__ out) {
-  for (int64_t t = gtid(); t < nup * 8; t += gstride()) {
-    uint64_t ck = (up[t >> 3] << 3) | uint64_t(t & 7);
-    bool internal = contains_sorted(uc, nuc, ck);
-    out[t] = internal ? ~0ull : okey(ck << (3u * (D - l)), l);
+// The leaves, in order, from the sorted internal octants: child c of internal
+// octant i is internal if its key is in the list, else a leaf.  Its place is
+// known from the number a of internal octants that sort before it.  Of the
+// octants before a leaf L of level d in the pre-order (a key's ancestors
+// before it): an internal one that is not an ancestor of L has all 8 children
+// before L; an ancestor has those before the path to L, plus the path's own
+// where that is internal.  With S the sum of the path's child numbers that is
+// 1 + 8 (a - d) + S + (d - 1) octants, a of them internal: 7 a - 7 d + S leaves.
+__global__ void balance_leaves(const uint64_t* __restrict__ u, int64_t nu, uint32_t D, uint64_t* __restrict__ out) {
+  for (int64_t t = gtid(); t < nu * 8; t += gstride()) {
+    const int64_t i = t >> 3;
+    const uint64_t k = u[i];
+    const uint32_t d = okey_l(k) + 1;
+    const uint64_t m = okey_m(k) | (uint64_t(t & 7) << (3u * (D - d)));
+    const uint64_t ck = okey(m, d);
+    const int64_t a = gallop(u, i + 1, nu, ck);
+    if (a < nu && u[a] == ck) continue;
+    const int64_t S = __popcll(m & 0x1249249249249249ull) + 2 * __popcll(m & 0x2492492492492492ull) +
+                      4 * __popcll(m & 0x4924924924924924ull);
+    out[7 * a - 7 * int64_t(d) + S] = ck;
   }
 }
 
@@ -175,77 +246,30 @@ __device__ __forceinline__ uint32_t child_of(uint64_t ok, uint32_t D) {
   if (l == 0) return 0;
   return uint32_t((okey_m(ok) >> (3u * (D - l))) & 7u);
 }
-__device__ __forceinline__ uint64_t parent_key(uint64_t ok, uint32_t D) {
-  uint32_t l = okey_l(ok);
-  uint32_t pl = l ? l - 1 : 0;
-  uint64_t m = okey_m(ok) & ~((1ull << (3u * (D - pl))) - 1ull);
-  return okey(m, pl);
-}
-
-// family start: a child-0 leaf followed by its 7 siblings as leaves
-__global__ void coarsen_mark(const uint64_t* __restrict__ k, int64_t n, uint32_t D, uint32_t* __restrict__ start) {
-  for (int64_t i = gtid(); i < n; i += gstride()) {
-    uint32_t s = 0;
-    if (i + 7 < n && okey_l(k[i]) > 0 && child_of(k[i], D) == 0 && okey_l(k[i + 7]) == okey_l(k[i]) &&
-        parent_key(k[i + 7], D) == parent_key(k[i], D))
-      s = 1;
-    start[i] = s;
+// A family (a child-0 leaf followed by its 7 siblings as leaves) becomes its
+// parent; other leaves stay.
+struct Coarsen {
+  const uint64_t* __restrict__ k;
+  int64_t n;
+  uint32_t D;
+  uint64_t* __restrict__ out;
+  __device__ bool family(int64_t i) const {
+    const uint64_t a = k[i];
+    if (i + 7 >= n || okey_l(a) == 0 || child_of(a, D) != 0) return false;
+    const uint64_t b = k[i + 7];
+    return okey_l(b) == okey_l(a) && parent_key(b, D) == parent_key(a, D);
   }
-}
-__global__ void coarsen_keep(const uint32_t* __restrict__ start, int64_t n, uint32_t* __restrict__ keep) {
-  for (int64_t i = gtid(); i < n; i += gstride()) {
-    uint32_t kp = 1;
+  __device__ uint32_t count(int64_t i) const {
     for (int d = 1; d <= 7 && i - d >= 0; ++d)
-      if (start[i - d]) kp = 0;
-    keep[i] = kp;
+      if (family(i - d)) return 0u;
+    return 1u;
   }
-}
-__global__ void coarsen_emit(const uint64_t* __restrict__ k, int64_t n, uint32_t D, const uint32_t* __restrict__ start,
-                             const uint32_t* __restrict__ keep, const uint32_t* __restrict__ pos, uint64_t* __restrict__ out) {
-  for (int64_t i = gtid(); i < n; i += gstride())
-    if (keep[i]) out[pos[i]] = start[i] ? parent_key(k[i], D) : k[i];
-}
-
-__global__ void count_not_sentinel(const uint64_t* __restrict__ k, int64_t n, uint32_t* __restrict__ flag) {
-  for (int64_t i = gtid(); i < n; i += gstride()) flag[i] = k[i] != ~0ull ? 1u : 0u;
-}
-
-__global__ void scatter_flagged(const uint64_t* __restrict__ k, int64_t n, const uint32_t* __restrict__ flag,
-                                const uint32_t* __restrict__ pos, uint64_t* __restrict__ out) {
-  for (int64_t i = gtid(); i < n; i += gstride())
-    if (flag[i]) out[pos[i]] = k[i];
-}
+  __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
+    if (c) out[off] = family(i) ? parent_key(k[i], D) : k[i];
+  }
+};
 
 }  // namespace
-
-// Keep the entries of keys[0, n) whose flag is set, in order; keys is
-// reallocated to the compacted length.
-static dg_status compact_by_flag(DBuf<uint64_t>& keys, int64_t n, const uint32_t* flag, int64_t* n_out,
-                                 cudaStream_t s) {
-  DBuf<uint32_t> pos;
-  DBuf<uint64_t> out;
-  DG_TRY(pos.alloc(n));
-  uint32_t total = 0;
-  DG_TRY(scan_u32(flag, pos.p, n, &total, s));
-  DG_TRY(out.alloc(total > 0 ? total : 1));
-  scatter_flagged<<<grid_for(n, 256), 256, 0, s>>>(keys.p, n, flag, pos.p, out.p);
-  DG_CUDA(cudaGetLastError());
-  DG_CUDA(cudaStreamSynchronize(s));
-  keys = std::move(out);
-  *n_out = total;
-  return DG_OK;
-}
-
-static dg_status drop_sentinels(DBuf<uint64_t>& keys, int64_t n, int64_t* n_out, cudaStream_t s) {
-  if (n == 0) {
-    *n_out = 0;
-    return DG_OK;
-  }
-  DBuf<uint32_t> flag;
-  DG_TRY(flag.alloc(n));
-  count_not_sentinel<<<grid_for(n, 256), 256, 0, s>>>(keys.p, n, flag.p);
-  return compact_by_flag(keys, n, flag.p, n_out, s);
-}
 
 static dg_status set_root(dg_octree* out, uint32_t D, cudaStream_t s) {
   out->max_depth = D;
@@ -263,42 +287,39 @@ dg_status points_to_octree(const double* d_pts, int64_t n, uint32_t D, uint32_t 
   DG_CHECK(n >= 0, DG_EINVAL, "negative point count");
   if (D == 0 || n <= int64_t(m)) return set_root(out, D, s);  // Construct.C:884-888,915-919
   DBuf<uint64_t> pk, tmp;
-  DBuf<uint32_t> bad;
+  DBuf<uint32_t> sums, cnt;  // cnt: [0] a point outside, [1] leaves with points, [2] leaves
+  const int64_t nb = tile_blocks(n + 1);
   DG_TRY(pk.alloc(n));
   DG_TRY(tmp.alloc(n));
-  DG_TRY(bad.alloc(1));
-  DG_CUDA(cudaMemsetAsync(bad.p, 0, 4, s));
-  quantise_points<<<grid_for(n, 256), 256, 0, s>>>(d_pts, n, D, pk.p, bad.p);
+  DG_TRY(sums.alloc(nb));
+  DG_TRY(cnt.alloc(3));
+  DG_CUDA(cudaMemsetAsync(cnt.p, 0, 12, s));
+  quantise_points<<<grid_for(n, 256), 256, 0, s>>>(d_pts, n, D, pk.p, cnt.p);
   DG_CUDA(cudaGetLastError());
-  uint32_t hbad = 0;
-  DG_CUDA(cudaMemcpyAsync(&hbad, bad.p, 4, cudaMemcpyDeviceToHost, s));
-  DG_CUDA(cudaStreamSynchronize(s));
-  DG_CHECK(!hbad, DG_EINVAL, "points must lie in [0,1)^3");
-  DG_TRY(radix_sort_u64(pk.p, tmp.p, n, int(3 * D), s));
+  DG_TRY(radix_sort_u64(pk, tmp, n, int(3 * D), s));
   // leaf of every point, then adjacent-unique
   point_leaves<<<grid_for(n, 256), 256, 0, s>>>(pk.p, n, D, m, tmp.p);
   DG_CUDA(cudaGetLastError());
-  int64_t u = 0;
-  DG_TRY(unique_u64(tmp.p, n, &u, s));
+  const UniqueKeys uq{tmp.p, pk.p};
+  DG_TRY(tile_scan(uq, ItemCount{n}, sums.p, cnt.p + 1, s));
+  DG_TRY(tile_emit(uq, ItemCount{n}, sums.p, s));
   // complete the gaps with the coarsest octants
-  DBuf<uint32_t> cnt;
-  DG_TRY(cnt.alloc(u + 1));
-  count_gaps<<<grid_for(u + 1, 256), 256, 0, s>>>(tmp.p, u, D, cnt.p);
-  uint32_t total = 0;
-  DG_TRY(scan_u32(cnt.p, cnt.p, u + 1, &total, s));
-  DG_TRY(out->keys.alloc(total));
-  emit_gaps<<<grid_for(u + 1, 256), 256, 0, s>>>(tmp.p, u, D, cnt.p, out->keys.p);
-  DG_CUDA(cudaGetLastError());
-  DG_CUDA(cudaStreamSynchronize(s));
-  out->n = total;
+  Gaps gaps{pk.p, cnt.p + 1, D, nullptr};
+  const ItemCount ng{n + 1, cnt.p + 1, 1};
+  DG_TRY(tile_scan(gaps, ng, sums.p, cnt.p + 2, s));
+  uint32_t h[3];
+  DG_TRY(read_words(cnt.p, h, 3, s));
+  DG_CHECK(!h[0], DG_EINVAL, "points must lie in [0,1)^3");
+  DG_TRY(out->keys.alloc(h[2]));
+  gaps.out = out->keys.p;
+  DG_TRY(tile_emit(gaps, ng, sums.p, s));
+  out->n = h[2];
   out->max_depth = D;
   return DG_OK;
 }
 
-// Coarsest 2:1 balanced refinement.  W_l (the octants that must exist at
-// level l) is the union of the input leaves at level l and the 3x3x3 blocks
-// around U_l = parents of W_{l+1}; the balanced leaves at level l are the
-// children of U_{l-1} that are not in U_l.
+// Coarsest 2:1 balanced refinement: the set of its internal octants
+// (InternalSet), sorted, and the children that are not in it.
 dg_status balance_octree(const dg_octree* in, dg_octree* out, cudaStream_t s) {
   const uint32_t D = in->max_depth;
   const int64_t n = in->n;
@@ -307,98 +328,43 @@ dg_status balance_octree(const dg_octree* in, dg_octree* out, cudaStream_t s) {
     out->max_depth = D;
     DG_TRY(out->keys.alloc(n > 0 ? n : 1));
     if (n) DG_CUDA(cudaMemcpyAsync(out->keys.p, in->keys.p, 8 * n, cudaMemcpyDeviceToDevice, s));
-    DG_CUDA(cudaStreamSynchronize(s));
     out->n = n;
     return DG_OK;
   }
-  // leaves grouped by level (stable sort on the level bits of a composite key)
-  DBuf<uint64_t> byl, tmp;
-  DBuf<uint32_t> hist;
-  DG_TRY(byl.alloc(n));
-  DG_TRY(tmp.alloc(n));
-  DG_TRY(hist.alloc(32));
-  DG_CUDA(cudaMemsetAsync(hist.p, 0, 128, s));
-  level_composite<<<grid_for(n, 256), 256, 0, s>>>(in->keys.p, n, D, byl.p, hist.p);
+  constexpr int kCounts = 2 + int(kMaxDepth) + 1;
+  DBuf<uint64_t> table, list;
+  DBuf<uint32_t> cnt;
+  DG_TRY(cnt.alloc(kCounts));
+  uint32_t h[kCounts];
+  int64_t nu = 0;
+  // room for 4 times the internal octants of a complete octree of n leaves
+  // (the benchmark's point clouds grow 1.6 to 1.8 times), at half load; a set
+  // that does not fit is built again with four times the room
+  for (int64_t lcap = std::max<int64_t>(4096, 4 * (n / 7)); nu == 0; lcap *= 4) {
+    DG_CHECK(lcap < (int64_t(1) << 30), DG_ENOMEM, "balance: too many octants");
+    DG_TRY(table.alloc(2 * lcap));
+    DG_TRY(list.alloc(lcap));
+    DG_CUDA(cudaMemsetAsync(table.p, 0xff, sizeof(uint64_t) * size_t(2 * lcap), s));
+    DG_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof h, s));
+    const InternalSet S{table.p, uint64_t(2 * lcap), list.p, uint32_t(lcap), cnt.p};
+    balance_leaf_parents<<<grid_for(n, 256), 256, 0, s>>>(in->keys.p, n, D, S);
+    for (uint32_t l = D; l-- > 1;) balance_level<<<grid_for(8 * lcap, 256), 256, 0, s>>>(l, D, S);
+    DG_CUDA(cudaGetLastError());
+    DG_TRY(read_words(cnt.p, h, kCounts, s));
+    if (h[1]) continue;
+    nu = h[0];
+    for (int l = 2; l < kCounts; ++l) nu += h[l];
+    if (nu == 0) return set_root(out, D, s);
+  }
+  table.reset();
+  DBuf<uint64_t> tmp;
+  DG_TRY(tmp.alloc(list.n));
+  DG_TRY(radix_sort_u64(list, tmp, nu, int(3 * D + 5), s));
+  const int64_t total = 7 * nu + 1;
+  DG_CHECK(total < (int64_t(1) << 31), DG_EINVAL, "balance: too many octants");
+  DG_TRY(out->keys.alloc(total));
+  balance_leaves<<<grid_for(8 * nu, 256), 256, 0, s>>>(list.p, nu, D, out->keys.p);
   DG_CUDA(cudaGetLastError());
-  DG_TRY(radix_sort_u64(byl.p, tmp.p, n, 5, s, 59));
-  strip_level<<<grid_for(n, 256), 256, 0, s>>>(byl.p, n);
-  uint32_t h[32];
-  DG_CUDA(cudaMemcpyAsync(h, hist.p, 128, cudaMemcpyDeviceToHost, s));
-  DG_CUDA(cudaStreamSynchronize(s));
-  int64_t off[33];
-  off[0] = 0;
-  for (int l = 0; l < 32; ++l) off[l + 1] = off[l] + h[l];
-
-  std::vector<DBuf<uint64_t>> U(D + 1);  // U[l]: internal octants at level l (sorted level keys)
-  std::vector<int64_t> nU(D + 1, 0);
-  DBuf<uint64_t> W;
-  int64_t nW = h[D];
-  DG_TRY(W.alloc(nW > 0 ? nW : 1));
-  if (nW) DG_CUDA(cudaMemcpyAsync(W.p, byl.p + off[D], 8 * nW, cudaMemcpyDeviceToDevice, s));
-  for (uint32_t l = D; l >= 1; --l) {
-    // U_{l-1} = unique parents of W_l
-    if (nW > 0) {
-      DBuf<uint32_t> flag, pos;
-      DG_TRY(flag.alloc(nW));
-      DG_TRY(pos.alloc(nW));
-      mark_parent_unique<<<grid_for(nW, 256), 256, 0, s>>>(W.p, nW, flag.p);
-      uint32_t tot = 0;
-      DG_TRY(scan_u32(flag.p, pos.p, nW, &tot, s));
-      DG_TRY(U[l - 1].alloc(tot));
-      scatter_parents<<<grid_for(nW, 256), 256, 0, s>>>(W.p, nW, flag.p, pos.p, U[l - 1].p);
-      DG_CUDA(cudaGetLastError());
-      DG_CUDA(cudaStreamSynchronize(s));
-      nU[l - 1] = tot;
-    }
-    if (l - 1 == 0) break;
-    // W_{l-1} = unique(block27(U_{l-1}) + leaves at level l-1)
-    const uint32_t lp = l - 1;
-    int64_t nc = nU[lp] * 27 + int64_t(h[lp]);
-    DBuf<uint64_t> cand, ctmp;
-    DG_TRY(cand.alloc(nc > 0 ? nc : 1));
-    DG_TRY(ctmp.alloc(nc > 0 ? nc : 1));
-    if (nU[lp]) block27<<<grid_for(nU[lp] * 27, 256), 256, 0, s>>>(U[lp].p, nU[lp], lp, cand.p);
-    if (h[lp]) DG_CUDA(cudaMemcpyAsync(cand.p + nU[lp] * 27, byl.p + off[lp], 8 * int64_t(h[lp]),
-                                       cudaMemcpyDeviceToDevice, s));
-    DG_CUDA(cudaGetLastError());
-    // the sentinel needs all 64 bits to sort last
-    DG_TRY(radix_sort_u64(cand.p, ctmp.p, nc, 64, s));
-    int64_t nu = 0;
-    DG_TRY(unique_u64(cand.p, nc, &nu, s));
-    if (nu > 0) {
-      uint64_t last = 0;
-      DG_CUDA(cudaMemcpyAsync(&last, cand.p + nu - 1, 8, cudaMemcpyDeviceToHost, s));
-      DG_CUDA(cudaStreamSynchronize(s));
-      if (last == ~0ull) --nu;
-    }
-    W = std::move(cand);
-    nW = nu;
-  }
-  if (nU[0] == 0) return set_root(out, D, s);
-  // assemble the leaves level by level
-  std::vector<DBuf<uint64_t>> leaves(D + 1);
-  std::vector<int64_t> nleaf(D + 1, 0);
-  int64_t total = 0;
-  for (uint32_t l = 1; l <= D; ++l) {
-    if (nU[l - 1] == 0) continue;
-    int64_t nk = nU[l - 1] * 8;
-    DG_TRY(leaves[l].alloc(nk));
-    const uint64_t* uc = nU[l] ? U[l].p : nullptr;
-    emit_children<<<grid_for(nk, 256), 256, 0, s>>>(U[l - 1].p, nU[l - 1], uc, nU[l], l, D, leaves[l].p);
-    DG_CUDA(cudaGetLastError());
-    DG_TRY(drop_sentinels(leaves[l], nk, &nleaf[l], s));
-    total += nleaf[l];
-  }
-  DBuf<uint64_t> all, atmp;
-  DG_TRY(all.alloc(total));
-  DG_TRY(atmp.alloc(total));
-  int64_t o = 0;
-  for (uint32_t l = 1; l <= D; ++l) {
-    if (nleaf[l]) DG_CUDA(cudaMemcpyAsync(all.p + o, leaves[l].p, 8 * nleaf[l], cudaMemcpyDeviceToDevice, s));
-    o += nleaf[l];
-  }
-  DG_TRY(radix_sort_u64(all.p, atmp.p, total, int(3 * D + 5), s));
-  out->keys = std::move(all);
   out->n = total;
   out->max_depth = D;
   return DG_OK;
@@ -411,23 +377,19 @@ dg_status coarsen_octree(const dg_octree* in, dg_octree* out, cudaStream_t s) {
   if (n < 8) {  // Coarsen.C:66-70
     DG_TRY(out->keys.alloc(n > 0 ? n : 1));
     if (n) DG_CUDA(cudaMemcpyAsync(out->keys.p, in->keys.p, 8 * n, cudaMemcpyDeviceToDevice, s));
-    DG_CUDA(cudaStreamSynchronize(s));
     out->n = n;
     return DG_OK;
   }
-  DBuf<uint32_t> start, keep, pos;
-  DG_TRY(start.alloc(n));
-  DG_TRY(keep.alloc(n));
-  DG_TRY(pos.alloc(n));
-  unsigned g = grid_for(n, 256);
-  coarsen_mark<<<g, 256, 0, s>>>(in->keys.p, n, D, start.p);
-  coarsen_keep<<<g, 256, 0, s>>>(start.p, n, keep.p);
+  const int64_t nb = tile_blocks(n);
+  DBuf<uint32_t> sums;
+  DG_TRY(sums.alloc(nb + 1));
+  Coarsen f{in->keys.p, n, D, nullptr};
+  DG_TRY(tile_scan(f, ItemCount{n}, sums.p, sums.p + nb, s));
   uint32_t total = 0;
-  DG_TRY(scan_u32(keep.p, pos.p, n, &total, s));
+  DG_TRY(read_words(sums.p + nb, &total, 1, s));
   DG_TRY(out->keys.alloc(total));
-  coarsen_emit<<<g, 256, 0, s>>>(in->keys.p, n, D, start.p, keep.p, pos.p, out->keys.p);
-  DG_CUDA(cudaGetLastError());
-  DG_CUDA(cudaStreamSynchronize(s));
+  f.out = out->keys.p;
+  DG_TRY(tile_emit(f, ItemCount{n}, sums.p, s));
   out->n = total;
   return DG_OK;
 }

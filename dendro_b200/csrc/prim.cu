@@ -1,76 +1,54 @@
 // Device-wide primitives: exclusive scan, LSD radix sort of 64-bit keys,
 // adjacent-duplicate removal.  Hand-written; no CUB/Thrust on the path.
-#include "dg_internal.h"
+#include <cstring>
+#include <utility>
+
+#include "prim.cuh"
 
 namespace dg {
 
 namespace {
 
-constexpr int kScanBlock = 1024;  // elements per scan block (256 threads x 4)
-
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
-  const int lane = threadIdx.x & 31;
+// Exclusive scan of nt values in place by one CTA of 1024 threads, 4
+// consecutive values per thread and step; the total to *total.
+__global__ void __launch_bounds__(1024) scan_small_kernel(uint32_t* __restrict__ v, int64_t nt,
+                                                          uint32_t* __restrict__ total) {
+  __shared__ uint32_t ws[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t carry = 0;
+  for (int64_t base = 0; base < nt; base += 4096) {
+    const int64_t i0 = base + int64_t(threadIdx.x) * 4;
+    uint32_t x[4], t = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += t;
+    for (int k = 0; k < 4; ++k) {
+      x[k] = i0 + k < nt ? v[i0 + k] : 0u;
+      t += x[k];
+    }
+    const uint32_t incl = warp_incl_scan(t);
+    if (lane == 31) ws[w] = incl;
+    __syncthreads();
+    const uint32_t wi = warp_incl_scan(ws[lane]);  // every warp scans the 32 warp sums
+    const uint32_t before = __shfl_sync(0xffffffffu, wi, w) - ws[w];
+    const uint32_t sum = __shfl_sync(0xffffffffu, wi, 31);
+    uint32_t run = carry + before + incl - t;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i0 + k < nt) v[i0 + k] = run;
+      run += x[k];
+    }
+    carry += sum;
+    __syncthreads();
   }
-  return v;
+  if (threadIdx.x == 0 && total) *total = carry;
 }
 
-// Block-level exclusive scan of 4 items per thread (256 threads).
-__device__ void block_scan4(uint32_t (&v)[4], uint32_t& block_total) {
-  __shared__ uint32_t warp_sums[8];
-  uint32_t t0 = v[0], t1 = t0 + v[1], t2 = t1 + v[2], t3 = t2 + v[3];
-  uint32_t incl = warp_incl_scan(t3);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 31) warp_sums[wid] = incl;
-  __syncthreads();
-  if (wid == 0) {
-    uint32_t w = lane < 8 ? warp_sums[lane] : 0;
-    uint32_t wi = warp_incl_scan(w);
-    if (lane < 8) warp_sums[lane] = wi - w;
-  }
-  __syncthreads();
-  uint32_t base = warp_sums[wid] + (incl - t3);
-  block_total = 0;
-  v[3] = base + t2;
-  v[2] = base + t1;
-  v[1] = base + t0;
-  v[0] = base;
-}
-
-__global__ void scan_block_sums(const uint32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ sums) {
-  int64_t base = int64_t(blockIdx.x) * kScanBlock + threadIdx.x * 4;
-  uint32_t s = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (base + i < n) s += in[base + i];
-  // block reduce
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  __shared__ uint32_t ws[8];
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int i = 0; i < 8; ++i) t += ws[i];
-    sums[blockIdx.x] = t;
-  }
-}
-
-__global__ void scan_apply(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int64_t n,
-                           const uint32_t* __restrict__ block_off) {
-  int64_t base = int64_t(blockIdx.x) * kScanBlock + threadIdx.x * 4;
-  uint32_t v[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = (base + i < n) ? in[base + i] : 0u;
-  uint32_t tot;
-  block_scan4(v, tot);
-  uint32_t off = block_off ? block_off[blockIdx.x] : 0u;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (base + i < n) out[base + i] = v[i] + off;
-}
+// scan_u32 as a tile emission: every item's output is its own offset.
+struct ScanItems {
+  const uint32_t* in;
+  uint32_t* out;
+  __device__ uint32_t count(int64_t i) const { return in[i]; }
+  __device__ void emit(int64_t i, uint32_t off, uint32_t) const { out[i] = off; }
+};
 
 // ------------------------------------------------------------ radix sort --
 constexpr int kRadixBits = 8;
@@ -79,6 +57,13 @@ constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;  // keys per thread
 constexpr int kSortTile = kSortThreads * kSortItems;
 
+// A pass of the sort is three launches whatever n is: a histogram per block
+// of kSortTile keys, the scan of each digit's row of block counts (a CTA per
+// digit, the row total to rowtot), and the scatter, which scans the 256 row
+// totals itself.  Nothing is allocated or waited for between passes; a
+// device-wide scan of the whole histogram took three more launches, an
+// allocation and a host wait per pass (92 passes of a mesh set-up from
+// 131,072 points: 2.9 ms of kernels and most of its 46 ms of wall time).
 __global__ void __launch_bounds__(kSortThreads)
 radix_hist(const uint64_t* __restrict__ keys, int64_t n, int shift, uint32_t* __restrict__ hist, int nblocks) {
   __shared__ uint32_t h[kBins];
@@ -93,13 +78,40 @@ radix_hist(const uint64_t* __restrict__ keys, int64_t n, int shift, uint32_t* __
   for (int i = threadIdx.x; i < kBins; i += blockDim.x) hist[int64_t(i) * nblocks + blockIdx.x] = h[i];
 }
 
+__global__ void __launch_bounds__(256) radix_rowscan(uint32_t* __restrict__ hist, int nblocks,
+                                                     uint32_t* __restrict__ rowtot) {
+  __shared__ uint32_t ws[8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t* row = hist + int64_t(blockIdx.x) * nblocks;
+  uint32_t carry = 0;
+  for (int base = 0; base < nblocks; base += 256) {
+    const int i = base + int(threadIdx.x);
+    const uint32_t x = i < nblocks ? row[i] : 0u;
+    const uint32_t incl = warp_incl_scan(x);
+    if (lane == 31) ws[w] = incl;
+    __syncthreads();
+    uint32_t before = 0, sum = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      before += k < w ? ws[k] : 0u;
+      sum += ws[k];
+    }
+    if (i < nblocks) row[i] = carry + before + incl - x;
+    carry += sum;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) rowtot[blockIdx.x] = carry;
+}
+
 // Stable scatter.  Warp w owns keys [base + w*512, base + (w+1)*512) in
 // slot-major, lane-minor order; ranks within the warp come from
 // __match_any_sync, and per-(warp, digit) counters give the warp offsets.
 __global__ void __launch_bounds__(kSortThreads)
 radix_scatter(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int64_t n, int shift,
-              const uint32_t* __restrict__ offs, int nblocks) {
+              const uint32_t* __restrict__ offs, int nblocks, const uint32_t* __restrict__ rowtot) {
+  static_assert(kBins == kSortThreads, "one thread per digit");
   __shared__ uint32_t cnt[kSortThreads / 32][kBins];
+  __shared__ uint32_t wtot[kSortThreads / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < (kSortThreads / 32) * kBins; i += blockDim.x) (&cnt[0][0])[i] = 0;
   __syncthreads();
@@ -122,9 +134,17 @@ radix_scatter(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int64
     rank[s] = pre + __popc(peers & lt);
   }
   __syncthreads();
-  // exclusive prefix over warps for each digit, plus the global block offset
-  for (int d = threadIdx.x; d < kBins; d += blockDim.x) {
-    uint32_t run = offs[int64_t(d) * nblocks + blockIdx.x];
+  // exclusive prefix over warps for each digit, plus the digit's first place
+  // (the row totals before it) and the block's place in the digit's row
+  const uint32_t rt = rowtot[threadIdx.x];
+  const uint32_t rincl = warp_incl_scan(rt);
+  if (lane == 31) wtot[wid] = rincl;
+  __syncthreads();
+  {
+    const int d = threadIdx.x;
+    uint32_t run = offs[int64_t(d) * nblocks + blockIdx.x] + rincl - rt;
+#pragma unroll
+    for (int k = 0; k < kSortThreads / 32; ++k) run += k < wid ? wtot[k] : 0u;
     for (int w = 0; w < kSortThreads / 32; ++w) {
       uint32_t c = cnt[w][d];
       cnt[w][d] = run;
@@ -142,17 +162,39 @@ radix_scatter(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int64
   }
 }
 
-__global__ void mark_unique(const uint64_t* __restrict__ k, int64_t n, uint32_t* __restrict__ flag) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    flag[i] = (i == 0 || k[i] != k[i - 1]) ? 1u : 0u;
-}
-__global__ void scatter_unique(const uint64_t* __restrict__ k, int64_t n, const uint32_t* __restrict__ flag,
-                               const uint32_t* __restrict__ pos, uint64_t* __restrict__ out) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    if (flag[i]) out[pos[i]] = k[i];
+}  // namespace
+
+dg_status scan_small(uint32_t* v, int64_t nt, uint32_t* total, cudaStream_t s) {
+  scan_small_kernel<<<1, 1024, 0, s>>>(v, nt, total);
+  DG_CUDA(cudaGetLastError());
+  return DG_OK;
 }
 
+namespace {
+struct HostWords {
+  uint32_t* p = nullptr;
+  uint32_t plain[64];
+  HostWords() {
+    if (cudaHostAlloc(&p, sizeof plain, cudaHostAllocPortable) != cudaSuccess) {
+      (void)cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~HostWords() {
+    if (p) cudaFreeHost(p);
+  }
+};
 }  // namespace
+
+dg_status read_words(const uint32_t* dev, uint32_t* host, int nw, cudaStream_t s) {
+  static thread_local HostWords w;
+  DG_CHECK(nw > 0 && nw <= 64, DG_EINVAL, "read_words: at most 64 words");
+  uint32_t* at = w.p ? w.p : w.plain;
+  DG_CUDA(cudaMemcpyAsync(at, dev, sizeof(uint32_t) * size_t(nw), cudaMemcpyDeviceToHost, s));
+  DG_CUDA(cudaStreamSynchronize(s));
+  memcpy(host, at, sizeof(uint32_t) * size_t(nw));
+  return DG_OK;
+}
 
 dg_status scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* total, cudaStream_t s) {
   if (n <= 0) {
@@ -160,79 +202,50 @@ dg_status scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* total
     return DG_OK;
   }
   DG_CHECK(n < (int64_t(1) << 31), DG_EINVAL, "scan: too many elements");
-  int64_t nb = (n + kScanBlock - 1) / kScanBlock;
-  uint32_t last_in = 0;
-  if (total) DG_CUDA(cudaMemcpyAsync(&last_in, in + n - 1, 4, cudaMemcpyDeviceToHost, s));
-  if (nb == 1) {
-    scan_apply<<<1, 256, 0, s>>>(in, out, n, nullptr);
-  } else {
-    DBuf<uint32_t> sums;
-    DG_TRY(sums.alloc(nb));
-    scan_block_sums<<<unsigned(nb), 256, 0, s>>>(in, n, sums.p);
-    DG_TRY(scan_u32(sums.p, sums.p, nb, nullptr, s));
-    scan_apply<<<unsigned(nb), 256, 0, s>>>(in, out, n, sums.p);
-    DG_CUDA(cudaGetLastError());
-    if (total) {
-      uint32_t last_out = 0;
-      DG_CUDA(cudaMemcpyAsync(&last_out, out + n - 1, 4, cudaMemcpyDeviceToHost, s));
-      DG_CUDA(cudaStreamSynchronize(s));
-      *total = last_out + last_in;
-    }
-    // `sums` is released when this scope ends: finish the work that reads it first
-    DG_CUDA(cudaStreamSynchronize(s));
-    return DG_OK;
-  }
-  DG_CUDA(cudaGetLastError());
-  if (total) {
-    uint32_t last_out = 0;
-    DG_CUDA(cudaMemcpyAsync(&last_out, out + n - 1, 4, cudaMemcpyDeviceToHost, s));
-    DG_CUDA(cudaStreamSynchronize(s));
-    *total = last_out + last_in;
-  }
+  const int64_t nb = tile_blocks(n);
+  DBuf<uint32_t> sums;
+  DG_TRY(sums.alloc(nb + 1));
+  const ScanItems f{in, out};
+  const ItemCount nc{n};
+  DG_TRY(tile_scan(f, nc, sums.p, sums.p + nb, s));
+  DG_TRY(tile_emit(f, nc, sums.p, s));
+  if (total) DG_TRY(read_words(sums.p + nb, total, 1, s));
   return DG_OK;
 }
 
-dg_status radix_sort_u64(uint64_t* keys, uint64_t* tmp, int64_t n, int bits, cudaStream_t s, int start_bit) {
+dg_status radix_sort_u64(DBuf<uint64_t>& keys, DBuf<uint64_t>& tmp, int64_t n, int bits, cudaStream_t s,
+                         int start_bit) {
   if (n <= 1) return DG_OK;
   DG_CHECK(n < (int64_t(1) << 31), DG_EINVAL, "radix sort: too many keys");
-  int nblocks = int((n + kSortTile - 1) / kSortTile);
+  const int nblocks = int((n + kSortTile - 1) / kSortTile);
   DBuf<uint32_t> hist;
-  DG_TRY(hist.alloc(int64_t(kBins) * nblocks));
-  int passes = (bits + kRadixBits - 1) / kRadixBits;
-  uint64_t* src = keys;
-  uint64_t* dst = tmp;
+  DG_TRY(hist.alloc(int64_t(kBins) * nblocks + kBins));
+  uint32_t* rowtot = hist.p + int64_t(kBins) * nblocks;
+  const int passes = (bits + kRadixBits - 1) / kRadixBits;
   for (int p = 0; p < passes; ++p) {
-    int shift = start_bit + p * kRadixBits;
-    radix_hist<<<nblocks, kSortThreads, 0, s>>>(src, n, shift, hist.p, nblocks);
-    DG_TRY(scan_u32(hist.p, hist.p, int64_t(kBins) * nblocks, nullptr, s));
-    radix_scatter<<<nblocks, kSortThreads, 0, s>>>(src, dst, n, shift, hist.p, nblocks);
-    DG_CUDA(cudaGetLastError());
-    uint64_t* t = src;
-    src = dst;
-    dst = t;
+    const int shift = start_bit + p * kRadixBits;
+    radix_hist<<<nblocks, kSortThreads, 0, s>>>(keys.p, n, shift, hist.p, nblocks);
+    radix_rowscan<<<kBins, 256, 0, s>>>(hist.p, nblocks, rowtot);
+    radix_scatter<<<nblocks, kSortThreads, 0, s>>>(keys.p, tmp.p, n, shift, hist.p, nblocks, rowtot);
+    std::swap(keys, tmp);
   }
-  if (src != keys) DG_CUDA(cudaMemcpyAsync(keys, src, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s));
-  DG_CUDA(cudaStreamSynchronize(s));
+  DG_CUDA(cudaGetLastError());
   return DG_OK;
 }
 
-dg_status unique_u64(uint64_t* keys, int64_t n, int64_t* n_out, cudaStream_t s) {
-  if (n <= 1) {
-    *n_out = n;
-    return DG_OK;
-  }
-  DBuf<uint32_t> flag, pos;
-  DBuf<uint64_t> out;
-  DG_TRY(flag.alloc(n));
-  DG_TRY(pos.alloc(n));
-  DG_TRY(out.alloc(n));
-  unsigned g = grid_for(n, 256);
-  mark_unique<<<g, 256, 0, s>>>(keys, n, flag.p);
+dg_status unique_u64(DBuf<uint64_t>& keys, DBuf<uint64_t>& tmp, int64_t n, int64_t* n_out, cudaStream_t s) {
+  *n_out = n;
+  if (n <= 1) return DG_OK;
+  const int64_t nb = tile_blocks(n);
+  DBuf<uint32_t> sums;
+  DG_TRY(sums.alloc(nb + 1));
+  const UniqueKeys f{keys.p, tmp.p};
+  const ItemCount nc{n};
+  DG_TRY(tile_scan(f, nc, sums.p, sums.p + nb, s));
+  DG_TRY(tile_emit(f, nc, sums.p, s));
   uint32_t total = 0;
-  DG_TRY(scan_u32(flag.p, pos.p, n, &total, s));
-  scatter_unique<<<g, 256, 0, s>>>(keys, n, flag.p, pos.p, out.p);
-  DG_CUDA(cudaMemcpyAsync(keys, out.p, sizeof(uint64_t) * total, cudaMemcpyDeviceToDevice, s));
-  DG_CUDA(cudaStreamSynchronize(s));
+  DG_TRY(read_words(sums.p + nb, &total, 1, s));
+  std::swap(keys, tmp);
   *n_out = total;
   return DG_OK;
 }

@@ -18,7 +18,8 @@
 
 #include <type_traits>
 
-#include "dg_internal.h"
+#include "octet.cuh"
+#include "prim.cuh"
 
 #include <cuda_bf16.h>
 
@@ -128,6 +129,21 @@ __global__ void zero_elems(double* __restrict__ coef, int64_t E, const uint32_t*
 // concatenation helpers for batches of meshes
 __global__ void copy_add_u32(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int64_t n, uint32_t add) {
   for (int64_t i = gtid(); i < n; i += gstride()) dst[i] = src[i] + add;
+}
+// Octet tables of one mesh into a batch's at octet oo: blockIdx.y = the row
+// (27 of node ids, 8 of element ids, the meta words).
+__global__ void concat_octets(int64_t n, const uint32_t* __restrict__ meta, const uint32_t* __restrict__ id,
+                              const uint32_t* __restrict__ elem, int64_t nt, int64_t oo, uint32_t node_add,
+                              uint32_t elem_add, uint32_t* __restrict__ tmeta, uint32_t* __restrict__ tid,
+                              uint32_t* __restrict__ telem) {
+  const int r = blockIdx.y;
+  const uint32_t* src = r < 27 ? id + int64_t(r) * n : r < 35 ? elem + int64_t(r - 27) * n : meta;
+  uint32_t* dst = (r < 27 ? tid + int64_t(r) * nt : r < 35 ? telem + int64_t(r - 27) * nt : tmeta) + oo;
+  const uint32_t add = r < 27 ? node_add : r < 35 ? elem_add : 0u;
+  for (int64_t i = gtid(); i < n; i += gstride()) {
+    const uint32_t v = src[i];
+    dst[i] = r < 35 && v == kNoNode ? kNoNode : v + add;
+  }
 }
 __global__ void fill_u16(uint16_t* __restrict__ d, int64_t n0, int64_t n1, uint16_t v) {
   for (int64_t i = n0 + gtid(); i < n1; i += gstride()) d[i] = v;
@@ -852,7 +868,7 @@ dg_status build_restriction(Level& F, int64_t Nc, cudaStream_t s) {
   DG_CUDA(cudaGetLastError());
   int bits = 1;
   while ((int64_t(1) << bits) < Nc) ++bits;
-  DG_TRY(radix_sort_u64(keys.p, tmp.p, nnz, bits, s, 32));
+  DG_TRY(radix_sort_u64(keys, tmp, nnz, bits, s, 32));
   uint32_t total = 0;
   DG_TRY(scan_u32(F.rptr.p, F.rptr.p, Nc + 1, &total, s));
   DG_CHECK(int64_t(total) == nnz, DG_EINVAL, "restriction: entry count mismatch");
@@ -1103,6 +1119,7 @@ dg_status set_elasticity_operators(dg_damg* m) {
     A->dof = 3;
     A->mu = m->cfg.mu;
     A->lam = m->cfg.lambda;
+    DG_TRY(ensure_octet_chunks(L.da.get(), s));
     DG_TRY(A->dirichlet.alloc(L.da->N));
     DG_TRY(node_boundary_flags(L.da.get(), A->dirichlet.p, s));
     L.A = std::move(A);
@@ -1388,7 +1405,7 @@ dg_status build_hierarchy(const dg_octree* finest, int nlevels, cudaStream_t s, 
   t0->max_depth = finest->max_depth;
   t0->n = finest->n;
   DG_TRY(t0->keys.alloc(finest->n));
-  DG_CUDA(cudaMemcpy(t0->keys.p, finest->keys.p, 8 * finest->n, cudaMemcpyDeviceToDevice));
+  DG_CUDA(cudaMemcpyAsync(t0->keys.p, finest->keys.p, 8 * finest->n, cudaMemcpyDeviceToDevice, s));
   trees.push_back(std::move(t0));
   int idx = -1;
   bool repeat = nlevels > 1;
@@ -1459,6 +1476,7 @@ dg_status finish_create(dg_damg* m) {
 // Concatenate per-mesh meshes of one level into one mesh (node ids offset).
 dg_status concat_das(const std::vector<dg_da*>& in, dg_da* out, cudaStream_t s) {
   out->D = in[0]->D;
+  out->meshes = int(in.size());
   int64_t E = 0, N = 0, P = 0;
   for (dg_da* d : in) {
     DG_CHECK(d->D == out->D, DG_EINVAL, "batched meshes must share maxDepth");
@@ -1486,9 +1504,28 @@ dg_status concat_das(const std::vector<dg_da*>& in, dg_da* out, cudaStream_t s) 
     no += d->N;
   }
   DG_CUDA(cudaGetLastError());
-  // no octet tables: the meshes' parent keys coincide across the batch, so
-  // the octet kernels are not offered for a concatenated level
-  return build_tiles(out, s);
+  // the octet tables of the meshes, one after another, with the same offsets
+  // (octets are told apart by their place, so parent keys may coincide)
+  OctetSet& O = out->octs;
+  int64_t n = 0;
+  for (dg_da* d : in) n += d->octs.n;
+  DG_TRY(O.meta.alloc(n));
+  DG_TRY(O.id.alloc(27 * n));
+  DG_TRY(O.elem.alloc(8 * n));
+  int64_t oo = 0;
+  eo = no = 0;
+  for (dg_da* d : in) {
+    const OctetSet& S = d->octs;
+    const dim3 g(grid_for(S.n, 256, 2), 36);
+    concat_octets<<<g, 256, 0, s>>>(S.n, S.meta.p, S.id.p, S.elem.p, n, oo, uint32_t(no), uint32_t(eo), O.meta.p,
+                                    O.id.p, O.elem.p);
+    oo += S.n;
+    eo += d->E;
+    no += d->N;
+  }
+  DG_CUDA(cudaGetLastError());
+  O.n = n;
+  return DG_OK;
 }
 
 // Concatenate per-mesh prolongations (block diagonal).
@@ -1537,6 +1574,7 @@ dg_status dg_damg_create_batch(const dg_octree* const* finest, int count, const 
            DG_ENOTIMPL, "damg_create: dof 3 (elasticity) is one mesh with the FP64 V-cycle and coarse_op 0");
   DG_CUDA(cudaStreamCreateWithFlags(&m->s, cudaStreamNonBlocking));
   cudaStream_t s = m->s;
+  PoolScope scope(s);  // ends before m, so m's buffers outlive no stream that they are freed on
   m->nmesh = count;
   if (count == 1) {
     DG_TRY(build_hierarchy(finest[0], m->cfg.nlevels, s, m->lv));
@@ -1578,6 +1616,7 @@ dg_status dg_damg_create_batch(const dg_octree* const* finest, int count, const 
     DG_CUDA(cudaStreamSynchronize(s));
   }
   DG_TRY(finish_create(m.get()));
+  DG_CUDA(cudaStreamSynchronize(s));
   *out = m.release();
   return DG_OK;
 }
@@ -1595,7 +1634,11 @@ dg_status dg_damg_batch_offsets(const dg_damg* m, int level, int64_t* elem_off, 
 
 dg_status dg_damg_set_lapmass(dg_damg* m, const double* coef) {
   DG_CHECK(m, DG_EINVAL, "damg_set_lapmass: null handle");
-  return set_operators(m, coef);
+  DG_CUDA(cudaDeviceSynchronize());  // the present operators may be in use on other streams
+  PoolScope scope(m->s);
+  DG_TRY(set_operators(m, coef));
+  DG_CUDA(cudaStreamSynchronize(m->s));
+  return DG_OK;
 }
 
 dg_status dg_damg_set_tolerances(dg_damg* m, double rtol, int maxit) {
@@ -1795,7 +1838,7 @@ dg_status dg_damg_solve(dg_damg* m, const double* b, double* x, int on_device, d
   return conv ? DG_OK : DG_ENOTCONVERGED;
 }
 
-void dg_damg_destroy(dg_damg* m) { delete m; }
+void dg_damg_destroy(dg_damg* m) { delete_drained(m); }
 
 }  // extern "C"
 

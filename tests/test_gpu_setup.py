@@ -1,0 +1,85 @@
+"""Octree and mesh set-up at the edges of its hash sets, counts and memory pool."""
+import threading
+
+import numpy as np
+import pytest
+
+from dendro_b200 import inputs as I
+
+pytestmark = pytest.mark.gpu
+
+
+def same(a, b):
+    return len(a) == len(b) and np.array_equal(a.view(np.uint32).reshape(-1, 4), b.view(np.uint32).reshape(-1, 4))
+
+
+def pairs_at_corners(places, depth):
+    """Pairs of points in neighbouring finest cells at corners of a coarse grid: balancing such an octree makes it
+    seven times larger, more than the set of internal octants first has room for."""
+    c = np.unique(np.round(np.random.default_rng(3).uniform(0.1, 0.9, (places, 3)) * 16) / 16, axis=0)
+    return np.concatenate([c + 2.0 ** -(depth + 1), c + 3 * 2.0 ** -(depth + 1)])
+
+
+def check_mesh(gpu, oracle, pts, depth):
+    lin = oracle.points2octree(pts, depth, 1)
+    ref = oracle.balance(lin, depth)
+    assert same(gpu.points2Octree(pts, depth, 1).to_numpy(), lin)
+    bal = gpu.balanceOctree(gpu.Octree.from_octants(lin, depth))
+    assert same(bal.to_numpy(), ref)
+    m = oracle.Mesh(ref, depth)
+    da = gpu.DA(bal)
+    got = da.export()
+    assert (da.E, da.N) == (m.E, m.N)
+    for k, want in (("nlist", m.nlist), ("hmask", m.hmask), ("cnum", m.cnum), ("etype", m.etype), ("level", m.elev),
+                    ("node_xyz", m.node_xyz)):
+        assert np.array_equal(got[k], want), k
+
+
+# one octet, one level, tiles of 2048 octants just filled or overrun, a set that is built again
+@pytest.mark.parametrize("n,depth", [(2, 1), (2, 2), (9, 3), (330, 6), (700, 5), (3000, 12)])
+def test_mesh_sizes(gpu, oracle, n, depth):
+    check_mesh(gpu, oracle, I.clamp_unit(I.uniform_cloud(n, n), depth), depth)
+
+
+def test_mesh_of_a_set_built_again(gpu, oracle):
+    pts = pairs_at_corners(64, 17)
+    lin = oracle.points2octree(pts, 17, 1)
+    assert (len(oracle.balance(lin, 17)) - 1) // 7 > max(4096, 4 * (len(lin) // 7))
+    check_mesh(gpu, oracle, pts, 17)
+
+
+def test_set_up_in_several_threads(gpu, oracle):
+    clouds = [I.clamp_unit(I.gaussian_cloud(1500 + 900 * i, i), 9) for i in range(4)]
+    refs = [oracle.balance(oracle.points2octree(p, 9, 1), 9) for p in clouds]
+    nls = [oracle.Mesh(r, 9).nlist for r in refs]
+    bad = []
+
+    def work(i):
+        for _ in range(5):
+            t = gpu.balanceOctree(gpu.points2Octree(clouds[i], 9, 1))
+            if not same(t.to_numpy(), refs[i]) or not np.array_equal(gpu.DA(t).export()["nlist"], nls[i]):
+                bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+def test_levels_of_a_batch_have_octets(gpu, oracle):
+    """Every octet launch shape on a batch's concatenated mesh, against the meshes one by one."""
+    import torch
+    clouds = [I.clamp_unit(I.gaussian_cloud(n, n), 8) for n in (300, 1700, 40)]
+    trees = [gpu.balanceOctree(gpu.points2Octree(p, 8, 1)) for p in clouds]
+    m = gpu.DAMG(trees, nlevels=3)
+    da = m.level_da(0)
+    _, no = m.batch_offsets(0)
+    x = np.random.default_rng(0).uniform(-1, 1, da.N)
+    want = np.concatenate([oracle.Mesh(t.to_numpy(), 8).matvec(x[no[i]:no[i + 1]]) for i, t in enumerate(trees)])
+    A = gpu.Jacobian2(da)
+    for v in range(A.kernel_count()):
+        A.set_kernel(v)
+        y = A.mult(torch.tensor(x, device="cuda")).cpu().numpy()
+        assert np.linalg.norm(y - want) <= 1e-12 * np.linalg.norm(want), v
