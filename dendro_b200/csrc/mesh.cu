@@ -44,28 +44,36 @@ __device__ __forceinline__ int64_t find_exact(const uint64_t* __restrict__ a, in
   return (lo < n && a[lo] == key) ? lo : -1;
 }
 
-// Hash map of 64-bit keys to 32-bit values: slots (key, value) of 16 bytes,
-// so that a look-up that hits on its first probe reads one 32-byte sector.
-// (Binary searches over the sorted node keys took 22 dependent loads each.)
+// Hash map from the keys of a key array to their places in it: slots of 8
+// bytes, a 32-bit tag of the key's hash above the place, so that a table for
+// the 3.2M nodes of the benchmark mesh at half load (51 MB) stays in L2; a slot
+// whose tag matches is checked against the key array, which is sorted or nearly
+// so and read with locality.  (Binary searches over the sorted node keys take
+// 22 dependent loads each.)
 struct KeyMap {
-  ulonglong2* slot;  // key kNoKey: empty
+  uint64_t* slot;  // kNoKey: empty
   uint64_t cap;
+  const uint64_t* keys;
 };
-__device__ __forceinline__ void map_insert(const KeyMap& M, uint64_t key, uint32_t val) {
-  // keys are distinct and fill at most half the slots, so this ends
+__device__ __forceinline__ uint32_t hash_tag(uint64_t key) { return uint32_t((key * 0xd6e8feb86659fd93ull) >> 33); }
+__device__ __forceinline__ void map_insert(const KeyMap& M, uint64_t key, uint32_t at) {
+  // entries fill at most half the slots, so this ends; tags are below 2^31, so
+  // no entry equals the empty slot
+  const uint64_t e = (uint64_t(hash_tag(key)) << 32) | at;
   uint64_t h = hash_slot(key, M.cap);
-  while (atomicCAS(&M.slot[h].x, kNoKey, key) != kNoKey) h = h + 1 == M.cap ? 0 : h + 1;
-  M.slot[h].y = val;
+  while (atomicCAS(reinterpret_cast<unsigned long long*>(M.slot + h), kNoKey, e) != kNoKey)
+    h = h + 1 == M.cap ? 0 : h + 1;
 }
-// The value of `key`, kNoNode when it is not there; `cur` is the slot at
-// hash_slot(key), read by the caller (so that several reads overlap).
-__device__ __forceinline__ uint32_t map_resolve(const KeyMap& M, uint64_t key, uint64_t h, ulonglong2 cur) {
-  while (cur.x != key) {
-    if (cur.x == kNoKey) return kNoNode;
+// The place of `key`, kNoNode when it is not there; `cur` is the slot at
+// h = hash_slot(key), read by the caller (so that several reads overlap).
+__device__ __forceinline__ uint32_t map_resolve(const KeyMap& M, uint64_t key, uint64_t h, uint64_t cur) {
+  const uint32_t tag = hash_tag(key);
+  while (cur != kNoKey) {
+    if (uint32_t(cur >> 32) == tag && M.keys[uint32_t(cur)] == key) return uint32_t(cur);
     h = h + 1 == M.cap ? 0 : h + 1;
     cur = M.slot[h];
   }
-  return uint32_t(cur.y);
+  return kNoNode;
 }
 __device__ __forceinline__ uint32_t map_find(const KeyMap& M, uint64_t key) {
   const uint64_t h = hash_slot(key, M.cap);
@@ -105,13 +113,46 @@ __device__ __forceinline__ uint64_t embedded_parent(uint64_t k, uint32_t D) {
   const uint32_t l = okey_l(k);
   return okey(okey_m(k) & ~((1ull << (3u * (D - l + 1))) - 1ull), l);
 }
-// The parents of the octants, once per run of siblings.
-struct ParentRuns {
+// The octets: the parents of the octants, each at its first leaf child, so in
+// the order of those and without a sort.  An octant whose predecessor is its
+// sibling is not the first; after a refined sibling the ones before that are
+// looked up, back over the sibling's own octants.
+struct Octets {
   const uint64_t* __restrict__ k;
   uint32_t D;
   uint64_t* __restrict__ out;
+  // first i in [0, hi) with k[i] >= key, searched back from hi
+  __device__ int64_t gallop_back(int64_t hi, uint64_t key) const {
+    int64_t lo = hi, step = 1;
+    while (lo > 0 && k[lo - 1] >= key) {
+      hi = lo - 1;
+      lo = lo > step ? lo - step : 0;
+      step <<= 1;
+      if (k[lo] < key) {
+        ++lo;
+        break;
+      }
+      hi = lo;
+    }
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (k[mid] < key) lo = mid + 1;
+      else hi = mid;
+    }
+    return lo;
+  }
   __device__ uint32_t count(int64_t i) const {
-    return i == 0 || embedded_parent(k[i], D) != embedded_parent(k[i - 1], D) ? 1u : 0u;
+    const uint64_t e = k[i], p = embedded_parent(e, D);
+    const uint32_t l = okey_l(e);
+    if (l == 0) return 1u;
+    const uint32_t sh = 3u * (D - l);
+    int64_t at = i;
+    for (int c = int((okey_m(e) >> sh) & 7u); c > 0; --c) {
+      // `at` is the first octant at or after the anchor of sibling c
+      if (at > 0 && okey_l(k[at - 1]) == l && embedded_parent(k[at - 1], D) == p) return 0u;
+      at = gallop_back(at, okey(okey_m(p) + (uint64_t(c - 1) << sh), 0));
+    }
+    return 1u;
   }
   __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
     if (c) out[off] = embedded_parent(k[i], D);
@@ -286,8 +327,8 @@ __constant__ LatticeTables c_lat = LatticeTables();
 // point p (27 look-ups per octet instead of 64 and more per 8 elements); a
 // vertex without a node hangs and lists its parent's vertex, an octet corner
 // (DA::buildNodeList).  A CTA works 32 octets and writes their rows together.
-// One look-up is a random 32-byte sector, so each warp issues the first probe
-// of its 4 octets before it follows any of them.
+// Each warp issues the first probe of its 4 octets' points before it follows
+// any of them.
 constexpr int kLatOctets = 32;
 __global__ void __launch_bounds__(256) octet_lattice(const uint64_t* __restrict__ okeys, int64_t n, uint32_t Dp,
                                                      const uint32_t* __restrict__ ometa,
@@ -301,15 +342,14 @@ __global__ void __launch_bounds__(256) octet_lattice(const uint64_t* __restrict_
   constexpr uint32_t kNever = (1u << 0) | (1u << 2) | (1u << 6) | (1u << 8) | (1u << 13) | (1u << 18) | (1u << 20) |
                               (1u << 24) | (1u << 26);  // corners and the centre do not hang
   for (int64_t o0 = int64_t(blockIdx.x) * kLatOctets; o0 < n; o0 += int64_t(gridDim.x) * kLatOctets) {
-    uint64_t key[kPer], h[kPer];
-    ulonglong2 cur[kPer];
+    uint64_t key[kPer], h[kPer], cur[kPer];
     uint32_t cm[kPer];
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
       const int64_t o = o0 + w * kPer + j;
       cm[j] = 0;
       key[j] = h[j] = 0;
-      cur[j] = make_ulonglong2(kNoKey, 0);
+      cur[j] = kNoKey;
       if (o < n && lane < 27) {
         const uint64_t k = okeys[o];
         cm[j] = ometa_cmask(ometa[o]);
@@ -628,50 +668,46 @@ dg_status build_mesh(const dg_octree* tree, dg_da* da, cudaStream_t s) {
   DG_TRY(upload_etype_lut());
   DG_CHECK(E < (int64_t(1) << 31), DG_EINVAL, "mesh above 2^31 elements");
   const uint32_t Dp = D + 1;
-  const int bits = int(3 * Dp + 5);
   OctetSet& O = da->octs;
   da->D = Dp;
   da->E = E;
   DG_TRY(da->ekey.alloc(E));
   const int64_t nb = tile_blocks(E);
-  DBuf<uint32_t> sums, cnt;  // cnt: [0] pseudo-octants, [1] sibling runs, [2] octets, [3] nodes, [4] children, [5] errors
+  DBuf<uint32_t> sums, cnt;  // cnt: [0] pseudo-octants, [1] octets, [2] nodes, [3] children, [4] errors
   DG_TRY(sums.alloc(2 * nb));
-  DG_TRY(cnt.alloc(6));
-  DG_CUDA(cudaMemsetAsync(cnt.p, 0, 24, s));
+  DG_TRY(cnt.alloc(5));
+  DG_CUDA(cudaMemsetAsync(cnt.p, 0, 20, s));
   PseudoOctants pf{tree->keys.p, D, da->ekey.p, nullptr};
-  ParentRuns rf{tree->keys.p, D, nullptr};
+  Octets of{tree->keys.p, D, nullptr};
   DG_TRY(tile_scan(pf, ItemCount{E}, sums.p, cnt.p, s));
-  DG_TRY(tile_scan(rf, ItemCount{E}, sums.p + nb, cnt.p + 1, s));
-  uint32_t h[6];
+  DG_TRY(tile_scan(of, ItemCount{E}, sums.p + nb, cnt.p + 1, s));
+  uint32_t h[5];
   DG_TRY(read_words(cnt.p, h, 2, s));
-  const int64_t P = h[0], runs = h[1];
+  const int64_t P = h[0], n = h[1];
   da->P = P;
-  DBuf<uint64_t> ps, pt, okeys, ot;
+  DBuf<uint64_t> ps, pt, okeys;
   DG_TRY(ps.alloc(P));
   DG_TRY(pt.alloc(P));
-  DG_TRY(okeys.alloc(runs));
-  DG_TRY(ot.alloc(runs));
+  DG_TRY(okeys.alloc(n));
   pf.out = ps.p;
-  rf.out = okeys.p;
+  of.out = okeys.p;
   DG_TRY(tile_emit(pf, ItemCount{E}, sums.p, s));
-  DG_TRY(tile_emit(rf, ItemCount{E}, sums.p + nb, s));
-  DG_TRY(radix_sort_u64(ps, pt, P, bits, s));
-  DG_TRY(radix_sort_u64(okeys, ot, runs, bits, s));
-  const UniqueKeys uq{okeys.p, ot.p};
-  DG_TRY(tile_scan(uq, ItemCount{runs}, sums.p, cnt.p + 2, s));
-  DG_TRY(tile_emit(uq, ItemCount{runs}, sums.p, s));
-  std::swap(okeys, ot);
-  DG_TRY(read_words(cnt.p, h, 3, s));
-  const int64_t n = h[2];
+  DG_TRY(tile_emit(of, ItemCount{E}, sums.p + nb, s));
+  // Pseudo-octants are made in the order of their octants.  The octants that
+  // touch a face of the domain are, in their order, ordered on that face (and
+  // so for edges), so the pseudo-octants beyond one face, edge or corner are
+  // sorted already, and those 7 kinds sort by the top bits of the coordinates:
+  // one stable pass on 3 bits sorts them all.
+  DG_TRY(radix_sort_u64(ps, pt, P, 3, s, int(5 + 3 * D)));
   O.n = n;
   DG_TRY(O.meta.alloc(n));
   DG_TRY(O.elem.alloc(8 * n));
-  DBuf<ulonglong2> oslots, nslots;
+  DBuf<uint64_t> oslots, nslots;
   DG_TRY(oslots.alloc(2 * n));
-  DG_CUDA(cudaMemsetAsync(oslots.p, 0xff, sizeof(ulonglong2) * size_t(oslots.n), s));
-  const KeyMap om{oslots.p, uint64_t(oslots.n)};
+  DG_CUDA(cudaMemsetAsync(oslots.p, 0xff, sizeof(uint64_t) * size_t(oslots.n), s));
+  const KeyMap om{oslots.p, uint64_t(oslots.n), okeys.p};
   octet_children<<<grid_for(n, 128), 128, 0, s>>>(okeys.p, n, Dp, da->ekey.p, E, O.meta.p, O.elem.p, om,
-                                                  cnt.p + 4);
+                                                  cnt.p + 3);
   DBuf<uint8_t> flag;
   DG_TRY(flag.alloc(E + P));
   flag_elements<<<grid_for(8 * n, 256), 256, 0, s>>>(okeys.p, n, Dp, O.meta.p, O.elem.p, om, flag.p);
@@ -680,26 +716,26 @@ dg_status build_mesh(const dg_octree* tree, dg_da* da, cudaStream_t s) {
   NodeKeys nf{flag.p, da->ekey.p, E, ps.p, nullptr, {}};
   DBuf<uint32_t> nsums;
   DG_TRY(nsums.alloc(tile_blocks(E + P)));
-  DG_TRY(tile_scan(nf, ItemCount{E + P}, nsums.p, cnt.p + 3, s));
-  DG_TRY(read_words(cnt.p, h, 5, s));
-  DG_CHECK(h[4] == uint32_t(E), DG_EUNBALANCED, "octants inside one another: octree not linear");
-  const int64_t N = h[3];
+  DG_TRY(tile_scan(nf, ItemCount{E + P}, nsums.p, cnt.p + 2, s));
+  DG_TRY(read_words(cnt.p, h, 4, s));
+  DG_CHECK(h[3] == uint32_t(E), DG_EUNBALANCED, "octants inside one another: octree not linear");
+  const int64_t N = h[2];
   da->N = N;
   DG_TRY(da->nkey.alloc(N));
   DG_TRY(nslots.alloc(2 * N));
-  DG_CUDA(cudaMemsetAsync(nslots.p, 0xff, sizeof(ulonglong2) * size_t(nslots.n), s));
+  DG_CUDA(cudaMemsetAsync(nslots.p, 0xff, sizeof(uint64_t) * size_t(nslots.n), s));
   nf.nkey = da->nkey.p;
-  nf.M = KeyMap{nslots.p, uint64_t(nslots.n)};
+  nf.M = KeyMap{nslots.p, uint64_t(nslots.n), da->nkey.p};
   DG_TRY(tile_emit(nf, ItemCount{E + P}, nsums.p, s));
   DG_TRY(da->nl.alloc(8 * E));
   DG_TRY(da->meta.alloc(E));
   DG_TRY(O.id.alloc(27 * n));
   octet_lattice<<<grid_for(n, kLatOctets, 8), 256, 0, s>>>(okeys.p, n, Dp, O.meta.p, O.elem.p, nf.M, E, O.id.p,
-                                                           da->nl.p, da->meta.p, cnt.p + 5);
+                                                           da->nl.p, da->meta.p, cnt.p + 4);
   DG_CUDA(cudaGetLastError());
-  DG_TRY(read_words(cnt.p, h, 6, s));
-  DG_CHECK(!(h[5] & 1u), DG_EUNBALANCED, "hanging vertex without a parent node: octree not 2:1 balanced");
-  DG_CHECK(!(h[5] & 2u), DG_EUNBALANCED, "hanging configuration outside the 18 element types");
+  DG_TRY(read_words(cnt.p, h, 5, s));
+  DG_CHECK(!(h[4] & 1u), DG_EUNBALANCED, "hanging vertex without a parent node: octree not 2:1 balanced");
+  DG_CHECK(!(h[4] & 2u), DG_EUNBALANCED, "hanging configuration outside the 18 element types");
   return DG_OK;
 }
 
