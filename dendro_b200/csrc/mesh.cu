@@ -80,27 +80,46 @@ __device__ __forceinline__ uint32_t map_find(const KeyMap& M, uint64_t key) {
   return map_resolve(M, key, h, M.slot[h]);
 }
 
-// Per octant its positive-boundary pseudo-octants (embedded keys); the
-// octant's own embedded key (level + 1, same anchor) goes to ekey.
+// Per octant its embedded key (level + 1, same anchor) and a byte: bits 0-2
+// the positive faces of the domain that it touches, bits 3-7 the number of
+// internal octants that it is the first element of.
+__global__ void classify_octants(const uint64_t* __restrict__ k, int64_t E, uint32_t D, uint64_t* __restrict__ ekey,
+                                 uint8_t* __restrict__ cls) {
+  for (int64_t i = gtid(); i < E; i += gstride()) {
+    const uint64_t key = k[i];
+    ekey[i] = key + 1;
+    const uint32_t l = okey_l(key);
+    // the coordinates' top l bits are all ones on an axis that touches
+    const uint64_t a = okey_m(key) >> (3u * (D - l)), axis = 0x1249249249249249ull & ((1ull << (3u * l)) - 1ull);
+    uint32_t f = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) f |= uint32_t(((a >> d) & axis) == axis) << d;
+    // its ancestors that do not hold the octant before it: those below the
+    // deepest one that holds both (an octree of the root alone: the embedded
+    // root, its parent)
+    uint32_t c = l ? l : 1u;
+    if (i) {
+      const uint64_t x = okey_m(key) ^ okey_m(k[i - 1]);
+      const uint32_t both = x ? (uint32_t(__clzll(x)) - (64u - 3u * D)) / 3u : D;
+      c = l > both + 1 ? l - 1 - both : 0u;
+    }
+    cls[i] = uint8_t(f | (c << 3));
+  }
+}
+
+// Per octant its positive-boundary pseudo-octants (embedded keys), one per
+// non-empty subset of the faces it touches.
 struct PseudoOctants {
+  const uint8_t* __restrict__ cls;
   const uint64_t* __restrict__ k;
   uint32_t D;
-  uint64_t* __restrict__ ekey;
   uint64_t* __restrict__ out;
-  __device__ uint32_t touching(int64_t i, uint32_t& x, uint32_t& y, uint32_t& z) const {
-    demorton(okey_m(k[i]), x, y, z);
-    const uint32_t blen = (1u << D) - (1u << (D - okey_l(k[i])));
-    return (x == blen) | (y == blen) << 1 | (z == blen) << 2;
-  }
-  __device__ uint32_t count(int64_t i) const {
-    uint32_t x, y, z;
-    return (1u << __popc(touching(i, x, y, z))) - 1u;  // the non-empty subsets of the touched faces
-  }
+  __device__ uint32_t count(int64_t i) const { return (1u << __popc(cls[i] & 7u)) - 1u; }
   __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
-    ekey[i] = k[i] + 1;
     if (!c) return;
     uint32_t x, y, z;
-    const uint32_t f = touching(i, x, y, z), top = 1u << D;
+    demorton(okey_m(k[i]), x, y, z);
+    const uint32_t f = cls[i] & 7u, top = 1u << D;
     uint64_t* o = out + off;
     for (uint32_t s = 1; s < 8; ++s)
       if ((s & f) == s)
@@ -108,80 +127,48 @@ struct PseudoOctants {
   }
 };
 
-// Embedded key of the parent of an octant with (unembedded) key k.
-__device__ __forceinline__ uint64_t embedded_parent(uint64_t k, uint32_t D) {
-  const uint32_t l = okey_l(k);
-  return okey(okey_m(k) & ~((1ull << (3u * (D - l + 1))) - 1ull), l);
-}
-// The octets: the parents of the octants, each at its first leaf child, so in
-// the order of those and without a sort.  An octant whose predecessor is its
-// sibling is not the first; after a refined sibling the ones before that are
-// looked up, back over the sibling's own octants.
-struct Octets {
-  const uint64_t* __restrict__ k;
-  uint32_t D;
+// The internal octants (embedded keys), each at its first element, coarser
+// first: in key order without a sort; `first` keeps that element.
+struct Internals {
+  const uint8_t* __restrict__ cls;
+  const uint64_t* __restrict__ ekey;
+  uint32_t Dp;
   uint64_t* __restrict__ out;
-  // first i in [0, hi) with k[i] >= key, searched back from hi
-  __device__ int64_t gallop_back(int64_t hi, uint64_t key) const {
-    int64_t lo = hi, step = 1;
-    while (lo > 0 && k[lo - 1] >= key) {
-      hi = lo - 1;
-      lo = lo > step ? lo - step : 0;
-      step <<= 1;
-      if (k[lo] < key) {
-        ++lo;
-        break;
-      }
-      hi = lo;
-    }
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (k[mid] < key) lo = mid + 1;
-      else hi = mid;
-    }
-    return lo;
-  }
-  __device__ uint32_t count(int64_t i) const {
-    const uint64_t e = k[i], p = embedded_parent(e, D);
-    const uint32_t l = okey_l(e);
-    if (l == 0) return 1u;
-    const uint32_t sh = 3u * (D - l);
-    int64_t at = i;
-    for (int c = int((okey_m(e) >> sh) & 7u); c > 0; --c) {
-      // `at` is the first octant at or after the anchor of sibling c
-      if (at > 0 && okey_l(k[at - 1]) == l && embedded_parent(k[at - 1], D) == p) return 0u;
-      at = gallop_back(at, okey(okey_m(p) + (uint64_t(c - 1) << sh), 0));
-    }
-    return 1u;
-  }
+  uint32_t* __restrict__ first;
+  __device__ uint32_t count(int64_t i) const { return cls[i] >> 3; }
   __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
-    if (c) out[off] = embedded_parent(k[i], D);
+    const uint64_t e = ekey[i];
+    for (uint32_t j = 0; j < c; ++j) {
+      const uint32_t l = okey_l(e) - c + j;
+      out[off + j] = okey(okey_m(e) & ~((1ull << (3u * (Dp - l))) - 1ull), l);
+      first[off + j] = uint32_t(i);
+    }
   }
 };
 
-// Per octet (parent with leaf children): the element ids of its children, its
-// meta word, and its place in the map of octet keys; *covered counts the
-// children, all E elements when no octant lies inside another.
-__global__ void octet_children(const uint64_t* __restrict__ okeys, int64_t n, uint32_t Dp,
-                               const uint64_t* __restrict__ ekey, int64_t E, uint32_t* __restrict__ ometa,
-                               uint32_t* __restrict__ oelem, KeyMap M, uint32_t* __restrict__ covered) {
+// Per internal octant: the element ids of its leaf children (kid), its meta
+// word, its place in the map of keys, and per child the element anchored at
+// the child's anchor (the child, or the first of its own elements; kNoNode in
+// an octree with holes).  *covered counts the children, all E elements when no
+// octant lies inside another.
+__global__ void octet_children(const uint64_t* __restrict__ ukey, const uint32_t* __restrict__ first, int64_t nu,
+                               uint32_t Dp, const uint64_t* __restrict__ ekey, int64_t E,
+                               uint32_t* __restrict__ umeta, uint32_t* __restrict__ kid,
+                               uint32_t* __restrict__ anchored, KeyMap M, uint32_t* __restrict__ covered) {
   uint32_t mine = 0;
-  for (int64_t o = gtid(); o < n; o += gstride()) {
-    const uint64_t k = okeys[o], am = okey_m(k);
+  for (int64_t o = gtid(); o < nu; o += gstride()) {
+    const uint64_t k = ukey[o], am = okey_m(k);
     const uint32_t m = okey_l(k) + 1;
     const uint32_t sh = 3u * (Dp - m);
-    int64_t lo = 0, hi = E;  // the first element at or after the parent's anchor
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (ekey[mid] < okey(am, 0)) lo = mid + 1;
-      else hi = mid;
-    }
+    int64_t lo = first[o];
     uint32_t mask = 0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const uint64_t ck = okey(am + (uint64_t(c) << sh), m);
-      const bool leaf = lo < E && ekey[lo] == ck;
-      oelem[int64_t(c) * n + o] = leaf ? uint32_t(lo) : kNoNode;
+      const uint64_t cm = am + (uint64_t(c) << sh);
+      const uint64_t at = lo < E ? ekey[lo] : kNoKey;
+      const bool leaf = at == okey(cm, m);
+      kid[int64_t(c) * nu + o] = leaf ? uint32_t(lo) : kNoNode;
+      anchored[int64_t(c) * nu + o] = lo < E && okey_m(at) == cm ? uint32_t(lo) : kNoNode;
       if (leaf) {
         mask |= 1u << c;
         ++lo;
@@ -189,21 +176,45 @@ __global__ void octet_children(const uint64_t* __restrict__ okeys, int64_t n, ui
         lo = gallop(ekey, lo, E, okey(am + (uint64_t(c + 1) << sh), 0));
       }
     }
-    ometa[o] = m | (mask << 8);
+    umeta[o] = m | (mask << 8);
     map_insert(M, k, uint32_t(o));
     mine += __popc(mask);
   }
-  atomicAdd(covered, mine);
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if (mine && (threadIdx.x & 31) == 0) atomicAdd(covered, mine);
 }
 
-// Whether the octant q (an embedded key inside the domain, level >= 1) is an
-// element: its parent is an octet with that child.
-__device__ __forceinline__ bool is_element(const KeyMap& M, const uint32_t* __restrict__ ometa, uint64_t q,
-                                           uint32_t Dp) {
+// The octets: the internal octants with leaf children, in order.
+struct Octets {
+  const uint32_t* __restrict__ umeta;
+  const uint32_t* __restrict__ kid;
+  int64_t nu, n;
+  uint32_t* __restrict__ at;  // [n] the octet's internal octant
+  uint32_t* __restrict__ ometa;
+  uint32_t* __restrict__ oelem;
+  __device__ uint32_t count(int64_t i) const { return ometa_cmask(umeta[i]) ? 1u : 0u; }
+  __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
+    if (!c) return;
+    at[off] = uint32_t(i);
+    ometa[off] = umeta[i];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) oelem[int64_t(k) * n + off] = kid[int64_t(k) * nu + i];
+  }
+};
+
+// The place among the internal octants of the parent of octant q (an embedded
+// key inside the domain, level >= 1) when q is an element -- when that parent
+// has it as a leaf child --, else kNoNode.
+__device__ __forceinline__ uint32_t element_parent(const KeyMap& M, const uint32_t* __restrict__ umeta, uint64_t q,
+                                                   uint32_t Dp) {
   const uint32_t l = okey_l(q);
   const uint64_t m = okey_m(q);
   const uint32_t o = map_find(M, okey(m & ~((1ull << (3u * (Dp - l + 1))) - 1ull), l - 1));
-  return o != kNoNode && ((ometa_cmask(ometa[o]) >> uint32_t((m >> (3u * (Dp - l))) & 7u)) & 1u);
+  return o != kNoNode && ((ometa_cmask(umeta[o]) >> uint32_t((m >> (3u * (Dp - l))) & 7u)) & 1u) ? o : kNoNode;
+}
+__device__ __forceinline__ bool is_element(const KeyMap& M, const uint32_t* __restrict__ umeta, uint64_t q,
+                                           uint32_t Dp) {
+  return element_parent(M, umeta, q, Dp) != kNoNode;
 }
 
 // NODE flags of the elements (flagNodesType3): the anchor of child c is
@@ -271,22 +282,35 @@ __global__ void flag_pseudo(const uint64_t* __restrict__ ps, int64_t P, uint32_t
 
 // The nodes: octants flagged NODE, elements then pseudo-octants, in key
 // order (pseudo-octants lie outside the domain child of the embedded root, so
-// they sort after every element); each node's key goes to the map too.
+// they sort after every element); rank[i] = the node id of octant i's anchor.
 struct NodeKeys {
   const uint8_t* __restrict__ flag;
   const uint64_t* __restrict__ ekey;
   int64_t E;
   const uint64_t* __restrict__ ps;
   uint64_t* __restrict__ nkey;
-  KeyMap M;
+  uint32_t* __restrict__ rank;
   __device__ uint32_t count(int64_t i) const { return flag[i]; }
   __device__ void emit(int64_t i, uint32_t off, uint32_t c) const {
-    if (!c) return;
-    const uint64_t m = okey_m(i < E ? ekey[i] : ps[i - E]);
-    nkey[off] = m;
-    map_insert(M, m, off);
+    rank[i] = c ? off : kNoNode;
+    if (c) nkey[off] = okey_m(i < E ? ekey[i] : ps[i - E]);
   }
 };
+
+// The node ids of the anchors of an internal octant's 8 children, 32 bytes each.
+__global__ void octet_own_nodes(int64_t nu, const uint32_t* __restrict__ anchored, const uint32_t* __restrict__ rank,
+                                uint32_t* __restrict__ own) {
+  for (int64_t o = gtid(); o < nu; o += gstride()) {
+    uint32_t v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const uint32_t e = anchored[int64_t(c) * nu + o];
+      v[c] = e != kNoNode ? rank[e] : kNoNode;
+    }
+    reinterpret_cast<uint4*>(own)[2 * o] = make_uint4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<uint4*>(own)[2 * o + 1] = make_uint4(v[4], v[5], v[6], v[7]);
+  }
+}
 
 // Children of an octet that have lattice point p as a vertex.
 __host__ __device__ constexpr uint32_t lat_children(int p) {
@@ -322,56 +346,114 @@ struct LatticeTables {
 };
 __constant__ LatticeTables c_lat = LatticeTables();
 
+// The node at point m outside the domain: a pseudo-octant's anchor or none.
+struct PseudoNodes {
+  const uint64_t* __restrict__ ps;
+  int64_t P;
+  const uint32_t* __restrict__ rank;  // node ids of the pseudo-octants
+  __device__ uint32_t operator()(uint64_t m) const {
+    const int64_t i = gallop(ps, 0, P, okey(m, 0));
+    return i < P && okey_m(ps[i]) == m ? rank[i] : kNoNode;
+  }
+};
+
 // Element -> node map, hanging masks, element types and the octets' lattice
-// ids from one look-up per lattice point: a warp per octet, lane p looks up
-// point p (27 look-ups per octet instead of 64 and more per 8 elements); a
-// vertex without a node hangs and lists its parent's vertex, an octet corner
-// (DA::buildNodeList).  A CTA works 32 octets and writes their rows together.
-// Each warp issues the first probe of its 4 octets' points before it follows
-// any of them.
+// ids.  An octet's lattice points with coordinates 0 and 1 are its children's
+// anchors; one with a coordinate 2 on the axes of S is a child's anchor of the
+// neighbour cell of the parent's size towards S, so 7 look-ups among the
+// internal octants give all 27 points (a look-up per point in a hash of the
+// nodes took 553 us on the 4.7M-element benchmark mesh, and 248 us to fill).  A
+// neighbour that is not internal is an element, which has a node at most at
+// its anchor, or lies inside an element of twice the size, with a node at most
+// where their anchors meet; both are found through their parents.  A vertex
+// without a node hangs and lists its parent's vertex, an octet corner
+// (DA::buildNodeList).  8 lanes per octet, lane S for the neighbour towards S
+// (0: the octet itself); a CTA works 32 octets and writes their rows together.
 constexpr int kLatOctets = 32;
-__global__ void __launch_bounds__(256) octet_lattice(const uint64_t* __restrict__ okeys, int64_t n, uint32_t Dp,
+__global__ void __launch_bounds__(256) octet_lattice(const uint64_t* __restrict__ ukey,
+                                                     const uint32_t* __restrict__ umeta,
+                                                     const uint32_t* __restrict__ own, KeyMap M,
+                                                     const uint32_t* __restrict__ oat, int64_t n, uint32_t Dp,
                                                      const uint32_t* __restrict__ ometa,
-                                                     const uint32_t* __restrict__ oelem, KeyMap M, int64_t E,
+                                                     const uint32_t* __restrict__ oelem, PseudoNodes F, int64_t E,
                                                      uint32_t* __restrict__ oid, uint32_t* __restrict__ nl,
                                                      uint32_t* __restrict__ meta, uint32_t* __restrict__ err) {
   __shared__ uint32_t sid[27][kLatOctets + 1], shang[kLatOctets];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const uint64_t outside = 1ull << (3u * (Dp - 1));
   constexpr int kPer = kLatOctets / 8;  // octets per warp
   const uint32_t touch = lane < 27 ? c_lat.children[lane] : 0u, corner = lane < 27 ? c_lat.corners[lane] : 0u;
   constexpr uint32_t kNever = (1u << 0) | (1u << 2) | (1u << 6) | (1u << 8) | (1u << 13) | (1u << 18) | (1u << 20) |
                               (1u << 24) | (1u << 26);  // corners and the centre do not hang
   for (int64_t o0 = int64_t(blockIdx.x) * kLatOctets; o0 < n; o0 += int64_t(gridDim.x) * kLatOctets) {
-    uint64_t key[kPer], h[kPer], cur[kPer];
-    uint32_t cm[kPer];
+    {
+      const int j = tid >> 3;
+      const uint32_t S = tid & 7;
+      const int64_t o = o0 + j;
+      if (o < n) {
+        uint32_t q = oat[o];
+        const uint64_t k = ukey[q];
+        const uint32_t pl = okey_l(k);
+        uint64_t am = okey_m(k);
+        if (S) {
+          uint32_t x, y, z;
+          demorton(am, x, y, z);
+          const uint32_t size = 1u << (Dp - pl);
+          am = morton(x + ((S & 1) ? size : 0), y + ((S & 2) ? size : 0), z + ((S & 4) ? size : 0));
+          q = am < outside ? map_find(M, okey(am, pl)) : kNoNode;
+        }
+        const uint32_t sh = 3u * (Dp - pl - 1);
+        uint32_t v[8];
+        if (am >= outside || pl == 0) {
+          // (the root octant alone: its octet's other children are outside)
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const int64_t o = o0 + w * kPer + j;
-      cm[j] = 0;
-      key[j] = h[j] = 0;
-      cur[j] = kNoKey;
-      if (o < n && lane < 27) {
-        const uint64_t k = okeys[o];
-        cm[j] = ometa_cmask(ometa[o]);
-        uint32_t x, y, z;
-        demorton(okey_m(k), x, y, z);
-        const uint32_t s = 1u << (Dp - okey_l(k) - 1);
-        key[j] = morton(x + s * (lane % 3), y + s * ((lane / 3) % 3), z + s * (lane / 9));
-        h[j] = hash_slot(key[j], M.cap);
-        cur[j] = M.slot[h[j]];
+          for (int c = 0; c < 8; ++c) {
+            const uint64_t m = am + (uint64_t(c) << sh);
+            v[c] = uint32_t(c) & S ? kNoNode : m >= outside ? F(m) : own[8 * int64_t(q) + c];
+          }
+        } else if (q != kNoNode) {
+          const uint4 a = reinterpret_cast<const uint4*>(own)[2 * int64_t(q)];
+          const uint4 b = reinterpret_cast<const uint4*>(own)[2 * int64_t(q) + 1];
+          v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+          v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        } else {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) v[c] = kNoNode;
+          // the cell an element, or the first child's place in one (or more
+          // than one) size up
+          for (uint32_t l = pl; l >= 1; --l) {
+            const uint32_t child = uint32_t((am >> (3u * (Dp - l))) & 7u);
+            const uint32_t par = element_parent(M, umeta, okey(am, l), Dp);
+            if (par != kNoNode) {
+              v[0] = own[8 * int64_t(par) + child];
+              break;
+            }
+            if (child) break;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (!(uint32_t(c) & S)) {
+            // per axis: 2 where S, else the child's bit
+            const int px = (S & 1) ? 2 : (c & 1), py = (S & 2) ? 2 : ((c >> 1) & 1), pz = (S & 4) ? 2 : (c >> 2);
+            sid[px + 3 * py + 9 * pz][j] = v[c];
+          }
       }
     }
+    __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const uint32_t id = map_resolve(M, key[j], h[j], cur[j]);
-      const bool present = (cm[j] & touch) != 0u, found = id != kNoNode;
+    for (int i = 0; i < kPer; ++i) {
+      const int j = w * kPer + i;
+      const int64_t o = o0 + j;
+      if (o >= n) break;  // the same for the whole warp
+      const uint32_t id = lane < 27 ? sid[lane][j] : kNoNode;
+      const bool present = (ometa_cmask(ometa[o]) & touch) != 0u, found = id != kNoNode;
       const uint32_t hang = __ballot_sync(0xffffffffu, present && !found);
       const uint32_t need = __reduce_or_sync(0xffffffffu, ((hang >> lane) & 1u) ? corner : 0u);
-      const bool use = (present && found) || ((need >> lane) & 1u);
       if (((need >> lane) & 1u) && !found) atomicOr(err, 1u);
-      if (lane < 27) sid[lane][w * kPer + j] = use ? id : kNoNode;
+      if (lane < 27 && !present && !((need >> lane) & 1u)) sid[lane][j] = kNoNode;
       if (lane == 0) {
-        shang[w * kPer + j] = hang;
+        shang[j] = hang;
         if (hang & kNever) atomicOr(err, 2u);
       }
     }
@@ -673,69 +755,90 @@ dg_status build_mesh(const dg_octree* tree, dg_da* da, cudaStream_t s) {
   da->E = E;
   DG_TRY(da->ekey.alloc(E));
   const int64_t nb = tile_blocks(E);
-  DBuf<uint32_t> sums, cnt;  // cnt: [0] pseudo-octants, [1] octets, [2] nodes, [3] children, [4] errors
+  DBuf<uint32_t> sums, cnt;  // cnt: [0] pseudo-octants, [1] internal octants, [2] nodes, [3] children, [4] errors, [5] octets
   DG_TRY(sums.alloc(2 * nb));
-  DG_TRY(cnt.alloc(5));
-  DG_CUDA(cudaMemsetAsync(cnt.p, 0, 20, s));
-  PseudoOctants pf{tree->keys.p, D, da->ekey.p, nullptr};
-  Octets of{tree->keys.p, D, nullptr};
+  DG_TRY(cnt.alloc(6));
+  DG_CUDA(cudaMemsetAsync(cnt.p, 0, 24, s));
+  DBuf<uint8_t> cls;
+  DG_TRY(cls.alloc(E));
+  classify_octants<<<grid_for(E, 256), 256, 0, s>>>(tree->keys.p, E, D, da->ekey.p, cls.p);
+  PseudoOctants pf{cls.p, tree->keys.p, D, nullptr};
+  Internals uf{cls.p, da->ekey.p, Dp, nullptr, nullptr};
   DG_TRY(tile_scan(pf, ItemCount{E}, sums.p, cnt.p, s));
-  DG_TRY(tile_scan(of, ItemCount{E}, sums.p + nb, cnt.p + 1, s));
-  uint32_t h[5];
+  DG_TRY(tile_scan(uf, ItemCount{E}, sums.p + nb, cnt.p + 1, s));
+  uint32_t h[6];
   DG_TRY(read_words(cnt.p, h, 2, s));
-  const int64_t P = h[0], n = h[1];
+  const int64_t P = h[0], nu = h[1];
   da->P = P;
-  DBuf<uint64_t> ps, pt, okeys;
+  DBuf<uint64_t> ps, pt, ukey;
+  DBuf<uint32_t> first;
   DG_TRY(ps.alloc(P));
   DG_TRY(pt.alloc(P));
-  DG_TRY(okeys.alloc(n));
+  DG_TRY(ukey.alloc(nu));
+  DG_TRY(first.alloc(nu));
   pf.out = ps.p;
-  of.out = okeys.p;
+  uf.out = ukey.p;
+  uf.first = first.p;
   DG_TRY(tile_emit(pf, ItemCount{E}, sums.p, s));
-  DG_TRY(tile_emit(of, ItemCount{E}, sums.p + nb, s));
+  DG_TRY(tile_emit(uf, ItemCount{E}, sums.p + nb, s));
   // Pseudo-octants are made in the order of their octants.  The octants that
   // touch a face of the domain are, in their order, ordered on that face (and
   // so for edges), so the pseudo-octants beyond one face, edge or corner are
   // sorted already, and those 7 kinds sort by the top bits of the coordinates:
   // one stable pass on 3 bits sorts them all.
   DG_TRY(radix_sort_u64(ps, pt, P, 3, s, int(5 + 3 * D)));
-  O.n = n;
-  DG_TRY(O.meta.alloc(n));
-  DG_TRY(O.elem.alloc(8 * n));
-  DBuf<uint64_t> oslots, nslots;
-  DG_TRY(oslots.alloc(2 * n));
-  DG_CUDA(cudaMemsetAsync(oslots.p, 0xff, sizeof(uint64_t) * size_t(oslots.n), s));
-  const KeyMap om{oslots.p, uint64_t(oslots.n), okeys.p};
-  octet_children<<<grid_for(n, 128), 128, 0, s>>>(okeys.p, n, Dp, da->ekey.p, E, O.meta.p, O.elem.p, om,
-                                                  cnt.p + 3);
+  DBuf<uint64_t> slots;
+  DBuf<uint32_t> anchored, kid, umeta;
+  DG_TRY(anchored.alloc(8 * nu));
+  DG_TRY(kid.alloc(8 * nu));
+  DG_TRY(umeta.alloc(nu));
+  DG_TRY(slots.alloc(2 * nu));
+  DG_CUDA(cudaMemsetAsync(slots.p, 0xff, sizeof(uint64_t) * size_t(slots.n), s));
+  const KeyMap um{slots.p, uint64_t(slots.n), ukey.p};
+  octet_children<<<grid_for(nu, 128), 128, 0, s>>>(ukey.p, first.p, nu, Dp, da->ekey.p, E, umeta.p, kid.p, anchored.p,
+                                                   um, cnt.p + 3);
   DBuf<uint8_t> flag;
   DG_TRY(flag.alloc(E + P));
-  flag_elements<<<grid_for(8 * n, 256), 256, 0, s>>>(okeys.p, n, Dp, O.meta.p, O.elem.p, om, flag.p);
-  if (P) flag_pseudo<<<grid_for(P, 128), 128, 0, s>>>(ps.p, P, Dp, O.meta.p, om, flag.p + E);
+  flag_elements<<<grid_for(8 * nu, 256), 256, 0, s>>>(ukey.p, nu, Dp, umeta.p, kid.p, um, flag.p);
+  if (P) flag_pseudo<<<grid_for(P, 128), 128, 0, s>>>(ps.p, P, Dp, umeta.p, um, flag.p + E);
   DG_CUDA(cudaGetLastError());
-  NodeKeys nf{flag.p, da->ekey.p, E, ps.p, nullptr, {}};
-  DBuf<uint32_t> nsums;
-  DG_TRY(nsums.alloc(tile_blocks(E + P)));
+  NodeKeys nf{flag.p, da->ekey.p, E, ps.p, nullptr, nullptr};
+  Octets of{umeta.p, kid.p, nu, 0, nullptr, nullptr, nullptr};
+  DBuf<uint32_t> nsums, rank, own, oat;
+  const int64_t nbn = tile_blocks(E + P);
+  DG_TRY(nsums.alloc(nbn + tile_blocks(nu)));
   DG_TRY(tile_scan(nf, ItemCount{E + P}, nsums.p, cnt.p + 2, s));
-  DG_TRY(read_words(cnt.p, h, 4, s));
+  DG_TRY(tile_scan(of, ItemCount{nu}, nsums.p + nbn, cnt.p + 5, s));
+  DG_TRY(read_words(cnt.p, h, 6, s));
   DG_CHECK(h[3] == uint32_t(E), DG_EUNBALANCED, "octants inside one another: octree not linear");
-  const int64_t N = h[2];
+  const int64_t N = h[2], n = h[5];
   da->N = N;
   DG_TRY(da->nkey.alloc(N));
-  DG_TRY(nslots.alloc(2 * N));
-  DG_CUDA(cudaMemsetAsync(nslots.p, 0xff, sizeof(uint64_t) * size_t(nslots.n), s));
+  DG_TRY(rank.alloc(E + P));
+  DG_TRY(own.alloc(8 * nu));
   nf.nkey = da->nkey.p;
-  nf.M = KeyMap{nslots.p, uint64_t(nslots.n), da->nkey.p};
+  nf.rank = rank.p;
   DG_TRY(tile_emit(nf, ItemCount{E + P}, nsums.p, s));
+  octet_own_nodes<<<grid_for(nu, 256), 256, 0, s>>>(nu, anchored.p, rank.p, own.p);
+  DG_TRY(oat.alloc(n));
+  DG_TRY(O.meta.alloc(n));
+  DG_TRY(O.elem.alloc(8 * n));
+  DG_TRY(O.id.alloc(27 * n));
   DG_TRY(da->nl.alloc(8 * E));
   DG_TRY(da->meta.alloc(E));
-  DG_TRY(O.id.alloc(27 * n));
-  octet_lattice<<<grid_for(n, kLatOctets, 8), 256, 0, s>>>(okeys.p, n, Dp, O.meta.p, O.elem.p, nf.M, E, O.id.p,
-                                                           da->nl.p, da->meta.p, cnt.p + 4);
+  of.n = n;
+  of.at = oat.p;
+  of.ometa = O.meta.p;
+  of.oelem = O.elem.p;
+  DG_TRY(tile_emit(of, ItemCount{nu}, nsums.p + nbn, s));
+  const PseudoNodes pn{ps.p, P, rank.p + E};
+  octet_lattice<<<grid_for(n, kLatOctets, 8), 256, 0, s>>>(ukey.p, umeta.p, own.p, um, oat.p, n, Dp, O.meta.p,
+                                                           O.elem.p, pn, E, O.id.p, da->nl.p, da->meta.p, cnt.p + 4);
   DG_CUDA(cudaGetLastError());
   DG_TRY(read_words(cnt.p, h, 5, s));
   DG_CHECK(!(h[4] & 1u), DG_EUNBALANCED, "hanging vertex without a parent node: octree not 2:1 balanced");
   DG_CHECK(!(h[4] & 2u), DG_EUNBALANCED, "hanging configuration outside the 18 element types");
+  O.n = n;
   return DG_OK;
 }
 

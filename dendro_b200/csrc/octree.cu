@@ -128,7 +128,7 @@ struct InternalSet {
                        // below leaves' parents
 };
 
-// Lanes whose key is new to the set; a full table raises the flag.
+// Whether the key is new to the set; a full table raises the flag.
 __device__ __forceinline__ bool set_insert(const InternalSet& S, uint64_t key) {
   uint64_t h = hash_slot(key, S.cap);
   for (int probe = 0; probe < kMaxProbes; ++probe) {
@@ -142,19 +142,39 @@ __device__ __forceinline__ bool set_insert(const InternalSet& S, uint64_t key) {
   S.count[1] = 1u;
   return false;
 }
-// Append `key` of the lanes with `is_new` behind the first `base` members,
-// counting them in *ctr: one atomic per warp.  All lanes of the warp call it.
-__device__ __forceinline__ void set_append(const InternalSet& S, bool is_new, uint64_t key, uint32_t base,
-                                           uint32_t* ctr) {
-  const uint32_t m = __ballot_sync(0xffffffffu, is_new);
-  if (!m) return;
-  const int lane = threadIdx.x & 31;
-  uint32_t at = 0;
-  if (lane == __ffs(m) - 1) at = atomicAdd(ctr, uint32_t(__popc(m)));
-  at = base + __shfl_sync(0xffffffffu, at, __ffs(m) - 1) + uint32_t(__popc(m & ((1u << lane) - 1u)));
-  if (!is_new) return;
-  if (at < S.lcap) S.list[at] = key;
-  else S.count[1] = 1u;
+// The CTA's new keys behind the first `base` members, counted in *ctr: one
+// atomic per kSetItems items of every thread.  (One per warp and item, all on
+// the same address, was most of the time of these kernels: 94K of them and
+// 125 us for the 3M leaves of the 1M-point benchmark octree.)  All threads of
+// the CTA call it.
+constexpr int kSetThreads = 256;
+constexpr int kSetItems = 4;
+__device__ __forceinline__ void set_append(const InternalSet& S, const bool (&is_new)[kSetItems],
+                                           const uint64_t (&key)[kSetItems], uint32_t base, uint32_t* ctr) {
+  __shared__ uint32_t ws[kSetThreads / 32], at0;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t mine = 0;
+#pragma unroll
+  for (int k = 0; k < kSetItems; ++k) mine += is_new[k];
+  const uint32_t incl = warp_incl_scan(mine);
+  if (lane == 31) ws[w] = incl;
+  __syncthreads();
+  uint32_t before = 0, sum = 0;
+#pragma unroll
+  for (int k = 0; k < kSetThreads / 32; ++k) {
+    before += k < w ? ws[k] : 0u;
+    sum += ws[k];
+  }
+  if (threadIdx.x == 0 && sum) at0 = atomicAdd(ctr, sum);
+  __syncthreads();
+  uint32_t at = base + at0 + before + incl - mine;
+#pragma unroll
+  for (int k = 0; k < kSetItems; ++k) {
+    if (!is_new[k]) continue;
+    if (at < S.lcap) S.list[at] = key[k];
+    else S.count[1] = 1u;
+    ++at;
+  }
 }
 
 __device__ __forceinline__ uint64_t parent_key(uint64_t ok, uint32_t D) {
@@ -164,15 +184,22 @@ __device__ __forceinline__ uint64_t parent_key(uint64_t ok, uint32_t D) {
   return okey(m, pl);
 }
 
-__global__ void balance_leaf_parents(const uint64_t* __restrict__ leaf, int64_t n, uint32_t D, InternalSet S) {
-  const int64_t nr = (n + 31) & ~int64_t(31);  // whole warps
-  for (int64_t i = gtid(); i < nr; i += gstride()) {
-    bool fresh = false;
-    uint64_t pk = 0;
-    if (i < n && okey_l(leaf[i]) > 0) {
-      pk = parent_key(leaf[i], D);
-      // siblings are mostly adjacent: only the first of a run inserts
-      if (i == 0 || okey_l(leaf[i - 1]) == 0 || parent_key(leaf[i - 1], D) != pk) fresh = set_insert(S, pk);
+__global__ void __launch_bounds__(kSetThreads) balance_leaf_parents(const uint64_t* __restrict__ leaf, int64_t n,
+                                                                    uint32_t D, InternalSet S) {
+  constexpr int64_t kStep = kSetThreads * kSetItems;
+  for (int64_t i0 = int64_t(blockIdx.x) * kStep; i0 < n; i0 += int64_t(gridDim.x) * kStep) {
+    bool fresh[kSetItems];
+    uint64_t pk[kSetItems];
+#pragma unroll
+    for (int k = 0; k < kSetItems; ++k) {
+      const int64_t i = i0 + k * kSetThreads + threadIdx.x;
+      fresh[k] = false;
+      pk[k] = 0;
+      if (i < n && okey_l(leaf[i]) > 0) {
+        pk[k] = parent_key(leaf[i], D);
+        // siblings are mostly adjacent: only the first of a run inserts
+        if (i == 0 || okey_l(leaf[i - 1]) == 0 || parent_key(leaf[i - 1], D) != pk[k]) fresh[k] = set_insert(S, pk[k]);
+      }
     }
     set_append(S, fresh, pk, 0u, S.count);
   }
@@ -180,40 +207,47 @@ __global__ void balance_leaf_parents(const uint64_t* __restrict__ leaf, int64_t 
 
 // The members of level l (those among the leaves' parents, and those that the
 // level below added) add theirs at level l - 1; 8 lanes per member.
-__global__ void balance_level(uint32_t l, uint32_t D, InternalSet S) {
+__global__ void __launch_bounds__(kSetThreads) balance_level(uint32_t l, uint32_t D, InternalSet S) {
+  constexpr int64_t kStep = kSetThreads * kSetItems;
   const uint32_t n0 = min(S.count[0], S.lcap);
   uint32_t base = n0;
   for (uint32_t k = l + 1; k < D; ++k) base += S.count[2 + k];
   const uint32_t nl = S.count[2 + l];
   const uint32_t wbase = base + nl;
-  const int64_t items = (int64_t(n0) + nl) * 8, nr = (items + 31) & ~int64_t(31);
+  const int64_t items = (int64_t(n0) + nl) * 8;
   const int64_t side = int64_t(1) << (l - 1);
-  for (int64_t t = gtid(); t < nr; t += gstride()) {
-    bool fresh = false;
-    uint64_t key = 0;
-    if (t < items) {
+  for (int64_t t0 = int64_t(blockIdx.x) * kStep; t0 < items; t0 += int64_t(gridDim.x) * kStep) {
+    bool fresh[kSetItems];
+    uint64_t key[kSetItems];
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < kSetItems; ++k) {
+      const int64_t t = t0 + k * kSetThreads + threadIdx.x;
+      fresh[k] = false;
+      key[k] = 0;
+      if (t >= items) continue;
       const uint32_t j = uint32_t(t >> 3);
       const uint64_t at = j < n0 ? j : uint64_t(base) + (j - n0);
-      const uint64_t u = at < S.lcap ? S.list[at] : 0ull;
-      if (at < S.lcap && okey_l(u) == l) {
-        uint32_t c[3];
-        demorton(okey_m(u) >> (3u * (D - l)), c[0], c[1], c[2]);
-        bool in = true;
-        uint32_t q[3];
+      if (at >= S.lcap) continue;
+      const uint64_t u = S.list[at];
+      if (okey_l(u) != l) continue;
+      uint32_t c[3];
+      demorton(okey_m(u) >> (3u * (D - l)), c[0], c[1], c[2]);
+      bool in = true;
+      uint32_t q[3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          int64_t p = int64_t(c[a] >> 1);
-          if ((t >> a) & 1) p += (c[a] & 1u) ? 1 : -1;
-          in = in && p >= 0 && p < side;
-          q[a] = uint32_t(p);
-        }
-        if (in) {
-          key = okey(morton(q[0], q[1], q[2]) << (3u * (D - l + 1)), l - 1);
-          fresh = set_insert(S, key);
-        }
+      for (int a = 0; a < 3; ++a) {
+        int64_t p = int64_t(c[a] >> 1);
+        if ((t >> a) & 1) p += (c[a] & 1u) ? 1 : -1;
+        in = in && p >= 0 && p < side;
+        q[a] = uint32_t(p);
       }
+      if (!in) continue;
+      key[k] = okey(morton(q[0], q[1], q[2]) << (3u * (D - l + 1)), l - 1);
+      fresh[k] = set_insert(S, key[k]);
+      any = any || fresh[k];
     }
-    set_append(S, fresh, key, wbase, S.count + 2 + (l - 1));
+    if (__syncthreads_or(any)) set_append(S, fresh, key, wbase, S.count + 2 + (l - 1));
   }
 }
 
@@ -347,8 +381,8 @@ dg_status balance_octree(const dg_octree* in, dg_octree* out, cudaStream_t s) {
     DG_CUDA(cudaMemsetAsync(table.p, 0xff, sizeof(uint64_t) * size_t(2 * lcap), s));
     DG_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof h, s));
     const InternalSet S{table.p, uint64_t(2 * lcap), list.p, uint32_t(lcap), cnt.p};
-    balance_leaf_parents<<<grid_for(n, 256), 256, 0, s>>>(in->keys.p, n, D, S);
-    for (uint32_t l = D; l-- > 1;) balance_level<<<grid_for(8 * lcap, 256), 256, 0, s>>>(l, D, S);
+    balance_leaf_parents<<<grid_for(n, kSetThreads * kSetItems), kSetThreads, 0, s>>>(in->keys.p, n, D, S);
+    for (uint32_t l = D; l-- > 1;) balance_level<<<grid_for(8 * lcap, kSetThreads * kSetItems), kSetThreads, 0, s>>>(l, D, S);
     DG_CUDA(cudaGetLastError());
     DG_TRY(read_words(cnt.p, h, kCounts, s));
     if (h[1]) continue;
