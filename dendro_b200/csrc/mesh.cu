@@ -46,38 +46,32 @@ __device__ __forceinline__ int64_t find_exact(const uint64_t* __restrict__ a, in
 
 // Hash map from the keys of a key array to their places in it: slots of 8
 // bytes, a 32-bit tag of the key's hash above the place, so that a table for
-// the 3.2M nodes of the benchmark mesh at half load (51 MB) stays in L2; a slot
+// the 672K internal octants of the benchmark mesh (17 MB) stays in L2; a slot
 // whose tag matches is checked against the key array, which is sorted or nearly
 // so and read with locality.  (Binary searches over the sorted node keys take
 // 22 dependent loads each.)
 struct KeyMap {
   uint64_t* slot;  // kNoKey: empty
-  uint64_t cap;
+  HashShape shape;
   const uint64_t* keys;
 };
-__device__ __forceinline__ uint32_t hash_tag(uint64_t key) { return uint32_t((key * 0xd6e8feb86659fd93ull) >> 33); }
 __device__ __forceinline__ void map_insert(const KeyMap& M, uint64_t key, uint32_t at) {
   // entries fill at most half the slots, so this ends; tags are below 2^31, so
   // no entry equals the empty slot
-  const uint64_t e = (uint64_t(hash_tag(key)) << 32) | at;
-  uint64_t h = hash_slot(key, M.cap);
-  while (atomicCAS(reinterpret_cast<unsigned long long*>(M.slot + h), kNoKey, e) != kNoKey)
-    h = h + 1 == M.cap ? 0 : h + 1;
+  const uint64_t mix = hash_mix(key), wrap = M.shape.slots() - 1;
+  const uint64_t e = (uint64_t(hash_tag(mix, M.shape)) << 32) | at;
+  uint64_t h = mix >> M.shape.shift;
+  while (atomicCAS(reinterpret_cast<unsigned long long*>(M.slot + h), kNoKey, e) != kNoKey) h = (h + 1) & wrap;
 }
-// The place of `key`, kNoNode when it is not there; `cur` is the slot at
-// h = hash_slot(key), read by the caller (so that several reads overlap).
-__device__ __forceinline__ uint32_t map_resolve(const KeyMap& M, uint64_t key, uint64_t h, uint64_t cur) {
-  const uint32_t tag = hash_tag(key);
-  while (cur != kNoKey) {
-    if (uint32_t(cur >> 32) == tag && M.keys[uint32_t(cur)] == key) return uint32_t(cur);
-    h = h + 1 == M.cap ? 0 : h + 1;
-    cur = M.slot[h];
-  }
-  return kNoNode;
-}
+// The place of `key`, kNoNode when it is not there.
 __device__ __forceinline__ uint32_t map_find(const KeyMap& M, uint64_t key) {
-  const uint64_t h = hash_slot(key, M.cap);
-  return map_resolve(M, key, h, M.slot[h]);
+  const uint64_t mix = hash_mix(key), wrap = M.shape.slots() - 1;
+  const uint32_t tag = hash_tag(mix, M.shape);
+  for (uint64_t h = mix >> M.shape.shift;; h = (h + 1) & wrap) {
+    const uint64_t cur = M.slot[h];
+    if (cur == kNoKey) return kNoNode;
+    if (uint32_t(cur >> 32) == tag && M.keys[uint32_t(cur)] == key) return uint32_t(cur);
+  }
 }
 
 // Per octant its embedded key (level + 1, same anchor) and a byte: bits 0-2
@@ -162,6 +156,23 @@ __global__ void octet_children(const uint64_t* __restrict__ ukey, const uint32_t
     const uint32_t sh = 3u * (Dp - m);
     int64_t lo = first[o];
     uint32_t mask = 0;
+    // mostly the 8 children are the next 8 elements: read them together
+    bool all = lo + 8 <= E;
+    if (all) {
+      uint64_t e[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) e[c] = ekey[lo + c];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) all = all && e[c] == okey(am + (uint64_t(c) << sh), m);
+    }
+    if (all) {
+      mask = 255u;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        kid[int64_t(c) * nu + o] = uint32_t(lo + c);
+        anchored[int64_t(c) * nu + o] = uint32_t(lo + c);
+      }
+    } else
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       const uint64_t cm = am + (uint64_t(c) << sh);
@@ -235,11 +246,12 @@ __global__ void flag_elements(const uint64_t* __restrict__ okeys, int64_t n, uin
       const uint64_t k = okeys[o];
       const uint32_t pl = okey_l(k);
       if (pl >= 1 && c != 0 && c != 7) {
-        uint32_t x, y, z;
-        demorton(okey_m(k), x, y, z);
-        const uint32_t S = 1u << (Dp - pl);
-        if (!(((c & 1) && !x) || ((c & 2) && !y) || ((c & 4) && !z)))
-          coarse = is_element(M, ometa, okey(morton(x - ((c & 1) ? S : 0), y - ((c & 2) ? S : 0), z - ((c & 4) ? S : 0)), pl), Dp);
+        const uint64_t unit = 1ull << (3u * (Dp - pl));
+        uint64_t q = okey_m(k);
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if ((c >> a) & 1) q = morton_dec(q, a, unit << a);
+        if (!(q >> (3u * Dp))) coarse = is_element(M, ometa, okey(q, pl), Dp);
       }
     }
     const uint32_t L = __ballot_sync(0xffffffffu, coarse) >> (threadIdx.x & 24);
@@ -396,10 +408,10 @@ __global__ void __launch_bounds__(256) octet_lattice(const uint64_t* __restrict_
         const uint32_t pl = okey_l(k);
         uint64_t am = okey_m(k);
         if (S) {
-          uint32_t x, y, z;
-          demorton(am, x, y, z);
-          const uint32_t size = 1u << (Dp - pl);
-          am = morton(x + ((S & 1) ? size : 0), y + ((S & 2) ? size : 0), z + ((S & 4) ? size : 0));
+          const uint64_t unit = 1ull << (3u * (Dp - pl));
+#pragma unroll
+          for (int a = 0; a < 3; ++a)
+            if ((S >> a) & 1) am = morton_inc(am, a, unit << a);
           q = am < outside ? map_find(M, okey(am, pl)) : kNoNode;
         }
         const uint32_t sh = 3u * (Dp - pl - 1);
@@ -792,10 +804,11 @@ dg_status build_mesh(const dg_octree* tree, dg_da* da, cudaStream_t s) {
   DG_TRY(anchored.alloc(8 * nu));
   DG_TRY(kid.alloc(8 * nu));
   DG_TRY(umeta.alloc(nu));
-  DG_TRY(slots.alloc(2 * nu));
+  const HashShape shape = hash_shape(nu);
+  DG_TRY(slots.alloc(int64_t(shape.slots())));
   DG_CUDA(cudaMemsetAsync(slots.p, 0xff, sizeof(uint64_t) * size_t(slots.n), s));
-  const KeyMap um{slots.p, uint64_t(slots.n), ukey.p};
-  octet_children<<<grid_for(nu, 128), 128, 0, s>>>(ukey.p, first.p, nu, Dp, da->ekey.p, E, umeta.p, kid.p, anchored.p,
+  const KeyMap um{slots.p, shape, ukey.p};
+  octet_children<<<grid_for(nu, 128, 16), 128, 0, s>>>(ukey.p, first.p, nu, Dp, da->ekey.p, E, umeta.p, kid.p, anchored.p,
                                                    um, cnt.p + 3);
   DBuf<uint8_t> flag;
   DG_TRY(flag.alloc(E + P));

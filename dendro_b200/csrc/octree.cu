@@ -120,35 +120,43 @@ struct Gaps {
 // per internal octant) was two thirds of the kernel time.  Levels are worked
 // from the finest up, one launch each, with all counts on the device.
 struct InternalSet {
-  uint64_t* table;     // [cap] okeys, kNoKey empty
-  uint64_t cap;
+  uint64_t* table;     // okeys, kNoKey empty
+  HashShape shape;
   uint64_t* list;      // [lcap] the set's members in order of insertion
   uint32_t lcap;
   uint32_t* count;     // [0] members from leaves, [1] flag: table or list full, [2 + l] members of level l added
                        // below leaves' parents
 };
 
-// Whether the key is new to the set; a full table raises the flag.
-__device__ __forceinline__ bool set_insert(const InternalSet& S, uint64_t key) {
-  uint64_t h = hash_slot(key, S.cap);
+// Whether the key is new to the set; a full table raises the flag.  `h` is the
+// key's slot and `cur` what the caller read there (reads of several keys
+// overlap).
+__device__ __forceinline__ uint64_t set_slot(const InternalSet& S, uint64_t key) {
+  return hash_mix(key) >> S.shape.shift;
+}
+__device__ __forceinline__ uint64_t set_peek(const InternalSet& S, uint64_t h) {
+  return *reinterpret_cast<volatile uint64_t*>(S.table + h);
+}
+__device__ __forceinline__ bool set_insert(const InternalSet& S, uint64_t key, uint64_t h, uint64_t cur) {
+  const uint64_t wrap = S.shape.slots() - 1;
   for (int probe = 0; probe < kMaxProbes; ++probe) {
-    uint64_t cur = *reinterpret_cast<volatile uint64_t*>(S.table + h);
-    if (cur == kNoKey)
-      cur = atomicCAS(reinterpret_cast<unsigned long long*>(S.table + h), kNoKey, key);
+    if (cur == kNoKey) cur = atomicCAS(reinterpret_cast<unsigned long long*>(S.table + h), kNoKey, key);
     if (cur == kNoKey) return true;
     if (cur == key) return false;
-    h = h + 1 == S.cap ? 0 : h + 1;
+    h = (h + 1) & wrap;
+    cur = set_peek(S, h);
   }
   S.count[1] = 1u;
   return false;
 }
+
 // The CTA's new keys behind the first `base` members, counted in *ctr: one
 // atomic per kSetItems items of every thread.  (One per warp and item, all on
-// the same address, was most of the time of these kernels: 94K of them and
-// 125 us for the 3M leaves of the 1M-point benchmark octree.)  All threads of
+// the same address, took most of the 125 us that the 3M leaves of the 1M-point
+// benchmark octree did: 94K atomics.)  All threads of
 // the CTA call it.
 constexpr int kSetThreads = 256;
-constexpr int kSetItems = 4;
+constexpr int kSetItems = 2;
 __device__ __forceinline__ void set_append(const InternalSet& S, const bool (&is_new)[kSetItems],
                                            const uint64_t (&key)[kSetItems], uint32_t base, uint32_t* ctr) {
   __shared__ uint32_t ws[kSetThreads / 32], at0;
@@ -198,7 +206,10 @@ __global__ void __launch_bounds__(kSetThreads) balance_leaf_parents(const uint64
       if (i < n && okey_l(leaf[i]) > 0) {
         pk[k] = parent_key(leaf[i], D);
         // siblings are mostly adjacent: only the first of a run inserts
-        if (i == 0 || okey_l(leaf[i - 1]) == 0 || parent_key(leaf[i - 1], D) != pk[k]) fresh[k] = set_insert(S, pk[k]);
+        if (i == 0 || okey_l(leaf[i - 1]) == 0 || parent_key(leaf[i - 1], D) != pk[k]) {
+          const uint64_t h = set_slot(S, pk[k]);
+          fresh[k] = set_insert(S, pk[k], h, set_peek(S, h));
+        }
       }
     }
     set_append(S, fresh, pk, 0u, S.count);
@@ -215,36 +226,40 @@ __global__ void __launch_bounds__(kSetThreads) balance_level(uint32_t l, uint32_
   const uint32_t nl = S.count[2 + l];
   const uint32_t wbase = base + nl;
   const int64_t items = (int64_t(n0) + nl) * 8;
-  const int64_t side = int64_t(1) << (l - 1);
   for (int64_t t0 = int64_t(blockIdx.x) * kStep; t0 < items; t0 += int64_t(gridDim.x) * kStep) {
-    bool fresh[kSetItems];
-    uint64_t key[kSetItems];
+    bool fresh[kSetItems], mine[kSetItems];
+    uint64_t key[kSetItems], h[kSetItems], cur[kSetItems];
     bool any = false;
 #pragma unroll
     for (int k = 0; k < kSetItems; ++k) {
       const int64_t t = t0 + k * kSetThreads + threadIdx.x;
-      fresh[k] = false;
-      key[k] = 0;
+      fresh[k] = mine[k] = false;
+      key[k] = h[k] = cur[k] = 0;
       if (t >= items) continue;
       const uint32_t j = uint32_t(t >> 3);
       const uint64_t at = j < n0 ? j : uint64_t(base) + (j - n0);
       if (at >= S.lcap) continue;
       const uint64_t u = S.list[at];
       if (okey_l(u) != l) continue;
-      uint32_t c[3];
-      demorton(okey_m(u) >> (3u * (D - l)), c[0], c[1], c[2]);
-      bool in = true;
-      uint32_t q[3];
+      // the parent's anchor, stepped towards u's side on the lane's axes
+      const uint32_t sh = 3u * (D - l + 1);
+      const uint64_t m = okey_m(u);
+      uint64_t q = (m >> sh) << sh;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        int64_t p = int64_t(c[a] >> 1);
-        if ((t >> a) & 1) p += (c[a] & 1u) ? 1 : -1;
-        in = in && p >= 0 && p < side;
-        q[a] = uint32_t(p);
-      }
-      if (!in) continue;
-      key[k] = okey(morton(q[0], q[1], q[2]) << (3u * (D - l + 1)), l - 1);
-      fresh[k] = set_insert(S, key[k]);
+      for (int a = 0; a < 3; ++a)
+        if ((t >> a) & 1) {
+          const uint64_t unit = 1ull << (sh + a);
+          q = ((m >> (sh - 3 + a)) & 1u) ? morton_inc(q, a, unit) : morton_dec(q, a, unit);
+        }
+      if (q >> (3u * D)) continue;  // outside the domain
+      mine[k] = true;
+      key[k] = okey(q, l - 1);
+      h[k] = set_slot(S, key[k]);
+      cur[k] = set_peek(S, h[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kSetItems; ++k) {
+      if (mine[k]) fresh[k] = set_insert(S, key[k], h[k], cur[k]);
       any = any || fresh[k];
     }
     if (__syncthreads_or(any)) set_append(S, fresh, key, wbase, S.count + 2 + (l - 1));
@@ -372,15 +387,16 @@ dg_status balance_octree(const dg_octree* in, dg_octree* out, cudaStream_t s) {
   uint32_t h[kCounts];
   int64_t nu = 0;
   // room for 4 times the internal octants of a complete octree of n leaves
-  // (the benchmark's point clouds grow 1.6 to 1.8 times), at half load; a set
-  // that does not fit is built again with four times the room
+  // (the benchmark's point clouds grow 1.6 to 1.8 times), at most half
+  // full; a set that does not fit is built again with four times the room
   for (int64_t lcap = std::max<int64_t>(4096, 4 * (n / 7)); nu == 0; lcap *= 4) {
     DG_CHECK(lcap < (int64_t(1) << 30), DG_ENOMEM, "balance: too many octants");
-    DG_TRY(table.alloc(2 * lcap));
+    const HashShape shape = hash_shape(lcap);
+    DG_TRY(table.alloc(int64_t(shape.slots())));
     DG_TRY(list.alloc(lcap));
-    DG_CUDA(cudaMemsetAsync(table.p, 0xff, sizeof(uint64_t) * size_t(2 * lcap), s));
+    DG_CUDA(cudaMemsetAsync(table.p, 0xff, sizeof(uint64_t) * size_t(shape.slots()), s));
     DG_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof h, s));
-    const InternalSet S{table.p, uint64_t(2 * lcap), list.p, uint32_t(lcap), cnt.p};
+    const InternalSet S{table.p, shape, list.p, uint32_t(lcap), cnt.p};
     balance_leaf_parents<<<grid_for(n, kSetThreads * kSetItems), kSetThreads, 0, s>>>(in->keys.p, n, D, S);
     for (uint32_t l = D; l-- > 1;) balance_level<<<grid_for(8 * lcap, kSetThreads * kSetItems), kSetThreads, 0, s>>>(l, D, S);
     DG_CUDA(cudaGetLastError());

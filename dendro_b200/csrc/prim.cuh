@@ -136,14 +136,46 @@ __device__ __forceinline__ int64_t gallop(const uint64_t* __restrict__ a, int64_
   return lo;
 }
 
-// Open-addressing hash of 64-bit keys (never all ones), linear probing.
+// Open-addressing hash of 64-bit keys (never all ones), linear probing, a
+// power of two of slots: the slot is the top bits of the key multiplied by odd
+// constants (2^64 over the golden ratio) twice, the halves folded between --
+// with one multiplication the regular keys of a cloud's octants run into long
+// probe sequences (building the map took twice as long), and a range reduction
+// by a 128-bit product made the kernels bound by integer arithmetic.
 constexpr uint64_t kNoKey = ~0ull;
 constexpr int kMaxProbes = 512;  // an insertion that probes further reports a full table
-__device__ __forceinline__ uint64_t hash_slot(uint64_t key, uint64_t cap) {
-  uint64_t h = key * 0x9e3779b97f4a7c15ull;
-  h ^= h >> 32;
-  h *= 0xd6e8feb86659fd93ull;
-  return __umul64hi(h, cap);
+struct HashShape {
+  uint32_t shift;  // 64 - log2(slots)
+  __host__ __device__ uint64_t slots() const { return 1ull << (64u - shift); }
+};
+inline HashShape hash_shape(int64_t entries) {  // at most half full
+  uint32_t b = 4;
+  while ((int64_t(1) << b) < 2 * entries) ++b;
+  return HashShape{64u - b};
+}
+__device__ __forceinline__ uint64_t hash_mix(uint64_t key) {
+  key *= 0x9e3779b97f4a7c15ull;
+  key ^= key >> 32;
+  return key * 0x9e3779b97f4a7c15ull;
+}
+// 31 bits of the mixed key below the slot's
+__device__ __forceinline__ uint32_t hash_tag(uint64_t mix, HashShape H) {
+  return uint32_t(mix >> (H.shift - 31u)) & 0x7fffffffu;
+}
+
+// Steps between cells in Morton order without taking coordinates apart: a
+// coordinate's bits sit at every third place, so adding with the other places
+// filled by ones carries from one of its bits to the next.  `unit` is the
+// coordinate's bit of the step; leaving the domain [0, 2^D) on a positive side
+// sets a bit at or above 3 D, so does leaving it on a negative one.
+__device__ __forceinline__ uint64_t axis_bits(int a) { return 0x1249249249249249ull << a; }
+__device__ __forceinline__ uint64_t morton_inc(uint64_t m, int a, uint64_t unit) {
+  const uint64_t A = axis_bits(a);
+  return (((m | ~A) + unit) & A) | (m & ~A);
+}
+__device__ __forceinline__ uint64_t morton_dec(uint64_t m, int a, uint64_t unit) {
+  const uint64_t A = axis_bits(a);
+  return (((m & A) - unit) & A) | (m & ~A);
 }
 
 // Copies nw device words to the host and waits for the stream (a page-locked
