@@ -431,7 +431,7 @@ dg_status dg_mat_create_elasticity(dg_da* da, double mu, double lambda, const ui
       st = node_boundary_flags(da, A->dirichlet.p, nullptr);
     }
   }
-  if (!st) st = ensure_octet_chunks(da, nullptr);
+  if (!st) st = ensure_octet_tiles(da, nullptr);
   if (st) { delete A; return st; }
   *out = A;
   return DG_OK;

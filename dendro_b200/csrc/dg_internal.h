@@ -19,9 +19,10 @@ struct TileSet {
   DBuf<uint32_t> nodes;      // [ptr[ntiles]]
   DBuf<uint16_t> nend;       // [ntiles * 8 te]: tile t, node k -> end of its run in inc
   DBuf<uint16_t> inc;        // [ntiles * 8 te]: tile t -> references ordered by node
-  DBuf<uint4> eloc;          // [E] per element the node positions of its 8 vertices (multi-RHS set only)
   // warp tiles (at most 256 nodes per tile), all in the child-number frame
   // (frame vertex j = vertex j ^ c of the element):
+  DBuf<uint4> eloc;          // [E] per element the node positions of its 8 vertices (multi-RHS set only)
+  // warp tiles
   DBuf<uint8_t> eloc8;       // [8 E] per element byte j = node rank of frame vertex j
   DBuf<uint32_t> wmeta;      // [E] level | frame hanging mask << 8
   DBuf<uint8_t> ref8;        // [ntiles * kWarpRefBytes] per tile: the references sorted by node as frame
@@ -52,12 +53,27 @@ struct OctetSet {
   DBuf<uint32_t> cel;     // [2 nchunk]: first element id, element range length
   DBuf<uint16_t> lidx;    // [27][n]
   DBuf<uint16_t> lelem;   // [8][n]
-  DBuf<uint16_t> lnl;     // [8][E]: per element, the chunk-local index of each vertex's node (the DA's nl)
   // [n + 1][kOctRec] per octet (and a padding octet without children): the
   // 27 lattice node ids, the mask of lattice points without a node, the meta
   // word, 3 words of padding -- one 128-byte record read by the lane-per-child
   // operator and the tensor-memory multi-RHS kernel
   DBuf<uint32_t> rec;
+};
+// Tiles of 32 consecutive octets, one per lane of a warp (octile.cu): their
+// lattices' distinct nodes, whose sums are merged before they leave.
+constexpr int kOctTile = 32;
+constexpr int kOctTileRefs = 27 * kOctTile;  // lattice positions: point * 32 + octet
+constexpr int kOctTileMaxRefs = 16;          // references to one node within a tile
+struct OctTiles {
+  bool tried = false;     // built, or found not to fit
+  int64_t ntiles = 0;
+  uint32_t max_nodes = 0;
+  DBuf<uint32_t> ptr;     // [ntiles] first entry of the tile's node list, a multiple of 4
+  DBuf<uint32_t> nodes;   // node ids by falling number of references; bit 31: in another tile's list too
+  DBuf<uint16_t> hdr;     // [ntiles][16]: nodes with at least 1, 2, ... references
+  DBuf<uint16_t> refs;    // [ntiles][kOctTileRefs]: the nodes' first references, the second ones, ...
+  DBuf<uint16_t> lidx;    // [27][n] rank of each octet's lattice nodes in the tile's list (0xffff: none)
+  DBuf<uint32_t> shared;  // the nodes that are not in exactly one tile's list, ascending
 };
 // Compressed element-to-node map (cmap.cuh), built on request.
 struct CompressedMap {
@@ -94,6 +110,7 @@ struct dg_da {
   // one's (kMultiTile elements per tile), both built on first use
   dg::TileSet tiles_w, tiles_mr;
   dg::OctetSet octs;  // elements grouped by parent (octet operator kernel)
+  dg::OctTiles otiles;  // tiles of octets (on first use)
   dg::CompressedMap cmap;  // compressed element map (on request)
   // operator launch shape picked by the autotuner on first use (-1: not yet)
   int tuned_f64 = -1, tuned_f32 = -1;
@@ -186,6 +203,7 @@ dg_status build_octets(dg_da* da, cudaStream_t s);  // da->octs from nl and meta
 dg_status ensure_tiles(dg_da* da, cudaStream_t s);
 dg_status ensure_octet_records(dg_da* da, cudaStream_t s);
 dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s);
+dg_status ensure_octet_tiles(dg_da* da, cudaStream_t s);  // da->otiles (octile.cu)
 // da->cmap with narrow quotients of qbits (1..16) bits (cmap.cu); nl_out
 // [8][E] receives the map decoded from it
 dg_status build_cmap(dg_da* da, int qbits, cudaStream_t s);
@@ -239,11 +257,11 @@ dg_status lapmass_residual_f32(const dg_mat* A, const float* x, const float* b, 
 const char* matvec_variant_name(int v);
 int matvec_variant_count();
 dg_status matvec_variant_tables(dg_da* da, int v, cudaStream_t s);
-// Y = A X for nrhs vectors (node-major [N][nrhs], FP32) on the tensor cores;
-// split 1: TF32 products, 3: high/low TF32 split (FP32-level accuracy).
+// Y = A X for nrhs vectors (node-major [N][nrhs], FP32): split 0, 1 and 3 the
+// octet form (exact FP32 products), 4 and 5 on tcgen05.
 dg_status mrhs_apply(const dg_mat* A, const float* X, float* Y, int nrhs, int split, cudaStream_t s);
 // Y = A X in the octet form (CUDA cores) in FP32 or FP64, node-major [N][R],
-// R a multiple of 32; coef = the operator's coefficients in that precision
+// R a multiple of 16; coef = the operator's coefficients in that precision
 // ([2][E], a then b; ignored when the operator has none).
 template <class T>
 dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int R, cudaStream_t s);

@@ -3070,7 +3070,10 @@ __device__ __forceinline__ void frame_scatter(double (&r)[8], uint32_t fm) {
     r[j] = t;
   }
 }
-// r = the element's 24 results in the frame from its 24 raw frame values.
+// r = the element's 24 results in the frame from its 24 raw frame values;
+// FOLD: with T^T applied (a hanging vertex's share goes to its corners), else
+// the caller folds.
+template <bool FOLD = true>
 __device__ __forceinline__ void elasticity_frame(double (&u0)[8], double (&u1)[8], double (&u2)[8], uint32_t fm,
                                                  uint32_t cn, double wl, double wg, double (&r0)[8],
                                                  double (&r1)[8], double (&r2)[8]) {
@@ -3090,6 +3093,8 @@ __device__ __forceinline__ void elasticity_frame(double (&u0)[8], double (&u1)[8
   wht8(u0);
   wht8(u1);
   wht8(u2);
+  wl *= 0.125;  // of the inverse transform
+  wg *= 0.125;
   const double s0 = (cn & 1u) ? -1.0 : 1.0, s1 = (cn & 2u) ? -1.0 : 1.0, s2 = (cn & 4u) ? -1.0 : 1.0;
   const double g01 = wg * s0 * s1, g02 = wg * s0 * s2, g12 = wg * s1 * s2;
 #pragma unroll
@@ -3107,14 +3112,14 @@ __device__ __forceinline__ void elasticity_frame(double (&u0)[8], double (&u1)[8
     if ((w & 2) && !(w & 4)) a1 += g12 * m0 * u2[w ^ 6];
     if ((w & 4) && !(w & 1)) a2 += g02 * m1 * u0[w ^ 5];
     if ((w & 4) && !(w & 2)) a2 += g12 * m0 * u1[w ^ 6];
-    r0[w] = a0 * 0.125;
-    r1[w] = a1 * 0.125;
-    r2[w] = a2 * 0.125;
+    r0[w] = a0;
+    r1[w] = a1;
+    r2[w] = a2;
   }
   wht8(r0);
   wht8(r1);
   wht8(r2);
-  if (fm) {
+  if (FOLD && fm) {
     frame_scatter(r0, fm);
     frame_scatter(r1, fm);
     frame_scatter(r2, fm);
@@ -3166,99 +3171,239 @@ __global__ void __launch_bounds__(128) elasticity_kernel(const uint32_t* __restr
   }
 }
 
-// Chunked form (the octet chunks of the mesh, OctetSet): a CTA per chunk
-// stages x at the chunk's nodes (3 components) and their Dirichlet flags in
-// shared memory with coalesced loads, applies every element of the chunk's
-// octets (one thread per element, the same element arithmetic as above) with
-// x read from shared memory and the 24 results added into a shared
-// accumulator, then writes the chunk's node sums with stores (nodes no other
-// chunk touches) or global reductions.  Dirichlet rows are set afterwards by
-// elasticity_dirichlet_rows, as for the kernel above.
-constexpr int kElasChunkThreads = 256;
-__global__ void __launch_bounds__(kElasChunkThreads, 2) elasticity_chunk_kernel(
-    int64_t n, int64_t nchunk, uint32_t node_cap, const uint32_t* __restrict__ oelem, const uint16_t* __restrict__ lnl,
-    const uint32_t* __restrict__ cptr, const uint32_t* __restrict__ cnodes, const uint32_t* __restrict__ meta,
-    const uint8_t* __restrict__ dir, int64_t E, double mu, double lam, const double* __restrict__ x,
-    double* __restrict__ y) {
-  extern __shared__ __align__(16) unsigned char el_smem[];
-  double* sx = reinterpret_cast<double*>(el_smem);
-  double* sy = sx + 3 * size_t(node_cap);
-  uint8_t* sd = reinterpret_cast<uint8_t*>(sy + 3 * size_t(node_cap));
-  for (int64_t q = blockIdx.x; q < nchunk; q += gridDim.x) {
-    const uint32_t p0 = __ldg(cptr + q), nn = __ldg(cptr + q + 1) - p0;
-    for (uint32_t k0 = threadIdx.x; k0 < nn; k0 += 4 * kElasChunkThreads) {
-      uint32_t id[4];
+// Octet-tile form: a CTA of 8 warps works a tile of 32 octets (OctTiles), warp
+// c the children c, one octet per lane.  Shared-memory FP64 atomics are
+// compare-and-swap loops (a form that added each element's 24 results with them
+// took 513 us on the 4.7M-element benchmark mesh and lost more on small ones;
+// this one takes 481 us), so no two threads add to one place:
+// x at the tile's nodes is staged once (zero at Dirichlet nodes); a thread
+// works its element in its child-number frame and writes the 24 results by
+// (frame vertex, child, octet); the frame vertex of a child at lattice point p
+// is the same for all children that touch p (bit a set where p's coordinate a
+// is 1), so a warp sums a lattice point over its children with the octets on
+// the lanes, free of bank conflicts; hanging points are folded onto the octet's
+// corners, corner 2c by the threads of child c, whose frame vertices 1 to 6 are
+// the points around it; then each node's references are summed and the node
+// leaves, stored, or added where another tile has it (those nodes are set by
+// elasticity_shared_rows first).  Dirichlet rows leave as x.  The next tile's x
+// is copied while this one's sums leave (552 us without).  What bounds it is
+// issue and shared memory at 16 warps per SM: 225 M warp instructions, 118
+// registers and 86 KB of shared memory per CTA.
+constexpr int kElasTileThreads = 256;
+__global__ void __launch_bounds__(kElasTileThreads, 2) elasticity_tile_kernel(
+    int64_t n, int64_t ntiles, uint32_t cap, const uint32_t* __restrict__ ometa, const uint32_t* __restrict__ tptr,
+    const uint32_t* __restrict__ nodes, const uint16_t* __restrict__ hdr, const uint16_t* __restrict__ refs,
+    const uint16_t* __restrict__ lidx, const uint8_t* __restrict__ dir, double mu, double lam,
+    const double* __restrict__ x, double* __restrict__ y) {
+  extern __shared__ __align__(16) unsigned char et_smem[];
+  double* rs = reinterpret_cast<double*>(et_smem);  // [3][8 frame vertices][8 children][32 octets]
+  double* sy = rs + 3 * 8 * 256;                    // [3][27][32]
+  double* sx = sy + 3 * kOctTileRefs;               // [cap][3]
+  uint16_t* sref = reinterpret_cast<uint16_t*>(sx + 3 * size_t(cap));
+  uint16_t* shdr = sref + kOctTileRefs;
+  uint32_t* sid = reinterpret_cast<uint32_t*>(shdr + kOctTileMaxRefs);  // [2][cap]
+  uint8_t* sd = reinterpret_cast<uint8_t*>(sid + 2 * size_t(cap));      // [2][cap]
+  const int tid = threadIdx.x, lane = tid & 31, c = tid >> 5;
+  const uint32_t cn = uint32_t(c);
+  // lattice point of frame vertex f: the child's corner q = 2 c, one step
+  // towards the centre on the axes of f
+  const int q = 2 * (c & 1) + 3 * (c & 2) + 9 * ((c & 4) / 2);
+  const int d0 = (c & 1) ? -1 : 1, d1 = (c & 2) ? -3 : 3, d2 = (c & 4) ? -9 : 9;
+  // children that touch the lattice points of frame vertices 1, 2, 4; of 3, 5, 6
+  const uint32_t t1 = (1u << c) | (1u << (c ^ 1)), t2 = (1u << c) | (1u << (c ^ 2)), t4 = (1u << c) | (1u << (c ^ 4));
+  const uint32_t t3 = t1 | t2 | (1u << (c ^ 3)), t5 = t1 | t4 | (1u << (c ^ 5)), t6 = t2 | t4 | (1u << (c ^ 6));
+  // x and the Dirichlet flags of a tile's nodes, ids in sid[buf]; x's copies
+  // are asynchronous, one group
+  auto fetch_x = [&](uint32_t count, int buf) {
+    for (uint32_t i = tid; i < count; i += kElasTileThreads) {
+      const uint32_t id = sid[buf * cap + i] & 0x7fffffffu;
+      const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(sx + 3 * i));
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t k = k0 + u * kElasChunkThreads;
-        id[u] = k < nn ? (__ldg(cnodes + p0 + k) & 0x7fffffffu) : 0u;
-      }
-      double v[4][3];
-      uint8_t dv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const bool in = k0 + u * kElasChunkThreads < nn;
-        dv[u] = in ? __ldg(dir + id[u]) : uint8_t(0);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) v[u][a] = in ? __ldg(x + 3 * int64_t(id[u]) + a) : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t k = k0 + u * kElasChunkThreads;
-        if (k >= nn) continue;
-        sd[k] = dv[u];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          sx[3 * k + a] = v[u][a];
-          sy[3 * k + a] = 0.0;
-        }
-      }
+      for (int a = 0; a < 3; ++a)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(at + 8 * a), "l"(x + 3 * int64_t(id) + a)
+                     : "memory");
+      sd[buf * cap + i] = __ldg(dir + id);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 8 * kOctChunk; i += kElasChunkThreads) {
-      const int c = i / kOctChunk;
-      const int64_t o = q * kOctChunk + (i - c * kOctChunk);
-      if (o >= n) continue;
-      const uint32_t e = __ldg(oelem + int64_t(c) * n + o);
-      if (e == kNoNode) continue;
-      const uint32_t m = __ldg(meta + e);
-      const uint32_t lev = meta_lev(m), cn = meta_cnum(m);
-      const uint32_t fm = frame_mask(meta_mask(m), cn);
-      const double fac = elem_h<double>(lev) / 2.0;
-      // frame vertex v is vertex v ^ cn: its node's chunk-local index
-      uint32_t li[8];
-      bool bd[8];
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // ranks of the frame vertices' nodes, and the octet's word
+  uint32_t li[8], m = 0;
+  auto fetch_ranks = [&](int64_t tt) {
+    const int64_t o = tt * kOctTile + lane;
+    const bool in = o < n;
+    m = in ? __ldg(ometa + o) : 0u;
+    const uint16_t* lo = lidx + (in ? o : 0);
+#pragma unroll
+    for (int f = 0; f < 8; ++f)
+      li[f] = __ldg(lo + int64_t(q + ((f & 1) ? d0 : 0) + ((f & 2) ? d1 : 0) + ((f & 4) ? d2 : 0)) * n);
+  };
+  int64_t t = blockIdx.x;
+  if (t >= ntiles) return;
+  uint32_t p0 = __ldg(tptr + t), c1 = __ldg(hdr + t * kOctTileMaxRefs);
+  for (uint32_t i = tid; i < c1; i += kElasTileThreads) sid[i] = __ldg(nodes + p0 + i);
+  fetch_ranks(t);
+  __syncthreads();
+  fetch_x(c1, 0);
+  for (int buf = 0; t < ntiles; buf ^= 1) {
+    const int64_t tn = t + gridDim.x;
+    const bool more = tn < ntiles;
+    uint32_t pn = 0, cnx = 0;
+    if (more) {
+      pn = __ldg(tptr + tn);
+      cnx = __ldg(hdr + tn * kOctTileMaxRefs);
+    }
+    // frame vertices that hang: without a node, and touched by a present child
+    const uint32_t cm = ometa_cmask(m);
+    const uint32_t touch[8] = {0, t1, t2, t3, t4, t5, t6, 0};
+    uint32_t hang = 0;
+#pragma unroll
+    for (int f = 1; f < 7; ++f) hang |= (li[f] == 0xffffu && (cm & touch[f])) ? (1u << f) : 0u;
+    const bool mine = (cm >> c) & 1u;
+    if (mine && hang) {  // a hanging vertex lists the octet corner 2 v, v = f ^ c
+      const uint16_t* lo = lidx + t * kOctTile + lane;
+#pragma unroll
+      for (int f = 1; f < 7; ++f)
+        if ((hang >> f) & 1u) {
+          const int p = q + ((f & 1) ? 2 * d0 : 0) + ((f & 2) ? 2 * d1 : 0) + ((f & 4) ? 2 * d2 : 0);
+          li[f] = __ldg(lo + int64_t(p) * n);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    for (uint32_t i = tid; i < c1; i += kElasTileThreads)  // columns of Dirichlet nodes are dropped
+      if (sd[buf * cap + i]) sx[3 * i] = sx[3 * i + 1] = sx[3 * i + 2] = 0.0;
+    __syncthreads();  // x of this tile is there; the last one is done with the lists below
+    for (int i = tid; i < kOctTileRefs / 8; i += kElasTileThreads)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       static_cast<uint32_t>(__cvta_generic_to_shared(sref + 8 * i))),
+                   "l"(refs + t * kOctTileRefs + 8 * i)
+                   : "memory");
+    if (tid < kOctTileMaxRefs / 8)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       static_cast<uint32_t>(__cvta_generic_to_shared(shdr + 8 * tid))),
+                   "l"(hdr + t * kOctTileMaxRefs + 8 * tid)
+                   : "memory");
+    for (uint32_t i = 4 * tid; i < cnx; i += 4 * kElasTileThreads)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       static_cast<uint32_t>(__cvta_generic_to_shared(sid + (buf ^ 1) * cap + i))),
+                   "l"(nodes + pn + i)
+                   : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    double r0[8], r1[8], r2[8];
+    if (mine) {
       double u0[8], u1[8], u2[8];
 #pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        li[v] = __ldg(lnl + int64_t(uint32_t(v) ^ cn) * E + e);
-        bd[v] = sd[li[v]] != 0;
-        u0[v] = bd[v] ? 0.0 : sx[3 * li[v]];
-        u1[v] = bd[v] ? 0.0 : sx[3 * li[v] + 1];
-        u2[v] = bd[v] ? 0.0 : sx[3 * li[v] + 2];
+      for (int f = 0; f < 8; ++f) {
+        const double* s = sx + 3 * li[f];
+        u0[f] = s[0];
+        u1[f] = s[1];
+        u2[f] = s[2];
       }
-      double r0[8], r1[8], r2[8];
-      elasticity_frame(u0, u1, u2, fm, cn, mu * fac, (mu + lam) * fac, r0, r1, r2);
+      const double fac = elem_h<double>(ometa_lev(m)) / 2.0;
+      elasticity_frame<false>(u0, u1, u2, hang, cn, mu * fac, (mu + lam) * fac, r0, r1, r2);
+    } else {
 #pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        if (bd[v]) continue;
-        double* t = sy + 3 * li[v];
-        if (r0[v] != 0.0) atomicAdd(t, r0[v]);
-        if (r1[v] != 0.0) atomicAdd(t + 1, r1[v]);
-        if (r2[v] != 0.0) atomicAdd(t + 2, r2[v]);
-      }
+      for (int f = 0; f < 8; ++f) r0[f] = r1[f] = r2[f] = 0.0;
     }
+#pragma unroll
+    for (int f = 0; f < 8; ++f) {
+      rs[f * 256 + tid] = r0[f];
+      rs[(8 + f) * 256 + tid] = r1[f];
+      rs[(16 + f) * 256 + tid] = r2[f];
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < nn; k += kElasChunkThreads) {
-      const uint32_t id = __ldg(cnodes + p0 + k);
-      double* dst = y + 3 * int64_t(id & 0x7fffffffu);
+    // x has been read: the next tile's comes in while this one's sums leave
+    fetch_x(cnx, buf ^ 1);
+    // lattice sums: warp c takes the points c, c + 8, c + 16 and c + 24
+    for (int p = c; p < 27; p += 8) {
+      const int px = p % 3, py = (p / 3) % 3, pz = p / 9;
+      const int f = (px == 1) | (py == 1) << 1 | (pz == 1) << 2;
+      const int base = (px == 2) | (py == 2) << 1 | (pz == 2) << 2;
+      const double* r = rs + f * 256 + base * 32 + lane;
+      double* s = sy + p * 32 + lane;
+      // the children towards each free axis are 1, 2 or 4 rows of 32 further on
+      const int e0 = (f & 1) ? 32 : (f & 2) ? 64 : 128, e1 = (f & 1) && (f & 2) ? 64 : 128;
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        st_if(dst + a, sy[3 * k + a], !(id >> 31));
-        red_add_if(dst + a, sy[3 * k + a], (id >> 31) && sy[3 * k + a] != 0.0);
+        const double* ra = r + a * 2048;
+        double v = ra[0];
+        if (f) {
+          v += ra[e0];
+          if (f & (f - 1)) {
+            v += ra[e1] + ra[e0 + e1];
+            if (f == 7) v += (ra[128] + ra[160]) + (ra[192] + ra[224]);
+          }
+        }
+        s[a * kOctTileRefs] = v;
       }
     }
     __syncthreads();
+    if (hang) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        double* s = sy + a * kOctTileRefs + q * 32 + lane;
+        double edge = 0.0, face = 0.0;
+        if (hang & 2u) edge += s[d0 * 32];
+        if (hang & 4u) edge += s[d1 * 32];
+        if (hang & 16u) edge += s[d2 * 32];
+        if (hang & 8u) face += s[(d0 + d1) * 32];
+        if (hang & 32u) face += s[(d0 + d2) * 32];
+        if (hang & 64u) face += s[(d1 + d2) * 32];
+        s[0] += 0.5 * edge + 0.25 * face;
+      }
+    }
+    __syncthreads();
+    if (more) fetch_ranks(tn);
+    for (uint32_t k = tid; k < c1; k += kElasTileThreads) {
+      const uint32_t id = sid[buf * cap + k];
+      const bool d = sd[buf * cap + k] != 0;
+      const uint16_t* rk = sref + k;
+      double s0 = sy[rk[0]], s1 = sy[kOctTileRefs + rk[0]], s2 = sy[2 * kOctTileRefs + rk[0]];
+      uint32_t cj = c1;
+      for (int j = 1; j < kOctTileMaxRefs; ++j) {
+        rk += cj;
+        cj = shdr[j];
+        if (k >= cj) break;
+        const double* s = sy + rk[0];
+        s0 += s[0];
+        s1 += s[kOctTileRefs];
+        s2 += s[2 * kOctTileRefs];
+      }
+      const int64_t at = 3 * int64_t(id & 0x7fffffffu);
+      if (!(id >> 31)) {
+        if (d) {
+          s0 = __ldg(x + at);
+          s1 = __ldg(x + at + 1);
+          s2 = __ldg(x + at + 2);
+        }
+        y[at] = s0;
+        y[at + 1] = s1;
+        y[at + 2] = s2;
+      } else if (!d) {
+        red_add_if(y + at, s0, s0 != 0.0);
+        red_add_if(y + at + 1, s1, s1 != 0.0);
+        red_add_if(y + at + 2, s2, s2 != 0.0);
+      }
+    }
+    t = tn;
+    p0 = pn;
+    c1 = cnx;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+constexpr size_t elasticity_tile_smem(uint32_t cap) {
+  return sizeof(double) * (3 * 8 * 256 + 3 * kOctTileRefs + 3 * size_t(cap)) +
+         sizeof(uint16_t) * (kOctTileRefs + kOctTileMaxRefs) + (2 * sizeof(uint32_t) + 2) * size_t(cap);
+}
+// Rows of the nodes that are not in exactly one tile, before the sums are
+// added: x at Dirichlet nodes, else zero.
+__global__ void elasticity_shared_rows(const uint32_t* __restrict__ shared, int64_t ns,
+                                       const uint8_t* __restrict__ dir, const double* __restrict__ x,
+                                       double* __restrict__ y) {
+  for (int64_t i = gtid(); i < 3 * ns; i += gstride()) {
+    const int64_t k = i / 3;
+    const int64_t id = shared[k], at = 3 * id + (i - 3 * k);
+    y[at] = dir[id] ? x[at] : 0.0;
   }
 }
 
@@ -3432,7 +3577,7 @@ __global__ void set_dirichlet_diag1(const uint8_t* __restrict__ dir, int64_t N, 
 }  // namespace
 
 // DG_ELASTICITY_KERNEL=element keeps the one-thread-per-element kernel (testing).
-static bool elasticity_chunks_off() {
+static bool elasticity_tiles_off() {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("DG_ELASTICITY_KERNEL");
@@ -3443,20 +3588,24 @@ static bool elasticity_chunks_off() {
 
 dg_status elasticity_apply_f64(const dg_mat* A, const double* x, double* y, cudaStream_t s) {
   const dg_da* da = A->da;
-  DG_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * 3 * da->N, s));
   const OctetSet& O = da->octs;
-  if (O.nchunk > 0 && O.lnl.p && !elasticity_chunks_off()) {
-    const size_t smem = 6 * sizeof(double) * O.max_nodes + O.max_nodes;
-    DG_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(elasticity_chunk_kernel),
-                              (6 * sizeof(double) + 1) * 27 * kOctChunk));
-    const unsigned g = unsigned(std::min<int64_t>(O.nchunk, int64_t(sm_count()) * 4));
-    elasticity_chunk_kernel<<<g, kElasChunkThreads, smem, s>>>(O.n, O.nchunk, O.max_nodes, O.elem.p, O.lnl.p,
-                                                               O.cptr.p, O.cnodes.p, da->meta.p, A->dirichlet.p,
-                                                               da->E, A->mu, A->lam, x, y);
-  } else {
-    elasticity_kernel<<<grid_for(da->E, 128, 16), 128, 0, s>>>(da->nl.p, da->meta.p, A->dirichlet.p, da->E, A->mu,
-                                                                 A->lam, x, y);
+  const OctTiles& Q = da->otiles;
+  if (Q.ntiles > 0 && !elasticity_tiles_off()) {
+    const uint32_t cap = (Q.max_nodes + 7u) & ~7u;
+    DG_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(elasticity_tile_kernel),
+                              elasticity_tile_smem(kOctTileRefs)));
+    if (Q.shared.n)
+      elasticity_shared_rows<<<grid_for(3 * Q.shared.n, 256), 256, 0, s>>>(Q.shared.p, Q.shared.n, A->dirichlet.p, x, y);
+    const unsigned g = unsigned(std::min<int64_t>(Q.ntiles, int64_t(sm_count()) * 2));
+    elasticity_tile_kernel<<<g, kElasTileThreads, elasticity_tile_smem(cap), s>>>(
+        O.n, Q.ntiles, cap, O.meta.p, Q.ptr.p, Q.nodes.p, Q.hdr.p, Q.refs.p, Q.lidx.p, A->dirichlet.p, A->mu, A->lam,
+        x, y);
+    DG_CUDA(cudaGetLastError());
+    return DG_OK;
   }
+  DG_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * 3 * da->N, s));
+  elasticity_kernel<<<grid_for(da->E, 128, 16), 128, 0, s>>>(da->nl.p, da->meta.p, A->dirichlet.p, da->E, A->mu,
+                                                              A->lam, x, y);
   elasticity_dirichlet_rows<<<grid_for(da->N, 256), 256, 0, s>>>(A->dirichlet.p, da->N, x, y);
   DG_CUDA(cudaGetLastError());
   return DG_OK;
