@@ -260,12 +260,11 @@ class _Mat:
 
     def mult_multi(self, X, Y=None, split: int = 3, stream=None):
         """Y = A X for the columns of X, a CUDA float32 tensor [N, nrhs]
-        (nrhs a multiple of 16), on the tensor cores (split 3: FP32-level
-        accuracy from three TF32 products; 1: one TF32 product; 5 and 4: the
-        same two precisions with tcgen05 and tensor-memory accumulators on
-        pairs of element parents, nrhs a multiple of 64), or with split 0 in
-        the octet form on the CUDA cores (exact FP32 products; nrhs a multiple
-        of 32)."""
+        (nrhs a multiple of 16), in exact FP32 products on the CUDA cores
+        (split 3, 1 or 0; 0 takes nrhs a multiple of 32), or on the tensor
+        cores with tcgen05 and tensor-memory accumulators on pairs of element
+        parents (nrhs a multiple of 64): split 5 in three TF32 products
+        (FP32-level accuracy), 4 in one."""
         import torch
         if not (X.is_cuda and X.dtype == torch.float32 and X.dim() == 2 and X.is_contiguous()):
             raise TypeError("X must be a contiguous CUDA float32 tensor [N, nrhs]")

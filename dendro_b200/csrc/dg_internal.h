@@ -21,8 +21,6 @@ struct TileSet {
   DBuf<uint16_t> inc;        // [ntiles * 8 te]: tile t -> references ordered by node
   // warp tiles (at most 256 nodes per tile), all in the child-number frame
   // (frame vertex j = vertex j ^ c of the element):
-  DBuf<uint4> eloc;          // [E] per element the node positions of its 8 vertices (multi-RHS set only)
-  // warp tiles
   DBuf<uint8_t> eloc8;       // [8 E] per element byte j = node rank of frame vertex j
   DBuf<uint32_t> wmeta;      // [E] level | frame hanging mask << 8
   DBuf<uint8_t> ref8;        // [ntiles * kWarpRefBytes] per tile: the references sorted by node as frame
@@ -105,10 +103,8 @@ struct dg_da {
   dg::DBuf<uint32_t> meta;   // [E] packed level / child number / hanging mask / type
   dg::DBuf<uint64_t> ekey;   // [E] element octant keys (embedded space)
   dg::DBuf<uint64_t> nkey;   // [N] node anchor Morton keys (embedded space), sorted
-  // element tiles of the shared-memory operator kernels: the scalar warp-tile
-  // operator's (kWarpTile elements per tile) and the multi-right-hand-side
-  // one's (kMultiTile elements per tile), both built on first use
-  dg::TileSet tiles_w, tiles_mr;
+  // element tiles of the warp-tile operator kernels (built on first use)
+  dg::TileSet tiles_w;
   dg::OctetSet octs;  // elements grouped by parent (octet operator kernel)
   dg::OctTiles otiles;  // tiles of octets (on first use)
   dg::CompressedMap cmap;  // compressed element map (on request)
@@ -141,9 +137,7 @@ struct dg_mat {
 
 namespace dg {
 
-// elements per tile of the multi-right-hand-side kernel and of the scalar
-// warp-tile kernel (one lane each)
-constexpr int kMultiTile = 128;
+// elements per tile of the warp-tile kernels (one lane each)
 constexpr int kWarpTile = 32;
 constexpr int kWarpRefBytes = 16 * kWarpTile + 4 * 32;  // per warp tile in TileSet::ref8
 // Slack after per-element arrays that the bulk-copy operator kernel reads in

@@ -533,7 +533,7 @@ template <int TE>
 __global__ void __launch_bounds__(TE) tile_lists(const uint32_t* __restrict__ nl, int64_t E, int64_t ntiles,
                                                  uint32_t* __restrict__ tmp, uint32_t* __restrict__ cnt,
                                                  uint16_t* __restrict__ nend, uint16_t* __restrict__ inc,
-                                                 uint4* __restrict__ eloc, uint8_t* __restrict__ eloc8) {
+                                                 uint8_t* __restrict__ eloc8) {
   constexpr int S = 8 * TE;
   constexpr int kPer = 8;  // sorted entries per thread
   static_assert(S <= 4096, "positions are 12-bit");
@@ -590,19 +590,7 @@ __global__ void __launch_bounds__(TE) tile_lists(const uint32_t* __restrict__ nl
     }
     if (tid == 0) cnt[t] = total;
     __syncthreads();
-    if (eloc) {  // per element the node ranks of its eight vertices
-      const int64_t e = t * TE + tid;
-      if (e < E) {
-        uint4 o;
-        o.x = uint32_t(slot[0 * TE + tid]) | (uint32_t(slot[1 * TE + tid]) << 16);
-        o.y = uint32_t(slot[2 * TE + tid]) | (uint32_t(slot[3 * TE + tid]) << 16);
-        o.z = uint32_t(slot[4 * TE + tid]) | (uint32_t(slot[5 * TE + tid]) << 16);
-        o.w = uint32_t(slot[6 * TE + tid]) | (uint32_t(slot[7 * TE + tid]) << 16);
-        eloc[e] = o;
-      }
-      __syncthreads();
-    }
-    if (eloc8) {  // the same as bytes (tiles of at most 256 nodes)
+    {  // per element the node ranks of its eight vertices (at most 256 nodes)
       const int64_t e = t * TE + tid;
       if (e < E) {
         uint2 o;
@@ -857,34 +845,29 @@ dg_status build_mesh(const dg_octree* tree, dg_da* da, cudaStream_t s) {
 
 template <int TE>
 static dg_status launch_tile_lists(const dg_da* da, int64_t nt, uint32_t* tmp, uint32_t* cnt, uint16_t* nend,
-                                   uint16_t* inc, uint4* eloc, uint8_t* eloc8, cudaStream_t s) {
+                                   uint16_t* inc, uint8_t* eloc8, cudaStream_t s) {
   const size_t smem = size_t(8 + 2) * 8 * TE;
   static bool set = false;
   if (!set && smem > 48 * 1024) {
     DG_CUDA(cudaFuncSetAttribute(tile_lists<TE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   }
   set = true;
-  tile_lists<TE><<<grid_for(nt, TE, 2048 / TE), TE, smem, s>>>(da->nl.p, da->E, nt, tmp, cnt, nend, inc, eloc, eloc8);
+  tile_lists<TE><<<grid_for(nt, TE, 2048 / TE), TE, smem, s>>>(da->nl.p, da->E, nt, tmp, cnt, nend, inc, eloc8);
   DG_CUDA(cudaGetLastError());
   return DG_OK;
 }
 
 dg_status build_tile_set(const dg_da* da, int te, TileSet& ts, cudaStream_t s) {
   DG_CHECK(da->N < (int64_t(1) << 31), DG_EINVAL, "mesh above 2^31 nodes");
-  DG_CHECK(te == kMultiTile || te == kWarpTile, DG_EINVAL, "unsupported tile size");
+  DG_CHECK(te == kWarpTile, DG_EINVAL, "unsupported tile size");
   const int64_t E = da->E, nt = (E + te - 1) / te, S = 8 * int64_t(te);
   DBuf<uint32_t> tmp, cnt, touch;
   DG_TRY(tmp.alloc(nt * S));
   DG_TRY(cnt.alloc(nt));
   DG_TRY(ts.nend.alloc(nt * S));
   DG_TRY(ts.inc.alloc(nt * S));
-  if (te == kWarpTile) {
-    DG_TRY(ts.eloc8.alloc(8 * nt * kWarpTile));  // whole tiles
-    DG_TRY(launch_tile_lists<kWarpTile>(da, nt, tmp.p, cnt.p, ts.nend.p, ts.inc.p, nullptr, ts.eloc8.p, s));
-  } else {
-    DG_TRY(ts.eloc.alloc(E));
-    DG_TRY(launch_tile_lists<kMultiTile>(da, nt, tmp.p, cnt.p, ts.nend.p, ts.inc.p, ts.eloc.p, nullptr, s));
-  }
+  DG_TRY(ts.eloc8.alloc(8 * nt * kWarpTile));  // whole tiles
+  DG_TRY(launch_tile_lists<kWarpTile>(da, nt, tmp.p, cnt.p, ts.nend.p, ts.inc.p, ts.eloc8.p, s));
   std::vector<uint32_t> hc(nt);
   DG_CUDA(cudaMemcpyAsync(hc.data(), cnt.p, 4 * nt, cudaMemcpyDeviceToHost, s));
   uint32_t total = 0;

@@ -26,6 +26,8 @@
 // octet's own children are done in registers, not in memory.
 #pragma once
 
+#include <type_traits>
+
 #include "dg_internal.h"
 #include "element.cuh"
 
@@ -55,6 +57,110 @@ __host__ __device__ constexpr int oct_s1(int p) {
 // Per-octet word: level of the children (embedded) | child mask << 8.
 __host__ __device__ __forceinline__ uint32_t ometa_lev(uint32_t m) { return m & 31u; }
 __host__ __device__ __forceinline__ uint32_t ometa_cmask(uint32_t m) { return (m >> 8) & 255u; }
+
+// yv = the sum of the present children's element operators on the lattice
+// values xv (a child's factors g1, g2 scaled by coef).
+//
+// FP32 (and pairs of FP32): the children's Walsh transforms (element.cuh) are
+// done for the octet as a whole, an axis at a time: along an axis the 3 lattice
+// values of a line give both children's sums and differences (4 additions), so
+// lines that several children share are transformed once, and on the way back
+// the children's sums at the shared points come out of the transform (5
+// additions per line): 397 operations per octet against 512 child by child.
+// FP64: child by child, because 128 registers hold the 27 + 27 doubles but not
+// the transform's lines as well (one-thread-per-octet kernel on the 4.7M-element
+// benchmark mesh with the next ids in flight, this form / the other: FP64 101 /
+// 110 us, FP32 84 / 80 us; 64 right-hand sides in FP32 pairs 1240 / 1165 us).
+template <class T, bool FULL, class Coef>
+__device__ __forceinline__ void octet_children(const T (&xv)[27], T (&yv)[27], uint32_t cm, T g1, T g2, Coef coef) {
+  if constexpr (std::is_same<T, double>::value) {
+#pragma unroll
+    for (int p = 0; p < 27; ++p) yv[p] = T(0);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      if (FULL || ((cm >> c) & 1u)) {
+        T f1 = g1, f2 = g2;
+        coef(c, f1, f2);
+        T u[8];
+#pragma unroll
+        for (int v = 0; v < 8; ++v) u[v] = xv[oct_lat(c, v)];
+        lapmass_ref(u, f1, f2);
+#pragma unroll
+        for (int v = 0; v < 8; ++v) yv[oct_lat(c, v)] += u[v];
+      }
+    }
+    return;
+  }
+  T w[4][9];  // [x coefficient of child bit cx: 2 cx sum, 2 cx + 1 difference][y + 3 z]
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const T p = xv[3 * r], q = xv[3 * r + 1], t = xv[3 * r + 2];
+    w[0][r] = p + q;
+    w[1][r] = p - q;
+    w[2][r] = q + t;
+    w[3][r] = q - t;
+  }
+#pragma unroll
+  for (int cx = 0; cx < 2; ++cx) {
+    T v[2][4][3];  // [x difference][y coefficient][z]
+#pragma unroll
+    for (int ex = 0; ex < 2; ++ex)
+#pragma unroll
+      for (int z = 0; z < 3; ++z) {
+        const T p = w[2 * cx + ex][3 * z], q = w[2 * cx + ex][3 * z + 1], t = w[2 * cx + ex][3 * z + 2];
+        v[ex][0][z] = p + q;
+        v[ex][1][z] = p - q;
+        v[ex][2][z] = q + t;
+        v[ex][3][z] = q - t;
+      }
+#pragma unroll
+    for (int cy = 0; cy < 2; ++cy) {
+      T l[2][4];  // eigenvalues of the two children by the number of differences
+      bool on[2];
+#pragma unroll
+      for (int cz = 0; cz < 2; ++cz) {
+        const int c = cx + 2 * cy + 4 * cz;
+        on[cz] = FULL || ((cm >> c) & 1u);
+        T f1 = g1, f2 = g2;
+        if (on[cz]) coef(c, f1, f2);
+        l[cz][0] = f2 * T(0.125);
+        l[cz][1] = (f2 * T(1.0 / 3.0) + f1) * T(0.125);
+        l[cz][2] = (f2 * T(1.0 / 9.0) + f1 * T(2.0 / 3.0)) * T(0.125);
+        l[cz][3] = (f2 * T(1.0 / 27.0) + f1 * T(1.0 / 3.0)) * T(0.125);
+      }
+#pragma unroll
+      for (int ex = 0; ex < 2; ++ex)
+#pragma unroll
+        for (int ey = 0; ey < 2; ++ey) {
+          T(&g)[3] = v[ex][2 * cy + ey];
+          const int k = ex + ey;
+          T s0 = g[0] + g[1], d0 = g[0] - g[1], s1 = g[1] + g[2], d1 = g[1] - g[2];
+          // an absent child contributes nothing, whatever its vertices hold
+          s0 = on[0] ? s0 * l[0][k] : T(0);
+          d0 = on[0] ? d0 * l[0][k + 1] : T(0);
+          s1 = on[1] ? s1 * l[1][k] : T(0);
+          d1 = on[1] ? d1 * l[1][k + 1] : T(0);
+          g[0] = s0 + d0;
+          g[1] = (s0 - d0) + (s1 + d1);
+          g[2] = s1 - d1;
+        }
+    }
+#pragma unroll
+    for (int ex = 0; ex < 2; ++ex)
+#pragma unroll
+      for (int z = 0; z < 3; ++z) {
+        w[2 * cx + ex][3 * z] = v[ex][0][z] + v[ex][1][z];
+        w[2 * cx + ex][3 * z + 1] = (v[ex][0][z] - v[ex][1][z]) + (v[ex][2][z] + v[ex][3][z]);
+        w[2 * cx + ex][3 * z + 2] = v[ex][2][z] - v[ex][3][z];
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    yv[3 * r] = w[0][r] + w[1][r];
+    yv[3 * r + 1] = (w[0][r] - w[1][r]) + (w[2][r] + w[3][r]);
+    yv[3 * r + 2] = w[2][r] - w[3][r];
+  }
+}
 
 // The arithmetic of one octet on its 27 lattice values xv: the
 // points flagged in `none` (no node: hanging, or not a vertex of a present
@@ -91,24 +197,10 @@ __device__ __forceinline__ void octet_apply(T (&xv)[27], T (&yv)[27], uint32_t n
       }
     }
   }
-#pragma unroll
-  for (int p = 0; p < 27; ++p) yv[p] = T(0);
   const uint32_t cm = FULL ? 255u : ometa_cmask(m);
   const T h = elem_h<T>(ometa_lev(m));
   const T g1 = h * T(0.5), g2 = h * h * h * T(0.125);
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    if (FULL || ((cm >> c) & 1u)) {
-      T f1 = g1, f2 = g2;
-      coef(c, f1, f2);
-      T u[8];
-#pragma unroll
-      for (int v = 0; v < 8; ++v) u[v] = xv[oct_lat(c, v)];
-      lapmass_ref(u, f1, f2);
-#pragma unroll
-      for (int v = 0; v < 8; ++v) yv[oct_lat(c, v)] += u[v];
-    }
-  }
+  octet_children<T, FULL>(xv, yv, cm, g1, g2, coef);
   if (fill) {
 #pragma unroll
     for (int p = 0; p < 27; ++p) {

@@ -247,16 +247,14 @@ int dg_mat_kernel_count(void);
 /* Y = A X for nrhs right-hand sides at once (no reference counterpart: the
  * reference's Jacobian2MatMult, omgNeumann.C:533, takes one Vec).  X and Y are
  * device arrays, node-major [N][nrhs] FP32, 16-byte aligned; nrhs a multiple
- * of 16.  The element contraction runs on the tensor cores with TF32 inputs
- * and FP32 accumulation; split = 3 splits each input into a TF32 high part and
- * a TF32 remainder (three products, FP32-level accuracy), split = 1 uses one
- * TF32 product (both with mma.sync on the warp tiles); split = 5 and split = 4
- * are the same two precisions on the 5th-generation tensor cores (tcgen05.mma
- * with accumulators in tensor memory: per pair of element parents their
- * assembled 27 x 27 lattice matrix times the lattice rows of X; nrhs a
- * multiple of 64); split = 0 runs the octet form on the CUDA cores instead (a
- * warp per element parent and 32 right-hand sides, exact FP32 products;
- * nrhs a multiple of 32).  Scalar Laplacian + mass operators only. */
+ * of 16.  split = 0, 1 and 3 run the octet form on the CUDA cores (a group of
+ * lanes per element parent, one or two right-hand sides per lane, exact FP32
+ * products; split 0 takes nrhs a multiple of 32); split = 5 and split = 4 run the
+ * contraction on the 5th-generation tensor cores in three TF32 products of high
+ * and low parts (FP32-level accuracy) or one TF32 product (tcgen05.mma with
+ * accumulators in tensor memory: per pair of element parents their assembled
+ * 27 x 27 lattice matrix times the lattice rows of X; nrhs a multiple of 64).
+ * Scalar Laplacian + mass operators only. */
 dg_status dg_mat_mult_multi(dg_mat* A, const float* X, float* Y, int nrhs, int split, void* stream);
 dg_status dg_mat_set_kernel(dg_mat* A, int prec, int variant);
 void dg_mat_destroy(dg_mat* A);
