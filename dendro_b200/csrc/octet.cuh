@@ -89,76 +89,76 @@ __device__ __forceinline__ void octet_children(const T (&xv)[27], T (&yv)[27], u
         for (int v = 0; v < 8; ++v) yv[oct_lat(c, v)] += u[v];
       }
     }
-    return;
-  }
-  T w[4][9];  // [x coefficient of child bit cx: 2 cx sum, 2 cx + 1 difference][y + 3 z]
+  } else {
+    T w[4][9];  // [x coefficient of child bit cx: 2 cx sum, 2 cx + 1 difference][y + 3 z]
 #pragma unroll
-  for (int r = 0; r < 9; ++r) {
-    const T p = xv[3 * r], q = xv[3 * r + 1], t = xv[3 * r + 2];
-    w[0][r] = p + q;
-    w[1][r] = p - q;
-    w[2][r] = q + t;
-    w[3][r] = q - t;
-  }
+    for (int r = 0; r < 9; ++r) {
+      const T p = xv[3 * r], q = xv[3 * r + 1], t = xv[3 * r + 2];
+      w[0][r] = p + q;
+      w[1][r] = p - q;
+      w[2][r] = q + t;
+      w[3][r] = q - t;
+    }
 #pragma unroll
-  for (int cx = 0; cx < 2; ++cx) {
-    T v[2][4][3];  // [x difference][y coefficient][z]
+    for (int cx = 0; cx < 2; ++cx) {
+      T v[2][4][3];  // [x difference][y coefficient][z]
 #pragma unroll
-    for (int ex = 0; ex < 2; ++ex)
+      for (int ex = 0; ex < 2; ++ex)
 #pragma unroll
-      for (int z = 0; z < 3; ++z) {
-        const T p = w[2 * cx + ex][3 * z], q = w[2 * cx + ex][3 * z + 1], t = w[2 * cx + ex][3 * z + 2];
-        v[ex][0][z] = p + q;
-        v[ex][1][z] = p - q;
-        v[ex][2][z] = q + t;
-        v[ex][3][z] = q - t;
-      }
+        for (int z = 0; z < 3; ++z) {
+          const T p = w[2 * cx + ex][3 * z], q = w[2 * cx + ex][3 * z + 1], t = w[2 * cx + ex][3 * z + 2];
+          v[ex][0][z] = p + q;
+          v[ex][1][z] = p - q;
+          v[ex][2][z] = q + t;
+          v[ex][3][z] = q - t;
+        }
 #pragma unroll
-    for (int cy = 0; cy < 2; ++cy) {
-      T l[2][4];  // eigenvalues of the two children by the number of differences
-      bool on[2];
+      for (int cy = 0; cy < 2; ++cy) {
+        T l[2][4];  // eigenvalues of the two children by the number of differences
+        bool on[2];
 #pragma unroll
-      for (int cz = 0; cz < 2; ++cz) {
-        const int c = cx + 2 * cy + 4 * cz;
-        on[cz] = FULL || ((cm >> c) & 1u);
-        T f1 = g1, f2 = g2;
-        if (on[cz]) coef(c, f1, f2);
-        l[cz][0] = f2 * T(0.125);
-        l[cz][1] = (f2 * T(1.0 / 3.0) + f1) * T(0.125);
-        l[cz][2] = (f2 * T(1.0 / 9.0) + f1 * T(2.0 / 3.0)) * T(0.125);
-        l[cz][3] = (f2 * T(1.0 / 27.0) + f1 * T(1.0 / 3.0)) * T(0.125);
+        for (int cz = 0; cz < 2; ++cz) {
+          const int c = cx + 2 * cy + 4 * cz;
+          on[cz] = FULL || ((cm >> c) & 1u);
+          T f1 = g1, f2 = g2;
+          if (on[cz]) coef(c, f1, f2);
+          l[cz][0] = f2 * T(0.125);
+          l[cz][1] = (f2 * T(1.0 / 3.0) + f1) * T(0.125);
+          l[cz][2] = (f2 * T(1.0 / 9.0) + f1 * T(2.0 / 3.0)) * T(0.125);
+          l[cz][3] = (f2 * T(1.0 / 27.0) + f1 * T(1.0 / 3.0)) * T(0.125);
+        }
+#pragma unroll
+        for (int ex = 0; ex < 2; ++ex)
+#pragma unroll
+          for (int ey = 0; ey < 2; ++ey) {
+            T(&g)[3] = v[ex][2 * cy + ey];
+            const int k = ex + ey;
+            T s0 = g[0] + g[1], d0 = g[0] - g[1], s1 = g[1] + g[2], d1 = g[1] - g[2];
+            // an absent child contributes nothing, whatever its vertices hold
+            s0 = on[0] ? s0 * l[0][k] : T(0);
+            d0 = on[0] ? d0 * l[0][k + 1] : T(0);
+            s1 = on[1] ? s1 * l[1][k] : T(0);
+            d1 = on[1] ? d1 * l[1][k + 1] : T(0);
+            g[0] = s0 + d0;
+            g[1] = (s0 - d0) + (s1 + d1);
+            g[2] = s1 - d1;
+          }
       }
 #pragma unroll
       for (int ex = 0; ex < 2; ++ex)
 #pragma unroll
-        for (int ey = 0; ey < 2; ++ey) {
-          T(&g)[3] = v[ex][2 * cy + ey];
-          const int k = ex + ey;
-          T s0 = g[0] + g[1], d0 = g[0] - g[1], s1 = g[1] + g[2], d1 = g[1] - g[2];
-          // an absent child contributes nothing, whatever its vertices hold
-          s0 = on[0] ? s0 * l[0][k] : T(0);
-          d0 = on[0] ? d0 * l[0][k + 1] : T(0);
-          s1 = on[1] ? s1 * l[1][k] : T(0);
-          d1 = on[1] ? d1 * l[1][k + 1] : T(0);
-          g[0] = s0 + d0;
-          g[1] = (s0 - d0) + (s1 + d1);
-          g[2] = s1 - d1;
+        for (int z = 0; z < 3; ++z) {
+          w[2 * cx + ex][3 * z] = v[ex][0][z] + v[ex][1][z];
+          w[2 * cx + ex][3 * z + 1] = (v[ex][0][z] - v[ex][1][z]) + (v[ex][2][z] + v[ex][3][z]);
+          w[2 * cx + ex][3 * z + 2] = v[ex][2][z] - v[ex][3][z];
         }
     }
 #pragma unroll
-    for (int ex = 0; ex < 2; ++ex)
-#pragma unroll
-      for (int z = 0; z < 3; ++z) {
-        w[2 * cx + ex][3 * z] = v[ex][0][z] + v[ex][1][z];
-        w[2 * cx + ex][3 * z + 1] = (v[ex][0][z] - v[ex][1][z]) + (v[ex][2][z] + v[ex][3][z]);
-        w[2 * cx + ex][3 * z + 2] = v[ex][2][z] - v[ex][3][z];
-      }
-  }
-#pragma unroll
-  for (int r = 0; r < 9; ++r) {
-    yv[3 * r] = w[0][r] + w[1][r];
-    yv[3 * r + 1] = (w[0][r] - w[1][r]) + (w[2][r] + w[3][r]);
-    yv[3 * r + 2] = w[2][r] - w[3][r];
+    for (int r = 0; r < 9; ++r) {
+      yv[3 * r] = w[0][r] + w[1][r];
+      yv[3 * r + 1] = (w[0][r] - w[1][r]) + (w[2][r] + w[3][r]);
+      yv[3 * r + 2] = w[2][r] - w[3][r];
+    }
   }
 }
 
