@@ -145,20 +145,6 @@ __global__ void concat_octets(int64_t n, const uint32_t* __restrict__ meta, cons
     dst[i] = r < 35 && v == kNoNode ? kNoNode : v + add;
   }
 }
-__global__ void fill_u16(uint16_t* __restrict__ d, int64_t n0, int64_t n1, uint16_t v) {
-  for (int64_t i = n0 + gtid(); i < n1; i += gstride()) d[i] = v;
-}
-// per-mesh squared norms (acc zeroed by the caller), one shared slot per mesh
-__global__ void seg_sqnorm(const double* __restrict__ r, int64_t n, const uint16_t* __restrict__ node_mesh, int nmesh,
-                           double* __restrict__ acc) {
-  extern __shared__ double sh[];
-  for (int i = threadIdx.x; i < nmesh; i += blockDim.x) sh[i] = 0;
-  __syncthreads();
-  for (int64_t i = gtid(); i < n; i += gstride()) atomicAdd(sh + node_mesh[i], r[i] * r[i]);
-  __syncthreads();
-  for (int i = threadIdx.x; i < nmesh; i += blockDim.x)
-    if (sh[i] != 0.0) atomicAdd(acc + i, sh[i]);
-}
 
 // ----------------------------------------------------------- prolongation --
 // Weights of the coarse element holding fine node f: the 8 trilinear values
@@ -623,6 +609,75 @@ __global__ void dense_gemv(const double* __restrict__ A, int64_t N, const uint32
   }
 }
 
+// x += Ainv b for one symmetric block, from its lower triangle: an entry a_ij
+// below the diagonal serves row i (a_ij b_j) and row j (a_ij b_i), so half of the
+// matrix is never read: one V-cycle of the 131,072-point configuration reads
+// its 17,845 x 17,845 inverse (2.5 GB, 573 us with a warp per row at 4.4 TB/s)
+// as 1.3 GB.  A CTA takes kSymRows rows up to the diagonal (the longest rows
+// first), its warps 32 columns of every 256 with a column per lane: the column
+// sums over the CTA's rows stay in a lane and leave with one reduction per
+// column, the row sums stay in registers to the end.  The next columns' loads
+// are in flight meanwhile.  (Square tiles of 128 rows, which need fewer
+// reductions, took 470 us: 128 rows are 18 MB apart, more pages than the
+// translation caches hold.)
+constexpr int kSymRows = 16;
+constexpr int64_t kSymFrom = 3000;  // rows from which the matrix (72 MB) leaves L2 between cycles
+__global__ void __launch_bounds__(256, 2) dense_symv(const double* __restrict__ A, int64_t n,
+                                                     const double* __restrict__ b, double* __restrict__ x) {
+  __shared__ double bi[kSymRows], rs[8][kSymRows];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t i0 = (int64_t(gridDim.x) - 1 - blockIdx.x) * kSymRows;
+  const int64_t i1 = i0 + kSymRows < n ? i0 + kSymRows : n;  // one past the last row
+  if (tid < kSymRows) bi[tid] = i0 + tid < n ? b[i0 + tid] : 0.0;
+  __syncthreads();
+  const double* A0 = A + i0 * n;
+  double row[kSymRows], a[kSymRows], an[kSymRows];
+#pragma unroll
+  for (int r = 0; r < kSymRows; ++r) row[r] = an[r] = 0.0;
+  auto load = [&](double (&v)[kSymRows], int64_t j) {  // column j of the rows, up to the diagonal
+    if (j <= i0) {
+#pragma unroll
+      for (int r = 0; r < kSymRows; ++r) v[r] = i0 + r < i1 ? __ldg(A0 + int64_t(r) * n + j) : 0.0;
+    } else {
+#pragma unroll
+      for (int r = 0; r < kSymRows; ++r) v[r] = i0 + r < i1 && j <= i0 + r ? __ldg(A0 + int64_t(r) * n + j) : 0.0;
+    }
+  };
+  int64_t j = 32 * w + lane;
+  load(an, j);
+  for (; j - lane < i1; j += 256) {
+#pragma unroll
+    for (int r = 0; r < kSymRows; ++r) a[r] = an[r];
+    load(an, j + 256);
+    const double xj = j < i1 ? __ldg(b + j) : 0.0;
+    double col = 0.0;
+#pragma unroll
+    for (int r = 0; r < kSymRows; ++r) {
+      row[r] = fma(a[r], xj, row[r]);
+      col = fma(a[r], bi[r], col);
+    }
+    if (j >= i0 && j < i1) {  // the diagonal entry counts once
+#pragma unroll
+      for (int r = 0; r < kSymRows; ++r)
+        if (j == i0 + r) col -= a[r] * bi[r];
+    }
+    if (j < i1) atomicAdd(x + j, col);
+  }
+#pragma unroll
+  for (int r = 0; r < kSymRows; ++r) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) row[r] += __shfl_xor_sync(0xffffffffu, row[r], o);
+    if (lane == r) rs[w][r] = row[r];
+  }
+  __syncthreads();
+  if (tid < kSymRows && i0 + tid < n) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += rs[k][tid];
+    atomicAdd(x + i0 + tid, s);
+  }
+}
+
 // -------------------------------------------------------------- reductions --
 constexpr int kRedBlocks = 1184;  // 8 x 148 SMs: enough loads in flight for HBM
 
@@ -640,6 +695,26 @@ __device__ __forceinline__ double block_sum(double v) {
   __syncthreads();
   return v;
 }
+// Squared norm of each mesh's part of r (nodes off[k] to off[k + 1] - 1):
+// blockIdx.y = the mesh, its CTAs' partial sums to part[y][gridDim.x], which
+// seg_finish adds up.  (One shared-memory FP64 atomic per value, all on a few
+// addresses, took 96 us per norm of 8 meshes with 1M nodes.)
+__global__ void __launch_bounds__(256) seg_sqnorm(const double* __restrict__ r, const int64_t* __restrict__ off,
+                                                  double* __restrict__ part) {
+  const int64_t e = off[blockIdx.y + 1];
+  double v = 0;
+  #pragma unroll 4
+  for (int64_t i = off[blockIdx.y] + gtid(); i < e; i += gstride()) v = fma(r[i], r[i], v);
+  v = block_sum(v);
+  if (threadIdx.x == 0) part[int64_t(blockIdx.y) * gridDim.x + blockIdx.x] = v;
+}
+__global__ void __launch_bounds__(256) seg_finish(const double* __restrict__ part, int np, double* __restrict__ out) {
+  double v = 0;
+  for (int i = threadIdx.x; i < np; i += blockDim.x) v += part[int64_t(blockIdx.x) * np + i];
+  v = block_sum(v);
+  if (threadIdx.x == 0) out[blockIdx.x] = v;
+}
+constexpr int kSegBlocks = 64;  // CTAs per mesh
 // deterministic second stage: one block sums the partials in a fixed order
 __global__ void finish_sum(const double* __restrict__ part, int np, double* __restrict__ out) {
   double v = 0;
@@ -797,8 +872,8 @@ struct dg_damg {
   // batches: mesh offsets of elements / nodes on every level
   int nmesh = 1;
   std::vector<std::vector<int64_t>> mesh_elem_off, mesh_node_off;  // [level][mesh + 1]
-  DBuf<uint16_t> d_node_mesh;   // finest-level node -> mesh
-  DBuf<double> mesh_part;       // per-mesh squared norms
+  DBuf<int64_t> d_node_off;     // finest-level node offsets of the meshes
+  DBuf<double> mesh_part;       // per-mesh squared norms, then their partial sums
   // learned post-smoother on the finest level (FP32 inner V-cycle only)
   dg_mlp* mlp = nullptr;
   int mlp_sweeps = 2;
@@ -826,6 +901,20 @@ struct dg_damg {
 };
 
 namespace {
+
+// x = the coarsest level's dense inverse times b (FP64).
+dg_status coarse_solve(const dg_damg* m, const double* b, double* x, cudaStream_t s) {
+  const int64_t n = m->nc;
+  if (m->cb_n.size() == 1 && n >= kSymFrom) {
+    DG_CUDA(cudaMemsetAsync(x, 0, 8 * n, s));
+    dense_symv<<<unsigned((n + kSymRows - 1) / kSymRows), 256, 0, s>>>(m->Ainv.p, n, b, x);
+  } else {
+    dense_gemv<<<grid_for(n * 32, 256), 256, 0, s>>>(m->Ainv.p, n, m->d_crow_blk.p, m->d_cb_off.p, m->d_cb_n.p,
+                                                     m->d_cb_aoff.p, b, x);
+  }
+  DG_CUDA(cudaGetLastError());
+  return DG_OK;
+}
 
 dg_status build_prolongation(Level& F, Level& C, cudaStream_t s) {
   const dg_da* fd = F.da.get();
@@ -1199,12 +1288,7 @@ dg_status vcycle3(dg_damg* m, size_t l, const double* b, double* x) {
   Level& L = m->lv[l];
   const int64_t nn = L.da->N, n = 3 * nn;
   const unsigned g = grid_for(n, 256, 16);
-  if (l + 1 == m->lv.size()) {
-    dense_gemv<<<grid_for(n * 32, 256), 256, 0, s>>>(m->Ainv.p, n, m->d_crow_blk.p, m->d_cb_off.p, m->d_cb_n.p,
-                                                     m->d_cb_aoff.p, b, x);
-    DG_CUDA(cudaGetLastError());
-    return DG_OK;
-  }
+  if (l + 1 == m->lv.size()) return coarse_solve(m, b, x, s);
   const double w = m->cfg.omega;
   if (m->cfg.nu_pre > 0) {
     jacobi_first<<<g, 256, 0, s>>>(x, b, L.dinv.p, w, n);
@@ -1237,12 +1321,7 @@ dg_status vcycle(dg_damg* m, size_t l, const double* b, double* x) {
   Level& L = m->lv[l];
   const int64_t n = L.da->N;
   const unsigned g = grid_for(n, 256, 16);
-  if (l + 1 == m->lv.size()) {
-    dense_gemv<<<grid_for(n * 32, 256), 256, 0, s>>>(m->Ainv.p, n, m->d_crow_blk.p, m->d_cb_off.p, m->d_cb_n.p,
-                                                     m->d_cb_aoff.p, b, x);
-    DG_CUDA(cudaGetLastError());
-    return DG_OK;
-  }
+  if (l + 1 == m->lv.size()) return coarse_solve(m, b, x, s);
   const double w = m->cfg.omega;
   // pre-smoothing from a zero initial guess; the sweeps after the first and
   // the residual are fused warp-tile operator applications
@@ -1272,8 +1351,7 @@ dg_status vcycle32(dg_damg* m, size_t l, const float* b, float* x) {
   const unsigned g = grid_for(n, 256, 16);
   if (l + 1 == m->lv.size()) {
     convert<float, double><<<g, 256, 0, s>>>(b, L.b.p, n);
-    dense_gemv<<<grid_for(n * 32, 256), 256, 0, s>>>(m->Ainv.p, n, m->d_crow_blk.p, m->d_cb_off.p, m->d_cb_n.p,
-                                                     m->d_cb_aoff.p, L.b.p, L.x.p);
+    DG_TRY(coarse_solve(m, L.b.p, L.x.p, s));
     convert<double, float><<<g, 256, 0, s>>>(L.x.p, x, n);
     DG_CUDA(cudaGetLastError());
     return DG_OK;
@@ -1460,12 +1538,9 @@ dg_status finish_create(dg_damg* m) {
   }
   DG_TRY(m->part.alloc(kRedBlocks));
   DG_TRY(m->scal.alloc(8));
-  DG_TRY(m->d_node_mesh.alloc(N));
-  DG_TRY(m->mesh_part.alloc(m->nmesh));
-  const std::vector<int64_t>& no = m->mesh_node_off[0];
-  for (int i = 0; i < m->nmesh; ++i)
-    fill_u16<<<grid_for(no[i + 1] - no[i], 256), 256, 0, m->s>>>(m->d_node_mesh.p, no[i], no[i + 1], uint16_t(i));
-  DG_CUDA(cudaGetLastError());
+  DG_TRY(m->d_node_off.alloc(m->nmesh + 1));
+  DG_TRY(m->mesh_part.alloc(int64_t(m->nmesh) * (1 + kSegBlocks)));
+  DG_CUDA(cudaMemcpyAsync(m->d_node_off.p, m->mesh_node_off[0].data(), 8 * (m->nmesh + 1), cudaMemcpyHostToDevice, m->s));
   for (size_t l = 0; l + 1 < m->lv.size(); ++l) {
     DG_TRY(build_restriction(m->lv[l], m->lv[l + 1].da->N, m->s));
     DG_TRY(build_weight_codes(m->lv[l], m->s));
@@ -1758,8 +1833,8 @@ dg_status dg_damg_solve(dg_damg* m, const double* b, double* x, int on_device, d
   const int nm = m->nmesh;
   std::vector<double> bb(nm, hb), rr(nm);
   auto mesh_norms = [&](const double* v, std::vector<double>& out) -> dg_status {
-    DG_CUDA(cudaMemsetAsync(m->mesh_part.p, 0, 8 * nm, s));
-    seg_sqnorm<<<kRedBlocks, 256, 8 * nm, s>>>(v, n, m->d_node_mesh.p, nm, m->mesh_part.p);
+    seg_sqnorm<<<dim3(kSegBlocks, unsigned(nm)), 256, 0, s>>>(v, m->d_node_off.p, m->mesh_part.p + nm);
+    seg_finish<<<unsigned(nm), 256, 0, s>>>(m->mesh_part.p + nm, kSegBlocks, m->mesh_part.p);
     DG_CUDA(cudaGetLastError());
     DG_CUDA(cudaMemcpyAsync(out.data(), m->mesh_part.p, 8 * nm, cudaMemcpyDeviceToHost, s));
     DG_CUDA(cudaStreamSynchronize(s));
@@ -2272,12 +2347,7 @@ dg_status dg_damg_level_coef(dg_damg* m, int level, double* coef) {
 dg_status dg_damg_coarse_solve(dg_damg* m, const double* b, double* x, void* stream) {
   DG_CHECK(m && b && x && !m->lv.empty(), DG_EINVAL, "damg_coarse_solve: bad arguments");
   DG_CHECK(m->lv.back().A, DG_EINVAL, "damg_coarse_solve: no operator set");
-  const int64_t n = int64_t(m->cfg.dof) * m->lv.back().da->N;
-  auto s = static_cast<cudaStream_t>(stream);
-  dense_gemv<<<grid_for(n * 32, 256), 256, 0, s>>>(m->Ainv.p, n, m->d_crow_blk.p, m->d_cb_off.p, m->d_cb_n.p,
-                                                   m->d_cb_aoff.p, b, x);
-  DG_CUDA(cudaGetLastError());
-  return DG_OK;
+  return coarse_solve(m, b, x, static_cast<cudaStream_t>(stream));
 }
 
 dg_status dg_damg_vcycle(dg_damg* m, const double* b, double* x) {
