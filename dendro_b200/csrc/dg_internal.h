@@ -256,9 +256,11 @@ dg_status matvec_variant_tables(dg_da* da, int v, cudaStream_t s);
 dg_status mrhs_apply(const dg_mat* A, const float* X, float* Y, int nrhs, int split, cudaStream_t s);
 // Y = A X in the octet form (CUDA cores) in FP32 or FP64, node-major [N][R],
 // R a multiple of 16; coef = the operator's coefficients in that precision
-// ([2][E], a then b; ignored when the operator has none).
+// ([2][E], a then b; ignored when the operator has none).  zeroed: Y holds
+// zeros already.
 template <class T>
-dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int R, cudaStream_t s);
+dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int R, cudaStream_t s,
+                           bool zeroed = false);
 // Multi-RHS operator on tcgen05 (mrhs_tc.cu): nrhs a multiple of 64, passes 1
 // (TF32 products) or 3 (hi/lo split, FP32-level).
 dg_status mrhs_tc_apply(const dg_mat* A, const float* X, float* Y, int R, int passes, cudaStream_t s);

@@ -210,11 +210,11 @@ void launch_octet(const dg_da* da, const T* ca, const T* cb, int R, int col0, in
 // FP32: blocks of 64 columns by the pair kernel, then 32, then 16; FP64: 32
 // and 16.
 template <class T>
-dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int R, cudaStream_t s) {
+dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int R, cudaStream_t s, bool zeroed) {
   const dg_da* da = A->da;
   const OctetSet& O = da->octs;
   DG_CHECK(A->kind == 0 && R % kRC == 0 && O.n > 0, DG_EINVAL, "multi-RHS octet operator: bad arguments");
-  DG_CUDA(cudaMemsetAsync(Y, 0, sizeof(T) * size_t(da->N) * R, s));
+  if (!zeroed) DG_CUDA(cudaMemsetAsync(Y, 0, sizeof(T) * size_t(da->N) * R, s));
   const T* ca = A->has_coef ? coef : nullptr;
   const T* cb = A->has_coef ? coef + da->E : nullptr;
   int col = 0;
@@ -234,9 +234,10 @@ dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int
   DG_CUDA(cudaGetLastError());
   return DG_OK;
 }
-template dg_status mrhs_octet_apply<float>(const dg_mat*, const float*, const float*, float*, int, cudaStream_t);
-template dg_status mrhs_octet_apply<double>(const dg_mat*, const double*, const double*, double*, int,
-                                            cudaStream_t);
+template dg_status mrhs_octet_apply<float>(const dg_mat*, const float*, const float*, float*, int, cudaStream_t,
+                                           bool);
+template dg_status mrhs_octet_apply<double>(const dg_mat*, const double*, const double*, double*, int, cudaStream_t,
+                                            bool);
 
 dg_status mrhs_apply(const dg_mat* A, const float* X, float* Y, int R, int split, cudaStream_t s) {
   dg_da* da = A->da;

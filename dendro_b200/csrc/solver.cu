@@ -1927,107 +1927,251 @@ void dg_damg_destroy(dg_damg* m) { delete_drained(m); }
 // over the R columns, the coarsest level the dense inverse times the block.
 namespace {
 
+// The elementwise kernels work 16 bytes (W values of one row) per thread and
+// step: i counts those, i >> sh is the row (R is a power of two, so no
+// divisions: those by a run-time R took most of the instructions).
+template <class T>
+struct alignas(16) Quad {
+  static constexpr int W = 16 / int(sizeof(T));
+  T v[W];
+};
 template <class T>
 __global__ void mv_jacobi_first(T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ dinv, T omega,
-                                int64_t n, int R) {
-  for (int64_t i = gtid(); i < n; i += gstride()) x[i] = omega * dinv[i / R] * b[i];
+                                int64_t nv, int sh) {
+  const Quad<T>* b4 = reinterpret_cast<const Quad<T>*>(b);
+  for (int64_t i = gtid(); i < nv; i += gstride()) {
+    Quad<T> q = b4[i];
+    const T w = omega * dinv[i >> sh];
+#pragma unroll
+    for (int k = 0; k < Quad<T>::W; ++k) q.v[k] = w * q.v[k];
+    reinterpret_cast<Quad<T>*>(x)[i] = q;
+  }
 }
+// x += omega dinv (b - t), and t = 0 for the next operator application
 template <class T>
 __global__ void mv_jacobi_update(T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ dinv,
-                                 const T* __restrict__ t, T omega, int64_t n, int R) {
-  for (int64_t i = gtid(); i < n; i += gstride()) x[i] += omega * dinv[i / R] * (b[i] - t[i]);
+                                 T* __restrict__ t, T omega, int64_t nv, int sh) {
+  using Q = Quad<T>;
+  Q zero;
+#pragma unroll
+  for (int k = 0; k < Q::W; ++k) zero.v[k] = T(0);
+  #pragma unroll 2
+  for (int64_t i = gtid(); i < nv; i += gstride()) {
+    Q xq = reinterpret_cast<Q*>(x)[i];
+    const Q bq = reinterpret_cast<const Q*>(b)[i], tq = reinterpret_cast<const Q*>(t)[i];
+    const T w = omega * dinv[i >> sh];
+#pragma unroll
+    for (int k = 0; k < Q::W; ++k) xq.v[k] += w * (bq.v[k] - tq.v[k]);
+    reinterpret_cast<Q*>(x)[i] = xq;
+    reinterpret_cast<Q*>(t)[i] = zero;
+  }
 }
+// t = b - t
 template <class T>
-__global__ void mv_residual(const T* __restrict__ b, const T* __restrict__ t, T* __restrict__ r, int64_t n) {
-  for (int64_t i = gtid(); i < n; i += gstride()) r[i] = b[i] - t[i];
+__global__ void mv_residual(const T* __restrict__ b, T* __restrict__ t, int64_t nv) {
+  using Q = Quad<T>;
+  #pragma unroll 2
+  for (int64_t i = gtid(); i < nv; i += gstride()) {
+    const Q bq = reinterpret_cast<const Q*>(b)[i];
+    Q tq = reinterpret_cast<Q*>(t)[i];
+#pragma unroll
+    for (int k = 0; k < Q::W; ++k) tq.v[k] = bq.v[k] - tq.v[k];
+    reinterpret_cast<Q*>(t)[i] = tq;
+  }
 }
-// rc[c][:] = sum_k R[c][k] rf[k][:]  (thread per (row, column): coalesced rows)
+// rc[c][:] = sum_k R[c][k] rf[k][:]  (a thread per row and 16 bytes: coalesced rows)
 template <class T>
 __global__ void mv_restrict(const uint32_t* __restrict__ rptr, const uint32_t* __restrict__ rcol,
-                            const T* __restrict__ rval, int64_t Nc, int R, const T* __restrict__ rf,
+                            const T* __restrict__ rval, int64_t nv, int sh, const T* __restrict__ rf,
                             T* __restrict__ rc) {
-  for (int64_t i = gtid(); i < Nc * R; i += gstride()) {
-    const int64_t c = i / R;
-    const int j = int(i - c * R);
-    T acc = T(0);
-    for (uint32_t k = rptr[c]; k < rptr[c + 1]; ++k) acc += rval[k] * rf[int64_t(rcol[k]) * R + j];
-    rc[i] = acc;
+  using Q = Quad<T>;
+  for (int64_t i = gtid(); i < nv; i += gstride()) {
+    const int64_t c = i >> sh, j = i - (c << sh);
+    Q acc;
+#pragma unroll
+    for (int k = 0; k < Q::W; ++k) acc.v[k] = T(0);
+    const uint32_t e = rptr[c + 1];
+    #pragma unroll 4
+    for (uint32_t k = rptr[c]; k < e; ++k) {
+      const T w = rval[k];
+      const Q q = reinterpret_cast<const Q*>(rf)[(int64_t(rcol[k]) << sh) + j];
+#pragma unroll
+      for (int u = 0; u < Q::W; ++u) acc.v[u] += w * q.v[u];
+    }
+    reinterpret_cast<Q*>(rc)[i] = acc;
   }
 }
 template <class T>
 __global__ void mv_prolong_add(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ pcol,
-                               const T* __restrict__ pval, int64_t Nf, int R, const T* __restrict__ xc,
+                               const T* __restrict__ pval, int64_t nv, int sh, const T* __restrict__ xc,
                                T* __restrict__ xf) {
-  for (int64_t i = gtid(); i < Nf * R; i += gstride()) {
-    const int64_t f = i / R;
-    const int j = int(i - f * R);
-    T acc = T(0);
-    for (uint32_t k = pptr[f]; k < pptr[f + 1]; ++k) acc += pval[k] * xc[int64_t(pcol[k]) * R + j];
-    xf[i] += acc;
+  using Q = Quad<T>;
+  for (int64_t i = gtid(); i < nv; i += gstride()) {
+    const int64_t f = i >> sh, j = i - (f << sh);
+    Q acc;
+#pragma unroll
+    for (int k = 0; k < Q::W; ++k) acc.v[k] = T(0);
+    const uint32_t e = pptr[f + 1];
+    #pragma unroll 2
+    for (uint32_t k = pptr[f]; k < e; ++k) {
+      const T w = pval[k];
+      const Q q = reinterpret_cast<const Q*>(xc)[(int64_t(pcol[k]) << sh) + j];
+#pragma unroll
+      for (int u = 0; u < Q::W; ++u) acc.v[u] += w * q.v[u];
+    }
+    Q xq = reinterpret_cast<Q*>(xf)[i];
+#pragma unroll
+    for (int u = 0; u < Q::W; ++u) xq.v[u] += acc.v[u];
+    reinterpret_cast<Q*>(xf)[i] = xq;
   }
 }
 // x = Ainv b for a block of R columns (one dense block: a single mesh)
-__global__ void mv_coarse(const double* __restrict__ Ainv, int64_t n, int R, const double* __restrict__ b,
+__global__ void mv_coarse(const double* __restrict__ Ainv, int64_t n, int R, int sh, const double* __restrict__ b,
                           double* __restrict__ x) {
   for (int64_t i = gtid(); i < n * R; i += gstride()) {
-    const int64_t r = i / R;
-    const int j = int(i - r * R);
+    const int64_t r = i >> sh, j = i - (r << sh);
     const double* a = Ainv + r * n;
-    double acc = 0;
-    for (int64_t k = 0; k < n; ++k) acc += a[k] * b[k * R + j];
-    x[i] = acc;
+    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;  // four sums: loads of four steps in flight
+    int64_t k = 0;
+    for (; k + 4 <= n; k += 4) {
+      s0 = fma(a[k], b[(k << sh) + j], s0);
+      s1 = fma(a[k + 1], b[((k + 1) << sh) + j], s1);
+      s2 = fma(a[k + 2], b[((k + 2) << sh) + j], s2);
+      s3 = fma(a[k + 3], b[((k + 3) << sh) + j], s3);
+    }
+    for (; k < n; ++k) s0 = fma(a[k], b[(k << sh) + j], s0);
+    x[i] = (s0 + s1) + (s2 + s3);
   }
 }
+// four values per thread and step
 template <class A, class B>
-__global__ void mv_convert(const A* __restrict__ a, B* __restrict__ b, int64_t n) {
-  for (int64_t i = gtid(); i < n; i += gstride()) b[i] = B(a[i]);
+__global__ void mv_convert(const A* __restrict__ a, B* __restrict__ b, int64_t n4) {
+  struct alignas(16) A4 {
+    A v[4];
+  };
+  struct alignas(16) B4 {
+    B v[4];
+  };
+  #pragma unroll 2
+  for (int64_t i = gtid(); i < n4; i += gstride()) {
+    const A4 p = reinterpret_cast<const A4*>(a)[i];
+    B4 q;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q.v[k] = B(p.v[k]);
+    reinterpret_cast<B4*>(b)[i] = q;
+  }
 }
-// Column sums of a[i][j] b[i][j] over the N rows: per block R partial sums
-// (256 / R rows at a time), then one pass over the blocks.
+// Column sums over the N rows: a thread takes 2 columns (16 bytes) of every
+// (512 / R)-th row of its CTA; the CTA's sums per column go to part, one pass
+// over the CTAs by mv_dot_finish.  `h` = R / 2 threads per row.
 constexpr int kMvDotBlocks = 592;
-__global__ void __launch_bounds__(256) mv_dot_partial(const double* __restrict__ a, const double* __restrict__ b,
-                                                      int64_t N, int R, double* __restrict__ part) {
-  __shared__ double acc[256];
-  const int rows = 256 / R, j = int(threadIdx.x) % R, r0 = int(threadIdx.x) / R;
-  double v = 0;
-  for (int64_t i = int64_t(blockIdx.x) * rows + r0; i < N; i += int64_t(gridDim.x) * rows)
-    v += a[i * R + j] * b[i * R + j];
+__device__ __forceinline__ void mv_block_columns(double2 v, int h, double* __restrict__ part, int R) {
+  __shared__ double2 acc[256];
   acc[threadIdx.x] = v;
   __syncthreads();
-  if (threadIdx.x < R) {
-    double t = 0;
-    for (int k = 0; k < rows; ++k) t += acc[k * R + threadIdx.x];
-    part[int64_t(blockIdx.x) * R + threadIdx.x] = t;
+  if (int(threadIdx.x) < h) {
+    double2 t = acc[threadIdx.x];
+    for (int k = int(threadIdx.x) + h; k < 256; k += h) {
+      t.x += acc[k].x;
+      t.y += acc[k].y;
+    }
+    reinterpret_cast<double2*>(part + int64_t(blockIdx.x) * R)[threadIdx.x] = t;
+  }
+  __syncthreads();
+}
+// sums of a b and, when c is given, of a c (part2)
+__global__ void __launch_bounds__(256) mv_dot_partial(const double* __restrict__ a, const double* __restrict__ b,
+                                                      const double* __restrict__ c, int64_t N, int R,
+                                                      double* __restrict__ part, double* __restrict__ part2) {
+  const int h = R / 2;
+  const int64_t n2 = N * h, S = int64_t(gridDim.x) * 256;
+  const double2 *a2 = reinterpret_cast<const double2*>(a), *b2 = reinterpret_cast<const double2*>(b),
+                *c2 = reinterpret_cast<const double2*>(c);
+  double2 v = make_double2(0, 0), w = make_double2(0, 0);
+  #pragma unroll 4
+  for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < n2; i += S) {  // 256 is a multiple of h: same columns
+    const double2 x = a2[i], y = b2[i];
+    v.x = fma(x.x, y.x, v.x);
+    v.y = fma(x.y, y.y, v.y);
+    if (c) {
+      const double2 z = c2[i];
+      w.x = fma(x.x, z.x, w.x);
+      w.y = fma(x.y, z.y, w.y);
+    }
+  }
+  mv_block_columns(v, h, part, R);
+  if (c) mv_block_columns(w, h, part2, R);
+}
+// 32 columns per CTA (blockIdx.x), the CTAs' sums spread over 8 groups of
+// lanes; blockIdx.y: the second set of sums.  (One CTA, a thread per column:
+// 70 us.)
+__global__ void __launch_bounds__(256) mv_dot_finish(const double* __restrict__ part, int nb, int R,
+                                                     double* __restrict__ out, double* __restrict__ out2) {
+  __shared__ double acc[8][32];
+  const int j = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
+  const double* p = part + int64_t(blockIdx.y) * nb * R;
+  double t = 0;
+  #pragma unroll 8
+  for (int k = g; k < nb; k += 8) t += p[int64_t(k) * R + j];
+  acc[g][threadIdx.x & 31] = t;
+  __syncthreads();
+  if (g == 0) {
+    for (int k = 1; k < 8; ++k) t += acc[k][threadIdx.x];
+    (blockIdx.y ? out2 : out)[j] = t;
   }
 }
-__global__ void mv_dot_finish(const double* __restrict__ part, int nb, int R, double* __restrict__ out) {
-  for (int j = threadIdx.x; j < R; j += blockDim.x) {
-    double t = 0;
-    for (int k = 0; k < nb; ++k) t += part[int64_t(k) * R + j];
-    out[j] = t;
+// The step of every column: x += alpha p, r -= alpha q with alpha = rz / pq
+// (zero for converged columns), and the sums of r r.
+__global__ void __launch_bounds__(256) mv_step(double* __restrict__ x, double* __restrict__ r,
+                                               const double* __restrict__ p, const double* __restrict__ q,
+                                               const double* __restrict__ rz, const double* __restrict__ pq,
+                                               const uint8_t* __restrict__ done, int64_t N, int R,
+                                               double* __restrict__ part) {
+  const int h = R / 2, j = 2 * (int(threadIdx.x) % h);
+  const double a0 = (done[j] || pq[j] == 0) ? 0.0 : rz[j] / pq[j];
+  const double a1 = (done[j + 1] || pq[j + 1] == 0) ? 0.0 : rz[j + 1] / pq[j + 1];
+  const int64_t n2 = N * h, S = int64_t(gridDim.x) * 256;
+  double2 *x2 = reinterpret_cast<double2*>(x), *r2 = reinterpret_cast<double2*>(r);
+  const double2 *p2 = reinterpret_cast<const double2*>(p), *q2 = reinterpret_cast<const double2*>(q);
+  double2 v = make_double2(0, 0);
+  #pragma unroll 2
+  for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < n2; i += S) {
+    double2 xi = x2[i], ri = r2[i];
+    const double2 pi = p2[i], qi = q2[i];
+    xi.x += a0 * pi.x;
+    xi.y += a1 * pi.y;
+    ri.x -= a0 * qi.x;
+    ri.y -= a1 * qi.y;
+    x2[i] = xi;
+    r2[i] = ri;
+    v.x = fma(ri.x, ri.x, v.x);
+    v.y = fma(ri.y, ri.y, v.y);
   }
+  mv_block_columns(v, h, part, R);
 }
-// per-column PCG steps: y += s a[j] x; p = z + b[j] p
-__global__ void mv_axpy(double* __restrict__ y, const double* __restrict__ x, const double* __restrict__ a,
-                        double sgn, int64_t n, int R) {
-  for (int64_t i = gtid(); i < n; i += gstride()) y[i] += sgn * a[i % R] * x[i];
-}
-__global__ void mv_direction(double* __restrict__ p, const double* __restrict__ z, const double* __restrict__ b,
-                             int64_t n, int R) {
-  for (int64_t i = gtid(); i < n; i += gstride()) p[i] = z[i] + b[i % R] * p[i];
-}
-// alpha = rz / pq and the flexible beta = (rz_new - (r, z_old)) / rz, zero for
-// converged columns (done[j]); rz <- rz_new
-__global__ void mv_alpha(const double* __restrict__ rz, const double* __restrict__ pq,
-                         const uint8_t* __restrict__ done, double* __restrict__ alpha, int R) {
-  for (int j = threadIdx.x; j < R; j += blockDim.x) alpha[j] = (done[j] || pq[j] == 0) ? 0.0 : rz[j] / pq[j];
-}
-__global__ void mv_beta(const double* __restrict__ rzn, const double* __restrict__ rzo, double* __restrict__ rz,
-                        const uint8_t* __restrict__ done, double* __restrict__ beta, int R, int flexible) {
-  for (int j = threadIdx.x; j < R; j += blockDim.x) {
-    const double num = flexible ? rzn[j] - rzo[j] : rzn[j];
-    beta[j] = (done[j] || rz[j] == 0) ? 0.0 : num / rz[j];
-    rz[j] = rzn[j];
+// The direction of every column: p = z + beta p, the flexible beta =
+// (rz_new - (r, z_old)) / rz or rz_new / rz, zero for converged columns.
+__global__ void __launch_bounds__(256) mv_direction(double* __restrict__ p, const double* __restrict__ z,
+                                                    const double* __restrict__ rzn, const double* __restrict__ rzo,
+                                                    const double* __restrict__ rz, const uint8_t* __restrict__ done,
+                                                    int flexible, int64_t N, int R) {
+  const int h = R / 2, j = 2 * (int(threadIdx.x) % h);
+  double be[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double num = flexible ? rzn[j + k] - rzo[j + k] : rzn[j + k];
+    be[k] = (done[j + k] || rz[j + k] == 0) ? 0.0 : num / rz[j + k];
+  }
+  const int64_t n2 = N * h, S = int64_t(gridDim.x) * 256;
+  double2* p2 = reinterpret_cast<double2*>(p);
+  const double2* z2 = reinterpret_cast<const double2*>(z);
+  #pragma unroll 2
+  for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < n2; i += S) {
+    double2 pi = p2[i];
+    const double2 zi = z2[i];
+    pi.x = zi.x + be[0] * pi.x;
+    pi.y = zi.y + be[1] * pi.y;
+    p2[i] = pi;
   }
 }
 
@@ -2042,15 +2186,20 @@ dg_status vcycle_multi(dg_damg* m, size_t l, const T* b, T* x, int R, MultiLevel
                        DBuf<double>& cx) {
   cudaStream_t s = m->s;
   Level& L = m->lv[l];
-  const int64_t N = L.da->N, n = N * R;
-  const unsigned g = grid_for(n, 256, 16);
+  constexpr int kW = Quad<T>::W;
+  int lr = 0;  // log2 R
+  while ((1 << lr) < R) ++lr;
+  const int sh = lr - (kW == 4 ? 2 : 1);
+  const int64_t N = L.da->N, n = N * R, nv = n / kW;
+  const unsigned g = grid_for(nv, 256, 16);
   if (l + 1 == m->lv.size()) {
+    const unsigned gc = grid_for(n, 256, 16);
     if constexpr (sizeof(T) == 8) {
-      mv_coarse<<<grid_for(n, 256, 16), 256, 0, s>>>(m->Ainv.p, N, R, b, x);
+      mv_coarse<<<gc, 256, 0, s>>>(m->Ainv.p, N, R, lr, b, x);
     } else {
-      mv_convert<float, double><<<g, 256, 0, s>>>(b, cb.p, n);
-      mv_coarse<<<grid_for(n, 256, 16), 256, 0, s>>>(m->Ainv.p, N, R, cb.p, cx.p);
-      mv_convert<double, float><<<g, 256, 0, s>>>(cx.p, x, n);
+      mv_convert<float, double><<<grid_for(n / 4, 256, 16), 256, 0, s>>>(b, cb.p, n / 4);
+      mv_coarse<<<gc, 256, 0, s>>>(m->Ainv.p, N, R, lr, cb.p, cx.p);
+      mv_convert<double, float><<<grid_for(n / 4, 256, 16), 256, 0, s>>>(cx.p, x, n / 4);
     }
     DG_CUDA(cudaGetLastError());
     return DG_OK;
@@ -2071,26 +2220,30 @@ dg_status vcycle_multi(dg_damg* m, size_t l, const T* b, T* x, int R, MultiLevel
   }
   const T w = T(m->cfg.omega);
   T* t = W.t[l].p;
+  bool zeroed = false;  // t holds zeros
   if (m->cfg.nu_pre > 0) {
-    mv_jacobi_first<T><<<g, 256, 0, s>>>(x, b, dinv, w, n, R);
+    mv_jacobi_first<T><<<g, 256, 0, s>>>(x, b, dinv, w, nv, sh);
     for (int k = 1; k < m->cfg.nu_pre; ++k) {
-      DG_TRY(mrhs_octet_apply<T>(L.A.get(), coef, x, t, R, s));
-      mv_jacobi_update<T><<<g, 256, 0, s>>>(x, b, dinv, t, w, n, R);
+      DG_TRY(mrhs_octet_apply<T>(L.A.get(), coef, x, t, R, s, zeroed));
+      mv_jacobi_update<T><<<g, 256, 0, s>>>(x, b, dinv, t, w, nv, sh);
+      zeroed = true;
     }
-    DG_TRY(mrhs_octet_apply<T>(L.A.get(), coef, x, t, R, s));
-    mv_residual<T><<<g, 256, 0, s>>>(b, t, t, n);
+    DG_TRY(mrhs_octet_apply<T>(L.A.get(), coef, x, t, R, s, zeroed));
+    mv_residual<T><<<g, 256, 0, s>>>(b, t, nv);
+    zeroed = false;
   } else {
     DG_CUDA(cudaMemsetAsync(x, 0, sizeof(T) * n, s));
   }
   Level& C = m->lv[l + 1];
-  const int64_t Nc = C.da->N;
-  mv_restrict<T><<<grid_for(Nc * R, 256, 16), 256, 0, s>>>(L.rptr.p, L.rcol.p, rval, Nc, R,
-                                                           m->cfg.nu_pre > 0 ? (const T*)t : b, W.b[l + 1].p);
+  const int64_t ncv = C.da->N * R / kW;
+  mv_restrict<T><<<grid_for(ncv, 128, 16), 128, 0, s>>>(L.rptr.p, L.rcol.p, rval, ncv, sh,
+                                                        m->cfg.nu_pre > 0 ? (const T*)t : b, W.b[l + 1].p);
   DG_TRY(vcycle_multi<T>(m, l + 1, W.b[l + 1].p, W.x[l + 1].p, R, W, cb, cx));
-  mv_prolong_add<T><<<g, 256, 0, s>>>(L.pptr.p, L.pcol.p, pval, N, R, W.x[l + 1].p, x);
+  mv_prolong_add<T><<<g, 256, 0, s>>>(L.pptr.p, L.pcol.p, pval, nv, sh, W.x[l + 1].p, x);
   for (int k = 0; k < m->cfg.nu_post; ++k) {
-    DG_TRY(mrhs_octet_apply<T>(L.A.get(), coef, x, t, R, s));
-    mv_jacobi_update<T><<<g, 256, 0, s>>>(x, b, dinv, t, w, n, R);
+    DG_TRY(mrhs_octet_apply<T>(L.A.get(), coef, x, t, R, s, zeroed));
+    mv_jacobi_update<T><<<g, 256, 0, s>>>(x, b, dinv, t, w, nv, sh);
+    zeroed = true;
   }
   DG_CUDA(cudaGetLastError());
   return DG_OK;
@@ -2130,12 +2283,22 @@ dg_status dg_damg_solve_multi(dg_damg* m, const double* B, double* X, int nrhs, 
   const int64_t N = L0.da->N, n = N * R;
   const bool f32 = m->cfg.inner_prec != DG_PREC_F64;
   if (on_device) DG_CUDA(cudaDeviceSynchronize());
-  DBuf<double> b, x, r, z, zo, p, q, part, sc, cb, cx;
+  // The work blocks come from the pool (about 30 allocations and releases a
+  // solve took as long as the solve); the solution is worked in the caller's
+  // array where that is device memory on a 16-byte boundary.
+  PoolScope scope(s);
+  DBuf<double> xb, r, za, zb, p, q, part, sc, cb, cx;
   DBuf<float> r32, z32;
   DBuf<uint8_t> done;
-  for (DBuf<double>* v : {&b, &x, &r, &z, &zo, &p, &q}) DG_TRY(v->alloc(n));
-  DG_TRY(part.alloc(int64_t(kMvDotBlocks) * R));
-  DG_TRY(sc.alloc(8 * int64_t(R)));  // bb, rz, pq, rr, rzn, rzo, alpha, beta
+  for (DBuf<double>* v : {&r, &za, &p, &q}) DG_TRY(v->alloc(n));
+  if (f32) DG_TRY(zb.alloc(n));  // the flexible direction needs the last z too
+  double* x = X;
+  if (!on_device || (reinterpret_cast<uintptr_t>(X) & 15) != 0) {
+    DG_TRY(xb.alloc(n));
+    x = xb.p;
+  }
+  DG_TRY(part.alloc(2 * int64_t(kMvDotBlocks) * R));
+  DG_TRY(sc.alloc(6 * int64_t(R)));  // bb, rz, pq, rr, rzn, rzo
   DG_TRY(done.alloc(R));
   const int64_t nc = m->lv.back().da->N * int64_t(R);
   DG_TRY(cb.alloc(nc));
@@ -2149,42 +2312,46 @@ dg_status dg_damg_solve_multi(dg_damg* m, const double* B, double* X, int nrhs, 
   } else {
     DG_TRY(alloc_multi_levels<double>(m, R, W64));
   }
-  double* bb = sc.p;
-  double *rz = sc.p + R, *pq = sc.p + 2 * R, *rr = sc.p + 3 * R, *rzn = sc.p + 4 * R, *rzo = sc.p + 5 * R;
-  double *alpha = sc.p + 6 * R, *beta = sc.p + 7 * R;
-  DG_CUDA(cudaMemcpyAsync(b.p, B, 8 * n, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
+  double *bb = sc.p, *rz = sc.p + R, *pq = sc.p + 2 * R, *rr = sc.p + 3 * R, *rzn = sc.p + 4 * R, *rzo = sc.p + 5 * R;
+  double *z = za.p, *zo = zb.p;
+  DG_CUDA(cudaMemcpyAsync(r.p, B, 8 * n, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
   DG_CUDA(cudaMemsetAsync(done.p, 0, R, s));
   DG_CUDA(cudaStreamSynchronize(s));
-  auto dots = [&](const double* u, const double* v, double* out) -> dg_status {
-    mv_dot_partial<<<kMvDotBlocks, 256, 0, s>>>(u, v, N, R, part.p);
-    mv_dot_finish<<<1, 256, 0, s>>>(part.p, kMvDotBlocks, R, out);
+  const int64_t step_rows = 512 / R;  // rows of a CTA's step in the column sums
+  const unsigned gd = unsigned(std::min<int64_t>((N + step_rows - 1) / step_rows, kMvDotBlocks));
+  auto finish = [&](double* out, double* out2) {
+    mv_dot_finish<<<dim3(unsigned(R / 32), out2 ? 2 : 1), 256, 0, s>>>(part.p, int(gd), R, out, out2);
+  };
+  auto dots = [&](const double* u, const double* v, double* out, const double* v2 = nullptr,
+                  double* out2 = nullptr) -> dg_status {
+    mv_dot_partial<<<gd, 256, 0, s>>>(u, v, v2, N, R, part.p, part.p + int64_t(gd) * R);
+    finish(out, out2);
     DG_CUDA(cudaGetLastError());
     return DG_OK;
   };
-  const unsigned g = grid_for(n, 256, 16);
   auto precond = [&]() -> dg_status {
     if (f32) {
-      mv_convert<double, float><<<g, 256, 0, s>>>(r.p, r32.p, n);
+      const unsigned g4 = grid_for(n / 4, 256, 16);
+      mv_convert<double, float><<<g4, 256, 0, s>>>(r.p, r32.p, n / 4);
       DG_TRY(vcycle_multi<float>(m, 0, r32.p, z32.p, R, W32, cb, cx));
-      mv_convert<float, double><<<g, 256, 0, s>>>(z32.p, z.p, n);
+      mv_convert<float, double><<<g4, 256, 0, s>>>(z32.p, z, n / 4);
       DG_CUDA(cudaGetLastError());
       return DG_OK;
     }
-    return vcycle_multi<double>(m, 0, r.p, z.p, R, W64, cb, cx);
+    return vcycle_multi<double>(m, 0, r.p, z, R, W64, cb, cx);
   };
   cudaEvent_t e0, e1;
   DG_CUDA(cudaEventCreate(&e0));
   DG_CUDA(cudaEventCreate(&e1));
   DG_CUDA(cudaEventRecord(e0, s));
-  DG_CUDA(cudaMemsetAsync(x.p, 0, 8 * n, s));
-  DG_CUDA(cudaMemcpyAsync(r.p, b.p, 8 * n, cudaMemcpyDeviceToDevice, s));
-  DG_TRY(dots(b.p, b.p, bb));
+  DG_CUDA(cudaMemsetAsync(x, 0, 8 * n, s));
+  DG_TRY(dots(r.p, r.p, bb));
   std::vector<double> hbb(R), hrr(R);
   std::vector<uint8_t> hdone(R, 0);
   DG_CUDA(cudaMemcpyAsync(hbb.data(), bb, 8 * R, cudaMemcpyDeviceToHost, s));
   DG_TRY(precond());
-  DG_CUDA(cudaMemcpyAsync(p.p, z.p, 8 * n, cudaMemcpyDeviceToDevice, s));
-  DG_TRY(dots(r.p, z.p, rz));
+  DG_CUDA(cudaMemcpyAsync(p.p, z, 8 * n, cudaMemcpyDeviceToDevice, s));
+  DG_TRY(dots(r.p, z, rz));
   const int flexible = f32 ? 1 : 0;
   int it = 0;
   double worst = 1.0;
@@ -2195,10 +2362,9 @@ dg_status dg_damg_solve_multi(dg_damg* m, const double* B, double* X, int nrhs, 
   for (it = 1; it <= m->cfg.maxit; ++it) {
     DG_TRY(mrhs_octet_apply<double>(L0.A.get(), L0.A->coef.p, p.p, q.p, R, s));
     DG_TRY(dots(p.p, q.p, pq));
-    mv_alpha<<<1, 256, 0, s>>>(rz, pq, done.p, alpha, R);
-    mv_axpy<<<g, 256, 0, s>>>(x.p, p.p, alpha, 1.0, n, R);
-    mv_axpy<<<g, 256, 0, s>>>(r.p, q.p, alpha, -1.0, n, R);
-    DG_TRY(dots(r.p, r.p, rr));
+    mv_step<<<gd, 256, 0, s>>>(x, r.p, p.p, q.p, rz, pq, done.p, N, R, part.p);
+    finish(rr, nullptr);
+    DG_CUDA(cudaGetLastError());
     DG_CUDA(cudaMemcpyAsync(hrr.data(), rr, 8 * R, cudaMemcpyDeviceToHost, s));
     DG_CUDA(cudaStreamSynchronize(s));
     worst = 0;
@@ -2216,12 +2382,13 @@ dg_status dg_damg_solve_multi(dg_damg* m, const double* B, double* X, int nrhs, 
       break;
     }
     DG_CUDA(cudaMemcpyAsync(done.p, hdone.data(), R, cudaMemcpyHostToDevice, s));
-    DG_CUDA(cudaMemcpyAsync(zo.p, z.p, 8 * n, cudaMemcpyDeviceToDevice, s));
+    if (flexible) std::swap(z, zo);
     DG_TRY(precond());
-    DG_TRY(dots(r.p, z.p, rzn));
-    if (flexible) DG_TRY(dots(r.p, zo.p, rzo));
-    mv_beta<<<1, 256, 0, s>>>(rzn, rzo, rz, done.p, beta, R, flexible);
-    mv_direction<<<g, 256, 0, s>>>(p.p, z.p, beta, n, R);
+    if (flexible) DG_TRY(dots(r.p, z, rzn, zo, rzo));
+    else DG_TRY(dots(r.p, z, rzn));
+    mv_direction<<<gd, 256, 0, s>>>(p.p, z, rzn, rzo, rz, done.p, flexible, N, R);
+    DG_CUDA(cudaGetLastError());
+    std::swap(rz, rzn);
   }
   DG_CUDA(cudaEventRecord(e1, s));
   DG_CUDA(cudaEventSynchronize(e1));
@@ -2229,7 +2396,8 @@ dg_status dg_damg_solve_multi(dg_damg* m, const double* B, double* X, int nrhs, 
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  DG_CUDA(cudaMemcpyAsync(X, x.p, 8 * n, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
+  if (x != X)
+    DG_CUDA(cudaMemcpyAsync(X, x, 8 * n, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
   DG_CUDA(cudaStreamSynchronize(s));
   if (rep) {
     rep->iterations = it > m->cfg.maxit ? m->cfg.maxit : it;
