@@ -2535,15 +2535,19 @@ static int forced_variant() {
 // untimed launch, then the best of two timed runs; for a mesh that L2 does not
 // hold, each after overwriting a buffer larger than L2.  y is used as scratch and left zero.  Inside a
 // capture an untuned mesh gets the default octet shape.  Timed are the shapes
-// that are fastest on some mesh: the element kernel (small meshes), the octet
-// kernels with the next ids in flight (the others), and the compressed-map
-// kernel where its map has been built; the tile, chunk, lane and quad shapes
-// need tables of their own and were 1.2 to 2 times slower on the benchmark
-// mesh, so they run only when fixed by the caller.
+// that are fastest on some mesh: the element kernel, the octet kernels with the
+// next ids in flight, the compressed-map kernel where its map has been built,
+// and up to kTilesMax elements the warp tiles (their tables are built for that;
+// FP64 / FP32 on the coarse levels of the 1M-point mesh, best tile against best
+// octet shape: 44 / 31 against 36 / 28 us with 1.6M elements, 15.1 / 11.9
+// against 15.5 / 12.8 with 469K, 6.9 / 5.9 against 8.1 / 6.8 with 127K, 4.7 / 4.3
+// against 7.8 / 6.3 with 32K).  The bulk-copy, chunk, lane and quad shapes were
+// 1.2 to 2 times slower on every mesh tried and run only when fixed by the caller.
 constexpr int kDefaultVariant = 28;  // "octet b128, next ids in flight, 4 CTAs/SM"
-static bool variant_timed(int v) {
+constexpr int64_t kTilesMax = int64_t(1) << 20;
+static bool variant_timed(int v, int64_t E) {
   const int k = kVariants[v].kind;
-  return k == 0 || k == 6 || k == 12 || k == 13 || k >= 15;
+  return k == 0 || k == 6 || k == 12 || k == 13 || k >= 15 || (k >= 2 && k <= 4 && E <= kTilesMax);
 }
 template <class T, class CT>
 static dg_status pick_variant(dg_da* da, int& choice, const CT* ca, const CT* cb, const T* x, T* y,
@@ -2565,34 +2569,36 @@ static dg_status pick_variant(dg_da* da, int& choice, const CT* ca, const CT* cb
     DG_CUDA(cudaEventCreate(&e1));
     // a mesh that stays in L2 between applications is timed there
     const int64_t flush_bytes = da->E * 64 > (int64_t(64) << 20) ? int64_t(192) << 20 : 0;
+    if (da->E <= kTilesMax) DG_TRY(ensure_tiles(da, s));
     PoolScope scope(s);
     DBuf<uint8_t> flush;
     DG_TRY(flush.alloc(flush_bytes));
     // A mesh in L2 is timed over several launches, queued before the first is
     // done: with one launch between the events, the host's own time to launch
     // it counts (a 45 MB mesh got a shape twice as slow as the best).
-    const int reps = flush_bytes ? 1 : 8;
+    const int reps = flush_bytes ? 1 : 4;
     float best = 1e30f;
     int bi = kDefaultVariant;
     DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
     for (int v = 0; v < kNumVariants; ++v) {
-      if (!variant_timed(v) || !variant_runs(kVariants[v].kind, da)) continue;
+      if (!variant_timed(v, da->E) || !variant_runs(kVariants[v].kind, da)) continue;
       DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));  // untimed: loads the kernel
       for (int trial = 0; trial < 2; ++trial) {
         if (flush_bytes) DG_CUDA(cudaMemsetAsync(flush.p, trial + 1, flush_bytes, s));
         DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
-        if (!flush_bytes)
-          for (int r = 0; r < 2; ++r) DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));
+        if (!flush_bytes) DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));
         DG_CUDA(cudaEventRecord(e0, s));
         for (int r = 0; r < reps; ++r) DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));
         DG_CUDA(cudaEventRecord(e1, s));
         DG_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
         DG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        const bool out = ms > 1.5f * best;  // no second run for a shape that is far off
         if (ms < best) {
           best = ms;
           bi = v;
         }
+        if (out) break;
       }
     }
     cudaEventDestroy(e0);
