@@ -722,11 +722,31 @@ __global__ void finish_sum(const double* __restrict__ part, int np, double* __re
   v = block_sum(v);
   if (threadIdx.x == 0) *out = v;
 }
+// The same in the kernel that made the partial sums, by its last CTA: each CTA
+// takes a ticket when its sum is written, and the one with the last ticket adds
+// them up, in finish_sum's order.  *ticket is zero before and after.
+__device__ __forceinline__ void finish_last(double v, double* __restrict__ part, double* __restrict__ out,
+                                            uint32_t* __restrict__ ticket) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = v;
+    __threadfence();
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    double t = 0;
+    for (int i = threadIdx.x; i < int(gridDim.x); i += blockDim.x) t += reinterpret_cast<volatile double*>(part)[i];
+    t = block_sum(t);
+    if (threadIdx.x == 0) *out = t;
+  }
+}
 // The FP64 vector kernels of the outer CG read 16-byte pairs (the solver's
 // vectors are whole allocations, so 16-byte aligned); an odd last element is
 // handled by thread 0.
 __global__ void dot_partial(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
-                            double* __restrict__ part) {
+                            double* __restrict__ part, double* __restrict__ out, uint32_t* __restrict__ ticket) {
   const double2* a2 = reinterpret_cast<const double2*>(a);
   const double2* b2 = reinterpret_cast<const double2*>(b);
   const int64_t n2 = n / 2;
@@ -739,7 +759,8 @@ __global__ void dot_partial(const double* __restrict__ a, const double* __restri
   }
   if (gtid() == 0 && (n & 1)) v0 = fma(a[n - 1], b[n - 1], v0);
   const double v = block_sum(v0 + v1);
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
+  if (out) finish_last(v, part, out, ticket);
+  else if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
 // the same for arrays of any alignment (caller-provided vectors)
 __global__ void dot_partial_any(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
@@ -750,20 +771,23 @@ __global__ void dot_partial_any(const double* __restrict__ a, const double* __re
   const double v = block_sum(v0);
   if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
-// x += alpha p; r -= alpha q; partial (r, r); alpha = num / den read on device
+// x += alpha p; r -= alpha q; (r, r) and, with z, (r, z) of the new r; alpha =
+// num / den read on device
 __global__ void cg_update(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
-                          const double* __restrict__ q, int64_t n, const double* __restrict__ num,
-                          const double* __restrict__ den, double* __restrict__ part) {
+                          const double* __restrict__ q, const double* __restrict__ z, int64_t n,
+                          const double* __restrict__ num, const double* __restrict__ den, double* __restrict__ part,
+                          double* __restrict__ rr, double* __restrict__ rz, uint32_t* __restrict__ ticket) {
   const double alpha = *num / *den;
   double2* x2 = reinterpret_cast<double2*>(x);
   double2* r2 = reinterpret_cast<double2*>(r);
   const double2* p2 = reinterpret_cast<const double2*>(p);
   const double2* q2 = reinterpret_cast<const double2*>(q);
+  const double2* z2 = reinterpret_cast<const double2*>(z);
   const int64_t n2 = n / 2, S = gstride();
-  double v0 = 0, v1 = 0;
+  double v0 = 0, v1 = 0, w0 = 0, w1 = 0;
   constexpr int U = 4;  // steps per thread, all loads first
   for (int64_t i0 = gtid(); i0 < n2; i0 += S * U) {
-    double2 xi[U], ri[U], pi[U], qi[U];
+    double2 xi[U], ri[U], pi[U], qi[U], zi[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t i = i0 + u * S;
@@ -772,6 +796,7 @@ __global__ void cg_update(double* __restrict__ x, double* __restrict__ r, const 
         ri[u] = r2[i];
         pi[u] = p2[i];
         qi[u] = q2[i];
+        if (z) zi[u] = z2[i];
       }
     }
 #pragma unroll
@@ -786,6 +811,10 @@ __global__ void cg_update(double* __restrict__ x, double* __restrict__ r, const 
       r2[i] = ri[u];
       v0 = fma(ri[u].x, ri[u].x, v0);
       v1 = fma(ri[u].y, ri[u].y, v1);
+      if (z) {
+        w0 = fma(ri[u].x, zi[u].x, w0);
+        w1 = fma(ri[u].y, zi[u].y, w1);
+      }
     }
   }
   if (gtid() == 0 && (n & 1)) {
@@ -793,9 +822,15 @@ __global__ void cg_update(double* __restrict__ x, double* __restrict__ r, const 
     const double rl = r[n - 1] - alpha * q[n - 1];
     r[n - 1] = rl;
     v0 = fma(rl, rl, v0);
+    if (z) w0 = fma(rl, z[n - 1], w0);
   }
   const double v = block_sum(v0 + v1);
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
+  finish_last(v, part, rr, ticket);
+  if (z) {
+    __syncthreads();
+    const double w = block_sum(w0 + w1);
+    finish_last(w, part + gridDim.x, rz, ticket + 1);
+  }
 }
 // p = z + beta p on 16-byte pairs
 __device__ __forceinline__ void axpby_pairs(double* __restrict__ p, const double* __restrict__ z, int64_t n,
@@ -881,7 +916,8 @@ struct dg_damg {
   bool mlp_active = false;
   DBuf<float> sm_s2;
   // PCG work vectors on the finest level and device scalars
-  DBuf<double> r, z, zold, p, q, part, scal;
+  DBuf<double> r, z, p, q, part, scal;
+  DBuf<uint32_t> ticket;  // of the reductions that end in their last CTA, zero between launches
   DBuf<float> r32, z32;
   cudaStream_t s = nullptr;
   // captured preconditioner, one per post-smoother (0 Jacobi, 1 learned), so
@@ -1445,9 +1481,11 @@ dg_status ensure_smoother_data(dg_damg* m) {
   return DG_OK;
 }
 
+// CTAs of a reduction over n values: fewer where each has less than a step
+unsigned red_blocks(int64_t n) { return unsigned(std::min<int64_t>(kRedBlocks, (n + 511) / 512 > 0 ? (n + 511) / 512 : 1)); }
+
 dg_status dot(dg_damg* m, const double* a, const double* b, int64_t n, double* out) {
-  dot_partial<<<kRedBlocks, 256, 0, m->s>>>(a, b, n, m->part.p);
-  finish_sum<<<1, 256, 0, m->s>>>(m->part.p, kRedBlocks, out);
+  dot_partial<<<red_blocks(n), 256, 0, m->s>>>(a, b, n, m->part.p, out, m->ticket.p);
   DG_CUDA(cudaGetLastError());
   return DG_OK;
 }
@@ -1531,12 +1569,13 @@ dg_status finish_create(dg_damg* m) {
   DG_TRY(m->z.alloc(N));
   DG_TRY(m->p.alloc(N));
   DG_TRY(m->q.alloc(N));
-  DG_TRY(m->zold.alloc(N));
   if (m->cfg.inner_prec != DG_PREC_F64) {
     DG_TRY(m->r32.alloc(N));
     DG_TRY(m->z32.alloc(N));
   }
-  DG_TRY(m->part.alloc(kRedBlocks));
+  DG_TRY(m->part.alloc(2 * kRedBlocks));
+  DG_TRY(m->ticket.alloc(2));
+  DG_CUDA(cudaMemsetAsync(m->ticket.p, 0, 8, m->s));
   DG_TRY(m->scal.alloc(8));
   DG_TRY(m->d_node_off.alloc(m->nmesh + 1));
   DG_TRY(m->mesh_part.alloc(int64_t(m->nmesh) * (1 + kSegBlocks)));
@@ -1821,7 +1860,9 @@ dg_status dg_damg_solve(dg_damg* m, const double* b, double* x, int on_device, d
   DG_CUDA(cudaEventCreate(&e0));
   DG_CUDA(cudaEventCreate(&e1));
   DG_CUDA(cudaEventRecord(e0, s));
-  double* sc = m->scal.p;  // [0] bb, [1] rz, [2] pq, [3] rr, [4] rz_new
+  // [0] bb, [2] pq, [3] rr, [5] (r, z_old); rz and the new rz change places
+  double* sc = m->scal.p;
+  double *rz = sc + 1, *rzn = sc + 4;
   DG_CUDA(cudaMemsetAsync(px, 0, 8 * n, s));
   DG_CUDA(cudaMemcpyAsync(m->r.p, pb, 8 * n, cudaMemcpyDeviceToDevice, s));
   DG_TRY(dot(m, pb, pb, n, sc + 0));
@@ -1851,12 +1892,14 @@ dg_status dg_damg_solve(dg_damg* m, const double* b, double* x, int on_device, d
   if (!conv) {
     DG_TRY(precond(m));
     DG_CUDA(cudaMemcpyAsync(m->p.p, m->z.p, 8 * n, cudaMemcpyDeviceToDevice, s));
-    DG_TRY(dot(m, m->r.p, m->z.p, n, sc + 1));
+    DG_TRY(dot(m, m->r.p, m->z.p, n, rz));
     for (it = 1; it <= m->cfg.maxit; ++it) {
       DG_TRY(level_op(L, m->p.p, m->q.p, s));
       DG_TRY(dot(m, m->p.p, m->q.p, n, sc + 2));
-      cg_update<<<kRedBlocks, 256, 0, s>>>(px, m->r.p, m->p.p, m->q.p, n, sc + 1, sc + 2, m->part.p);
-      finish_sum<<<1, 256, 0, s>>>(m->part.p, kRedBlocks, sc + 3);
+      // the flexible direction's (r, z_old) while z still holds the last z
+      cg_update<<<red_blocks(n), 256, 0, s>>>(px, m->r.p, m->p.p, m->q.p, flexible ? m->z.p : nullptr, n, rz, sc + 2,
+                                              m->part.p, sc + 3, sc + 5, m->ticket.p);
+      DG_CUDA(cudaGetLastError());
       if (nm > 1) {
         DG_TRY(mesh_norms(m->r.p, rr));
         rel = 0;
@@ -1864,8 +1907,9 @@ dg_status dg_damg_solve(dg_damg* m, const double* b, double* x, int on_device, d
           if (bb[i] > 0) rel = std::max(rel, std::sqrt(rr[i] / bb[i]));
       } else {
         double hr = 0;
-        DG_CUDA(cudaMemcpyAsync(&hr, sc + 3, 8, cudaMemcpyDeviceToHost, s));
-        DG_CUDA(cudaStreamSynchronize(s));
+        uint32_t hw[2];
+        DG_TRY(read_words(reinterpret_cast<const uint32_t*>(sc + 3), hw, 2, s));
+        memcpy(&hr, hw, 8);
         rel = std::sqrt(hr) / bnorm;
       }
       if (!(rel == rel)) break;  // NaN: stop and report
@@ -1880,16 +1924,12 @@ dg_status dg_damg_solve(dg_damg* m, const double* b, double* x, int on_device, d
         ++fallbacks;
       }
       prev_rel = rel;
-      if (flexible) DG_CUDA(cudaMemcpyAsync(m->zold.p, m->z.p, 8 * n, cudaMemcpyDeviceToDevice, s));
       DG_TRY(precond(m));
-      DG_TRY(dot(m, m->r.p, m->z.p, n, sc + 4));
-      if (flexible) {
-        DG_TRY(dot(m, m->r.p, m->zold.p, n, sc + 5));
-        cg_direction_flex<<<g, 256, 0, s>>>(m->p.p, m->z.p, n, sc + 4, sc + 5, sc + 1);
-      } else {
-        cg_direction<<<g, 256, 0, s>>>(m->p.p, m->z.p, n, sc + 4, sc + 1);
-      }
-      DG_CUDA(cudaMemcpyAsync(sc + 1, sc + 4, 8, cudaMemcpyDeviceToDevice, s));
+      DG_TRY(dot(m, m->r.p, m->z.p, n, rzn));
+      if (flexible) cg_direction_flex<<<g, 256, 0, s>>>(m->p.p, m->z.p, n, rzn, sc + 5, rz);
+      else cg_direction<<<g, 256, 0, s>>>(m->p.p, m->z.p, n, rzn, rz);
+      DG_CUDA(cudaGetLastError());
+      std::swap(rz, rzn);
     }
   }
   DG_CUDA(cudaEventRecord(e1, s));
@@ -2415,7 +2455,7 @@ dg_status dg_vec_dot(const double* x, const double* y, int64_t n, double* result
   DBuf<double> part;  // one partial sum per reduction block
   DG_TRY(part.alloc(kRedBlocks));
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0)
-    dot_partial<<<kRedBlocks, 256, 0, s>>>(x, y, n, part.p);
+    dot_partial<<<kRedBlocks, 256, 0, s>>>(x, y, n, part.p, nullptr, nullptr);
   else
     dot_partial_any<<<kRedBlocks, 256, 0, s>>>(x, y, n, part.p);
   finish_sum<<<1, 256, 0, s>>>(part.p, kRedBlocks, result);
