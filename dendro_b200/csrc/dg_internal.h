@@ -2,6 +2,7 @@
 #pragma once
 
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "dg_common.cuh"
@@ -110,6 +111,9 @@ struct dg_da {
   dg::CompressedMap cmap;  // compressed element map (on request)
   // operator launch shape picked by the autotuner on first use (-1: not yet)
   int tuned_f64 = -1, tuned_f32 = -1;
+  // held while a table is built on first use: threads may share a mesh, each
+  // with its own operators and streams
+  std::mutex tables;
 };
 
 struct dg_mlp {

@@ -2536,7 +2536,7 @@ static int forced_variant() {
 // hold, each after overwriting a buffer larger than L2.  y is used as scratch and left zero.  Inside a
 // capture an untuned mesh gets the default octet shape.  Timed are the shapes
 // that are fastest on some mesh: the element kernel, the octet kernels with the
-// next ids in flight, the compressed-map kernel where its map has been built,
+// lattice in registers, the compressed-map kernel where its map has been built,
 // and up to kTilesMax elements the warp tiles (their tables are built for that;
 // FP64 / FP32 on the coarse levels of the 1M-point mesh, best tile against best
 // octet shape: 44 / 31 against 36 / 28 us with 1.6M elements, 15.1 / 11.9

@@ -918,6 +918,7 @@ dg_status build_tile_set(const dg_da* da, int te, TileSet& ts, cudaStream_t s) {
 }
 
 dg_status ensure_tiles(dg_da* da, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(da->tables);
   if (da->tiles_w.ntiles) return DG_OK;
   PoolScope scope(s);
   DG_TRY(build_tile_set(da, kWarpTile, da->tiles_w, s));

@@ -392,6 +392,7 @@ dg_status build_octets(dg_da* da, cudaStream_t s) {
 }
 
 dg_status ensure_octet_records(dg_da* da, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(da->tables);
   OctetSet& O = da->octs;
   if (O.rec.n || !O.n) return DG_OK;
   PoolScope scope(s);
@@ -403,6 +404,7 @@ dg_status ensure_octet_records(dg_da* da, cudaStream_t s) {
 }
 
 dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(da->tables);
   if (da->octs.chunks_tried || !da->octs.n) return DG_OK;
   PoolScope scope(s);
   DG_TRY(build_chunks(da, s));

@@ -210,6 +210,7 @@ dg_status build(dg_da* da, cudaStream_t s) {
 }  // namespace
 
 dg_status ensure_octet_tiles(dg_da* da, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(da->tables);
   if (da->otiles.tried || !da->octs.n) return DG_OK;
   PoolScope scope(s);
   DG_TRY(build(da, s));

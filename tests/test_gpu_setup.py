@@ -68,6 +68,41 @@ def test_set_up_in_several_threads(gpu, oracle):
     assert not bad
 
 
+def test_first_use_of_a_mesh_in_several_threads(gpu):
+    """Threads that share a new mesh, each with its own operators and stream, all find its tables built once."""
+    import torch
+    da = gpu.DA(gpu.balanceOctree(gpu.points2Octree(I.clamp_unit(I.gaussian_cloud(20000, 3), 10), 10, 1)))
+    one = gpu.DA(gpu.balanceOctree(gpu.points2Octree(I.clamp_unit(I.gaussian_cloud(20000, 3), 10), 10, 1)))
+    x = torch.rand(da.N, dtype=torch.float64, device="cuda")
+    x3 = torch.rand(3 * da.N, dtype=torch.float64, device="cuda")
+    X = torch.rand(da.N, 64, dtype=torch.float32, device="cuda")
+
+    def forms(d):
+        st = torch.cuda.current_stream()
+        e, J = gpu.Elasticity(d, 0.4, 0.6), gpu.Jacobian2(d)
+        return [J.mult(x, stream=st), e.mult(x3, stream=st), J.mult_multi(X, split=5, stream=st)]
+
+    want = forms(one)
+    torch.cuda.synchronize()
+    start = threading.Barrier(4)
+    got = [None] * 4
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            start.wait()
+            got[i] = forms(da)
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for g in got:
+        for a, b, tol in zip(g, want, (1e-13, 1e-13, 1e-5)):
+            assert (a - b).abs().max() <= tol * b.abs().max()
+
+
 def test_levels_of_a_batch_have_octets(gpu, oracle):
     """Every octet launch shape on a batch's concatenated mesh, against the meshes one by one."""
     import torch
