@@ -611,58 +611,96 @@ __global__ void dense_gemv(const double* __restrict__ A, int64_t N, const uint32
 
 // x += Ainv b for one symmetric block, from its lower triangle: an entry a_ij
 // below the diagonal serves row i (a_ij b_j) and row j (a_ij b_i), so half of the
-// matrix is never read: one V-cycle of the 131,072-point configuration reads
-// its 17,845 x 17,845 inverse (2.5 GB, 573 us with a warp per row at 4.4 TB/s)
-// as 1.3 GB.  A CTA takes kSymRows rows up to the diagonal (the longest rows
-// first), its warps 32 columns of every 256 with a column per lane: the column
-// sums over the CTA's rows stay in a lane and leave with one reduction per
-// column, the row sums stay in registers to the end.  The next columns' loads
-// are in flight meanwhile.  (Square tiles of 128 rows, which need fewer
-// reductions, took 470 us: 128 rows are 18 MB apart, more pages than the
-// translation caches hold.)
-constexpr int kSymRows = 16;
-constexpr int64_t kSymFrom = 3000;  // rows from which the matrix (72 MB) leaves L2 between cycles
-__global__ void __launch_bounds__(256, 2) dense_symv(const double* __restrict__ A, int64_t n,
-                                                     const double* __restrict__ b, double* __restrict__ x) {
-  __shared__ double bi[kSymRows], rs[8][kSymRows];
+// matrix is never read.  The triangle is packed once, when the inverse is made:
+// strips of kSymRows rows, in each the blocks of 32 columns up to the diagonal
+// one after another, 4 KB apiece.  Bound by HBM: one V-cycle of the
+// 131,072-point configuration reads its 17,845 x 17,845 inverse (2.5 GB, 573 us
+// with a warp per row at 4.4 TB/s) as 1.27 GB in 180 us (7.1 TB/s); from the
+// rows of the full matrix, 16 rows of 143 KB apart at a time, it took 316 us.
+// A CTA takes a strip (the longest first), each warp every eighth block with a
+// column per lane: the column's sum over the strip leaves with one reduction,
+// the row sums stay in registers to the end.  A warp's next two blocks are on
+// their way into its own slots by 16-byte cp.async, 192 KB per SM, without a
+// block barrier.  (Blocks in registers, one ahead: 240 us; 32 rows: 184 us.)
+constexpr int kSymRows = 16, kSymWarps = 8, kSymStages = 3;
+constexpr int kSymBlock = 32 * kSymRows;  // values
+constexpr int kSymSmem = kSymWarps * kSymStages * kSymBlock * int(sizeof(double));
+// Rows from which it is used: there the full matrix (72 MB) no longer stays in
+// L2 between cycles.  A warp per row of it, against clearing x and this: 10.2
+// and 11.1 us for 1,000 rows, 14.2 and 15.2 for 3,001 (both in L2), 38.9 and
+// 19.5 for 4,000, 467 and 183 for 17,845.
+constexpr int64_t kSymFrom = 3000;
+__host__ __device__ inline int64_t sym_blocks(int64_t s) { return (s + 2) / 2; }  // of strip s
+__host__ __device__ inline int64_t sym_first(int64_t s) {                         // blocks before strip s
+  const int64_t h = s / 2;
+  return (h + (s & 1)) * (h + 1);
+}
+static_assert(kSymRows == 16, "sym_blocks and sym_first hold for 16 rows against 32 columns");
+__global__ void sym_pack(const double* __restrict__ A, int64_t n, double* __restrict__ P) {
+  const int64_t s = blockIdx.x;
+  double* o = P + sym_first(s) * kSymBlock;
+  const int64_t m = sym_blocks(s) * kSymBlock;
+  for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
+    const int64_t i = s * kSymRows + (k >> 5) % kSymRows, j = 32 * (k / kSymBlock) + (k & 31);
+    o[k] = i < n && j <= i ? A[i * n + j] : 0.0;
+  }
+}
+__global__ void __launch_bounds__(32 * kSymWarps, 2) dense_symv(const double* __restrict__ P, int64_t n,
+                                                                const double* __restrict__ b, double* __restrict__ x) {
+  extern __shared__ __align__(16) double sym_slots[];
+  __shared__ double bi[kSymRows], rs[kSymWarps][kSymRows];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int64_t i0 = (int64_t(gridDim.x) - 1 - blockIdx.x) * kSymRows;
-  const int64_t i1 = i0 + kSymRows < n ? i0 + kSymRows : n;  // one past the last row
+  const int64_t strip = int64_t(gridDim.x) - 1 - blockIdx.x, i0 = strip * kSymRows;
+  const int64_t nb = sym_blocks(strip);
   if (tid < kSymRows) bi[tid] = i0 + tid < n ? b[i0 + tid] : 0.0;
   __syncthreads();
-  const double* A0 = A + i0 * n;
-  double row[kSymRows], a[kSymRows], an[kSymRows];
+  const char* src = reinterpret_cast<const char*>(P + sym_first(strip) * kSymBlock) + 16 * lane;
+  double* slots = sym_slots + w * kSymStages * kSymBlock;
+  auto get = [&](int64_t k, int st) {
+    if (k < nb) {
+      const uint32_t d = uint32_t(__cvta_generic_to_shared(slots + st * kSymBlock)) + 16 * lane;
+      const char* p = src + k * (kSymBlock * 8);
 #pragma unroll
-  for (int r = 0; r < kSymRows; ++r) row[r] = an[r] = 0.0;
-  auto load = [&](double (&v)[kSymRows], int64_t j) {  // column j of the rows, up to the diagonal
-    if (j <= i0) {
-#pragma unroll
-      for (int r = 0; r < kSymRows; ++r) v[r] = i0 + r < i1 ? __ldg(A0 + int64_t(r) * n + j) : 0.0;
-    } else {
-#pragma unroll
-      for (int r = 0; r < kSymRows; ++r) v[r] = i0 + r < i1 && j <= i0 + r ? __ldg(A0 + int64_t(r) * n + j) : 0.0;
+      for (int q = 0; q < kSymBlock * 8; q += 512)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + q), "l"(p + q) : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  int64_t j = 32 * w + lane;
-  load(an, j);
-  for (; j - lane < i1; j += 256) {
+  double row[kSymRows];
 #pragma unroll
-    for (int r = 0; r < kSymRows; ++r) a[r] = an[r];
-    load(an, j + 256);
-    const double xj = j < i1 ? __ldg(b + j) : 0.0;
+  for (int r = 0; r < kSymRows; ++r) row[r] = 0.0;
+#pragma unroll
+  for (int t = 0; t < kSymStages - 1; ++t) get(w + t * kSymWarps, t);
+  int st = 0;
+  for (int64_t k = w; k < nb; k += kSymWarps) {
+    __syncwarp();  // the slot that is filled next has been read by every lane
+    get(k + (kSymStages - 1) * kSymWarps, (st + kSymStages - 1) % kSymStages);
+    const int64_t j = 32 * k + lane;
+    const double xj = j < n ? __ldg(b + j) : 0.0;
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSymStages - 1) : "memory");
+    __syncwarp();  // the other lanes' copies too
+    const double* a = slots + st * kSymBlock + lane;
     double col = 0.0;
+    if (32 * k + 32 <= i0) {
 #pragma unroll
-    for (int r = 0; r < kSymRows; ++r) {
-      row[r] = fma(a[r], xj, row[r]);
-      col = fma(a[r], bi[r], col);
-    }
-    if (j >= i0 && j < i1) {  // the diagonal entry counts once
+      for (int r = 0; r < kSymRows; ++r) {
+        const double v = a[32 * r];
+        row[r] = fma(v, xj, row[r]);
+        col = fma(v, bi[r], col);
+      }
+      atomicAdd(x + j, col);
+    } else {  // the diagonal, whose entry counts once, and nothing beyond it
 #pragma unroll
-      for (int r = 0; r < kSymRows; ++r)
-        if (j == i0 + r) col -= a[r] * bi[r];
+      for (int r = 0; r < kSymRows; ++r) {
+        const double v = a[32 * r];
+        if (j <= i0 + r) row[r] = fma(v, xj, row[r]);
+        if (j < i0 + r) col = fma(v, bi[r], col);
+      }
+      if (j < n && j < i0 + kSymRows) atomicAdd(x + j, col);
     }
-    if (j < i1) atomicAdd(x + j, col);
+    st = (st + 1) % kSymStages;
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
   for (int r = 0; r < kSymRows; ++r) {
 #pragma unroll
@@ -673,7 +711,7 @@ __global__ void __launch_bounds__(256, 2) dense_symv(const double* __restrict__ 
   if (tid < kSymRows && i0 + tid < n) {
     double s = 0.0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) s += rs[k][tid];
+    for (int k = 0; k < kSymWarps; ++k) s += rs[k][tid];
     atomicAdd(x + i0 + tid, s);
   }
 }
@@ -899,6 +937,7 @@ struct dg_damg {
   dg_damg_config cfg;
   std::vector<Level> lv;
   DBuf<double> Ainv;  // dense inverses of the coarsest operator, one block per mesh
+  DBuf<double> Asym;  // one large block's lower triangle, packed (dense_symv)
   int64_t nc = 0;
   // block structure of the coarsest level (one block per independent mesh)
   std::vector<int64_t> cb_off, cb_n, cb_aoff;
@@ -941,9 +980,9 @@ namespace {
 // x = the coarsest level's dense inverse times b (FP64).
 dg_status coarse_solve(const dg_damg* m, const double* b, double* x, cudaStream_t s) {
   const int64_t n = m->nc;
-  if (m->cb_n.size() == 1 && n >= kSymFrom) {
+  if (m->Asym.n) {
     DG_CUDA(cudaMemsetAsync(x, 0, 8 * n, s));
-    dense_symv<<<unsigned((n + kSymRows - 1) / kSymRows), 256, 0, s>>>(m->Ainv.p, n, b, x);
+    dense_symv<<<unsigned((n + kSymRows - 1) / kSymRows), 32 * kSymWarps, kSymSmem, s>>>(m->Asym.p, n, b, x);
   } else {
     dense_gemv<<<grid_for(n * 32, 256), 256, 0, s>>>(m->Ainv.p, n, m->d_crow_blk.p, m->d_cb_off.p, m->d_cb_n.p,
                                                      m->d_cb_aoff.p, b, x);
@@ -1108,6 +1147,7 @@ __global__ void fill_row_blk(uint32_t* __restrict__ rb, int64_t n0, int64_t n1, 
 constexpr int64_t kMaxCoarseNodes = 32768;
 constexpr int64_t kGjBlockedFrom = 1024;
 dg_status gj_invert(dg_damg* m, int64_t maxn, int nb);
+dg_status pack_inverse(dg_damg* m);
 
 dg_status setup_coarse(dg_damg* m) {
   Level& L = m->lv.back();
@@ -1130,7 +1170,8 @@ dg_status setup_coarse(dg_damg* m) {
     DG_CUDA(cudaMemcpyAsync(m->d_cb_aoff.p, m->cb_aoff.data(), 8, cudaMemcpyHostToDevice, m->s));
     DG_CUDA(cudaMemsetAsync(m->d_crow_blk.p, 0, 4 * n3, m->s));
     DG_TRY(elasticity_assemble_dense(L.A.get(), m->Ainv.p, m->s));
-    return gj_invert(m, n3, 1);
+    DG_TRY(gj_invert(m, n3, 1));
+    return pack_inverse(m);
   }
   const int64_t N = L.da->N;
   const std::vector<int64_t>& noff = m->mesh_node_off.back();
@@ -1160,7 +1201,8 @@ dg_status setup_coarse(dg_damg* m) {
     fill_row_blk<<<grid_for(m->cb_n[b], 256), 256, 0, m->s>>>(m->d_crow_blk.p, noff[b], noff[b + 1], uint32_t(b));
   DG_TRY(lapmass_assemble_dense(L.A.get(), m->Ainv.p, total, m->d_crow_blk.p, m->d_cb_off.p, m->d_cb_n.p,
                                 m->d_cb_aoff.p, m->s, L.jcoef(), L.jset()));
-  return gj_invert(m, maxn, nb);
+  DG_TRY(gj_invert(m, maxn, nb));
+  return pack_inverse(m);
 }
 
 // The dense inverse of the coarsest operator in m->Ainv: the blocked sweep
@@ -1176,6 +1218,22 @@ dg_status gj_invert(dg_damg* m, int64_t maxn, int nb) {
     gj_row<<<g1, 256, 0, m->s>>>(m->Ainv.p, m->d_cb_n.p, m->d_cb_aoff.p, k, colk.p, m->d_cb_off.p);
     gj_elim<<<g2, 256, 0, m->s>>>(m->Ainv.p, m->d_cb_n.p, m->d_cb_aoff.p, k, colk.p, m->d_cb_off.p);
   }
+  DG_CUDA(cudaGetLastError());
+  DG_CUDA(cudaStreamSynchronize(m->s));
+  return DG_OK;
+}
+
+// The packed triangle of one large inverse; without the memory for it (half
+// as much again) the coarse solve reads the full matrix.
+dg_status pack_inverse(dg_damg* m) {
+  if (m->cb_n.size() != 1 || m->nc < kSymFrom) return DG_OK;
+  const int64_t strips = (m->nc + kSymRows - 1) / kSymRows;
+  if (m->Asym.alloc(sym_first(strips) * kSymBlock) != DG_OK) {
+    m->Asym.reset();
+    return DG_OK;
+  }
+  DG_CUDA(cudaFuncSetAttribute(dense_symv, cudaFuncAttributeMaxDynamicSharedMemorySize, kSymSmem));
+  sym_pack<<<unsigned(strips), 256, 0, m->s>>>(m->Ainv.p, m->nc, m->Asym.p);
   DG_CUDA(cudaGetLastError());
   DG_CUDA(cudaStreamSynchronize(m->s));
   return DG_OK;

@@ -64,3 +64,22 @@ def test_infinity_stays_in_its_elements(gpu, oracle):
     X = torch.tensor(np.repeat(x[:, None], 112, 1), dtype=torch.float32, device="cuda")
     Y = A.mult_multi(X).cpu().numpy()
     assert np.isfinite(Y[~reach]).all()
+
+
+# the packed triangle of a large dense inverse: strips of 16 rows, blocks of 32 columns, the last ones cut short
+# (3115, 4071, 5728 and 5244 nodes)
+@pytest.mark.parametrize("n", [600, 900, 1200, 1300])
+def test_large_dense_coarse_solve(gpu, n):
+    import torch
+    from dendro_b200._lib import check, lib, ptr
+    tree = gpu.balanceOctree(gpu.points2Octree(I.clamp_unit(I.gaussian_cloud(n, n), 8), 8, 1))
+    m = gpu.DAMG(tree, nlevels=1)
+    m.setKSP()
+    da = m.level_da(0)
+    assert da.N >= 3000
+    b = torch.from_numpy(np.random.default_rng(n).uniform(-1, 1, da.N)).cuda()
+    x = torch.empty_like(b)
+    check(lib().dg_damg_coarse_solve(m.h, ptr(b), ptr(x), None), "damg_coarse_solve")
+    r = b - gpu.Jacobian2(da).mult(x)
+    torch.cuda.synchronize()
+    assert float(r.norm() / b.norm()) < 1e-9  # rounding times the matrix's condition (h from 1 to 1/256)
