@@ -18,7 +18,7 @@ namespace {
 
 constexpr int kRC = 16;  // right-hand sides come in multiples of this
 
-// A group of G lanes (32, or 16 for the last 16 right-hand sides) per octet
+// FP64: a group of G lanes (32, or 16 for the last 16 right-hand sides) per octet
 // and G right-hand sides, one lane per right-hand side.  Each lane holds its
 // column's 27 lattice values of the octet in registers and runs the octet
 // arithmetic of the scalar kernel (octet_apply: hanging points, the children's
@@ -126,43 +126,53 @@ __device__ __forceinline__ F2 operator-(F2 a, F2 b) {
 }
 __device__ __forceinline__ bool nonzero(F2 a) { return (a.v & 0x7fffffff7fffffffull) != 0ull; }
 
-// The octet form with two right-hand sides per lane (64 per warp): X rows
-// read as 8-byte pairs, Y rows added with 8-byte vector reductions, the
-// element arithmetic on packed pairs.  Works the first 64 nb columns (R even).
+// The octet form with two right-hand sides per lane and G lanes per octet: X
+// rows read as 8-byte pairs, Y rows added with 8-byte vector reductions, the
+// element arithmetic on packed pairs.  Works nb blocks of 2 G columns from
+// column col0 on (R and col0 even), G = 32, 16 or 8: with fewer lanes per octet
+// a warp works 2 or 4 octets at once, whose missing children and hanging points
+// differ, but at half the instructions per right-hand side.  Bound by their
+// issue.  On the 2.9M-element benchmark mesh, against one right-hand side per
+// lane: 32 columns 634 and 817 us, 16 columns 330 and 444, 48 columns 989 and
+// 1261; 64 columns 1138.
+template <int G>
 __global__ void __launch_bounds__(128) mrhs_octet_pair_kernel(int64_t n, const uint32_t* __restrict__ ometa,
                                                               const uint32_t* __restrict__ oid,
                                                               const uint32_t* __restrict__ oelem,
                                                               const float* __restrict__ ca,
-                                                              const float* __restrict__ cb, int R, int nb,
+                                                              const float* __restrict__ cb, int R, int col0, int nb,
                                                               const float* __restrict__ X, float* __restrict__ Y) {
-  __shared__ uint32_t slot[4][2][kMoWords];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr int S = 32 / G;  // groups per warp
+  __shared__ uint32_t slot[4 * S][2][kMoWords];
+  const int gl = threadIdx.x % G, grp = threadIdx.x / G;
   const int64_t tasks = n * nb;
-  const int64_t wstride = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  const int64_t stride = (int64_t(gridDim.x) * blockDim.x) / G;
   auto fetch = [&](int64_t t, int sl) {
     if (t < tasks) {
       const int64_t o = t / nb;
-      for (int k = lane; k < kMoWords; k += 32) {
+      for (int k = gl; k < kMoWords; k += G) {
         const uint32_t* src = k < 27 ? oid + int64_t(k) * n + o : k == 27 ? ometa + o : oelem + int64_t(k - 28) * n + o;
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
-                         static_cast<uint32_t>(__cvta_generic_to_shared(&slot[w][sl][k]))),
+                         static_cast<uint32_t>(__cvta_generic_to_shared(&slot[grp][sl][k]))),
                      "l"(src)
                      : "memory");
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  int64_t t = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+  // tw: the task of the warp's first group, the same for all its lanes
+  int64_t t = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / G, tw = t - grp % S;
   fetch(t, 0);
-  for (int it = 0; t < tasks; t += wstride, ++it) {
+  for (int it = 0; tw < tasks; t += stride, tw += stride, ++it) {
     const int sl = it & 1;
     __syncwarp();
-    fetch(t + wstride, sl ^ 1);
+    fetch(t + stride, sl ^ 1);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
-    const uint32_t* W = slot[w][sl];
+    if (S > 1 && t >= tasks) continue;
+    const uint32_t* W = slot[grp][sl];
     const int64_t o = t / nb;
-    const int col = int(t - o * nb) * 64 + 2 * lane;
+    const int col = col0 + int(t - o * nb) * (2 * G) + 2 * gl;
     const uint32_t m = W[27];
     uint32_t none = 0;
     F2 xv[27], yv[27];
@@ -204,11 +214,19 @@ void launch_octet(const dg_da* da, const T* ca, const T* cb, int R, int col0, in
   const unsigned grid = unsigned(std::min<int64_t>((warps + 3) / 4, int64_t(sm_count()) * 16));
   mrhs_octet_pf_kernel<T, G><<<grid, 128, 0, s>>>(O.n, O.meta.p, O.id.p, O.elem.p, ca, cb, R, col0, nb, X, Y);
 }
+template <int G>
+void launch_pairs(const dg_da* da, const float* ca, const float* cb, int R, int col0, int nb, const float* X, float* Y,
+                  cudaStream_t s) {
+  const OctetSet& O = da->octs;
+  const int64_t warps = (O.n * nb + 32 / G - 1) / (32 / G);
+  const unsigned grid = unsigned(std::min<int64_t>((warps + 3) / 4, int64_t(sm_count()) * 16));
+  mrhs_octet_pair_kernel<G><<<grid, 128, 0, s>>>(O.n, O.meta.p, O.id.p, O.elem.p, ca, cb, R, col0, nb, X, Y);
+}
 
 }  // namespace
 
-// FP32: blocks of 64 columns by the pair kernel, then 32, then 16; FP64: 32
-// and 16.
+// FP32: blocks of 64 columns by pairs, then 32, then 16 (2 and 4 octets per
+// warp); FP64: 32 and 16.
 template <class T>
 dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int R, cudaStream_t s, bool zeroed) {
   const dg_da* da = A->da;
@@ -219,18 +237,16 @@ dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int
   const T* cb = A->has_coef ? coef + da->E : nullptr;
   int col = 0;
   if constexpr (sizeof(T) == 4) {
-    if (const int nb = R / 64) {
-      const int64_t warps = O.n * nb;
-      const unsigned grid = unsigned(std::min<int64_t>((warps + 3) / 4, int64_t(sm_count()) * 16));
-      mrhs_octet_pair_kernel<<<grid, 128, 0, s>>>(O.n, O.meta.p, O.id.p, O.elem.p, ca, cb, R, nb, X, Y);
-      col = 64 * nb;
-    }
+    if (const int nb = R / 64) launch_pairs<32>(da, ca, cb, R, col, nb, X, Y, s);
+    col = R & ~63;
+    if ((R - col) & 32) launch_pairs<16>(da, ca, cb, R, col, 1, X, Y, s);
+    col = R & ~31;
+    if (R > col) launch_pairs<8>(da, ca, cb, R, col, 1, X, Y, s);
+  } else {
+    if (const int nb = R / 32) launch_octet<T, 32>(da, ca, cb, R, col, nb, X, Y, s);
+    col = R & ~31;
+    if (R > col) launch_octet<T, 16>(da, ca, cb, R, col, 1, X, Y, s);
   }
-  if (const int nb = (R - col) / 32) {
-    launch_octet<T, 32>(da, ca, cb, R, col, nb, X, Y, s);
-    col += 32 * nb;
-  }
-  if (R > col) launch_octet<T, 16>(da, ca, cb, R, col, 1, X, Y, s);
   DG_CUDA(cudaGetLastError());
   return DG_OK;
 }
