@@ -597,8 +597,8 @@ def run_multi(dev, steps, nrhs=64):
                                               "element parents the assembled 27 x 27 lattice matrices times the "
                                               "lattice values of 64 right-hand sides (M 128, N 64, K 32; split5: "
                                               "hi/lo split, three passes)",
-                     "octet_cuda_cores": "a warp per (parent octant, 32 right-hand sides), Walsh-form element "
-                                         "operators in FP32 registers, coalesced rows of X and Y"}
+                     "octet_cuda_cores": "a warp per (parent octant, 64 right-hand sides), Walsh-form element "
+                                         "operators on packed FP32 pairs, coalesced rows of X and Y"}
     return out
 
 
