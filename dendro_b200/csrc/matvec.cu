@@ -1964,39 +1964,41 @@ __global__ void lapmass_diag_kernel(const uint32_t* __restrict__ nl, const uint3
   }
 }
 
-// The diagonals of T^T K T and T^T M T for the 18 frame hanging patterns
-// (kFrameMasks), by frame vertex, and each 7-bit pattern's index.
+// The diagonals of T^T K T and T^T M T by frame vertex, for every frame hanging
+// pattern fm of the vertices 1 to 6 (row fm / 2).  An octree has 18 of these
+// (kFrameMasks); a mesh made from maps may have others, and T is then what the
+// element kernels apply (interp_hanging): a hanging vertex takes the mean of
+// the slots between it and its element's own corner of the parent.
 struct DiagTables {
-  double k[18][8], m[18][8];
-  uint8_t type[128];
-  constexpr DiagTables() : k(), m(), type() {
-    for (int t = 0; t < 18; ++t) {
-      const uint32_t fm = kFrameMasks[t];
-      type[fm] = uint8_t(t);
+  double k[64][8], m[64][8];
+  constexpr DiagTables() : k(), m() {
+    for (int t = 0; t < 64; ++t) {
       double T[8][8] = {};
-      for (int i = 0; i < 8; ++i)
-        for (int j = 0; j < 8; ++j) {
-          const int bits = (i & 1) + ((i >> 1) & 1) + (i >> 2);
-          if (!((fm >> i) & 1u)) T[i][j] = i == j ? 1.0 : 0.0;
-          else T[i][j] = (j & ~i) == 0 ? (bits == 1 ? 0.5 : 0.25) : 0.0;
-        }
+      for (int i = 0; i < 8; ++i) {
+        const int bits = (i & 1) + ((i >> 1) & 1) + (i >> 2);
+        if (!((2 * t) >> i & 1)) T[i][i] = 1.0;
+        else
+          for (int j = 0; j < 8; ++j)
+            if ((j & ~i) == 0) T[i][j] = bits == 1 ? 0.5 : 0.25;
+      }
       for (int j = 0; j < 8; ++j)
         for (int p = 0; p < 8; ++p)
           for (int q = 0; q < 8; ++q) {
+            const double w = T[p][j] * T[q][j];
+            if (w == 0.0) continue;
             double mm[3] = {}, kk[3] = {};
             for (int a = 0; a < 3; ++a) {
               const bool same = ((p ^ q) >> a & 1) == 0;
               mm[a] = same ? 2.0 / 3.0 : 1.0 / 3.0;
               kk[a] = same ? 0.5 : -0.5;
             }
-            const double w = T[p][j] * T[q][j];
             m[t][j] += w * mm[0] * mm[1] * mm[2];
             k[t][j] += w * (kk[0] * mm[1] * mm[2] + mm[0] * kk[1] * mm[2] + mm[0] * mm[1] * kk[2]);
           }
     }
   }
 };
-__constant__ DiagTables c_diag = DiagTables();
+__device__ const DiagTables c_diag = DiagTables();
 
 // The diagonal, one thread per octet: each child's 8 entries (a table row for
 // its hanging pattern, the same value everywhere without hanging vertices) are
@@ -2011,13 +2013,11 @@ __global__ void __launch_bounds__(128) lapmass_diag_octet_kernel(int64_t n, cons
                                                                  const uint32_t* __restrict__ oelem,
                                                                  const CT* __restrict__ ca, const CT* __restrict__ cb,
                                                                  double* __restrict__ d) {
-  __shared__ double sk[18][8], sm[18][8];
-  __shared__ uint8_t st[128];
-  for (int i = threadIdx.x; i < 18 * 8; i += blockDim.x) {
+  __shared__ double sk[64][8], sm[64][8];
+  for (int i = threadIdx.x; i < 64 * 8; i += blockDim.x) {
     sk[i / 8][i % 8] = c_diag.k[i / 8][i % 8];
     sm[i / 8][i % 8] = c_diag.m[i / 8][i % 8];
   }
-  for (int i = threadIdx.x; i < 128; i += blockDim.x) st[i] = c_diag.type[i];
   __syncthreads();
   for (int64_t o = gtid(); o < n; o += gstride()) {
     const uint32_t m = __ldg(ometa + o), cm = ometa_cmask(m);
@@ -2045,7 +2045,7 @@ __global__ void __launch_bounds__(128) lapmass_diag_octet_kernel(int64_t n, cons
 #pragma unroll
         for (int f = 0; f < 8; ++f) yv[oct_lat(c, f)] += v;
       } else {
-        const int t = st[fm];
+        const int t = int(fm >> 1);
 #pragma unroll
         for (int f = 0; f < 8; ++f) {
           const double v = f1 * sk[t][f] + f2 * sm[t][f];
