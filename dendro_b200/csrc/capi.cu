@@ -32,6 +32,9 @@ __global__ void octants_to_keys(const dg_octant* __restrict__ o, int64_t n, uint
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     uint32_t l = o[i].level_flags & kLevelMask;
     if (l > D) atomicOr(bad, 1u);
+    // outside the domain, whose octants have all their ancestors in it (the
+    // set-up kernels count on that)
+    if ((o[i].x | o[i].y | o[i].z) >> D) atomicOr(bad, 4u);
     k[i] = okey(morton(o[i].x, o[i].y, o[i].z), l);
     if (i > 0) {
       uint32_t pl = o[i - 1].level_flags & kLevelMask;
@@ -185,7 +188,9 @@ dg_status dg_octree_from_octants(const dg_octant* octs, int64_t n, int on_device
   if (cudaMemcpy(&h, bad.p, 4, cudaMemcpyDeviceToHost) != cudaSuccess) { delete t; DG_CUDA(cudaGetLastError()); }
   if (h) {
     delete t;
-    set_error(__FILE__, __LINE__, (h & 1) ? "octant level above maxDepth" : "octants not strictly Morton sorted");
+    set_error(__FILE__, __LINE__, (h & 1)   ? "octant level above maxDepth"
+                                  : (h & 4) ? "octant anchor outside the domain of side 2^maxDepth"
+                                            : "octants not strictly Morton sorted");
     return DG_EUNBALANCED;
   }
   *out = t;

@@ -274,6 +274,8 @@ __global__ void __launch_bounds__(kSetThreads) balance_level(uint32_t l, uint32_
 // before L; an ancestor has those before the path to L, plus the path's own
 // where that is internal.  With S the sum of the path's child numbers that is
 // 1 + 8 (a - d) + S + (d - 1) octants, a of them internal: 7 a - 7 d + S leaves.
+// (With every ancestor in the list, as the set has for octants inside the
+// domain, places lie in [0, 7 nu + 1); no other is written.)
 __global__ void balance_leaves(const uint64_t* __restrict__ u, int64_t nu, uint32_t D, uint64_t* __restrict__ out) {
   for (int64_t t = gtid(); t < nu * 8; t += gstride()) {
     const int64_t i = t >> 3;
@@ -285,7 +287,8 @@ __global__ void balance_leaves(const uint64_t* __restrict__ u, int64_t nu, uint3
     if (a < nu && u[a] == ck) continue;
     const int64_t S = __popcll(m & 0x1249249249249249ull) + 2 * __popcll(m & 0x2492492492492492ull) +
                       4 * __popcll(m & 0x4924924924924924ull);
-    out[7 * a - 7 * int64_t(d) + S] = ck;
+    const int64_t at = 7 * a - 7 * int64_t(d) + S;
+    if (at >= 0 && at <= 7 * nu) out[at] = ck;
   }
 }
 

@@ -63,7 +63,9 @@ int dg_device_count(void);
 dg_status dg_points2octree(const double* pts, int64_t n, int pts_on_device, uint32_t max_depth,
                            uint32_t max_num_pts, dg_octree** out);
 
-/* Wrap an existing sorted linear octree (e.g. read from an .ot file). */
+/* Wrap an existing sorted linear octree (e.g. read from an .ot file).
+ * DG_EUNBALANCED for octants out of Morton order, deeper than max_depth or
+ * with an anchor outside the domain [0, 2^max_depth)^3. */
 dg_status dg_octree_from_octants(const dg_octant* octs, int64_t n, int on_device, uint32_t max_depth,
                                  dg_octree** out);
 

@@ -118,3 +118,26 @@ def test_levels_of_a_batch_have_octets(gpu, oracle):
         A.set_kernel(v)
         y = A.mult(torch.tensor(x, device="cuda")).cpu().numpy()
         assert np.linalg.norm(y - want) <= 1e-12 * np.linalg.norm(want), v
+
+
+# only the import is called: what it refuses reaches no other kernel
+@pytest.mark.parametrize("octants,depth", [([(16, 0, 0, 4), (17, 0, 0, 4)], 4), ([(0, 0, 0, 4), (0, 16, 0, 4)], 4),
+                                           ([(0, 0, 0, 1), (0, 0, 1 << 21, 1)], 4), ([(0, 0, 0, 3), (8, 8, 8, 3)], 3),
+                                           ([(1, 0, 0, 0)], 0), ([(1 << 19, 0, 0, 19)], 19)])
+def test_octants_outside_the_domain_are_refused(gpu, tmp_path, octants, depth):
+    from dendro_b200._lib import OCT_DTYPE
+    with pytest.raises(gpu.DendroError) as err:
+        gpu.Octree.from_octants(np.array(octants, OCT_DTYPE), depth)
+    assert err.value.status == 6  # DG_EUNBALANCED
+    f = tmp_path / "o.ot"
+    f.write_text(f"3 {depth}\n{len(octants)}\n" + "".join("%d %d %d %d\n" % o for o in octants))
+    with pytest.raises(gpu.DendroError):
+        gpu.readNodesFromFile(f)
+
+
+@pytest.mark.parametrize("depth", [1, 4, 19])
+def test_octants_at_the_far_corner_are_kept(gpu, depth):
+    from dendro_b200._lib import OCT_DTYPE
+    top = (1 << depth) - 1
+    a = np.array([(0, 0, 0, depth), (top, top, top, depth)], OCT_DTYPE)
+    assert same(gpu.Octree.from_octants(a, depth).to_numpy(), a)
