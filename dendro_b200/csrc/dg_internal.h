@@ -194,14 +194,42 @@ void set_wait_limit(long long cycles);
 long long wait_limit();  // clock cycles a bounded device wait may take
 dg_status device_wait_status(cudaStream_t s);
 dg_status build_octets(dg_da* da, cudaStream_t s);  // da->octs from nl and meta (octet.cu)
-// Tables that only some launch shapes read, built when one of those is chosen
-// (not inside a stream capture: they allocate and synchronise s): the warp
-// tiles (da->tiles_w), the octets' records, the octet chunks (none when a
-// chunk's elements are too far apart).
+// Tables that only some launch shapes read, built when one of those is chosen:
+// the warp tiles (da->tiles_w), the octets' records, the octet chunks (none
+// when a chunk's elements are too far apart).  Each is complete when its call
+// returns, and left empty by one that fails.
 dg_status ensure_tiles(dg_da* da, cudaStream_t s);
 dg_status ensure_octet_records(dg_da* da, cudaStream_t s);
 dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s);
 dg_status ensure_octet_tiles(dg_da* da, cudaStream_t s);  // da->otiles (octile.cu)
+// build(stream), its allocations from the pool, then a wait: on s, or while s
+// is being captured on a stream of its own -- a table is needed now, and what
+// a captured stream allocates and launches is there only once the graph runs.
+// undo() gives back what a build that failed had allocated.
+template <class Build, class Undo>
+dg_status build_table(cudaStream_t s, Build&& build, Undo&& undo) {
+  auto on = [&](cudaStream_t t) -> dg_status {
+    PoolScope scope(t);
+    dg_status st = build(t);
+    if (!st) {
+      const cudaError_t e = cudaStreamSynchronize(t);
+      if (e != cudaSuccess) {
+        set_error(__FILE__, __LINE__, cudaGetErrorString(e));
+        st = DG_ECUDA;
+      }
+    }
+    if (st) undo();
+    return st;
+  };
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  DG_CUDA(cudaStreamIsCapturing(s, &cap));
+  if (cap == cudaStreamCaptureStatusNone) return on(s);
+  cudaStream_t own = nullptr;
+  DG_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+  const dg_status st = on(own);
+  cudaStreamDestroy(own);
+  return st;
+}
 // da->cmap with narrow quotients of qbits (1..16) bits (cmap.cu); nl_out
 // [8][E] receives the map decoded from it
 dg_status build_cmap(dg_da* da, int qbits, cudaStream_t s);

@@ -395,21 +395,29 @@ dg_status ensure_octet_records(dg_da* da, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(da->tables);
   OctetSet& O = da->octs;
   if (O.rec.n || !O.n) return DG_OK;
-  PoolScope scope(s);
-  DG_TRY(O.rec.alloc((O.n + 1) * kOctRec));
-  octet_records<<<grid_for(O.n + 1, 256), 256, 0, s>>>(O.n, O.meta.p, O.id.p, O.rec.p);
-  DG_CUDA(cudaGetLastError());
-  DG_CUDA(cudaStreamSynchronize(s));
-  return DG_OK;
+  auto build = [&](cudaStream_t t) -> dg_status {
+    DG_TRY(O.rec.alloc((O.n + 1) * kOctRec));
+    octet_records<<<grid_for(O.n + 1, 256), 256, 0, t>>>(O.n, O.meta.p, O.id.p, O.rec.p);
+    DG_CUDA(cudaGetLastError());
+    return DG_OK;
+  };
+  return build_table(s, build, [&] { O.rec.reset(); });
 }
 
 dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(da->tables);
-  if (da->octs.chunks_tried || !da->octs.n) return DG_OK;
-  PoolScope scope(s);
-  DG_TRY(build_chunks(da, s));
-  da->octs.chunks_tried = true;
-  DG_CUDA(cudaStreamSynchronize(s));
+  OctetSet& O = da->octs;
+  if (O.chunks_tried || !O.n) return DG_OK;
+  auto undo = [&] {
+    O.nchunk = 0;
+    O.cptr.reset();
+    O.cnodes.reset();
+    O.cel.reset();
+    O.lidx.reset();
+    O.lelem.reset();
+  };
+  DG_TRY(build_table(s, [&](cudaStream_t t) { return build_chunks(da, t); }, undo));
+  O.chunks_tried = true;
   return DG_OK;
 }
 

@@ -212,10 +212,8 @@ dg_status build(dg_da* da, cudaStream_t s) {
 dg_status ensure_octet_tiles(dg_da* da, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(da->tables);
   if (da->otiles.tried || !da->octs.n) return DG_OK;
-  PoolScope scope(s);
-  DG_TRY(build(da, s));
+  DG_TRY(build_table(s, [&](cudaStream_t t) { return build(da, t); }, [&] { da->otiles = OctTiles(); }));
   da->otiles.tried = true;
-  DG_CUDA(cudaStreamSynchronize(s));
   return DG_OK;
 }
 

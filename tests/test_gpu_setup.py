@@ -103,6 +103,29 @@ def test_first_use_of_a_mesh_in_several_threads(gpu):
             assert (a - b).abs().max() <= tol * b.abs().max()
 
 
+def test_first_use_of_a_mesh_inside_a_capture(gpu):
+    """A table that a captured call is the first to need is there when the call returns, for the graph and for the
+    calls after it."""
+    import torch
+    pts = I.clamp_unit(I.gaussian_cloud(5000, 3), 10)
+    da, one = (gpu.DA(gpu.balanceOctree(gpu.points2Octree(pts, 10, 1))) for _ in range(2))
+    X = torch.rand(da.N, 64, dtype=torch.float32, device="cuda")
+    want = gpu.Jacobian2(one).mult_multi(X, split=5)
+    Y = torch.zeros_like(X)
+    A = gpu.Jacobian2(da)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="relaxed"):
+        A.mult_multi(X, Y, split=5, stream=torch.cuda.current_stream())
+    for _ in range(2):
+        Y.fill_(7.0)
+        g.replay()
+        torch.cuda.synchronize()
+        assert (Y - want).abs().max() <= 1e-5 * want.abs().max()
+    del g
+    Y = A.mult_multi(X, split=5)
+    assert (Y - want).abs().max() <= 1e-5 * want.abs().max()
+
+
 def test_levels_of_a_batch_have_octets(gpu, oracle):
     """Every octet launch shape on a batch's concatenated mesh, against the meshes one by one."""
     import torch
