@@ -169,7 +169,8 @@ inline unsigned grid_for(int64_t n, int block, int per_sm = 8) {
 // The pool keeps at most kPoolKeep unused bytes between calls, gives the rest
 // back to the device at the next synchronisation, and gives everything back
 // when an allocation fails.  Outside a scope a pool buffer is released as
-// cudaFree would: after the device has finished.
+// cudaFree would: after the device has finished (and not at all when that
+// cannot be waited for, in a thread that captures a stream).
 constexpr uint64_t kPoolKeep = uint64_t(2) << 30;
 struct PoolScope {
   explicit PoolScope(cudaStream_t s);
@@ -185,14 +186,21 @@ struct PoolScope {
 // device's ordinal), else cudaMalloc (*dev = -1).
 cudaError_t device_alloc(void** p, size_t bytes, int* dev);
 void device_free(void* p, int dev);
+// Waits until the current device has finished all it was given, as cudaFree
+// does: also while another thread captures a stream, where
+// cudaDeviceSynchronize fails and ends that thread's capture.
+cudaError_t drain_device();
 // Deletes an object made of device buffers: waits for the device once (its
 // buffers may be in use on any stream), then releases them together.
 template <class T>
 void delete_drained(T* p) {
   if (!p) return;
-  cudaDeviceSynchronize();
-  PoolScope scope(nullptr);
-  delete p;
+  if (drain_device() == cudaSuccess) {
+    PoolScope scope(nullptr);
+    delete p;
+  } else {
+    delete p;
+  }
 }
 
 // Device buffer with RAII ownership.

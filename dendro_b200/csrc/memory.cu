@@ -45,6 +45,28 @@ cudaMemPool_t device_pool(int dev) {
 
 }  // namespace
 
+// A small block allocated and freed.  Another one is kept per device, so that
+// the 2 MB they lie in stay mapped: 5 us (cudaDeviceSynchronize 3; 600 with the
+// mapping undone each time).
+cudaError_t drain_device() {
+  static std::mutex mu;
+  static void* kept[kMaxDevices] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  constexpr size_t kSmall = 256;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < kMaxDevices && !kept[dev] && cudaMalloc(&kept[dev], kSmall) != cudaSuccess) kept[dev] = nullptr;
+  }
+  void* p = nullptr;
+  e = cudaMalloc(&p, kSmall);
+  if (e == cudaSuccess) e = cudaFree(p);
+  if (e == cudaErrorMemoryAllocation) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
+}
+
 PoolScope::PoolScope(cudaStream_t s) : prev_(t_scope.stream), prev_on_(t_scope.on) {
   t_scope.stream = s;
   t_scope.on = true;
@@ -72,7 +94,7 @@ cudaError_t device_alloc(void** p, size_t bytes, int* dev) {
     if (e != cudaErrorMemoryAllocation || attempt) break;
     // what the pool holds unused may be what is missing
     cudaMemPool_t held = device_pool(cur);
-    if (!held || cudaDeviceSynchronize() != cudaSuccess || cudaMemPoolTrimTo(held, 0) != cudaSuccess) {
+    if (!held || drain_device() != cudaSuccess || cudaMemPoolTrimTo(held, 0) != cudaSuccess) {
       (void)cudaGetLastError();
       break;
     }
@@ -93,8 +115,7 @@ void device_free(void* p, int dev) {
   }
   // outside a scope (or with another device current): any stream may still use it
   if (cur != dev) cudaSetDevice(dev);
-  cudaDeviceSynchronize();
-  cudaFreeAsync(p, nullptr);
+  if (drain_device() == cudaSuccess) cudaFreeAsync(p, nullptr);
   if (cur != dev) cudaSetDevice(cur);
 }
 

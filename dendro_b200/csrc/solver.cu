@@ -1806,7 +1806,7 @@ dg_status dg_damg_batch_offsets(const dg_damg* m, int level, int64_t* elem_off, 
 
 dg_status dg_damg_set_lapmass(dg_damg* m, const double* coef) {
   DG_CHECK(m, DG_EINVAL, "damg_set_lapmass: null handle");
-  DG_CUDA(cudaDeviceSynchronize());  // the present operators may be in use on other streams
+  DG_CUDA(drain_device());  // the present operators may be in use on other streams
   PoolScope scope(m->s);
   DG_TRY(set_operators(m, coef));
   DG_CUDA(cudaStreamSynchronize(m->s));

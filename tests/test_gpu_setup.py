@@ -126,6 +126,44 @@ def test_first_use_of_a_mesh_inside_a_capture(gpu):
     assert (Y - want).abs().max() <= 1e-5 * want.abs().max()
 
 
+def test_set_up_and_release_beside_a_capture(gpu):
+    """A thread that makes, uses and releases octrees, meshes, operators and hierarchies does not end the capture of
+    another thread's stream."""
+    import torch
+    pts = I.clamp_unit(I.gaussian_cloud(3000, 3), 9)
+    x = torch.rand(1000, dtype=torch.float64, device="cuda")
+    y = torch.zeros_like(x)
+    st = torch.cuda.Stream()
+    bad = []
+
+    def work():
+        try:
+            t = gpu.balanceOctree(gpu.points2Octree(pts, 9, 1))
+            da = gpu.DA(t)
+            A = gpu.Jacobian2(da)
+            A.mult(v[0][:da.N], v[1][:da.N], stream=st)
+            m = gpu.DAMG(t, nlevels=3)
+            m.setKSP()
+            m.setKSP(np.full((da.E, 2), 2.0))
+            del A, m, da, t
+        except Exception as e:  # noqa: BLE001 -- the test's thread reports it
+            bad.append(e)
+
+    v = torch.ones((2, 100000), dtype=torch.float64, device="cuda")
+    work()  # loads the kernels
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        torch.mul(x, 2.0, out=y)
+        th = threading.Thread(target=work)
+        th.start()
+        th.join()
+        y.add_(1.0)
+    assert not bad
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, 2 * x + 1)
+
+
 def test_levels_of_a_batch_have_octets(gpu, oracle):
     """Every octet launch shape on a batch's concatenated mesh, against the meshes one by one."""
     import torch
