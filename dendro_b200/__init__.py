@@ -18,5 +18,6 @@ does not load it until first use, and every use fails loudly without it.
 from .api import (DA, DAMG, DirichletJacobian, DirichletLaplacian, Elasticity, Jacobian2,  # noqa: F401
                   Octree, balanceOctree, coarsenOctree,
                   deviceCheck, points2Octree, readDataPtsFromFile, readNodesFromFile, readPtsFromFile,
-                  setDeviceWaitLimit, vecDot, writeDataPtsToFile, writeNodesToFile, writePtsToFile)
+                  setAllocationLimit, setDeviceWaitLimit, vecDot, writeDataPtsToFile, writeNodesToFile,
+                  writePtsToFile)
 from ._lib import DendroError, OCT_DTYPE  # noqa: F401

@@ -127,6 +127,7 @@ def lib():
         "dg_damg_level_apply": ([P, I, P, P, I], I),
         "dg_mat_create_dirichlet": ([P, I, P, PP], I),
         "dg_set_device_wait_limit": ([I64], I),
+        "dg_set_allocation_limit": ([I64], I),
         "dg_partition_weighted": ([I64, P, I, P], I),
         "dg_halo_create": ([I64, I64, U32, P, P, P, P, P, P, P, I, I, PP], I),
         "dg_halo_create_from_da": ([P, P, I, I, PP], I),
@@ -179,7 +180,7 @@ def exported_symbols():
         "dg_mlp_param_count", "dg_mlp_create", "dg_mlp_get_params", "dg_mlp_set_params", "dg_mlp_forward",
         "dg_mlp_gradient", "dg_mlp_train_step", "dg_mlp_destroy", "dg_damg_set_smoother", "dg_damg_features",
         "dg_vec_dot_noalloc", "dg_mat_kernel_count", "dg_mat_set_kernel", "dg_device_check",
-        "dg_set_device_wait_limit", "dg_write_pts", "dg_read_pts", "dg_write_data_pts", "dg_read_data_pts",
+        "dg_set_device_wait_limit", "dg_set_allocation_limit", "dg_write_pts", "dg_read_pts", "dg_write_data_pts", "dg_read_data_pts",
         "dg_octree_write", "dg_octree_read", "dg_da_dump_mesh", "dg_damg_level_apply",
         "dg_mat_create_dirichlet",
         "dg_mat_mult_multi", "dg_damg_set_tolerances",

@@ -489,3 +489,9 @@ def setDeviceWaitLimit(cycles: int) -> None:
     """Test hook: clock64 cycles a staged operator kernel waits for its copies
     before giving up (<= 0 restores the default of 2^31 cycles)."""
     check(lib().dg_set_device_wait_limit(int(cycles)), "set_device_wait_limit")
+
+
+def setAllocationLimit(nbytes: int) -> None:
+    """Test hook: the largest block of device memory that this thread's calls may allocate,
+    larger ones fail as on a full device (<= 0: no limit)."""
+    check(lib().dg_set_allocation_limit(int(nbytes)), "set_allocation_limit")

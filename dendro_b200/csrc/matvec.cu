@@ -2530,6 +2530,10 @@ static int forced_variant() {
   return v;
 }
 
+// A table that cannot be had for want of memory: the shapes that read it do
+// not run on this mesh, and no call fails for it.
+static dg_status if_memory(dg_status st) { return st == DG_ENOMEM ? DG_OK : st; }
+
 // The launch shape for a mesh and precision: the forced one, the tuned one,
 // or -- on first use outside a stream capture -- tune now: per variant one
 // untimed launch, then the best of two timed runs; for a mesh that L2 does not
@@ -2556,7 +2560,7 @@ static dg_status pick_variant(dg_da* da, int& choice, const CT* ca, const CT* cb
   if (choice < 0 || forced_variant() >= 0) DG_CUDA(cudaStreamIsCapturing(s, &cap));
   if (forced_variant() >= 0) {
     *v_out = forced_variant();
-    if (cap == cudaStreamCaptureStatusNone) DG_TRY(matvec_variant_tables(da, *v_out, s));
+    if (cap == cudaStreamCaptureStatusNone) DG_TRY(if_memory(matvec_variant_tables(da, *v_out, s)));
     return DG_OK;
   }
   if (choice < 0 && cap != cudaStreamCaptureStatusNone) {  // no timing inside a graph capture
@@ -2567,12 +2571,12 @@ static dg_status pick_variant(dg_da* da, int& choice, const CT* ca, const CT* cb
     cudaEvent_t e0, e1;
     DG_CUDA(cudaEventCreate(&e0));
     DG_CUDA(cudaEventCreate(&e1));
-    // a mesh that stays in L2 between applications is timed there
-    const int64_t flush_bytes = da->E * 64 > (int64_t(64) << 20) ? int64_t(192) << 20 : 0;
-    if (da->E <= kTilesMax) DG_TRY(ensure_tiles(da, s));
+    if (da->E <= kTilesMax) DG_TRY(if_memory(ensure_tiles(da, s)));
     PoolScope scope(s);
     DBuf<uint8_t> flush;
-    DG_TRY(flush.alloc(flush_bytes));
+    // a mesh that stays in L2 between applications is timed there
+    if (da->E * 64 > (int64_t(64) << 20)) DG_TRY(if_memory(flush.alloc(int64_t(192) << 20)));
+    const int64_t flush_bytes = flush.n;
     // A mesh in L2 is timed over several launches, queued before the first is
     // done: with one launch between the events, the host's own time to launch
     // it counts (a 45 MB mesh got a shape twice as slow as the best).
@@ -2859,7 +2863,8 @@ dg_status lapmass_apply_host_pipelined_f64(dg_mat* A, const double* hx, double* 
   if (!page_locked(hx) || !page_locked(hy)) return DG_ENOTIMPL;
   if (!A->pipe) {
     auto P = std::make_shared<HostPipe>();
-    DG_TRY(ensure_tiles(da, nullptr));
+    const dg_status st = ensure_tiles(da, nullptr);
+    if (st) return st == DG_ENOMEM ? DG_ENOTIMPL : st;
     DG_TRY(build_host_pipe(da, *P));
     A->pipe = P;
   }

@@ -14,6 +14,7 @@ struct ScopeState {
   bool on = false;
 };
 thread_local ScopeState t_scope;
+thread_local size_t t_largest = 0;  // no limit
 
 // The pool of a device, made on first use and kept for the process (its
 // unused memory is bounded by kPoolKeep); nullptr where pools are not
@@ -79,6 +80,7 @@ PoolScope::~PoolScope() {
 cudaError_t device_alloc(void** p, size_t bytes, int* dev) {
   *p = nullptr;
   *dev = -1;
+  if (t_largest && bytes > t_largest) return cudaErrorMemoryAllocation;
   int cur = 0;
   cudaError_t e = cudaGetDevice(&cur);
   if (e != cudaSuccess) return e;
@@ -120,3 +122,8 @@ void device_free(void* p, int dev) {
 }
 
 }  // namespace dg
+
+extern "C" dg_status dg_set_allocation_limit(int64_t bytes) {
+  dg::t_largest = bytes > 0 ? size_t(bytes) : 0;
+  return DG_OK;
+}

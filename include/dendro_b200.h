@@ -238,6 +238,9 @@ dg_status dg_device_check(void* stream);
 /* Test hook: the clock64 cycles such a wait lasts before it gives up
  * (<= 0 restores the default of 2^31 cycles, about one second). */
 dg_status dg_set_device_wait_limit(int64_t cycles);
+/* Test hook: the largest block of device memory that calls of this thread may
+ * allocate, larger ones fail as on a full device (<= 0: no limit). */
+dg_status dg_set_allocation_limit(int64_t bytes);
 int64_t dg_mat_size(const dg_mat* A); /* rows = dof * nodes */
 /* Launch shape of the scalar operator kernel that the autotuner picked on the
  * first application in the given precision ("untuned" before it). */

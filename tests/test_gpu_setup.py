@@ -181,6 +181,28 @@ def test_levels_of_a_batch_have_octets(gpu, oracle):
         assert np.linalg.norm(y - want) <= 1e-12 * np.linalg.norm(want), v
 
 
+@pytest.fixture
+def no_memory(gpu):
+    """Calls of this thread find no memory for blocks above the given size."""
+    yield gpu.setAllocationLimit
+    gpu.setAllocationLimit(0)
+
+
+# FP64 and FP32 on a mesh timed in L2 and on one timed from HBM
+@pytest.mark.parametrize("n,depth", [(3000, 9), (262144, 13)])
+def test_operator_without_memory_for_tables(gpu, no_memory, n, depth):
+    import torch
+    das = [gpu.DA(gpu.balanceOctree(gpu.points2Octree(I.clamp_unit(I.lognormal_cloud(n, 5), depth), depth, 1)))
+           for _ in range(2)]
+    for dt, tol in ((torch.float64, 1e-13), (torch.float32, 1e-5)):
+        x = torch.rand(das[0].N, dtype=dt, device="cuda")
+        want = gpu.Jacobian2(das[0]).mult(x)
+        no_memory(1)
+        y = gpu.Jacobian2(das[1]).mult(x)
+        no_memory(0)
+        assert (y - want).abs().max() <= tol * want.abs().max()
+
+
 # only the import is called: what it refuses reaches no other kernel
 @pytest.mark.parametrize("octants,depth", [([(16, 0, 0, 4), (17, 0, 0, 4)], 4), ([(0, 0, 0, 4), (0, 16, 0, 4)], 4),
                                            ([(0, 0, 0, 1), (0, 0, 1 << 21, 1)], 4), ([(0, 0, 0, 3), (8, 8, 8, 3)], 3),
