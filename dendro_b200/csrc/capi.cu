@@ -436,7 +436,7 @@ dg_status dg_mat_create_elasticity(dg_da* da, double mu, double lambda, const ui
       st = node_boundary_flags(da, A->dirichlet.p, nullptr);
     }
   }
-  if (!st) st = ensure_octet_tiles(da, nullptr);
+  if (!st) st = elasticity_tiles(A, nullptr);
   if (st) { delete A; return st; }
   *out = A;
   return DG_OK;

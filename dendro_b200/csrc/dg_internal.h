@@ -133,6 +133,7 @@ struct dg_mat {
   dg::DBuf<double> coef;       // [2][E] (a then b), FP64
   dg::DBuf<float> coef32;      // [2][E] FP32 copy for the inner solver
   double mu = 0, lam = 0;
+  bool tiles = false;          // elasticity on the mesh's octet tiles (there since the operator was made)
   dg::DBuf<uint8_t> dirichlet; // [N]
   dg::DBuf<double> host_x, host_y;  // device staging of dg_mat_mult_host, kept between calls
   mutable dg::DBuf<float> tc_coef;  // [octets + 1][16] element scale factors of the tensor-memory multi-RHS kernel
@@ -202,6 +203,9 @@ dg_status ensure_tiles(dg_da* da, cudaStream_t s);
 dg_status ensure_octet_records(dg_da* da, cudaStream_t s);
 dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s);
 dg_status ensure_octet_tiles(dg_da* da, cudaStream_t s);  // da->otiles (octile.cu)
+// A table that cannot be had for want of memory: the kernels that read it do
+// not run on this mesh, and no call fails for it.
+inline dg_status if_memory(dg_status st) { return st == DG_ENOMEM ? DG_OK : st; }
 // build(stream), its allocations from the pool, then a wait: on s, or while s
 // is being captured on a stream of its own -- a table is needed now, and what
 // a captured stream allocates and launches is there only once the graph runs.
@@ -298,6 +302,9 @@ dg_status mrhs_octet_apply(const dg_mat* A, const T* coef, const T* X, T* Y, int
 dg_status mrhs_tc_apply(const dg_mat* A, const float* X, float* Y, int R, int passes, cudaStream_t s);
 // DG_ETIMEOUT (then cleared) when a bounded wait of that kernel ran out.
 dg_status mrhs_tc_take_status();
+// Octet tiles for an elasticity operator; without memory for them it runs on
+// the element kernel.
+dg_status elasticity_tiles(dg_mat* A, cudaStream_t s);
 dg_status elasticity_apply_f64(const dg_mat* A, const double* x, double* y, cudaStream_t s);
 dg_status elasticity_diag(const dg_mat* A, double* d, cudaStream_t s);
 // Dense row-major (3 N) x (3 N) matrix of the elasticity operator, Dirichlet

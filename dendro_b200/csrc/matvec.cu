@@ -2530,10 +2530,6 @@ static int forced_variant() {
   return v;
 }
 
-// A table that cannot be had for want of memory: the shapes that read it do
-// not run on this mesh, and no call fails for it.
-static dg_status if_memory(dg_status st) { return st == DG_ENOMEM ? DG_OK : st; }
-
 // The launch shape for a mesh and precision: the forced one, the tuned one,
 // or -- on first use outside a stream capture -- tune now: per variant one
 // untimed launch, then the best of two timed runs; for a mesh that L2 does not
@@ -3603,11 +3599,17 @@ static bool elasticity_tiles_off() {
   return v == 1;
 }
 
+dg_status elasticity_tiles(dg_mat* A, cudaStream_t s) {
+  const dg_status st = ensure_octet_tiles(A->da, s);
+  A->tiles = st == DG_OK && A->da->otiles.ntiles > 0;
+  return if_memory(st);
+}
+
 dg_status elasticity_apply_f64(const dg_mat* A, const double* x, double* y, cudaStream_t s) {
   const dg_da* da = A->da;
   const OctetSet& O = da->octs;
   const OctTiles& Q = da->otiles;
-  if (Q.ntiles > 0 && !elasticity_tiles_off()) {
+  if (A->tiles && !elasticity_tiles_off()) {
     const uint32_t cap = (Q.max_nodes + 7u) & ~7u;
     DG_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(elasticity_tile_kernel),
                               elasticity_tile_smem(kOctTileRefs)));

@@ -1302,7 +1302,7 @@ dg_status set_elasticity_operators(dg_damg* m) {
     A->dof = 3;
     A->mu = m->cfg.mu;
     A->lam = m->cfg.lambda;
-    DG_TRY(ensure_octet_tiles(L.da.get(), s));
+    DG_TRY(elasticity_tiles(A.get(), s));
     DG_TRY(A->dirichlet.alloc(L.da->N));
     DG_TRY(node_boundary_flags(L.da.get(), A->dirichlet.p, s));
     L.A = std::move(A);

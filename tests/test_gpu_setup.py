@@ -203,6 +203,19 @@ def test_operator_without_memory_for_tables(gpu, no_memory, n, depth):
         assert (y - want).abs().max() <= tol * want.abs().max()
 
 
+def test_elasticity_without_memory_for_tiles(gpu, oracle, no_memory):
+    import torch
+    octs = oracle.balance(oracle.points2octree(I.clamp_unit(I.gaussian_cloud(2000, 5), 9), 9, 1), 9)
+    ref, da = oracle.Mesh(octs, 9), gpu.DA(gpu.Octree.from_octants(octs, 9))
+    x = np.random.default_rng(2).uniform(-1, 1, 3 * ref.N)
+    want = ref.elasticity_matvec(x, 0.4, 0.6, ref.node_bdy)
+    no_memory(2 * ref.N)  # the operator's own flags, one byte per node, and no tile table
+    few = gpu.Elasticity(da, 0.4, 0.6)
+    for A in (few, no_memory(0) or gpu.Elasticity(da, 0.4, 0.6), few):  # with the tiles that the second one builds
+        y = A.mult(torch.tensor(x, device="cuda")).cpu().numpy()
+        assert np.linalg.norm(y - want) <= 1e-12 * np.linalg.norm(want)
+
+
 # only the import is called: what it refuses reaches no other kernel
 @pytest.mark.parametrize("octants,depth", [([(16, 0, 0, 4), (17, 0, 0, 4)], 4), ([(0, 0, 0, 4), (0, 16, 0, 4)], 4),
                                            ([(0, 0, 0, 1), (0, 0, 1 << 21, 1)], 4), ([(0, 0, 0, 3), (8, 8, 8, 3)], 3),
