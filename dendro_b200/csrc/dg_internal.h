@@ -1,6 +1,7 @@
 // Internal device-side objects behind the opaque C-ABI handles.
 #pragma once
 
+#include <atomic>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -109,11 +110,15 @@ struct dg_da {
   dg::OctetSet octs;  // elements grouped by parent (octet operator kernel)
   dg::OctTiles otiles;  // tiles of octets (on first use)
   dg::CompressedMap cmap;  // compressed element map (on request)
-  // operator launch shape picked by the autotuner on first use (-1: not yet)
-  int tuned_f64 = -1, tuned_f32 = -1;
-  // held while a table is built on first use: threads may share a mesh, each
-  // with its own operators and streams
+  // Threads may share a mesh, each with its own operators and streams.
+  // Operator launch shape picked by the autotuner on first use (-1: not yet),
+  // by one thread, which holds `tuning` meanwhile.
+  std::atomic<int> tuned_f64{-1}, tuned_f32{-1};
+  std::mutex tuning;
+  // Tables built on first use, under `tables`; a flag is set when its table's
+  // contents are there, and only then does a kernel of any thread read them.
   std::mutex tables;
+  std::atomic<bool> tiles_ready{false}, records_ready{false}, chunks_ready{false};
 };
 
 struct dg_mlp {

@@ -2336,9 +2336,9 @@ constexpr int kNumVariants = int(sizeof(kVariants) / sizeof(kVariants[0]));
 static bool variant_runs(int k, const dg_da* da) {
   if (k == 16) return da->cmap.qbits != 0;
   if ((k == 6 || k >= 10) && da->octs.n == 0) return false;
-  if ((k == 10 || k == 11) && da->octs.rec.n == 0) return false;
-  if (k >= 7 && k <= 9 && da->octs.nchunk == 0) return false;
-  if (k >= 2 && k <= 5 && da->tiles_w.ntiles == 0) return false;
+  if ((k == 10 || k == 11) && !da->records_ready) return false;
+  if (k >= 7 && k <= 9 && !da->chunks_ready) return false;
+  if (k >= 2 && k <= 5 && !da->tiles_ready) return false;
   return true;
 }
 
@@ -2550,19 +2550,23 @@ static bool variant_timed(int v, int64_t E) {
   return k == 0 || k == 6 || k == 12 || k == 13 || k >= 15 || (k >= 2 && k <= 4 && E <= kTilesMax);
 }
 template <class T, class CT>
-static dg_status pick_variant(dg_da* da, int& choice, const CT* ca, const CT* cb, const T* x, T* y,
+static dg_status pick_variant(dg_da* da, std::atomic<int>& choice, const CT* ca, const CT* cb, const T* x, T* y,
                               cudaStream_t s, int* v_out) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (choice < 0 || forced_variant() >= 0) DG_CUDA(cudaStreamIsCapturing(s, &cap));
+  *v_out = choice;
+  if (*v_out < 0 || forced_variant() >= 0) DG_CUDA(cudaStreamIsCapturing(s, &cap));
   if (forced_variant() >= 0) {
     *v_out = forced_variant();
     if (cap == cudaStreamCaptureStatusNone) DG_TRY(if_memory(matvec_variant_tables(da, *v_out, s)));
     return DG_OK;
   }
-  if (choice < 0 && cap != cudaStreamCaptureStatusNone) {  // no timing inside a graph capture
+  if (*v_out < 0 && cap != cudaStreamCaptureStatusNone) {  // no timing inside a graph capture
     *v_out = kDefaultVariant;
     return DG_OK;
   }
+  if (*v_out >= 0) return DG_OK;
+  // one thread tunes, the others wait for its choice
+  std::lock_guard<std::mutex> lock(da->tuning);
   if (choice < 0) {
     cudaEvent_t e0, e1;
     DG_CUDA(cudaEventCreate(&e0));
@@ -2603,8 +2607,8 @@ static dg_status pick_variant(dg_da* da, int& choice, const CT* ca, const CT* cb
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    choice = bi;
     DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
+    choice = bi;
   }
   *v_out = choice;
   return DG_OK;
@@ -2612,7 +2616,7 @@ static dg_status pick_variant(dg_da* da, int& choice, const CT* ca, const CT* cb
 
 // y = A x with the mesh's launch shape.
 template <class T, class CT>
-static dg_status lapmass_launch(dg_da* da, int& choice, const CT* ca, const CT* cb, const T* x, T* y,
+static dg_status lapmass_launch(dg_da* da, std::atomic<int>& choice, const CT* ca, const CT* cb, const T* x, T* y,
                                 cudaStream_t s) {
   int v = 0;
   DG_TRY((pick_variant<T, CT>(da, choice, ca, cb, x, y, s, &v)));
@@ -2853,7 +2857,8 @@ static bool page_locked(const void* p) {
 
 dg_status lapmass_apply_host_pipelined_f64(dg_mat* A, const double* hx, double* hy) {
   dg_da* da = A->da;
-  if (A->kind != 0 || da->E < kPipeMinElements || da->tuned_f64 < 0) return DG_ENOTIMPL;
+  const int tuned = da->tuned_f64;
+  if (A->kind != 0 || da->E < kPipeMinElements || tuned < 0) return DG_ENOTIMPL;
   // pageable buffers: each chunk copy would block the host until its group
   // has run, serialising the pipeline, so the caller copies, applies, copies
   if (!page_locked(hx) || !page_locked(hy)) return DG_ENOTIMPL;
@@ -2866,8 +2871,8 @@ dg_status lapmass_apply_host_pipelined_f64(dg_mat* A, const double* hx, double* 
   }
   HostPipe& P = *A->pipe;
   // the mesh's shape when it is a plain warp-tile one, else the widest of them
-  const int kind = kVariants[da->tuned_f64].kind;
-  P.variant = (kind >= 2 && kind <= 4) ? da->tuned_f64 : kPipeVariant;
+  const int kind = kVariants[tuned].kind;
+  P.variant = (kind >= 2 && kind <= 4) ? tuned : kPipeVariant;
   DG_TRY(enqueue_host_pipe(A, P, hx, hy));
   DG_CUDA(cudaStreamSynchronize(P.sk));
   return DG_OK;
@@ -2896,7 +2901,7 @@ static dg_status apply_to_zeroed(const dg_mat* A, const CT* coef, const T* x, T*
   dg_da* da = A->da;
   const CT* ca = A->has_coef ? coef : nullptr;
   const CT* cb = A->has_coef ? coef + da->E : nullptr;
-  int& choice = sizeof(T) == 8 ? da->tuned_f64 : da->tuned_f32;
+  std::atomic<int>& choice = sizeof(T) == 8 ? da->tuned_f64 : da->tuned_f32;
   int v = 0;
   DG_TRY((pick_variant<T, CT>(da, choice, ca, cb, x, t, s, &v)));
   return launch_variant<T, CT>(v, da, ca, cb, x, t, s);

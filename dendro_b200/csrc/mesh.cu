@@ -919,10 +919,12 @@ dg_status build_tile_set(const dg_da* da, int te, TileSet& ts, cudaStream_t s) {
 
 dg_status ensure_tiles(dg_da* da, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(da->tables);
-  if (da->tiles_w.ntiles) return DG_OK;
-  return build_table(
+  if (da->tiles_ready) return DG_OK;
+  DG_TRY(build_table(
       s, [&](cudaStream_t t) { return build_tile_set(da, kWarpTile, da->tiles_w, t); },
-      [&] { da->tiles_w = TileSet(); });
+      [&] { da->tiles_w = TileSet(); }));
+  da->tiles_ready = true;
+  return DG_OK;
 }
 
 uint32_t etype_mask(int c, int t) { return kEtypeMask[c & 7][t % 18]; }

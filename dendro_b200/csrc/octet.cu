@@ -394,14 +394,16 @@ dg_status build_octets(dg_da* da, cudaStream_t s) {
 dg_status ensure_octet_records(dg_da* da, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(da->tables);
   OctetSet& O = da->octs;
-  if (O.rec.n || !O.n) return DG_OK;
+  if (da->records_ready || !O.n) return DG_OK;
   auto build = [&](cudaStream_t t) -> dg_status {
     DG_TRY(O.rec.alloc((O.n + 1) * kOctRec));
     octet_records<<<grid_for(O.n + 1, 256), 256, 0, t>>>(O.n, O.meta.p, O.id.p, O.rec.p);
     DG_CUDA(cudaGetLastError());
     return DG_OK;
   };
-  return build_table(s, build, [&] { O.rec.reset(); });
+  DG_TRY(build_table(s, build, [&] { O.rec.reset(); }));
+  da->records_ready = true;
+  return DG_OK;
 }
 
 dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s) {
@@ -418,6 +420,7 @@ dg_status ensure_octet_chunks(dg_da* da, cudaStream_t s) {
   };
   DG_TRY(build_table(s, [&](cudaStream_t t) { return build_chunks(da, t); }, undo));
   O.chunks_tried = true;
+  da->chunks_ready = O.nchunk > 0;
   return DG_OK;
 }
 

@@ -103,6 +103,31 @@ def test_first_use_of_a_mesh_in_several_threads(gpu):
             assert (a - b).abs().max() <= tol * b.abs().max()
 
 
+def test_a_mesh_is_tuned_once_by_threads_that_share_it(gpu):
+    """Whichever thread times the launch shapes, all threads run the one that it chose."""
+    import torch
+    pts = I.clamp_unit(I.gaussian_cloud(4000, 3), 10)
+    for _ in range(6):
+        da = gpu.DA(gpu.balanceOctree(gpu.points2Octree(pts, 10, 1)))
+        x = torch.rand(da.N, dtype=torch.float64, device="cuda")
+        names, start = [None] * 4, threading.Barrier(4)
+
+        def work(i):
+            st = torch.cuda.Stream()
+            J = gpu.Jacobian2(da)
+            start.wait()
+            J.mult(x, torch.empty_like(x), stream=st)
+            names[i] = J.kernel_name()
+            st.synchronize()
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert names == [gpu.Jacobian2(da).kernel_name()] * 4
+
+
 def test_first_use_of_a_mesh_inside_a_capture(gpu):
     """A table that a captured call is the first to need is there when the call returns, for the graph and for the
     calls after it."""
