@@ -9,27 +9,20 @@
 #include "dg_common.cuh"
 
 namespace dg {
-// Tiles of `te` consecutive elements for the shared-memory operator kernels.
-// Per tile: its distinct node ids (ascending; bit 31 set when another tile
-// also references the node) and, grouped by node, the tile's references to
-// them, each as position v * te + element of its (element, vertex) slot.
+// Warp tiles: te = kWarpTile consecutive elements each, for the warp-tile
+// operator kernels.  Per tile its distinct node ids (at most 8 te, ascending;
+// bit 31 set when another tile also references the node, or its sum arrives in
+// parts) and, in the child-number frame (frame vertex j = vertex j ^ c of the
+// element):
 struct TileSet {
-  int te = 0;                // elements per tile
   int64_t ntiles = 0;
-  uint32_t max_nodes = 0;    // largest node count of a tile
   DBuf<uint32_t> ptr;        // [ntiles + 1] offsets of the tiles' node lists
   DBuf<uint32_t> nodes;      // [ptr[ntiles]]
-  DBuf<uint16_t> nend;       // [ntiles * 8 te]: tile t, node k -> end of its run in inc
-  DBuf<uint16_t> inc;        // [ntiles * 8 te]: tile t -> references ordered by node
-  // warp tiles (at most 256 nodes per tile), all in the child-number frame
-  // (frame vertex j = vertex j ^ c of the element):
   DBuf<uint8_t> eloc8;       // [8 E] per element byte j = node rank of frame vertex j
   DBuf<uint32_t> wmeta;      // [E] level | frame hanging mask << 8
   DBuf<uint8_t> ref8;        // [ntiles * kWarpRefBytes] per tile: the references sorted by node as frame
                              // positions j * te + element [8 te], their node ranks [8 te], then per lane
                              // one flag word [32 x u32] (bit q valid, 8 + q start, 16 + q leave, 24 + q store)
-  DBuf<uint32_t> shared;     // ascending ids of the nodes several tiles reference
-  int64_t nshared = 0;
 };
 // Elements grouped by parent octant for the octet operator kernel (octet.cuh):
 // one entry per parent with at least one leaf child, in Morton order of the
@@ -245,7 +238,6 @@ dg_status build_cmap(dg_da* da, int qbits, cudaStream_t s);
 dg_status cmap_decode(const dg_da* da, uint32_t* nl_out, cudaStream_t s);
 // b = the load vector of a force sampled at the element centres (matvec.cu)
 dg_status load_vector(const dg_da* da, const double* force, double* b, cudaStream_t s);
-dg_status build_tile_set(const dg_da* da, int te, TileSet& ts, cudaStream_t s);
 // Hanging mask of element type t (0..17) for child number c
 // (include/oda/cnumEtypes.h:19-229).
 uint32_t etype_mask(int c, int t);

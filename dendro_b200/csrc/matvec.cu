@@ -2530,25 +2530,90 @@ static int forced_variant() {
   return v;
 }
 
-// The launch shape for a mesh and precision: the forced one, the tuned one,
-// or -- on first use outside a stream capture -- tune now: per variant one
-// untimed launch, then the best of two timed runs; for a mesh that L2 does not
-// hold, each after overwriting a buffer larger than L2.  y is used as scratch and left zero.  Inside a
-// capture an untuned mesh gets the default octet shape.  Timed are the shapes
-// that are fastest on some mesh: the element kernel, the octet kernels with the
-// lattice in registers, the compressed-map kernel where its map has been built,
-// and up to kTilesMax elements the warp tiles (their tables are built for that;
-// FP64 / FP32 on the coarse levels of the 1M-point mesh, best tile against best
-// octet shape: 44 / 31 against 36 / 28 us with 1.6M elements, 15.1 / 11.9
-// against 15.5 / 12.8 with 469K, 6.9 / 5.9 against 8.1 / 6.8 with 127K, 4.7 / 4.3
-// against 7.8 / 6.3 with 32K).  The bulk-copy, chunk, lane and quad shapes were
-// 1.2 to 2 times slower on every mesh tried and run only when fixed by the caller.
+// Events of a timed run, released whichever way the timing ends.
+struct EventPair {
+  cudaEvent_t e[2] = {nullptr, nullptr};
+  ~EventPair() {
+    for (cudaEvent_t x : e)
+      if (x) cudaEventDestroy(x);
+  }
+};
+
+// Times the launch shapes for a mesh and precision on stream s: y is scratch
+// and left zero.  Each shape that is fastest on some mesh runs once untimed and
+// is then timed, all of them queued before the host waits; the best three are
+// timed twice more and the fastest of those runs is the choice.  (Every shape
+// timed twice, with a wait for each run, took 7.7 ms of a first application on
+// 707K elements.)  A mesh that L2 does not hold is timed after overwriting a
+// buffer larger than L2, one that it holds over several launches, queued
+// before the first is done: with the host's own time to launch between the
+// events a 45 MB mesh got a shape twice as slow as the best.  Timed are the
+// element kernel, the octet kernels with the lattice in registers, the
+// compressed-map kernel where its map has been built, and up to kTilesMax
+// elements the warp tiles, whose tables are built for that (FP64 / FP32 on the
+// coarse levels of the 1M-point mesh, best tile against best octet shape:
+// 44 / 31 against 36 / 28 us with 1.6M elements, 15.1 / 11.9 against 15.5 / 12.8
+// with 469K, 6.9 / 5.9 against 8.1 / 6.8 with 127K, 4.7 / 4.3 against 7.8 / 6.3
+// with 32K; with 707K and 1.0M no tile shape was chosen).  The bulk-copy,
+// chunk, lane and quad shapes were 1.2 to 2 times slower on every mesh tried
+// and run only when fixed by the caller.
 constexpr int kDefaultVariant = 28;  // "octet b128, next ids in flight, 4 CTAs/SM"
-constexpr int64_t kTilesMax = int64_t(1) << 20;
+constexpr int64_t kTilesMax = int64_t(1) << 19;
 static bool variant_timed(int v, int64_t E) {
   const int k = kVariants[v].kind;
   return k == 0 || k == 6 || k == 12 || k == 13 || k >= 15 || (k >= 2 && k <= 4 && E <= kTilesMax);
 }
+template <class T, class CT>
+static dg_status tune(dg_da* da, const CT* ca, const CT* cb, const T* x, T* y, cudaStream_t s, int* choice) {
+  if (da->E <= kTilesMax) DG_TRY(if_memory(ensure_tiles(da, s)));
+  PoolScope scope(s);
+  DBuf<uint8_t> flush;
+  if (da->E * 64 > (int64_t(64) << 20)) DG_TRY(if_memory(flush.alloc(int64_t(192) << 20)));
+  std::vector<int> shapes;
+  for (int v = 0; v < kNumVariants; ++v)
+    if (variant_timed(v, da->E) && variant_runs(kVariants[v].kind, da)) shapes.push_back(v);
+  // ms[i] of shapes[i], i < n: the least of `runs` runs of `reps` launches each
+  auto time = [&](size_t n, int runs, int reps, std::vector<float>& ms) -> dg_status {
+    std::vector<EventPair> ev(n * size_t(runs));
+    for (size_t k = 0; k < ev.size(); ++k) {
+      const int v = shapes[k / size_t(runs)];
+      for (cudaEvent_t& e : ev[k].e) DG_CUDA(cudaEventCreate(&e));
+      if (flush.n) DG_CUDA(cudaMemsetAsync(flush.p, int(k), flush.n, s));
+      else DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));
+      DG_CUDA(cudaEventRecord(ev[k].e[0], s));
+      for (int r = 0; r < reps; ++r) DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));
+      DG_CUDA(cudaEventRecord(ev[k].e[1], s));
+    }
+    DG_CUDA(cudaStreamSynchronize(s));
+    ms.assign(n, 1e30f);
+    for (size_t k = 0; k < ev.size(); ++k) {
+      float t = 0;
+      DG_CUDA(cudaEventElapsedTime(&t, ev[k].e[0], ev[k].e[1]));
+      ms[k / size_t(runs)] = std::min(ms[k / size_t(runs)], t);
+    }
+    return DG_OK;
+  };
+  auto rank = [&](const std::vector<float>& ms) {
+    std::vector<std::pair<float, int>> by;
+    for (size_t i = 0; i < ms.size(); ++i) by.push_back({ms[i], shapes[i]});
+    std::sort(by.begin(), by.end());
+    for (size_t i = 0; i < ms.size(); ++i) shapes[i] = by[i].second;
+  };
+  std::vector<float> ms;
+  DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
+  for (int v : shapes) DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));  // loads the kernels
+  DG_TRY(time(shapes.size(), 1, flush.n ? 1 : 2, ms));
+  rank(ms);
+  DG_TRY(time(std::min<size_t>(3, shapes.size()), 2, flush.n ? 1 : 4, ms));
+  rank(ms);
+  DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
+  *choice = shapes[0];
+  return DG_OK;
+}
+
+// The launch shape for a mesh and precision: the forced one, the tuned one,
+// or -- on first use outside a stream capture -- tune now.  Inside a capture
+// an untuned mesh gets the default octet shape.
 template <class T, class CT>
 static dg_status pick_variant(dg_da* da, std::atomic<int>& choice, const CT* ca, const CT* cb, const T* x, T* y,
                               cudaStream_t s, int* v_out) {
@@ -2560,57 +2625,14 @@ static dg_status pick_variant(dg_da* da, std::atomic<int>& choice, const CT* ca,
     if (cap == cudaStreamCaptureStatusNone) DG_TRY(if_memory(matvec_variant_tables(da, *v_out, s)));
     return DG_OK;
   }
-  if (*v_out < 0 && cap != cudaStreamCaptureStatusNone) {  // no timing inside a graph capture
-    *v_out = kDefaultVariant;
-    return DG_OK;
-  }
+  if (*v_out < 0 && cap != cudaStreamCaptureStatusNone) *v_out = kDefaultVariant;
   if (*v_out >= 0) return DG_OK;
   // one thread tunes, the others wait for its choice
   std::lock_guard<std::mutex> lock(da->tuning);
-  if (choice < 0) {
-    cudaEvent_t e0, e1;
-    DG_CUDA(cudaEventCreate(&e0));
-    DG_CUDA(cudaEventCreate(&e1));
-    if (da->E <= kTilesMax) DG_TRY(if_memory(ensure_tiles(da, s)));
-    PoolScope scope(s);
-    DBuf<uint8_t> flush;
-    // a mesh that stays in L2 between applications is timed there
-    if (da->E * 64 > (int64_t(64) << 20)) DG_TRY(if_memory(flush.alloc(int64_t(192) << 20)));
-    const int64_t flush_bytes = flush.n;
-    // A mesh in L2 is timed over several launches, queued before the first is
-    // done: with one launch between the events, the host's own time to launch
-    // it counts (a 45 MB mesh got a shape twice as slow as the best).
-    const int reps = flush_bytes ? 1 : 4;
-    float best = 1e30f;
-    int bi = kDefaultVariant;
-    DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
-    for (int v = 0; v < kNumVariants; ++v) {
-      if (!variant_timed(v, da->E) || !variant_runs(kVariants[v].kind, da)) continue;
-      DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));  // untimed: loads the kernel
-      for (int trial = 0; trial < 2; ++trial) {
-        if (flush_bytes) DG_CUDA(cudaMemsetAsync(flush.p, trial + 1, flush_bytes, s));
-        DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
-        if (!flush_bytes) DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));
-        DG_CUDA(cudaEventRecord(e0, s));
-        for (int r = 0; r < reps; ++r) DG_TRY((launch_variant<T, CT>(v, da, ca, cb, x, y, s)));
-        DG_CUDA(cudaEventRecord(e1, s));
-        DG_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        DG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        const bool out = ms > 1.5f * best;  // no second run for a shape that is far off
-        if (ms < best) {
-          best = ms;
-          bi = v;
-        }
-        if (out) break;
-      }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    DG_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * da->N, s));
-    choice = bi;
-  }
   *v_out = choice;
+  if (*v_out >= 0) return DG_OK;
+  DG_TRY((tune<T, CT>(da, ca, cb, x, y, s, v_out)));
+  choice = *v_out;
   return DG_OK;
 }
 

@@ -710,21 +710,12 @@ __global__ void warp_split_runs(const uint16_t* __restrict__ nend, const uint32_
 }
 
 // Bit 31 of a list entry: the node is referenced by more than one tile, so its
-// sum must be accumulated with a global atomic.  The shared nodes are also
-// flagged per node for the compact list of them.
+// sum must be accumulated with a global atomic.
 __global__ void tile_local_mark(uint32_t* __restrict__ nodes, int64_t n, const uint32_t* __restrict__ touch) {
   for (int64_t i = gtid(); i < n; i += gstride()) {
     const uint32_t id = nodes[i] & 0x7fffffffu;
     if (touch[id] > 1u) nodes[i] = id | 0x80000000u;
   }
-}
-__global__ void shared_flag(uint32_t* __restrict__ touch, int64_t N) {
-  for (int64_t i = gtid(); i < N; i += gstride()) touch[i] = touch[i] > 1u ? 1u : 0u;
-}
-__global__ void shared_emit(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos, int64_t N,
-                            uint32_t* __restrict__ out) {
-  for (int64_t i = gtid(); i < N; i += gstride())
-    if (flag[i]) out[pos[i]] = uint32_t(i);
 }
 
 }  // namespace
@@ -857,62 +848,40 @@ static dg_status launch_tile_lists(const dg_da* da, int64_t nt, uint32_t* tmp, u
   return DG_OK;
 }
 
-dg_status build_tile_set(const dg_da* da, int te, TileSet& ts, cudaStream_t s) {
+// One wait, for the length of the node lists: the first application on a mesh
+// has this before it.
+static dg_status build_tile_set(const dg_da* da, TileSet& ts, cudaStream_t s) {
   DG_CHECK(da->N < (int64_t(1) << 31), DG_EINVAL, "mesh above 2^31 nodes");
-  DG_CHECK(te == kWarpTile, DG_EINVAL, "unsupported tile size");
-  const int64_t E = da->E, nt = (E + te - 1) / te, S = 8 * int64_t(te);
+  constexpr int S = 8 * kWarpTile;
+  const int64_t E = da->E, nt = (E + kWarpTile - 1) / kWarpTile;
   DBuf<uint32_t> tmp, cnt, touch;
+  DBuf<uint16_t> nend, inc;  // tile t, node k -> end of its run in inc, the references ordered by node
+  DBuf<uint8_t> r3;
   DG_TRY(tmp.alloc(nt * S));
-  DG_TRY(cnt.alloc(nt));
-  DG_TRY(ts.nend.alloc(nt * S));
-  DG_TRY(ts.inc.alloc(nt * S));
+  DG_TRY(cnt.alloc(nt + 1));
+  DG_TRY(nend.alloc(nt * S));
+  DG_TRY(inc.alloc(nt * S));
   DG_TRY(ts.eloc8.alloc(8 * nt * kWarpTile));  // whole tiles
-  DG_TRY(launch_tile_lists<kWarpTile>(da, nt, tmp.p, cnt.p, ts.nend.p, ts.inc.p, ts.eloc8.p, s));
-  std::vector<uint32_t> hc(nt);
-  DG_CUDA(cudaMemcpyAsync(hc.data(), cnt.p, 4 * nt, cudaMemcpyDeviceToHost, s));
-  uint32_t total = 0;
+  DG_CUDA(cudaMemsetAsync(cnt.p + nt, 0, 4, s));
+  DG_TRY(launch_tile_lists<kWarpTile>(da, nt, tmp.p, cnt.p, nend.p, inc.p, ts.eloc8.p, s));
   DG_TRY(ts.ptr.alloc(nt + 1));
-  DG_TRY(scan_u32(cnt.p, ts.ptr.p, nt, &total, s));
-  DG_CUDA(cudaMemcpyAsync(ts.ptr.p + nt, &total, 4, cudaMemcpyHostToDevice, s));
-  DG_CUDA(cudaStreamSynchronize(s));
-  uint32_t mx = 0;
-  for (uint32_t c : hc) mx = c > mx ? c : mx;
-  ts.max_nodes = mx;
+  DG_TRY(scan_u32(cnt.p, ts.ptr.p, nt + 1, nullptr, s));
+  uint32_t total = 0;
+  DG_TRY(read_words(ts.ptr.p + nt, &total, 1, s));
   DG_TRY(ts.nodes.alloc(total + kNodePad));
-  tile_compact<<<grid_for(nt, 256, 8), 256, 0, s>>>(tmp.p, int(S), ts.ptr.p, nt, ts.nodes.p);
+  tile_compact<<<grid_for(nt, 256, 8), 256, 0, s>>>(tmp.p, S, ts.ptr.p, nt, ts.nodes.p);
   DG_TRY(touch.alloc(da->N));
   DG_CUDA(cudaMemsetAsync(touch.p, 0, 4 * da->N, s));
-  if (te == kWarpTile)
-    warp_split_runs<<<grid_for(nt * 32, 256, 8), 256, 0, s>>>(ts.nend.p, ts.ptr.p, nt, ts.nodes.p);
+  warp_split_runs<<<grid_for(nt * 32, 256, 8), 256, 0, s>>>(nend.p, ts.ptr.p, nt, ts.nodes.p);
   tile_touch<<<grid_for(total, 256), 256, 0, s>>>(ts.nodes.p, total, touch.p);
   tile_local_mark<<<grid_for(total, 256), 256, 0, s>>>(ts.nodes.p, total, touch.p);
-  shared_flag<<<grid_for(da->N, 256), 256, 0, s>>>(touch.p, da->N);
+  DG_TRY(r3.alloc(nt * 3 * S));
+  DG_TRY(ts.ref8.alloc(nt * kWarpRefBytes));
+  warp_refs<<<grid_for(nt * 32, 256, 8), 256, 0, s>>>(inc.p, nend.p, ts.ptr.p, ts.nodes.p, da->meta.p, nt, r3.p,
+                                                       ts.ref8.p);
+  DG_TRY(ts.wmeta.alloc(nt * kWarpTile));  // whole tiles
+  warp_frame<<<grid_for(E, 256), 256, 0, s>>>(da->meta.p, E, reinterpret_cast<uint2*>(ts.eloc8.p), ts.wmeta.p);
   DG_CUDA(cudaGetLastError());
-  DBuf<uint32_t> pos;
-  DG_TRY(pos.alloc(da->N));
-  uint32_t ns = 0;
-  DG_TRY(scan_u32(touch.p, pos.p, da->N, &ns, s));
-  ts.nshared = ns;
-  DG_TRY(ts.shared.alloc(ns > 0 ? ns : 1));
-  shared_emit<<<grid_for(da->N, 256), 256, 0, s>>>(touch.p, pos.p, da->N, ts.shared.p);
-  if (te == kWarpTile) {  // byte lists with flags replace the uint16 ones
-    DBuf<uint8_t> r3;
-    DG_TRY(r3.alloc(nt * 3 * S));
-    DG_TRY(ts.ref8.alloc(nt * kWarpRefBytes));
-    warp_refs<<<grid_for(nt * 32, 256, 8), 256, 0, s>>>(ts.inc.p, ts.nend.p, ts.ptr.p, ts.nodes.p, da->meta.p, nt,
-                                                         r3.p, ts.ref8.p);
-    DG_TRY(ts.wmeta.alloc(nt * kWarpTile));  // whole tiles
-    warp_frame<<<grid_for(E, 256), 256, 0, s>>>(da->meta.p, E, reinterpret_cast<uint2*>(ts.eloc8.p), ts.wmeta.p);
-    DG_CUDA(cudaGetLastError());
-    DG_CUDA(cudaStreamSynchronize(s));  // r3 is freed on return
-  }
-  DG_CUDA(cudaGetLastError());
-  DG_CUDA(cudaStreamSynchronize(s));
-  if (te == kWarpTile) {
-    ts.inc.reset();
-    ts.nend.reset();
-  }
-  ts.te = te;
   ts.ntiles = nt;
   return DG_OK;
 }
@@ -921,7 +890,7 @@ dg_status ensure_tiles(dg_da* da, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(da->tables);
   if (da->tiles_ready) return DG_OK;
   DG_TRY(build_table(
-      s, [&](cudaStream_t t) { return build_tile_set(da, kWarpTile, da->tiles_w, t); },
+      s, [&](cudaStream_t t) { return build_tile_set(da, da->tiles_w, t); },
       [&] { da->tiles_w = TileSet(); }));
   da->tiles_ready = true;
   return DG_OK;
