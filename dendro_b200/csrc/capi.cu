@@ -414,6 +414,7 @@ dg_status dg_mat_create_lapmass(dg_da* da, const double* coef, dg_mat** out) {
     }
     if (!st) st = A->coef32.alloc(2 * da->E + kCoefPad);
     if (!st) st = convert_f64_to_f32(A->coef.p, A->coef32.p, 2 * da->E, nullptr);
+    if (!st) st = finish_stream(nullptr);
     if (st) { delete A; return st; }
   }
   *out = A;
@@ -437,6 +438,7 @@ dg_status dg_mat_create_elasticity(dg_da* da, double mu, double lambda, const ui
     }
   }
   if (!st) st = elasticity_tiles(A, nullptr);
+  if (!st) st = finish_stream(nullptr);
   if (st) { delete A; return st; }
   *out = A;
   return DG_OK;
@@ -456,6 +458,7 @@ dg_status dg_mat_create_dirichlet(dg_da* da, int with_mass, const uint8_t* diric
       st = node_boundary_flags(da, A->dirichlet.p, nullptr);
     }
   }
+  if (!st) st = finish_stream(nullptr);
   if (st) { delete A; return st; }
   *out = A;
   return DG_OK;

@@ -189,6 +189,26 @@ def test_set_up_and_release_beside_a_capture(gpu):
     assert torch.equal(y, 2 * x + 1)
 
 
+def test_operators_are_ready_on_any_stream(gpu):
+    """What creating an operator computes is there when the call returns, although the default stream is busy."""
+    import torch
+    da = gpu.DA(gpu.balanceOctree(gpu.points2Octree(I.clamp_unit(I.gaussian_cloud(3000, 3), 9), 9, 1)))
+    st = torch.cuda.Stream()
+    for make in (lambda: gpu.Elasticity(da, 0.4, 0.6), lambda: gpu.DirichletLaplacian(da),
+                 lambda: gpu.Jacobian2(da, np.full((da.E, 2), 3.0))):
+        A = make()
+        x = torch.rand(A.n, dtype=torch.float64, device="cuda")
+        want = A.mult(x)
+        y = torch.empty_like(x)
+        torch.cuda.synchronize()
+        del A
+        torch.full((da.N + 64 * da.E,), 255, dtype=torch.uint8, device="cuda")  # what new flags may find
+        torch.cuda._sleep(100_000_000)
+        make().mult(x, y, stream=st)
+        st.synchronize()
+        assert (y - want).abs().max() <= 1e-13 * want.abs().max()
+
+
 def test_levels_of_a_batch_have_octets(gpu, oracle):
     """Every octet launch shape on a batch's concatenated mesh, against the meshes one by one."""
     import torch
