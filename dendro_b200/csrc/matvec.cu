@@ -1942,28 +1942,6 @@ __global__ void __launch_bounds__(32 * kTmaWarps, MINB) lapmass_warp_tma_kernel(
   }
 }
 
-template <class CT>
-__global__ void lapmass_diag_kernel(const uint32_t* __restrict__ nl, const uint32_t* __restrict__ meta,
-                                    const CT* __restrict__ ca, const CT* __restrict__ cb, int64_t E,
-                                    double* __restrict__ d) {
-  for (int64_t e = gtid(); e < E; e += gstride()) {
-    const uint32_t m = meta[e];
-    const uint32_t lev = meta_lev(m), c = meta_cnum(m), mask = meta_mask(m);
-    const double h = elem_h<double>(lev);
-    const double a = ca ? double(ca[e]) : 1.0, b = cb ? double(cb[e]) : 1.0;
-    const double f1 = a * h / 2.0, f2 = b * h * h * h / 8.0;
-    for (int j = 0; j < 8; ++j) {
-      double u[8];
-#pragma unroll
-      for (int v = 0; v < 8; ++v) u[v] = v == j ? 1.0 : 0.0;
-      if (mask) interp_hanging(u, c, mask);
-      lapmass_ref(u, f1, f2);
-      if (mask) scatter_hanging(u, c, mask);
-      atomicAdd(d + nl[int64_t(j) * E + e], u[j]);
-    }
-  }
-}
-
 // The diagonals of T^T K T and T^T M T by frame vertex, for every frame hanging
 // pattern fm of the vertices 1 to 6 (row fm / 2).  An octree has 18 of these
 // (kFrameMasks); a mesh made from maps may have others, and T is then what the
@@ -2004,9 +1982,9 @@ __device__ const DiagTables c_diag = DiagTables();
 // its hanging pattern, the same value everywhere without hanging vertices) are
 // summed over the octet's lattice points in registers -- a hanging vertex's
 // slot belongs to the octet corner that the element lists for it -- and each
-// node's sum leaves with one reduction: 27 per 8 elements.  The element kernel
-// above makes 64, each after applying the element operator to a unit vector:
-// 1268 us on the 4.7M-element benchmark mesh.
+// node's sum leaves with one reduction: 27 per 8 elements.  120 us on the
+// 4.7M-element benchmark mesh; a thread per element that applied the element
+// operator to 8 unit vectors, with 64 reductions per 8 elements, took 1268.
 template <class CT>
 __global__ void __launch_bounds__(128) lapmass_diag_octet_kernel(int64_t n, const uint32_t* __restrict__ ometa,
                                                                  const uint32_t* __restrict__ oid,
@@ -2331,11 +2309,11 @@ static dg_status allow_dynamic_smem(const void* kern, size_t bytes) {
 }
 constexpr int kNumVariants = int(sizeof(kVariants) / sizeof(kVariants[0]));
 
-// Whether the mesh has the structure a launch shape of this kind reads:
-// octets, octet records, octet chunks, warp tiles or the compressed map.
+// Whether the mesh has the tables a launch shape of this kind reads: octet
+// records, octet chunks, warp tiles or the compressed map (every mesh has
+// octets).
 static bool variant_runs(int k, const dg_da* da) {
   if (k == 16) return da->cmap.qbits != 0;
-  if ((k == 6 || k >= 10) && da->octs.n == 0) return false;
   if ((k == 10 || k == 11) && !da->records_ready) return false;
   if (k >= 7 && k <= 9 && !da->chunks_ready) return false;
   if (k >= 2 && k <= 5 && !da->tiles_ready) return false;
@@ -2354,12 +2332,10 @@ dg_status matvec_variant_tables(dg_da* da, int v, cudaStream_t s) {
 template <class T, class CT>
 static dg_status launch_variant(int v, const dg_da* da, const CT* ca, const CT* cb, const T* x, T* y,
                                 cudaStream_t s) {
-  // a shape fixed by the caller that this mesh cannot run (no octets, no
-  // octet chunks or no warp tiles, e.g. a batch of meshes) falls back to
-  // the element kernel rather than leaving y unwritten
-  {
-    if (!variant_runs(kVariants[v].kind, da)) v = 0;
-  }
+  // a shape fixed by the caller that this mesh cannot run (no octet chunks, no
+  // compressed map, or no memory for its tables) falls back to the element
+  // kernel rather than leaving y unwritten
+  if (!variant_runs(kVariants[v].kind, da)) v = 0;
   const MatvecVariant& V = kVariants[v];
   const unsigned g = V.per_sm ? grid_for(da->E, V.block, V.per_sm)
                               : unsigned((da->E + V.block - 1) / V.block > 0 ? (da->E + V.block - 1) / V.block : 1);
@@ -3003,10 +2979,7 @@ dg_status lapmass_diag(const dg_mat* A, double* d, cudaStream_t s) {
   const double* ca = A->has_coef ? A->coef.p : nullptr;
   const double* cb = A->has_coef ? A->coef.p + da->E : nullptr;
   const OctetSet& O = da->octs;
-  if (O.n)
-    lapmass_diag_octet_kernel<double><<<grid_for(O.n, 128, 8), 128, 0, s>>>(O.n, O.meta.p, O.id.p, O.elem.p, ca, cb, d);
-  else
-    lapmass_diag_kernel<double><<<grid_for(da->E, 256, 8), 256, 0, s>>>(da->nl.p, da->meta.p, ca, cb, da->E, d);
+  lapmass_diag_octet_kernel<double><<<grid_for(O.n, 128, 8), 128, 0, s>>>(O.n, O.meta.p, O.id.p, O.elem.p, ca, cb, d);
   DG_CUDA(cudaGetLastError());
   return DG_OK;
 }

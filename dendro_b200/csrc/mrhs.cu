@@ -264,6 +264,8 @@ dg_status mrhs_apply(const dg_mat* A, const float* X, float* Y, int R, int split
   DG_CHECK((reinterpret_cast<uintptr_t>(X) & 15) == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0, DG_EINVAL,
            "mat_mult_multi: X and Y must be 16-byte aligned");
   if (split >= 4) return mrhs_tc_apply(A, X, Y, R, split == 4 ? 1 : 3, s);
+  // split 3 and 1 run the same kernels; split 0 keeps refusing what it refused
+  // when they did not, so that a caller's error check still sees it
   if (split == 0)
     DG_CHECK(R % 32 == 0 && da->meshes == 1, DG_EINVAL,
              "mat_mult_multi: split 0 takes nrhs a multiple of 32 on one mesh");

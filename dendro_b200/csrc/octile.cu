@@ -179,7 +179,7 @@ dg_status build(dg_da* da, cudaStream_t s) {
   DG_TRY(scan_u32(cnt.p, cnt.p, nt + 1, nullptr, s));
   uint32_t h[3];
   DG_TRY(read_words(cnt.p + nt, h, 3, s));
-  if (h[1]) {  // a node that 16 and more octets of a tile list: no such mesh is known
+  if (h[1]) {  // a node that more than 16 octets of a tile list: no such mesh is known
     T.hdr.reset();
     T.refs.reset();
     T.lidx.reset();
