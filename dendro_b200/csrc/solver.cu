@@ -1171,7 +1171,10 @@ dg_status setup_coarse(dg_damg* m) {
     DG_CUDA(cudaMemsetAsync(m->d_crow_blk.p, 0, 4 * n3, m->s));
     DG_TRY(elasticity_assemble_dense(L.A.get(), m->Ainv.p, m->s));
     DG_TRY(gj_invert(m, n3, 1));
-    return pack_inverse(m);
+    DG_TRY(pack_inverse(m));
+    // only solve_multi, which takes dof 1, reads the full matrix beside the triangle
+    if (m->Asym.n) m->Ainv.reset();
+    return DG_OK;
   }
   const int64_t N = L.da->N;
   const std::vector<int64_t>& noff = m->mesh_node_off.back();

@@ -66,6 +66,24 @@ def test_infinity_stays_in_its_elements(gpu, oracle):
     assert np.isfinite(Y[~reach]).all()
 
 
+# with 3 values per node (3 x 1874 rows), also after a second set-up: the full inverse has been given back by then
+def test_large_dense_coarse_solve_of_elasticity(gpu):
+    import torch
+    from dendro_b200._lib import check, lib, ptr
+    tree = gpu.balanceOctree(gpu.points2Octree(I.clamp_unit(I.gaussian_cloud(250, 7), 7), 7, 1))
+    m = gpu.DAMG(tree, nlevels=1, dof=3, mu=0.4, lam=0.2)
+    da = m.level_da(0)
+    assert 3 * da.N >= 3000
+    b = torch.from_numpy(np.random.default_rng(7).uniform(-1, 1, 3 * da.N)).cuda()
+    x = torch.empty_like(b)
+    for _ in range(2):
+        m.setKSP()
+        check(lib().dg_damg_coarse_solve(m.h, ptr(b), ptr(x), None), "damg_coarse_solve")
+        r = b - gpu.Elasticity(da, 0.4, 0.2).mult(x)
+        torch.cuda.synchronize()
+        assert float(r.norm() / b.norm()) < 1e-9  # as below
+
+
 # the packed triangle of a large dense inverse: strips of 16 rows, blocks of 32 columns, the last ones cut short
 # (3115, 4071, 5728 and 5244 nodes)
 @pytest.mark.parametrize("n", [600, 900, 1200, 1300])
