@@ -233,7 +233,11 @@ dg_status dg_octree_export(const dg_octree* t, dg_octant* host_out) {
   return DG_OK;
 }
 
-void dg_octree_destroy(dg_octree* t) { delete_drained(t); }
+// Every call that reads an octree has finished with it when it returns.
+void dg_octree_destroy(dg_octree* t) {
+  PoolScope scope(nullptr);
+  delete t;
+}
 
 // -------------------------------------------------------------------- mesh
 dg_status dg_da_create(const dg_octree* balanced, dg_da** out) {

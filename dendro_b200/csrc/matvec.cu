@@ -3187,8 +3187,8 @@ __global__ void __launch_bounds__(128) elasticity_kernel(const uint32_t* __restr
 // Octet-tile form: a CTA of 8 warps works a tile of 32 octets (OctTiles), warp
 // c the children c, one octet per lane.  Shared-memory FP64 atomics are
 // compare-and-swap loops (a form that added each element's 24 results with them
-// took 513 us on the 4.7M-element benchmark mesh and lost more on small ones;
-// this one takes 481 us), so no two threads add to one place:
+// took 526 us from 1M log-normal points, 5.1M elements, and lost more on small
+// meshes; this one takes 490), so no two threads add to one place:
 // x at the tile's nodes is staged once (zero at Dirichlet nodes); a thread
 // works its element in its child-number frame and writes the 24 results by
 // (frame vertex, child, octet); the frame vertex of a child at lattice point p
@@ -3199,9 +3199,12 @@ __global__ void __launch_bounds__(128) elasticity_kernel(const uint32_t* __restr
 // the points around it; then each node's references are summed and the node
 // leaves, stored, or added where another tile has it (those nodes are set by
 // elasticity_shared_rows first).  Dirichlet rows leave as x.  The next tile's x
-// is copied while this one's sums leave (552 us without).  What bounds it is
-// issue and shared memory at 16 warps per SM: 225 M warp instructions, 118
-// registers and 86 KB of shared memory per CTA.
+// is copied while this one's sums leave (552 us without).  No unit is full: L1,
+// mostly shared memory (73 M wavefronts, 26 M of its bank conflicts), at 64 %,
+// 43 % of the issue slots, the FP64 pipe at 20 %, DRAM at 8 %.  It waits: with 16
+// warps per SM (118 registers, 86 KB of shared memory per CTA) a warp takes 9
+// cycles per instruction, of them 1.8 for fixed latencies, 1.5 for shared
+// memory, 1.4 at barriers and 1.1 for ids and x.
 constexpr int kElasTileThreads = 256;
 __global__ void __launch_bounds__(kElasTileThreads, 2) elasticity_tile_kernel(
     int64_t n, int64_t ntiles, uint32_t cap, const uint32_t* __restrict__ ometa, const uint32_t* __restrict__ tptr,

@@ -7,7 +7,7 @@
 // vectors' precision; mrhs_tc.cu has the contraction on the 5th-generation
 // tensor cores.  (Contractions per element on mma.sync, TF32 in one or three
 // products, took 2120 and 2231 us for 64 right-hand sides on the 2.9M-element
-// benchmark mesh, bound by L1, where the pair kernel takes 1165 us.)
+// benchmark mesh, bound by L1, where the pair kernel takes 1140 us.)
 #include <algorithm>
 
 #include "octet.cuh"
@@ -131,10 +131,12 @@ __device__ __forceinline__ bool nonzero(F2 a) { return (a.v & 0x7fffffff7fffffff
 // element arithmetic on packed pairs.  Works nb blocks of 2 G columns from
 // column col0 on (R and col0 even), G = 32, 16 or 8: with fewer lanes per octet
 // a warp works 2 or 4 octets at once, whose missing children and hanging points
-// differ, but at half the instructions per right-hand side.  Bound by their
-// issue.  On the 2.9M-element benchmark mesh, against one right-hand side per
+// differ, but at half the instructions per right-hand side.  64 columns are 711 M
+// warp instructions, which fill 59 % of the issue slots (FMA pipe 46 %, L1 28 %,
+// DRAM 21 %): dependent arithmetic with the 12 warps per SM that 168 registers
+// leave.  On the 2.9M-element benchmark mesh, against one right-hand side per
 // lane: 32 columns 634 and 817 us, 16 columns 330 and 444, 48 columns 989 and
-// 1261; 64 columns 1138.
+// 1261; 64 columns 1140.
 template <int G>
 __global__ void __launch_bounds__(128) mrhs_octet_pair_kernel(int64_t n, const uint32_t* __restrict__ ometa,
                                                               const uint32_t* __restrict__ oid,

@@ -70,7 +70,7 @@ __host__ __device__ __forceinline__ uint32_t ometa_cmask(uint32_t m) { return (m
 // FP64: child by child, because 128 registers hold the 27 + 27 doubles but not
 // the transform's lines as well (one-thread-per-octet kernel on the 4.7M-element
 // benchmark mesh with the next ids in flight, this form / the other: FP64 101 /
-// 110 us, FP32 84 / 80 us; 64 right-hand sides in FP32 pairs 1240 / 1165 us).
+// 110 us, FP32 84 / 80 us; 64 right-hand sides in FP32 pairs 1240 / 1140 us).
 template <class T, bool FULL, class Coef>
 __device__ __forceinline__ void octet_children(const T (&xv)[27], T (&yv)[27], uint32_t cm, T g1, T g2, Coef coef) {
   if constexpr (std::is_same<T, double>::value) {

@@ -615,7 +615,7 @@ __global__ void dense_gemv(const double* __restrict__ A, int64_t N, const uint32
 // strips of kSymRows rows, in each the blocks of 32 columns up to the diagonal
 // one after another, 4 KB apiece.  Bound by HBM: one V-cycle of the
 // 131,072-point configuration reads its 17,845 x 17,845 inverse (2.5 GB, 573 us
-// with a warp per row at 4.4 TB/s) as 1.27 GB in 180 us (7.1 TB/s); from the
+// with a warp per row between a cycle's other kernels) as 1.27 GB in 180 us; from the
 // rows of the full matrix, 16 rows of 143 KB apart at a time, it took 316 us.
 // A CTA takes a strip (the longest first), each warp every eighth block with a
 // column per lane: the column's sum over the strip leaves with one reduction,
@@ -628,7 +628,7 @@ constexpr int kSymSmem = kSymWarps * kSymStages * kSymBlock * int(sizeof(double)
 // Rows from which it is used: there the full matrix (72 MB) no longer stays in
 // L2 between cycles.  A warp per row of it, against clearing x and this: 10.2
 // and 11.1 us for 1,000 rows, 14.2 and 15.2 for 3,001 (both in L2), 38.9 and
-// 19.5 for 4,000, 467 and 183 for 17,845.
+// 19.5 for 4,000, 467 and 183 for 17,845 (launches of one kind in a row).
 constexpr int64_t kSymFrom = 3000;
 __host__ __device__ inline int64_t sym_blocks(int64_t s) { return (s + 2) / 2; }  // of strip s
 __host__ __device__ inline int64_t sym_first(int64_t s) {                         // blocks before strip s
