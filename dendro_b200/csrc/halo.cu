@@ -154,10 +154,14 @@ jacobi_update(T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ 
     x[i] += omega * dinv[i] * (b[i] - ax[i]);
 }
 
+// Complete on return, for kernels on any stream: a copy from pageable memory
+// may still be on its way to the device when cudaMemcpy returns.
 template <class T>
 dg_status upload_vec(DBuf<T>& d, const std::vector<T>& h) {
   DG_TRY(d.alloc(int64_t(h.size())));
-  if (!h.empty()) DG_CUDA(cudaMemcpy(d.p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
+  if (h.empty()) return DG_OK;
+  DG_CUDA(cudaMemcpy(d.p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
+  DG_CUDA(cudaStreamSynchronize(nullptr));
   return DG_OK;
 }
 

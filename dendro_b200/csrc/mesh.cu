@@ -728,6 +728,7 @@ static dg_status upload_etype_lut() {
   for (int c = 0; c < 8; ++c)
     for (int t = 0; t < 18; ++t) lut[c][kEtypeMask[c][t]] = uint8_t(t);
   DG_CUDA(cudaMemcpyToSymbol(c_etype_lut, lut, sizeof lut));
+  DG_CUDA(cudaStreamSynchronize(nullptr));  // there before kernels on other streams
   done = true;
   return DG_OK;
 }

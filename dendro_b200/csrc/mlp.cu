@@ -509,6 +509,7 @@ dg_status dg_mlp_create(const float* params, dg_mlp** out) {
     cudaMemset(m->params.p, 0, 4 * kMlpParams);
   }
   *out = m;
+  DG_CUDA(cudaStreamSynchronize(nullptr));  // copies and clears are done, for any stream
   return DG_OK;
 }
 
@@ -524,6 +525,7 @@ dg_status dg_mlp_set_params(dg_mlp* m, const float* host) {
   m->step = 0;
   DG_CUDA(cudaMemset(m->m1.p, 0, 4 * kMlpParams));
   DG_CUDA(cudaMemset(m->m2.p, 0, 4 * kMlpParams));
+  DG_CUDA(cudaStreamSynchronize(nullptr));
   return DG_OK;
 }
 

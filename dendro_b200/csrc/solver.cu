@@ -1852,8 +1852,10 @@ dg_status dg_damg_prolong(dg_damg* m, int level, const double* xc, double* xf, i
   if (!on_device) {
     DG_TRY(dc.alloc(nc));
     DG_TRY(df.alloc(nf));
-    DG_CUDA(cudaMemcpy(dc.p, xc, 8 * nc, cudaMemcpyHostToDevice));
-    DG_CUDA(cudaMemcpy(df.p, xf, 8 * nf, cudaMemcpyHostToDevice));
+    // on the stream of the kernel: a cudaMemcpy from pageable memory may return
+    // before its last part has reached the device
+    DG_CUDA(cudaMemcpyAsync(dc.p, xc, 8 * nc, cudaMemcpyHostToDevice, m->s));
+    DG_CUDA(cudaMemcpyAsync(df.p, xf, 8 * nf, cudaMemcpyHostToDevice, m->s));
     pc = dc.p;
     pf = df.p;
   }
@@ -1880,7 +1882,7 @@ dg_status dg_damg_restrict(dg_damg* m, int level, const double* rf, double* rc, 
   if (!on_device) {
     DG_TRY(dc.alloc(nc));
     DG_TRY(df.alloc(nf));
-    DG_CUDA(cudaMemcpy(df.p, rf, 8 * nf, cudaMemcpyHostToDevice));
+    DG_CUDA(cudaMemcpyAsync(df.p, rf, 8 * nf, cudaMemcpyHostToDevice, m->s));
     pf = df.p;
     pc = dc.p;
   }

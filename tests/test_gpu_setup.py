@@ -282,3 +282,16 @@ def test_octants_at_the_far_corner_are_kept(gpu, depth):
     top = (1 << depth) - 1
     a = np.array([(0, 0, 0, depth), (top, top, top, depth)], OCT_DTYPE)
     assert same(gpu.Octree.from_octants(a, depth).to_numpy(), a)
+
+
+def test_transfers_of_host_vectors_see_this_call_s_data(gpu):
+    """The prolongation keeps constants and the restriction is linear, also where the vector's last part has only just
+    been copied."""
+    m = gpu.DAMG(gpu.balanceOctree(gpu.points2Octree(I.clamp_unit(I.lognormal_cloud(20000, 3), 12), 12, 1)), nlevels=2)
+    nf, nc = int(m.N[0]), int(m.N[1])
+    one = m.restrict(0, np.ones(nf))
+    for k in range(40):
+        c = 1.0 + k
+        xf = m.prolong(0, np.full(nc, c), np.zeros(nf))
+        assert (np.abs(xf - c) <= 1e-14 * c).all()
+        assert (np.abs(m.restrict(0, np.full(nf, c)) - c * one) <= 1e-13 * c * one).all()
