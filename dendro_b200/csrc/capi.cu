@@ -306,7 +306,7 @@ dg_status dg_da_load_vector(const dg_da* da, const double* force, double* b, int
   DG_CHECK(da && force && b, DG_EINVAL, "da_load_vector: bad arguments");
   if (on_device) {
     DG_TRY(load_vector(da, force, b, 0));
-    DG_CUDA(cudaDeviceSynchronize());
+    DG_CUDA(wait_device());
     return DG_OK;
   }
   DBuf<double> df, db;
@@ -321,7 +321,7 @@ dg_status dg_da_load_vector(const dg_da* da, const double* force, double* b, int
 dg_status dg_da_compress_maps(dg_da* da, int quotient_bits) {
   DG_CHECK(da, DG_EINVAL, "compress_maps: null mesh");
   DG_TRY(build_cmap(da, quotient_bits, 0));
-  DG_CUDA(cudaDeviceSynchronize());
+  DG_CUDA(wait_device());
   return DG_OK;
 }
 

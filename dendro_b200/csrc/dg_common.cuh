@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
+#include <shared_mutex>
 #include <string>
 
 #include "../../include/dendro_b200.h"
@@ -190,6 +191,10 @@ void device_free(void* p, int dev);
 // does: also while another thread captures a stream, where
 // cudaDeviceSynchronize fails and ends that thread's capture.
 cudaError_t drain_device();
+// cudaDeviceSynchronize, but not while another thread of this library captures
+// a stream (capture_lock held shared), which it would end.
+cudaError_t wait_device();
+std::shared_mutex& capture_lock();
 // Deletes an object made of device buffers: waits for the device once (its
 // buffers may be in use on any stream), then releases them together.
 template <class T>

@@ -63,9 +63,18 @@ cudaError_t drain_device() {
   void* p = nullptr;
   e = cudaMalloc(&p, kSmall);
   if (e == cudaSuccess) e = cudaFree(p);
-  if (e == cudaErrorMemoryAllocation) e = cudaDeviceSynchronize();
+  if (e == cudaErrorMemoryAllocation) e = wait_device();
   if (e != cudaSuccess) (void)cudaGetLastError();
   return e;
+}
+
+std::shared_mutex& capture_lock() {
+  static std::shared_mutex mu;
+  return mu;
+}
+cudaError_t wait_device() {
+  std::unique_lock<std::shared_mutex> lock(capture_lock());
+  return cudaDeviceSynchronize();
 }
 
 PoolScope::PoolScope(cudaStream_t s) : prev_(t_scope.stream), prev_on_(t_scope.on) {

@@ -537,7 +537,7 @@ dg_status dg_mlp_forward(dg_mlp* m, const float* F, int64_t n, float* out, int e
 dg_status dg_mlp_gradient(dg_mlp* m, const float* F, const float* T, int64_t n, int exact_fp32, float* grad_host,
                           double* loss_host) {
   DG_CHECK(m && F && T && n > 0, DG_EINVAL, "mlp_gradient: bad arguments");
-  DG_CUDA(cudaDeviceSynchronize());
+  DG_CUDA(wait_device());
   DG_CUDA(cudaMemset(m->grad.p, 0, 4 * kMlpParams));
   DG_CUDA(cudaMemset(m->loss.p, 0, 4));
   DG_TRY(mlp_gradient(m->params.p, F, T, n, m->grad.p, m->loss.p, exact_fp32 != 0, nullptr));
@@ -555,7 +555,7 @@ dg_status dg_mlp_train_step(dg_mlp* m, const float* F, const float* T, int64_t n
   DG_TRY(dg_mlp_gradient(m, F, T, n, 0, nullptr, loss_host));
   m->step += 1;
   DG_TRY(mlp_adam(m->params.p, m->grad.p, m->m1.p, m->m2.p, m->step, lr, nullptr));
-  DG_CUDA(cudaDeviceSynchronize());
+  DG_CUDA(wait_device());
   return DG_OK;
 }
 

@@ -1504,9 +1504,14 @@ dg_status precond(dg_damg* m) {
     // happen outside the capture
     DG_TRY(precond_body(m));
     cudaGraph_t graph = nullptr;
-    DG_CUDA(cudaStreamBeginCapture(m->s, cudaStreamCaptureModeThreadLocal));
-    dg_status st = precond_body(m);
-    cudaError_t e = cudaStreamEndCapture(m->s, &graph);
+    dg_status st = DG_OK;
+    cudaError_t e = cudaSuccess;
+    {
+      std::shared_lock<std::shared_mutex> lock(capture_lock());
+      DG_CUDA(cudaStreamBeginCapture(m->s, cudaStreamCaptureModeThreadLocal));
+      st = precond_body(m);
+      e = cudaStreamEndCapture(m->s, &graph);
+    }
     if (st != DG_OK) {
       if (graph) cudaGraphDestroy(graph);
       return st;
@@ -1859,7 +1864,7 @@ dg_status dg_damg_prolong(dg_damg* m, int level, const double* xc, double* xf, i
     pc = dc.p;
     pf = df.p;
   }
-  if (on_device) DG_CUDA(cudaDeviceSynchronize());
+  if (on_device) DG_CUDA(wait_device());
   if (dof == 3)
     prolong_add3<<<grid_for(F.da->N, 256), 256, 0, m->s>>>(F.pptr.p, F.pcol.p, F.pval.p, F.da->N, pc, pf);
   else
@@ -1886,7 +1891,7 @@ dg_status dg_damg_restrict(dg_damg* m, int level, const double* rf, double* rc, 
     pf = df.p;
     pc = dc.p;
   }
-  if (on_device) DG_CUDA(cudaDeviceSynchronize());
+  if (on_device) DG_CUDA(wait_device());
   if (dof == 3)
     restrict_gather3<<<grid_for(C.da->N, 256, 16), 256, 0, m->s>>>(F.rptr.p, F.rcol.p, F.rval.p, C.da->N, pf, pc);
   else
@@ -1908,7 +1913,7 @@ dg_status dg_damg_solve(dg_damg* m, const double* b, double* x, int on_device, d
   const double* pb = b;
   double* px = x;
   // the caller's device data may come from any stream
-  if (on_device) DG_CUDA(cudaDeviceSynchronize());
+  if (on_device) DG_CUDA(wait_device());
   // the vector kernels read 16-byte pairs: host data, and device data not
   // 16-byte aligned, go through the solver's own buffers
   const bool staged = !on_device || ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(x)) & 15) != 0;
@@ -2385,7 +2390,7 @@ dg_status dg_damg_solve_multi(dg_damg* m, const double* B, double* X, int nrhs, 
   const Level& L0 = m->lv[0];
   const int64_t N = L0.da->N, n = N * R;
   const bool f32 = m->cfg.inner_prec != DG_PREC_F64;
-  if (on_device) DG_CUDA(cudaDeviceSynchronize());
+  if (on_device) DG_CUDA(wait_device());
   // The work blocks come from the pool (about 30 allocations and releases a
   // solve took as long as the solve); the solution is worked in the caller's
   // array where that is device memory on a 16-byte boundary.
@@ -2544,7 +2549,7 @@ dg_status dg_damg_set_smoother(dg_damg* m, dg_mlp* mlp, int sweeps, double fallb
 
 dg_status dg_damg_features(dg_damg* m, const double* r, float* F, float* scale) {
   DG_CHECK(m && r && F, DG_EINVAL, "damg_features: bad arguments");
-  DG_CUDA(cudaDeviceSynchronize());
+  DG_CUDA(wait_device());
   DG_TRY(ensure_smoother_data(m));
   Level& L = m->lv[0];
   DBuf<float> d32, sc;
@@ -2624,7 +2629,7 @@ dg_status dg_damg_coarse_solve(dg_damg* m, const double* b, double* x, void* str
 dg_status dg_damg_vcycle(dg_damg* m, const double* b, double* x) {
   DG_CHECK(m && b && x, DG_EINVAL, "damg_vcycle: bad arguments");
   const int64_t n = int64_t(m->cfg.dof) * m->lv[0].da->N;
-  DG_CUDA(cudaDeviceSynchronize());
+  DG_CUDA(wait_device());
   DG_CUDA(cudaMemcpyAsync(m->r.p, b, 8 * n, cudaMemcpyDeviceToDevice, m->s));
   DG_TRY(precond_body(m));
   DG_CUDA(cudaMemcpyAsync(x, m->z.p, 8 * n, cudaMemcpyDeviceToDevice, m->s));

@@ -209,6 +209,43 @@ def test_operators_are_ready_on_any_stream(gpu):
         assert (y - want).abs().max() <= 1e-13 * want.abs().max()
 
 
+def test_solves_beside_another_threads_graph(gpu):
+    """One thread captures its V-cycle, again after every change of its operator, while others solve: a solve waits
+    for the device before it starts, which would end the capture."""
+    import torch
+    trees = [gpu.balanceOctree(gpu.points2Octree(I.clamp_unit(I.gaussian_cloud(n, n), 11), 11, 1))
+             for n in (20000, 50, 60, 70)]
+    ms = [gpu.DAMG(t, inner_prec=1, use_graph=i == 0) for i, t in enumerate(trees)]
+    for m in ms:
+        m.setKSP()
+    bs = [torch.rand(int(m.N[0]), dtype=torch.float64, device="cuda") for m in ms]
+    for m, b in zip(ms, bs):
+        m.solve(b)
+    bad, start, done = [], threading.Barrier(4), threading.Event()
+
+    def work(i):
+        try:
+            start.wait()
+            if i == 0:
+                for _ in range(30):
+                    ms[0].setKSP()
+                    ms[0].solve(bs[0])
+            while i and not done.is_set():
+                ms[i].solve(bs[i])
+        except Exception as e:  # noqa: BLE001 -- the test's thread reports it
+            bad.append((i, e))
+        finally:
+            if i == 0:
+                done.set()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
+
+
 def test_levels_of_a_batch_have_octets(gpu, oracle):
     """Every octet launch shape on a batch's concatenated mesh, against the meshes one by one."""
     import torch
