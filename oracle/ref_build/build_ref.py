@@ -83,7 +83,7 @@ def patched_headers():
 
 
 def main():
-    if not os.path.isdir(REF):
+    if not os.path.isdir(os.path.join(REF, "src")):  # not there, or empty
         print("reference tree not present; skipping the reference build")
         return 0
     os.makedirs(os.path.join(OUT, "obj"), exist_ok=True)
